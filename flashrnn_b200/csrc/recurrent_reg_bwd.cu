@@ -1,0 +1,511 @@
+// Reverse-time recurrence of narrow heads with R in the register file (see recurrent_reg.cuh).
+//
+// Groups, CTAs and the unit each thread owns are those of recurrent_reg_fwd.cu. Per step t a thread
+//   1. adds up the partial dh_t of its unit and two batch rows (fixed order), the external gradient and the pointwise
+//      carry, runs the cell backward and writes round_bf16(dg_t) to shared memory for ldmatrix (one CTA barrier),
+//   2. multiplies with its warp's fragments of R_slice^T [D x GR*U] (rows = units p of h_{t-1}, k = gate rows of this CTA),
+//   3. hands the accumulators to the owners of those units: two lanes swap halves so that each packet is 4 batch rows of
+//      one unit, 16 bytes.
+// LOCAL: D / 16 row tiles for D / 8 warps, so two warps share a tile and take half of k each: their two partial results
+//        are the "sources" of step 1.  else: the sources are the CTAs of the cluster, packets travel by st.async.
+// The state of step t - 1 stays in registers as the new state of the next iteration, and only the planes that the cell's
+// derivative reads are fetched: an LSTM reads one history plane per step where reading both states at t and t - 1 takes four.
+//
+// Safe reuse: dg is double-buffered because a warp may still read dg_t when another has begun step t - 1; the partial
+// sums of a parity are overwritten only after the CTA barrier of the step that read them; a TMA stage is refilled by the I/O
+// warp after every warp has staged its outputs of the step that used it.
+#include "recurrent_reg.cuh"
+
+namespace frnn {
+
+namespace {
+
+// History planes the cell's derivative reads: [first, first + count).
+template <int CELL> struct HistPlanes;
+template <> struct HistPlanes<kLSTM> { static constexpr int first = 1, count = 1; };
+template <> struct HistPlanes<kSLSTM> { static constexpr int first = 1, count = 3; };
+template <> struct HistPlanes<kGRU> { static constexpr int first = 0, count = 1; };
+template <> struct HistPlanes<kElman> { static constexpr int first = 0, count = 1; };
+
+template <int CELL, int KT, bool LOCAL>
+struct BwdRegCfg {
+  using CT = CellTraits<CELL>;
+  static constexpr int MTW = LOCAL ? 1 : (KT + 3) / 4;                    // row tiles of a warp
+  static constexpr int KTW = LOCAL ? (CT::GR * KT + 1) / 2 : 2 * CT::GR;  // k tiles of a warp
+  static constexpr int DG_BYTES = ((LOCAL ? 2 : 1) * KTW * 16 * 16 + 511) / 512 * 512;  // two of them: the tiles stay 1 KB aligned
+  static constexpr int GCL = CELL == kElman ? 0 : CT::GC;
+  static constexpr int HP = HistPlanes<CELL>::first, HS = HistPlanes<CELL>::count;
+  static constexpr int PLANE4 = kRegRows * kRegChunk * 4, PLANEC = kRegRows * kRegChunk * CT::CES;
+  static constexpr int CHUNK = GCL * PLANEC + (HS + CT::S) * PLANE4;  // cache, state of step t - 1, external gradient
+};
+
+template <int CELL, int KT, bool LOCAL>
+__global__ void __launch_bounds__(LOCAL ? 64 * KT + 32 : 160, reg_min_blocks(CELL, KT, LOCAL))
+frnn_bwd_reg_kernel(const BwdParams p, const float* history, const __grid_constant__ CUtensorMap cache_map,
+                    const __grid_constant__ CUtensorMap hist_map, const __grid_constant__ CUtensorMap init_map,
+                    const __grid_constant__ CUtensorMap dhist_map, const __grid_constant__ CUtensorMap dgr_map,
+                    const __grid_constant__ CUtensorMap dwx_map, const int wx_bf16, const int own_dwx, const int nst) {
+  using Cfg = BwdRegCfg<CELL, KT, LOCAL>;
+  using CT = CellTraits<CELL>;
+  constexpr int S = CT::S, MTW = Cfg::MTW, KTW = Cfg::KTW, GCL = Cfg::GCL, HP = Cfg::HP, HS = Cfg::HS;
+
+  extern __shared__ __align__(1024) uint8_t smem[];
+  __shared__ __align__(8) uint64_t s_part_bar[2];
+  __shared__ __align__(8) uint64_t s_full[kRegMaxStages];
+  __shared__ int s_gave_up;  // a compute warp of this CTA has stopped waiting (the flag in global memory is an L2 round trip away)
+  __shared__ __align__(8) uint64_t s_out_full[kRegMaxSlots];  // outputs of a step staged by every warp
+
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, q = lane >> 2, c = lane & 3;
+  const long long t_entry = clock64();
+  const int D = p.D, N = p.N, T = p.T, B = p.B;
+  const int nwarps = LOCAL ? (blockDim.x >> 5) - 1 : 4, U = nwarps * kRegUnitsPerWarp;
+  const int C = LOCAL ? 1 : p.C;
+  const int rank = LOCAL ? 0 : static_cast<int>(blockIdx.x % C), gid = blockIdx.x / C;
+  const int n = gid % N, b0 = gid / N * kRegRows;
+  const int sources = LOCAL ? 2 : C;
+  const int part_bytes = sources * U * kRegRows * 4;  // one parity: [source][unit][8 batch rows] fp32
+  const int chunks = (U + kRegChunk - 1) / kRegChunk, stage_bytes = chunks * Cfg::CHUNK;
+  uint8_t* const dgbuf = smem;
+  uint8_t* const part = smem + 2 * Cfg::DG_BYTES;
+  uint8_t* const stages = part + 2 * part_bytes;
+  uint8_t* const outs = stages + nst * stage_bytes;
+  // Outputs of a step, staged per 32 units: dWx where it is a tensor of its own, and dg as the dR contraction wants it.
+  const int slots = nst + 1;
+  const int dwx_bytes = own_dwx ? CT::GW * (wx_bf16 ? kRegPlane<2> : kRegPlane<4>) : 0;
+  const int out_chunk = reg_round_1k(dwx_bytes + CT::GR * kRegPlane<2>), out_slot = chunks * out_chunk;
+  const volatile int* abort_flag = p.err;
+  const uint64_t limit = p.wait_limit_ns;
+  const int mute_from = p.err[4] != 0 ? p.err[5] : 0x7fffffff;            // test hook: nobody publishes from this iteration on
+  const uint32_t jitter = wx_bf16 ? 0u : static_cast<uint32_t>(p.err[6]); // test hook (fp32 Wx): see jitter_stall
+  const bool prof = p.err[3] != 0 && blockIdx.x == 0 && tid == 0;
+
+  if (tid == 0) {
+    for (int i = 0; i < 2; ++i) mbar_init(smem_u32(&s_part_bar[i]), LOCAL ? nwarps : 1);
+    for (int s = 0; s < nst; ++s) mbar_init(smem_u32(&s_full[s]), 1);
+    for (int i = 0; i < slots; ++i) mbar_init(smem_u32(&s_out_full[i]), nwarps);
+    s_gave_up = 0;
+    fence_mbar_init();
+  }
+  for (int i = tid; i < 2 * Cfg::DG_BYTES / 16; i += blockDim.x)
+    reinterpret_cast<uint4*>(dgbuf)[i] = make_uint4(0u, 0u, 0u, 0u);
+  __syncthreads();
+  // the packets carry all 8 columns whatever the number of batch rows in use
+  const uint32_t part_tx = static_cast<uint32_t>(part_bytes);
+  if (tid == 0 && !LOCAL) {
+    mbar_arrive_expect_tx(smem_u32(&s_part_bar[1]), part_tx);              // iteration 1 (the last one if T == 1)
+    if (T >= 2) mbar_arrive_expect_tx(smem_u32(&s_part_bar[0]), part_tx);  // iteration 2
+  }
+
+  if (warp == nwarps) {
+    // ---------------- I/O warp: tiles in, staged outputs out ----------------
+    if (!LOCAL) cluster_sync_all();
+    if (lane == 0) {
+      auto fill = [&](int it, int s) {  // the operands of iteration `it`, step t
+        const int t = T - 1 - it;
+        const uint32_t bar = smem_u32(&s_full[s]);
+        mbar_arrive_expect_tx(bar, static_cast<uint32_t>(stage_bytes));
+        for (int i = 0; i < chunks; ++i) {
+          uint32_t dst = smem_u32(stages + s * stage_bytes + i * Cfg::CHUNK);
+          const int x = rank * U + i * kRegChunk;
+          if (GCL > 0) tma_load_5d(dst, &cache_map, bar, x, n, b0, 0, t);
+          dst += GCL * Cfg::PLANEC;
+          if (t > 0) tma_load_5d(dst, &hist_map, bar, x, n, b0, HP, t - 1);
+          else tma_load_5d(dst, &init_map, bar, x, n, b0, HP, 0);
+          dst += HS * Cfg::PLANE4;
+          tma_load_5d(dst, &dhist_map, bar, x, n, b0, 0, t);
+        }
+      };
+      for (int it = 0; it < nst && it < T; ++it) fill(it, it);
+      int stage = 0, slot = 0;
+      uint32_t phase = 0;
+      for (int it = 0; it < T; ++it) {
+        // released by the CTA's own warps, whose waits have the plain limit: theirs run out first
+        if (!mbar_wait_bounded<false, true>(smem_u32(&s_out_full[slot]), phase, 2 * limit, abort_flag)) {
+          reg_report(p.err, kErrWaitEmpty, it);
+          break;
+        }
+        for (int i = 0; i < chunks; ++i) {
+          const uint32_t src = smem_u32(outs + slot * out_slot + i * out_chunk);
+          const int x = rank * U + i * kRegChunk;
+          if (own_dwx) tma_store_5d(&dwx_map, src, x, n, b0, 0, T - 1 - it);
+          tma_store_5d(&dgr_map, src + dwx_bytes, x, n, b0, 0, T - 1 - it);
+        }
+        tma_store_commit();
+        tma_store_wait_read<1>();  // the copies of the previous step have read their slot: see kRegMaxSlots
+        // a warp that gave up on a wait may not have seen the stage filled: a copy could be on its way into it
+        if (*reinterpret_cast<volatile int*>(&s_gave_up) != 0) break;
+        if (it + nst < T) fill(it + nst, stage);
+        if (++stage == nst) stage = 0;
+        if (++slot == slots) { slot = 0; phase ^= 1u; }
+      }
+      tma_store_wait<0>();
+    }
+    __syncwarp();
+  } else {
+    // A fragments of R_slice^T: 8x8 blocks of R are loaded as they lie (gate rows x units p) and transposed in the warp.
+    const int n_tiles = D / 16;
+    const int khalf = LOCAL ? warp / n_tiles : 0;
+    const int tile0 = LOCAL ? warp % n_tiles : warp;
+    uint32_t a[MTW][KTW][4];
+#pragma unroll
+    for (int m = 0; m < MTW; ++m)
+#pragma unroll
+      for (int kt = 0; kt < KTW; ++kt)
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+          const int k8 = (khalf * KTW + kt) * 2 + (r >> 1);  // block of 8 gate rows
+          const int g = k8 * 8 / U, u = k8 * 8 % U + q;
+          const int pcol = (tile0 + (LOCAL ? 0 : 4 * m)) * 16 + 8 * (r & 1) + 2 * c;
+          uint32_t v = 0u;
+          if (g < CT::GR && pcol < D)
+            v = __ldg(reinterpret_cast<const uint32_t*>(p.R + ((static_cast<size_t>(g) * N + n) * D + rank * U + u) * D + pcol));
+          a[m][kt][r] = movmatrix_trans(v);
+        }
+
+    const int ul = warp * kRegUnitsPerWarp + q, d = rank * U + ul;
+    const size_t ND = static_cast<size_t>(N) * D, BND = static_cast<size_t>(B) * ND;
+    const size_t sBTND = static_cast<size_t>(T) * BND;
+    bool act[2];
+    float dcar[S][2], dbacc[CT::GB], sn[HS][2];
+#pragma unroll
+    for (int g = 0; g < CT::GB; ++g) dbacc[g] = 0.0f;
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const size_t b = static_cast<size_t>(b0 + 2 * c + e);
+      act[e] = b < static_cast<size_t>(B);
+#pragma unroll
+      for (int k = 0; k < S; ++k) dcar[k][e] = act[e] ? p.d_carry[k * BND + b * ND + static_cast<size_t>(n) * D + d] : 0.0f;
+#pragma unroll
+      for (int k = 0; k < HS; ++k)
+        sn[k][e] = act[e] ? history[(HP + k) * sBTND + ((b * T + T - 1) * N + n) * D + d] : 0.0f;
+    }
+    const int uc = (warp & 3) * kRegUnitsPerWarp + q;  // unit inside the staged 32
+    const uint32_t off_q = reg_tile_offset<2>(q, (warp & 3) * kRegUnitsPerWarp + 2 * c);
+    uint8_t* const my_chunk = stages + (warp >> 2) * Cfg::CHUNK;
+    uint8_t* const my_out = outs + (warp >> 2) * out_chunk;
+    uint8_t* out = my_out;
+    const int compute_threads = nwarps * 32;
+    const bool v1 = p.slstm_v1 != 0, zero_first = p.slstm_zero_first != 0, cut = p.cut_recurrent != 0, clip_on = p.grad_clip > 0.0f;
+    const float grad_clip = p.grad_clip;
+    // where this lane's packets of a tile go: the row q or q + 8 of the tile, four batch rows
+    const uint32_t row_off = static_cast<uint32_t>((q + 8 * (c & 1)) * (kRegRows * 4) + (c >> 1) * 16);
+    uint32_t dst_part[MTW], dst_bar[MTW];
+#pragma unroll
+    for (int m = 0; m < MTW; ++m) {
+      const int tile = tile0 + (LOCAL ? 0 : 4 * m);
+      if (LOCAL) {
+        dst_part[m] = smem_u32(part) + (khalf * U + tile * 16) * (kRegRows * 4) + row_off;
+        dst_bar[m] = 0u;
+      } else {
+        const int owner = tile < n_tiles ? tile / 2 : rank;  // 32 units, two tiles
+        dst_part[m] = map_to_cta(smem_u32(part) + (rank * U + (tile & 1) * 16) * (kRegRows * 4) + row_off, owner);
+        dst_bar[m] = map_to_cta(smem_u32(&s_part_bar[0]), owner);
+      }
+    }
+
+    bool dead = false;  // warp-uniform: after a failed wait the warp walks on without waiting
+    auto give_up = [&](int code, int it) {
+      if (lane == 0) reg_report(p.err, code, it);
+      dead = true;
+      *reinterpret_cast<volatile int*>(&s_gave_up) = 1;
+    };
+    float cache[CT::GC][2], sp[HS][2], dh[S][2];
+    int in_stage = 0, slot = 0;
+    uint32_t in_phase = 0;
+    auto read_stage = [&](int it) {
+      if (!dead && !mbar_wait_warp<false>(smem_u32(&s_full[in_stage]), in_phase, limit, abort_flag)) give_up(kErrWaitWx, it);
+      const uint8_t* sb = my_chunk + in_stage * stage_bytes;
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int row = 2 * c + e;
+#pragma unroll
+        for (int g = 0; g < GCL; ++g) cache[g][e] = ld_cache<CT::CES>(sb + g * Cfg::PLANEC + reg_tile_offset<CT::CES>(row, uc), 0);
+        const uint8_t* f = sb + GCL * Cfg::PLANEC + reg_tile_offset<4>(row, uc);
+#pragma unroll
+        for (int k = 0; k < HS; ++k) sp[k][e] = *reinterpret_cast<const float*>(f + k * Cfg::PLANE4);
+        f += HS * Cfg::PLANE4;
+#pragma unroll
+        for (int k = 0; k < S; ++k) dh[k][e] = *reinterpret_cast<const float*>(f + k * Cfg::PLANE4);
+      }
+      if (++in_stage == nst) { in_stage = 0; in_phase ^= 1u; }
+    };
+    if (!LOCAL) cluster_sync_all();
+    if (prof) p.err[20] = static_cast<int>(clock64() - t_entry);
+
+    read_stage(0);
+    long long pc[6] = {0, 0, 0, 0, 0, 0};
+    for (int it = 0; it <= T; ++it) {
+      if (jitter != 0u) { jitter_stall(jitter, static_cast<uint32_t>(warp), static_cast<uint32_t>(it)); __syncwarp(); }
+      const int t = T - 1 - it;
+      float ds[S][2];
+#pragma unroll
+      for (int k = 0; k < S; ++k)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) ds[k][e] = it < T ? dcar[k][e] + dh[k][e] : dcar[k][e];
+      const long long c1 = prof ? clock64() : 0;
+      long long cw = c1;
+      if (it >= 1) {
+        const int pb = it & 1;
+        if (!dead && !mbar_wait_warp<!LOCAL>(smem_u32(&s_part_bar[pb]), ((it - 1) >> 1) & 1, limit, abort_flag)) give_up(kErrWaitPart, it);
+        cw = prof ? clock64() : 0;
+        if (!cut) {
+          constexpr int kSrc = LOCAL ? 2 : 8;
+          const uint8_t* pbuf = part + pb * part_bytes + ul * (kRegRows * 4) + c * 8;
+          float2 v[kSrc];
+#pragma unroll
+          for (int k = 0; k < kSrc; ++k)
+            v[k] = k < sources ? *reinterpret_cast<const float2*>(pbuf + k * U * (kRegRows * 4)) : make_float2(0.0f, 0.0f);
+#pragma unroll
+          for (int k = 0; k < kSrc; ++k) { ds[0][0] += v[k].x; ds[0][1] += v[k].y; }
+        }
+      }
+      if (clip_on && it >= 1 && it < T) {
+        // the gradient carried into h_t from step t + 1 (total minus the external part) is complete here: clip it
+#pragma unroll
+        for (int e = 0; e < 2; ++e) ds[0][e] = clip_sym(ds[0][e] - dh[0][e], grad_clip) + dh[0][e];
+      }
+      const long long c2 = prof ? clock64() : 0;
+      if (it == T) {
+#pragma unroll
+        for (int e = 0; e < 2; ++e)
+          if (act[e]) {
+#pragma unroll
+            for (int k = 0; k < S; ++k)
+              p.d_initial[k * BND + static_cast<size_t>(b0 + 2 * c + e) * ND + static_cast<size_t>(n) * D + d] = ds[k][e];
+          }
+        break;
+      }
+      float dgr[CT::GR][2], dgw[CT::GW][2];
+      const bool take_i = CELL == kSLSTM && t == 0 && zero_first;
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        float cj[CT::GC], snj[S], spj[S], dsj[S], gr[CT::GR], gw[CT::GW], gb[CT::GB];
+#pragma unroll
+        for (int g = 0; g < GCL; ++g) cj[g] = cache[g][e];
+#pragma unroll
+        for (int k = 0; k < S; ++k) {
+          snj[k] = k >= HP && k < HP + HS ? sn[k >= HP ? k - HP : 0][e] : 0.0f;
+          spj[k] = k >= HP && k < HP + HS ? sp[k >= HP ? k - HP : 0][e] : 0.0f;
+          dsj[k] = ds[k][e];
+        }
+        cell_backward<CELL>(cj, spj, snj, dsj, gr, gw, gb, take_i, v1);
+        // rows past the batch hold zeros where the cell divides: their gradients are dropped
+#pragma unroll
+        for (int k = 0; k < S; ++k) dcar[k][e] = act[e] ? dsj[k] : 0.0f;
+#pragma unroll
+        for (int g = 0; g < CT::GR; ++g) dgr[g][e] = act[e] ? gr[g] : 0.0f;
+#pragma unroll
+        for (int g = 0; g < CT::GW; ++g) dgw[g][e] = gw[g];
+#pragma unroll
+        for (int g = 0; g < CT::GB; ++g) dbacc[g] += act[e] ? gb[g] : 0.0f;
+      }
+      uint32_t dgp[CT::GR];
+      const uint32_t dgs = smem_u32(dgbuf) + (it & 1) * Cfg::DG_BYTES;
+#pragma unroll
+      for (int g = 0; g < CT::GR; ++g) {
+        dgp[g] = pack_bf16x2(dgr[g][0], dgr[g][1]);
+        asm volatile("st.shared.b32 [%0], %1;" ::"r"(dgs + (g * nwarps + warp) * 128 + lane * 4), "r"(dgp[g]) : "memory");
+      }
+#pragma unroll
+      for (int k = 0; k < HS; ++k) { sn[k][0] = sp[k][0]; sn[k][1] = sp[k][1]; }
+      asm volatile("bar.sync 1, %0;" ::"r"(compute_threads) : "memory");
+      const long long c3 = prof ? clock64() : 0;
+      const int nb = (it + 1) & 1;
+      {
+        constexpr int CH = LOCAL ? 2 : 1;  // a single tile runs as two independent chains
+        float acc[CH][MTW][4];
+#pragma unroll
+        for (int h = 0; h < CH; ++h)
+#pragma unroll
+          for (int m = 0; m < MTW; ++m)
+#pragma unroll
+            for (int r = 0; r < 4; ++r) acc[h][m][r] = 0.0f;
+        const uint32_t ab = dgs + khalf * KTW * 256;
+#pragma unroll
+        for (int k2 = 0; k2 < (KTW + 1) / 2; ++k2) {
+          uint32_t bf[4];
+          if (2 * k2 + 1 < KTW) ldsm_x4_trans(ab + lane * 16 + k2 * 512, bf);
+          else ldsm_x2_trans(ab + (lane & 15) * 16 + k2 * 512, bf[0], bf[1]);
+#pragma unroll
+          for (int m = 0; m < MTW; ++m) mma_bf16_16816(acc[0][m], a[m][2 * k2], bf[0], bf[1]);
+          if (2 * k2 + 1 < KTW) {
+#pragma unroll
+            for (int m = 0; m < MTW; ++m) mma_bf16_16816(acc[CH - 1][m], a[m][2 * k2 + 1 < KTW ? 2 * k2 + 1 : 0], bf[2], bf[3]);
+          }
+        }
+        const bool publish = !dead && it < mute_from;
+#pragma unroll
+        for (int m = 0; m < MTW; ++m) {
+          float v[4];
+#pragma unroll
+          for (int r = 0; r < 4; ++r) v[r] = CH == 2 ? acc[0][m][r] + acc[CH - 1][m][r] : acc[0][m][r];
+          // rows q / q + 8, columns 2c, 2c + 1 -> even lanes: row q, columns 2c .. 2c + 3; odd lanes: row q + 8, 2c - 2 .. 2c + 1
+          const float x0 = __shfl_xor_sync(0xffffffffu, (c & 1) ? v[0] : v[2], 1);
+          const float x1 = __shfl_xor_sync(0xffffffffu, (c & 1) ? v[1] : v[3], 1);
+          const float4 w = (c & 1) ? make_float4(x0, x1, v[2], v[3]) : make_float4(v[0], v[1], x0, x1);
+          if constexpr (LOCAL) {
+            if (publish)
+              asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(dst_part[m] + nb * part_bytes), "f"(w.x), "f"(w.y),
+                           "f"(w.z), "f"(w.w) : "memory");
+          } else {
+            if (publish && tile0 + 4 * m < n_tiles)
+              st_async_v4_b32(dst_part[m] + nb * part_bytes, __float_as_uint(w.x), __float_as_uint(w.y), __float_as_uint(w.z),
+                              __float_as_uint(w.w), dst_bar[m] + nb * 8);
+          }
+        }
+        if constexpr (LOCAL) {
+          __syncwarp();
+          if (lane == 0 && publish) mbar_arrive(smem_u32(&s_part_bar[nb]));
+        }
+      }
+      // this parity's partial sums were complete at the wait above: armed for iteration it + 2
+      if (!LOCAL && tid == 0 && !dead && it >= 1 && it + 2 <= T) mbar_arrive_expect_tx(smem_u32(&s_part_bar[it & 1]), part_tx);
+      const long long c4 = prof ? clock64() : 0;
+      // outputs, while the partial sums of the next step are on their way
+#pragma unroll
+      for (int g = 0; g < CT::GR; ++g) reg_stage_16(out + dwx_bytes + g * kRegPlane<2>, off_q, dgp[g]);
+      if (own_dwx) {
+#pragma unroll
+        for (int g = 0; g < CT::GW; ++g) {
+          if (wx_bf16) reg_stage_16(out + g * kRegPlane<2>, off_q, pack_bf16x2(dgw[g][0], dgw[g][1]));
+          else reg_stage_f32(out + g * kRegPlane<4>, c, uc, dgw[g][0], dgw[g][1]);
+        }
+      }
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(smem_u32(&s_out_full[slot]));
+      out += out_slot;
+      if (++slot == slots) { slot = 0; out = my_out; }
+      const long long c5 = prof ? clock64() : 0;
+      if (it + 1 < T) read_stage(it + 1);
+      if (prof) {
+        pc[0] += clock64() - c5; pc[1] += c2 - c1; pc[2] += c3 - c2; pc[3] += c5 - c4; pc[4] += c4 - c3; pc[5] += cw - c1;
+      }
+    }
+    if (prof) {  // the slots of the tcgen05 kernels' phase timers that have a counterpart here
+      p.err[8] = static_cast<int>(pc[0]);   // stage wait and read
+      p.err[9] = static_cast<int>(pc[1]);   // wait for the partial sums and their sum
+      p.err[10] = static_cast<int>(pc[2]);  // cell, dg to shared memory, CTA barrier
+      p.err[11] = static_cast<int>(pc[3]);  // outputs staged
+      p.err[12] = static_cast<int>(pc[4]);  // mma and scatter
+      p.err[13] = static_cast<int>(pc[5]);  // wait alone
+    }
+    // bias gradient of the 8 batch rows: the four lanes of a unit in fixed order
+#pragma unroll
+    for (int g = 0; g < CT::GB; ++g) {
+      float v = dbacc[g];
+      v += __shfl_xor_sync(0xffffffffu, v, 1);
+      v += __shfl_xor_sync(0xffffffffu, v, 2);
+      if (c == 0) {
+        float* dst = p.db_part + ((static_cast<size_t>(b0 / p.db_rows) * CT::GB + g) * N + n) * D + d;
+        // an entry of 16 rows gets at most two addends on top of the launcher's zeros: the order cannot matter
+        if (p.db_rows == kRegRows) *dst = v;
+        else atomicAdd(dst, v);
+      }
+    }
+  }
+  if (*abort_flag != 0) {
+    const uint64_t t0 = global_timer_ns();
+    while (global_timer_ns() - t0 < 200000ull) __nanosleep(1000);
+  }
+  __syncthreads();
+  if (!LOCAL) cluster_sync_all();
+}
+
+template <int CELL, int KT, bool LOCAL>
+int launch_bwd_reg(const BwdParams& p, const void* cache, const float* history, const float* initial,
+                   const float* d_history, int wx_bf16, cudaStream_t stream) {
+  using Cfg = BwdRegCfg<CELL, KT, LOCAL>;
+  using CT = CellTraits<CELL>;
+  const int U = LOCAL ? p.D : kRegClusterUnits, C = p.D / U;
+  const int stage = reg_chunks(U) * Cfg::CHUNK;
+  // cells whose W-gates are their R-gates may have one bf16 buffer for dWx and dg
+  const bool own_dwx = !wx_bf16 || CELL == kGRU || p.dwx != static_cast<void*>(p.dgr);
+  const int out_slot = reg_chunks(U) * reg_round_1k(kRegRows * kRegChunk * (CT::GR * 2 + (own_dwx ? CT::GW * (wx_bf16 ? 2 : 4) : 0)));
+  // prefetch depth: 4 steps, 2 where only that lets two CTAs share an SM
+  const auto bytes = [&](int st) {
+    return 2 * Cfg::DG_BYTES + 2 * (LOCAL ? 2 : C) * U * kRegRows * 4 + st * stage + (st + 1) * out_slot;
+  };
+  const int nst = bytes(kRegMaxStages) <= 110 * 1024 ? kRegMaxStages : 2;
+  const int smem = bytes(nst);
+  const int D = p.D, N = p.N, B = p.B;
+  const uint64_t nd = static_cast<uint64_t>(N) * D, uT = p.T, uB = p.B;
+  CUtensorMap cache_map, hist_map, init_map, dhist_map, dgr_map, dwx_map;
+  if (reg_tile_map(&hist_map, history, 4, D, N, B, CT::S, p.T, uT * nd, uB * uT * nd, nd, Cfg::HS) != 0 ||
+      reg_tile_map(&dhist_map, d_history, 4, D, N, B, CT::S, p.T, uT * nd, uB * uT * nd, nd, CT::S) != 0 ||
+      reg_tile_map(&init_map, initial, 4, D, N, B, CT::S, 1, nd, uB * nd, nd, Cfg::HS) != 0 ||
+      reg_tile_map(&dgr_map, p.dgr, 2, D, N, B, CT::GR, p.T, uT * CT::GR * nd, nd, CT::GR * nd, CT::GR) != 0)
+    return -4;
+  cache_map = hist_map;  // Elman has no cache: a valid map that is never used
+  if (Cfg::GCL > 0 &&
+      reg_tile_map(&cache_map, cache, CT::CES, D, N, B, CT::GC, p.T, uT * CT::GC * nd, nd, CT::GC * nd, CT::GC) != 0)
+    return -4;
+  dwx_map = dgr_map;
+  if (own_dwx &&
+      reg_tile_map(&dwx_map, p.dwx, wx_bf16 ? 2 : 4, D, N, B, CT::GW, p.T, uT * CT::GW * nd, nd, CT::GW * nd, CT::GW) != 0)
+    return -4;
+  auto kern = frnn_bwd_reg_kernel<CELL, KT, LOCAL>;
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (e != cudaSuccess) return static_cast<int>(e);
+  BwdParams q = p;
+  q.C = C;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(p.N * reg_batch_tiles(p.B) * C));
+  cfg.blockDim = dim3(static_cast<unsigned>(U / kRegUnitsPerWarp * 32 + 32));
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = static_cast<unsigned>(C);
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = LOCAL ? 0 : 1;
+  if (!LOCAL) {
+    int clusters = 0;
+    e = cudaOccupancyMaxActiveClusters(&clusters, kern, &cfg);
+    if (e != cudaSuccess) return static_cast<int>(e);
+    if (p.N * reg_batch_tiles(p.B) > clusters) return kRegNoRoom;
+  }
+  if (p.db_rows != kRegRows) {
+    const size_t tiles = static_cast<size_t>((p.B + p.db_rows - 1) / p.db_rows);
+    e = cudaMemsetAsync(p.db_part, 0, tiles * CT::GB * p.N * p.D * sizeof(float), stream);
+    if (e != cudaSuccess) return static_cast<int>(e);
+  }
+  e = cudaLaunchKernelEx(&cfg, kern, q, history, cache_map, hist_map, init_map, dhist_map, dgr_map, dwx_map, wx_bf16,
+                         own_dwx ? 1 : 0, nst);
+  return static_cast<int>(e);
+}
+
+template <int CELL>
+int launch_bwd_reg_cell(const BwdParams& p, const void* cache, const float* history, const float* initial,
+                        const float* d_history, int wx_bf16, cudaStream_t s) {
+  switch (reg_k_tiles(p.D)) {
+    case 2: return launch_bwd_reg<CELL, 2, true>(p, cache, history, initial, d_history, wx_bf16, s);
+    case 4:
+      return reg_local(CELL, p.D) ? launch_bwd_reg<CELL, 4, true>(p, cache, history, initial, d_history, wx_bf16, s)
+                                  : launch_bwd_reg<CELL, 4, false>(p, cache, history, initial, d_history, wx_bf16, s);
+    case 6: return launch_bwd_reg<CELL, 6, false>(p, cache, history, initial, d_history, wx_bf16, s);
+    case 8: return launch_bwd_reg<CELL, 8, false>(p, cache, history, initial, d_history, wx_bf16, s);
+    case 10: return launch_bwd_reg<CELL, 10, false>(p, cache, history, initial, d_history, wx_bf16, s);
+    case 12: return launch_bwd_reg<CELL, 12, false>(p, cache, history, initial, d_history, wx_bf16, s);
+    case 14: return launch_bwd_reg<CELL, 14, false>(p, cache, history, initial, d_history, wx_bf16, s);
+    case 16: return launch_bwd_reg<CELL, 16, false>(p, cache, history, initial, d_history, wx_bf16, s);
+    default: return -2;
+  }
+}
+
+}  // namespace
+
+int backward_reg_dispatch(int cell, const BwdParams& p, const void* cache, const float* history, const float* initial,
+                          const float* d_history, int wx_bf16, cudaStream_t s) {
+  switch (cell) {
+    case kLSTM: return launch_bwd_reg_cell<kLSTM>(p, cache, history, initial, d_history, wx_bf16, s);
+    case kSLSTM: return launch_bwd_reg_cell<kSLSTM>(p, cache, history, initial, d_history, wx_bf16, s);
+    case kGRU: return launch_bwd_reg_cell<kGRU>(p, cache, history, initial, d_history, wx_bf16, s);
+    case kElman: return launch_bwd_reg_cell<kElman>(p, cache, history, initial, d_history, wx_bf16, s);
+    default: return -1;
+  }
+}
+
+}  // namespace frnn

@@ -124,6 +124,27 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t parity,
   }
 }
 
+// The same wait made by a whole warp at once: every lane polls, the warp leaves together (all lanes get the same answer),
+// so that warp-wide instructions may follow without a divergence.
+template <bool kClusterScope>
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, uint64_t limit_ns, const volatile int* abort_flag) {
+  auto poll = [&]() -> bool {
+    const bool ok = kClusterScope ? mbar_try_wait_cluster_spin(bar, parity) : mbar_try_wait_spin(bar, parity);
+    return __all_sync(0xffffffffu, ok);
+  };
+  for (int fast = 0; fast < 64; ++fast) {
+    if (poll()) return true;
+  }
+  const uint64_t t0 = global_timer_ns();
+  uint32_t spins = 0;
+  while (true) {
+    if (poll()) return true;
+    if ((++spins & 255u) == 0u &&
+        __any_sync(0xffffffffu, (abort_flag != nullptr && *abort_flag != 0) || global_timer_ns() - t0 > limit_ns))
+      return false;
+  }
+}
+
 // ----------------------------------------------------------------------------------------------
 // proxies / fences
 // ----------------------------------------------------------------------------------------------
@@ -210,6 +231,10 @@ __device__ __forceinline__ void bulk_copy_to_cluster(uint32_t dst_cluster, uint3
 __device__ __forceinline__ void tma_store_2d(const void* tmap, uint32_t src, int c0, int c1) {
   asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];"
                :: "l"(tmap), "r"(src), "r"(c0), "r"(c1) : "memory");
+}
+__device__ __forceinline__ void tma_store_5d(const void* tmap, uint32_t src, int c0, int c1, int c2, int c3, int c4) {
+  asm volatile("cp.async.bulk.tensor.5d.global.shared::cta.bulk_group [%0, {%2, %3, %4, %5, %6}], [%1];"
+               ::"l"(reinterpret_cast<uint64_t>(tmap)), "r"(src), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4) : "memory");
 }
 __device__ __forceinline__ void tma_store_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 // Wait until at most N of this thread's bulk groups still READ their shared-memory source.
@@ -363,6 +388,29 @@ __device__ __forceinline__ void umma_bf16_ts(uint32_t tmem_d, uint32_t tmem_a, u
       :
       : "r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
+}
+
+// ----------------------------------------------------------------------------------------------
+// warp-level tensor-core path (operands in registers): m16n8k16, bf16 operands, fp32 accumulators
+// ----------------------------------------------------------------------------------------------
+__device__ __forceinline__ void mma_bf16_16816(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+// Four / two 8x8 blocks of 16-bit values, transposed on the way in; lane i gives the address of row i % 8 of block i / 8.
+__device__ __forceinline__ void ldsm_x4_trans(uint32_t addr, uint32_t (&r)[4]) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void ldsm_x2_trans(uint32_t addr, uint32_t& r0, uint32_t& r1) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0, %1}, [%2];" : "=r"(r0), "=r"(r1) : "r"(addr) : "memory");
+}
+// 8x8 block of 16-bit values held by a warp (lane i: row i / 4, columns 2 (i % 4), + 1) -> its transpose, same layout.
+__device__ __forceinline__ uint32_t movmatrix_trans(uint32_t v) {
+  uint32_t r;
+  asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(r) : "r"(v));
+  return r;
 }
 
 // Asynchronous stores into the shared memory of a CTA of the cluster. Each store also reports
