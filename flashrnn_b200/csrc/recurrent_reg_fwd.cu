@@ -15,7 +15,10 @@
 // A group cannot overtake itself: a half of the operand double buffer is written again only after every warp has published
 // the step in between, and a warp publishes after its own reads of that half.
 //
-// Bound: the serial chain of a step (operand wait, ldmatrix, mma chain, activations, exchange), not memory or math.
+// Bound: the serial chain of a step, mostly instruction issue of one warp per scheduler: at LSTM B8 N3 D256, 1331 cycles =
+// operand wait 150 + Wx read and 32 mma 471 + cell 161 + publication 221 + staging of the outputs 318. Per step there, against
+// the tcgen05 kernel: 0.80 us against 1.29; GRU B16 N24 D32 0.63 against 0.68; Elman B16 N12 D64 0.52 against 0.66. A wait of
+// its own for the Wx tile cost 150 cycles more (D256: 0.85 us).
 #include "recurrent_reg.cuh"
 
 namespace frnn {
@@ -63,7 +66,7 @@ frnn_fwd_reg_kernel(const FwdParams p, const __grid_constant__ CUtensorMap wx_ma
   const bool prof = p.err[3] != 0 && blockIdx.x == 0 && tid == 0;
 
   if (tid == 0) {
-    for (int i = 0; i < 2; ++i) mbar_init(smem_u32(&s_hbar[i]), LOCAL ? nwarps : 1);
+    for (int i = 0; i < 2; ++i) mbar_init(smem_u32(&s_hbar[i]), (LOCAL ? nwarps : 1) + 1);  // + the I/O warp: Wx has landed
     for (int i = 0; i < slots; ++i) mbar_init(smem_u32(&s_out_full[i]), nwarps);
     for (int s = 0; s < nst; ++s) mbar_init(smem_u32(&s_wx_full[s]), 1);
     s_gave_up = 0;
@@ -98,14 +101,31 @@ frnn_fwd_reg_kernel(const FwdParams p, const __grid_constant__ CUtensorMap wx_ma
           tma_load_5d(dst + i * chunk_bytes, &wx_map, bar, rank * U + i * kRegChunk, n, b0, 0, p.t0 + t);
       };
       for (int t = 0; t < nst && t < T; ++t) fill(t, t);
-      int stage = 0, slot = 0;
-      uint32_t phase = 0;
-      for (int t = 0; t < T; ++t) {
+      int stage = 0, slot = 0, next = 1 % nst;
+      uint32_t phase = 0, next_phase = 1 / nst;
+      // The operand barrier of step t also stands for its Wx tile: one wait per step on the compute warps' chain, not two.
+      auto announce = [&](int t) -> bool {
+        if (!mbar_wait_bounded<false, true>(smem_u32(&s_wx_full[next]), next_phase & 1, limit, abort_flag)) {
+          reg_report(p.err, kErrWaitWx, t);
+          return false;
+        }
+        if (++next == nst) { next = 0; next_phase ^= 1u; }
+        mbar_arrive(smem_u32(&s_hbar[t & 1]));
+        return true;
+      };
+      bool ok = true;
+      for (int t = 1; t <= 2 && t < nst && t < T && ok; ++t) ok = announce(t);
+      for (int t = 0; t < T && ok; ++t) {
         // released by the CTA's own warps, whose waits have the plain limit: theirs run out first
         if (!mbar_wait_bounded<false, true>(smem_u32(&s_out_full[slot]), phase, 2 * limit, abort_flag)) {
           reg_report(p.err, kErrWaitEpi, t);
           break;
         }
+        // A warp that gave up on a wait sets the flag before it stages. Then the phase that the barrier is in may never
+        // complete (another arrival would overrun its count), and a copy could be on its way into the stage: stop here.
+        if (*reinterpret_cast<volatile int*>(&s_gave_up) != 0) break;
+        // step t + 2 uses the barrier of step t, which every warp has left
+        if (nst > 2 && t >= 1 && t + 2 < T) ok = announce(t + 2);
         for (int i = 0; i < chunks; ++i) {
           const uint32_t src = smem_u32(outs + slot * out_slot + i * out_chunk);
           const int x = rank * U + i * kRegChunk;
@@ -115,10 +135,8 @@ frnn_fwd_reg_kernel(const FwdParams p, const __grid_constant__ CUtensorMap wx_ma
         }
         tma_store_commit();
         tma_store_wait_read<1>();  // the copies of step t - 1 have read their slot: see kRegMaxSlots
-        // every warp that staged step t had read its Wx; a warp that gave up on a wait may not have, and a copy could be
-        // on its way into the stage
-        if (*reinterpret_cast<volatile int*>(&s_gave_up) != 0) break;
         if (t + nst < T) fill(t + nst, stage);
+        if (nst <= 2 && t + 2 < T) ok = announce(t + 2);
         if (++stage == nst) stage = 0;
         if (++slot == slots) { slot = 0; phase ^= 1u; }
       }
@@ -163,7 +181,6 @@ frnn_fwd_reg_kernel(const FwdParams p, const __grid_constant__ CUtensorMap wx_ma
     uint8_t* const my_out = outs + (warp >> 2) * out_chunk;
     uint8_t* out = my_out;
     int slot = 0, in_stage = 0;
-    uint32_t in_phase = 0;
     bool dead = false;  // warp-uniform: after a failed wait the warp walks on without waiting
     auto give_up = [&](int code, int t) {
       if (lane == 0) reg_report(p.err, code, t);
@@ -171,8 +188,7 @@ frnn_fwd_reg_kernel(const FwdParams p, const __grid_constant__ CUtensorMap wx_ma
       *reinterpret_cast<volatile int*>(&s_gave_up) = 1;
     };
     float wx[CT::GW][2];
-    auto read_wx = [&](int t) {
-      if (!dead && !mbar_wait_warp<false>(smem_u32(&s_wx_full[in_stage]), in_phase, limit, abort_flag)) give_up(kErrWaitWx, t);
+    auto read_wx = [&]() {
       const uint8_t* ws = my_chunk + in_stage * stage_bytes;
 #pragma unroll
       for (int g = 0; g < CT::GW; ++g)
@@ -181,7 +197,7 @@ frnn_fwd_reg_kernel(const FwdParams p, const __grid_constant__ CUtensorMap wx_ma
           if (wx_bf16) wx[g][e] = __bfloat162float(*reinterpret_cast<const __nv_bfloat16*>(ws + g * kRegPlane<2> + reg_tile_offset<2>(2 * c + e, uc)));
           else wx[g][e] = *reinterpret_cast<const float*>(ws + g * kRegPlane<4> + reg_tile_offset<4>(2 * c + e, uc));
         }
-      if (++in_stage == nst) { in_stage = 0; in_phase ^= 1u; }
+      if (++in_stage == nst) in_stage = 0;
     };
 
     uint32_t peer_delta[2] = {0u, 0u};  // C <= 8: a lane of a quad sends to the peers c and c + 4
@@ -193,7 +209,7 @@ frnn_fwd_reg_kernel(const FwdParams p, const __grid_constant__ CUtensorMap wx_ma
     }
     if (prof) p.err[20] = static_cast<int>(clock64() - t_entry);
 
-    read_wx(0);
+    if (!mbar_wait_warp<false>(smem_u32(&s_wx_full[0]), 0, limit, abort_flag)) give_up(kErrWaitWx, 0);
     long long pc[6] = {0, 0, 0, 0, 0, 0};
     for (int t = 0; t < T; ++t) {
       if (jitter != 0u) { jitter_stall(jitter, static_cast<uint32_t>(warp), static_cast<uint32_t>(t)); __syncwarp(); }
@@ -201,6 +217,7 @@ frnn_fwd_reg_kernel(const FwdParams p, const __grid_constant__ CUtensorMap wx_ma
       const long long c1 = prof ? clock64() : 0;
       if (t >= 1 && !dead && !mbar_wait_warp<!LOCAL>(smem_u32(&s_hbar[pb]), ((t - 1) >> 1) & 1, limit, abort_flag)) give_up(kErrWaitH, t);
       const long long c2 = prof ? clock64() : 0;
+      read_wx();
       float acc[2][NT][4];  // even and odd k tiles: twice the independent chains
 #pragma unroll
       for (int h = 0; h < 2; ++h)
@@ -285,18 +302,17 @@ frnn_fwd_reg_kernel(const FwdParams p, const __grid_constant__ CUtensorMap wx_ma
       out += out_slot;
       if (++slot == slots) { slot = 0; out = my_out; }
       const long long c6 = prof ? clock64() : 0;
-      if (t + 1 < T) read_wx(t + 1);
       if (prof) {
-        pc[0] += clock64() - c6; pc[1] += c2 - c1; pc[2] += c3 - c2; pc[3] += c4 - c3; pc[4] += c5 - c4; pc[5] += c6 - c5;
+        pc[0] += clock64() - c1; pc[1] += c2 - c1; pc[2] += c3 - c2; pc[3] += c4 - c3; pc[4] += c5 - c4; pc[5] += c6 - c5;
       }
     }
     if (prof) {  // the slots of the tcgen05 kernels' phase timers that have a counterpart here
-      p.err[8] = static_cast<int>(pc[0]);    // Wx stage wait and read
+      p.err[15] = static_cast<int>(pc[0]);   // the whole step
       p.err[12] = static_cast<int>(pc[3]);   // accumulators -> h_t
       p.err[13] = static_cast<int>(pc[4]);   // publication
       p.err[14] = static_cast<int>(pc[5]);   // outputs staged
       p.err[16] = static_cast<int>(pc[1]);   // operand wait
-      p.err[17] = static_cast<int>(pc[2]);   // ldmatrix + mma issue
+      p.err[17] = static_cast<int>(pc[2]);   // Wx read, ldmatrix, mma
     }
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
@@ -375,7 +391,7 @@ int launch_fwd_reg_cell(const FwdParams& p, const void* wx, int wx_bf16, cudaStr
   switch (reg_k_tiles(p.D)) {
     case 2: return launch_fwd_reg<CELL, 2, true>(p, wx, wx_bf16, s);
     case 4:
-      return reg_local(CELL, p.D) ? launch_fwd_reg<CELL, 4, true>(p, wx, wx_bf16, s)
+      return reg_local(p.D) ? launch_fwd_reg<CELL, 4, true>(p, wx, wx_bf16, s)
                                   : launch_fwd_reg<CELL, 4, false>(p, wx, wx_bf16, s);
     case 6: return launch_fwd_reg<CELL, 6, false>(p, wx, wx_bf16, s);
     case 8: return launch_fwd_reg<CELL, 8, false>(p, wx, wx_bf16, s);
