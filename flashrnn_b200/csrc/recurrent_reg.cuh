@@ -14,7 +14,7 @@ namespace frnn {
 constexpr int kRegUnitsPerWarp = 8;
 constexpr int kRegRows = 8;           // batch rows of a group: the column extent of one mma
 constexpr int kRegClusterUnits = 32;  // units of a CTA where a group is a thread-block cluster
-constexpr int kRegNoRoom = -100;      // a launch would need more than one wave of clusters
+constexpr int kRegNoRoom = -100;      // not taken: more than one wave of clusters, or outputs off the 16-byte grid
 
 // Widths of these kernels. One CTA holds a head of 16, 32 or 48 units whole; other widths run as a cluster of D / 32 CTAs.
 // At 64 units one CTA's 8 warps share each scheduler two by two and its I/O warp moves two 32-unit tiles per step: LSTM, 8

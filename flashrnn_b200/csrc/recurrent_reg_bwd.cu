@@ -453,6 +453,8 @@ int launch_bwd_reg(const BwdParams& p, const void* cache, const float* history, 
   const int smem = bytes(nst);
   const int D = p.D, N = p.N, B = p.B;
   const uint64_t nd = static_cast<uint64_t>(N) * D, uT = p.T, uB = p.B;
+  // bulk stores start on 16-byte boundaries; the tcgen05 kernels write these outputs with plain stores
+  if (((reinterpret_cast<uintptr_t>(p.dwx) | reinterpret_cast<uintptr_t>(p.dgr)) & 15u) != 0) return kRegNoRoom;
   CUtensorMap cache_map, hist_map, init_map, dhist_map, dgr_map, dwx_map;
   if (reg_tile_map(&hist_map, history, 4, D, N, B, CT::S, p.T, uT * nd, uB * uT * nd, nd, Cfg::HS) != 0 ||
       reg_tile_map(&dhist_map, d_history, 4, D, N, B, CT::S, p.T, uT * nd, uB * uT * nd, nd, CT::S) != 0 ||

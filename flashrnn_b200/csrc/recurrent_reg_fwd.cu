@@ -348,6 +348,9 @@ int launch_fwd_reg(const FwdParams& p, const void* wx, int wx_bf16, cudaStream_t
   const auto bytes = [&](int st) { return 2 * KT * 16 * 16 + st * stage + (st + 1) * out_slot; };
   const int nst = bytes(kRegMaxStages) <= 110 * 1024 ? kRegMaxStages : 2;
   const int smem = bytes(nst);
+  // bulk stores start on 16-byte boundaries; the tcgen05 kernels write these outputs with plain stores
+  if (((reinterpret_cast<uintptr_t>(p.history) | reinterpret_cast<uintptr_t>(p.cache) | reinterpret_cast<uintptr_t>(p.hbf)) & 15u) != 0)
+    return kRegNoRoom;
   CUtensorMap map, hist_map, cache_map, hbf_map;
   const uint64_t nd = static_cast<uint64_t>(p.N) * p.D, T = p.T, Tt = p.T_total;
   if (reg_tile_map(&map, wx, es, p.D, p.N, p.B, CT::GW, p.T_total, Tt * CT::GW * nd, nd, CT::GW * nd, CT::GW) != 0) return -4;
