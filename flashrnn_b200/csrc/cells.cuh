@@ -165,9 +165,9 @@ __device__ __forceinline__ void cell_backward(const float* cache, const float* s
     float d_logf = d_fg * fg;
     const float dm = slstm_v1 ? 0.0f : ds[3] - d_i - d_logf;
     if (slstm_take_i) {
-      d_i += dm;
+      d_i = __fmaf_rn(d_ig, ig, dm);
     } else if (i > logf) {
-      d_i += dm;
+      d_i = __fmaf_rn(d_ig, ig, dm);
     } else if (i < logf) {
       d_logf += dm;
     } else {

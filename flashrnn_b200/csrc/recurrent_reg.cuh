@@ -51,10 +51,15 @@ inline int reg_tile_map(CUtensorMap* map, const void* base, int es, int D, int N
 }
 
 // CTAs per SM the register budget is cut for. Two CTAs of 5 warps leave 168 registers a thread: enough up to 128 units of
-// contraction (and for the one-gate cell), while wider slices would spill their fragments, 468 bytes at 256.
-constexpr int reg_min_blocks(int cell, int kt, bool local) {
-  return local ? (kt <= 2 ? 4 : (cell == kSLSTM ? 1 : 2)) : (kt <= 8 || cell == kElman ? 2 : 1);
+// contraction (and for the one-gate cell), while wider slices would spill their fragments, 468 bytes at 256. One-CTA backward
+// kernels hold the fragments of all gates of a tile (one sum per tile): four-gate cells would spill at four CTAs per SM, sLSTM
+// B16 T1024 N24 D32 2133 us forward and backward against 1849 at three.
+constexpr int reg_min_blocks(int cell, int kt, bool local, bool backward) {
+  return local ? (kt <= 2 ? (backward && (cell == kLSTM || cell == kSLSTM) ? 3 : 4) : (cell == kSLSTM ? 1 : 2)) : (kt <= 8 || cell == kElman ? 2 : 1);
 }
+
+// Threads of a CTA: a warp per 8 units (4 in a cluster; up to 32 units with two k tiles, 48 with four) and the I/O warp.
+constexpr int reg_max_threads(int kt, bool local) { return local && kt > 2 ? 7 * 32 : 5 * 32; }
 
 #ifdef __CUDACC__
 template <int ES> constexpr int kRegPlane = kRegRows * kRegChunk * ES;  // bytes of a staged plane

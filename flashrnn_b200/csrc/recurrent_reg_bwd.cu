@@ -6,8 +6,12 @@
 //   2. multiplies with its warp's fragments of R_slice^T [D x GR*U] (rows = units p of h_{t-1}, k = gate rows of this CTA),
 //   3. hands the accumulators to the owners of those units: two lanes swap halves so that each packet is 4 batch rows of
 //      one unit, 16 bytes.
-// LOCAL: D / 16 row tiles for D / 8 warps, so two warps share a tile and take half of k each: their two partial results
-//        are the "sources" of step 1.  else: the sources are the CTAs of the cluster, packets travel by st.async.
+// The sums of step 2 run over the same gate rows in the same order as in the tcgen05 kernels, whose CTAs own 32 units (16
+// where the width is not a multiple of 32), and step 1 adds them in the same order: every gradient is the same bits, whichever
+// kernels a call takes.
+//   LOCAL: D / 16 row tiles for D / 8 warps. 16 and 32 units: one sum per tile, which half of the warps run; 48 units: three
+//          "sources" of 16 units each, two for the first half of the warps and one for the second.
+//   else:  the sources are the CTAs of the cluster, packets travel by st.async.
 // The state of step t - 1 stays in registers as the new state of the next iteration, and only the planes that the cell's
 // derivative reads are fetched: an LSTM reads one history plane per step where reading both states at t and t - 1 takes four.
 //
@@ -34,9 +38,13 @@ template <> struct HistPlanes<kElman> { static constexpr int first = 0, count = 
 template <int CELL, int KT, bool LOCAL>
 struct BwdRegCfg {
   using CT = CellTraits<CELL>;
-  static constexpr int MTW = LOCAL ? 1 : (KT + 3) / 4;                    // row tiles of a warp
-  static constexpr int KTW = LOCAL ? (CT::GR * KT + 1) / 2 : 2 * CT::GR;  // k tiles of a warp
-  static constexpr int DG_BYTES = ((LOCAL ? 2 : 1) * KTW * 16 * 16 + 511) / 512 * 512;  // two of them: the tiles stay 1 KB aligned
+  static constexpr int MTW = LOCAL ? 1 : (KT + 3) / 4;  // row tiles of a warp
+  static constexpr int KTW = 2 * CT::GR;                // k tiles of a warp
+  // Sums of a tile: one over all gate rows of the CTA, except in a 48-unit CTA, where units 0 .. 15, 16 .. 31 and 32 .. 47
+  // have one each and a warp of the first half of the warps runs two of them.
+  static constexpr int CH = LOCAL && KT == 4 ? 2 : 1;
+  static constexpr int MAX_SOURCES = LOCAL ? (KT == 4 ? 3 : 1) : 8;
+  static constexpr int DG_BYTES = (CT::GR * (LOCAL ? KT * 16 : 32) * 16 + 511) / 512 * 512;  // two of them: the tiles stay 1 KB aligned
   static constexpr int GCL = CELL == kElman ? 0 : CT::GC;
   static constexpr int HP = HistPlanes<CELL>::first, HS = HistPlanes<CELL>::count;
   static constexpr int PLANE4 = kRegRows * kRegChunk * 4, PLANEC = kRegRows * kRegChunk * CT::CES;
@@ -44,14 +52,14 @@ struct BwdRegCfg {
 };
 
 template <int CELL, int KT, bool LOCAL>
-__global__ void __launch_bounds__(LOCAL ? 64 * KT + 32 : 160, reg_min_blocks(CELL, KT, LOCAL))
+__global__ void __launch_bounds__(reg_max_threads(KT, LOCAL), reg_min_blocks(CELL, KT, LOCAL, true))
 frnn_bwd_reg_kernel(const BwdParams p, const float* history, const __grid_constant__ CUtensorMap cache_map,
                     const __grid_constant__ CUtensorMap hist_map, const __grid_constant__ CUtensorMap init_map,
                     const __grid_constant__ CUtensorMap dhist_map, const __grid_constant__ CUtensorMap dgr_map,
                     const __grid_constant__ CUtensorMap dwx_map, const int wx_bf16, const int own_dwx, const int nst) {
   using Cfg = BwdRegCfg<CELL, KT, LOCAL>;
   using CT = CellTraits<CELL>;
-  constexpr int S = CT::S, MTW = Cfg::MTW, KTW = Cfg::KTW, GCL = Cfg::GCL, HP = Cfg::HP, HS = Cfg::HS;
+  constexpr int S = CT::S, MTW = Cfg::MTW, KTW = Cfg::KTW, CH = Cfg::CH, GCL = Cfg::GCL, HP = Cfg::HP, HS = Cfg::HS;
 
   extern __shared__ __align__(1024) uint8_t smem[];
   __shared__ __align__(8) uint64_t s_part_bar[2];
@@ -66,7 +74,7 @@ frnn_bwd_reg_kernel(const BwdParams p, const float* history, const __grid_consta
   const int C = LOCAL ? 1 : p.C;
   const int rank = LOCAL ? 0 : static_cast<int>(blockIdx.x % C), gid = blockIdx.x / C;
   const int n = gid % N, b0 = gid / N * kRegRows;
-  const int sources = LOCAL ? 2 : C;
+  const int sources = LOCAL ? Cfg::MAX_SOURCES : C;
   const int part_bytes = sources * U * kRegRows * 4;  // one parity: [source][unit][8 batch rows] fp32
   const int chunks = (U + kRegChunk - 1) / kRegChunk, stage_bytes = chunks * Cfg::CHUNK;
   uint8_t* const dgbuf = smem;
@@ -167,7 +175,7 @@ frnn_bwd_reg_kernel(const BwdParams p, const float* history, const __grid_consta
   } else {
     // A fragments of R_slice^T: 8x8 blocks of R are loaded as they lie (gate rows x units p) and transposed in the warp.
     const int n_tiles = D / 16;
-    const int khalf = LOCAL ? warp / n_tiles : 0;
+    const int part0 = LOCAL ? warp / n_tiles * Cfg::CH : 0;  // first source of this warp
     const int tile0 = LOCAL ? warp % n_tiles : warp;
     uint32_t a[MTW][KTW][4];
 #pragma unroll
@@ -176,11 +184,12 @@ frnn_bwd_reg_kernel(const BwdParams p, const float* history, const __grid_consta
       for (int kt = 0; kt < KTW; ++kt)
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
-          const int k8 = (khalf * KTW + kt) * 2 + (r >> 1);  // block of 8 gate rows
+          // block of 8 gate rows: tile kt of the gate-major rows; with CH sums per warp, gate kt % GR of 16 units
+          const int k8 = CH == 1 ? kt * 2 + (r >> 1) : kt % CT::GR * nwarps + 2 * (part0 + kt / CT::GR) + (r >> 1);
           const int g = k8 * 8 / U, u = k8 * 8 % U + q;
           const int pcol = (tile0 + (LOCAL ? 0 : 4 * m)) * 16 + 8 * (r & 1) + 2 * c;
           uint32_t v = 0u;
-          if (g < CT::GR && pcol < D)
+          if (g < CT::GR && pcol < D && part0 + (CH == 1 ? 0 : kt / CT::GR) < sources)
             v = __ldg(reinterpret_cast<const uint32_t*>(p.R + ((static_cast<size_t>(g) * N + n) * D + rank * U + u) * D + pcol));
           a[m][kt][r] = movmatrix_trans(v);
         }
@@ -189,9 +198,9 @@ frnn_bwd_reg_kernel(const BwdParams p, const float* history, const __grid_consta
     const size_t ND = static_cast<size_t>(N) * D, BND = static_cast<size_t>(B) * ND;
     const size_t sBTND = static_cast<size_t>(T) * BND;
     bool act[2];
-    float dcar[S][2], dbacc[CT::GB], sn[HS][2];
+    float dcar[S][2], dbacc[CT::GB][2], sn[HS][2];
 #pragma unroll
-    for (int g = 0; g < CT::GB; ++g) dbacc[g] = 0.0f;
+    for (int g = 0; g < CT::GB; ++g) dbacc[g][0] = dbacc[g][1] = 0.0f;
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
       const size_t b = static_cast<size_t>(b0 + 2 * c + e);
@@ -217,7 +226,7 @@ frnn_bwd_reg_kernel(const BwdParams p, const float* history, const __grid_consta
     for (int m = 0; m < MTW; ++m) {
       const int tile = tile0 + (LOCAL ? 0 : 4 * m);
       if (LOCAL) {
-        dst_part[m] = smem_u32(part) + (khalf * U + tile * 16) * (kRegRows * 4) + row_off;
+        dst_part[m] = smem_u32(part) + (part0 * U + tile * 16) * (kRegRows * 4) + row_off;
         dst_bar[m] = 0u;
       } else {
         const int owner = tile < n_tiles ? tile / 2 : rank;  // 32 units, two tiles
@@ -254,7 +263,7 @@ frnn_bwd_reg_kernel(const BwdParams p, const float* history, const __grid_consta
     if (prof) p.err[20] = static_cast<int>(clock64() - t_entry);
 
     if (!mbar_wait_warp<false>(smem_u32(&s_full[0]), 0, limit, abort_flag)) give_up(kErrWaitWx, 0);
-    constexpr int kSrc = LOCAL ? 2 : 8;
+    constexpr int kSrc = Cfg::MAX_SOURCES;
     long long pc[6] = {0, 0, 0, 0, 0, 0};
     for (int it = 0; it <= T; ++it) {
       if (jitter != 0u) { jitter_stall(jitter, static_cast<uint32_t>(warp), static_cast<uint32_t>(it)); __syncwarp(); }
@@ -319,9 +328,7 @@ frnn_bwd_reg_kernel(const BwdParams p, const float* history, const __grid_consta
 #pragma unroll
         for (int g = 0; g < CT::GR; ++g) dgr[g][e] = act[e] ? gr[g] : 0.0f;
 #pragma unroll
-        for (int g = 0; g < CT::GW; ++g) dgw[g][e] = gw[g];
-#pragma unroll
-        for (int g = 0; g < CT::GB; ++g) dbacc[g] += act[e] ? gb[g] : 0.0f;
+        for (int g = 0; g < CT::GW; ++g) dgw[g][e] = act[e] ? gw[g] : 0.0f;
       }
       uint32_t dgp[CT::GR];
       const uint32_t dgs = smem_u32(dgbuf) + (it & 1) * Cfg::DG_BYTES;
@@ -335,8 +342,8 @@ frnn_bwd_reg_kernel(const BwdParams p, const float* history, const __grid_consta
       asm volatile("bar.sync 1, %0;" ::"r"(compute_threads) : "memory");
       const long long c3 = prof ? clock64() : 0;
       const int nb = (it + 1) & 1;
-      {
-        constexpr int CH = LOCAL ? 2 : 1;  // a single tile runs as two independent chains
+      const bool publish = !dead && it < mute_from;
+      if (!LOCAL || part0 < sources) {
         float acc[CH][MTW][4];
 #pragma unroll
         for (int h = 0; h < CH; ++h)
@@ -344,48 +351,59 @@ frnn_bwd_reg_kernel(const BwdParams p, const float* history, const __grid_consta
           for (int m = 0; m < MTW; ++m)
 #pragma unroll
             for (int r = 0; r < 4; ++r) acc[h][m][r] = 0.0f;
-        const uint32_t ab = dgs + khalf * KTW * 256;
+        if constexpr (CH == 1) {
 #pragma unroll
-        for (int k2 = 0; k2 < (KTW + 1) / 2; ++k2) {
-          uint32_t bf[4];
-          if (2 * k2 + 1 < KTW) ldsm_x4_trans(ab + lane * 16 + k2 * 512, bf);
-          else ldsm_x2_trans(ab + (lane & 15) * 16 + k2 * 512, bf[0], bf[1]);
+          for (int k2 = 0; k2 < KTW / 2; ++k2) {
+            uint32_t bf[4];
+            ldsm_x4_trans(dgs + lane * 16 + k2 * 512, bf);
 #pragma unroll
-          for (int m = 0; m < MTW; ++m) mma_bf16_16816(acc[0][m], a[m][2 * k2], bf[0], bf[1]);
-          if (2 * k2 + 1 < KTW) {
+            for (int m = 0; m < MTW; ++m) mma_bf16_16816(acc[0][m], a[m][2 * k2], bf[0], bf[1]);
 #pragma unroll
-            for (int m = 0; m < MTW; ++m) mma_bf16_16816(acc[CH - 1][m], a[m][2 * k2 + 1 < KTW ? 2 * k2 + 1 : 0], bf[2], bf[3]);
+            for (int m = 0; m < MTW; ++m) mma_bf16_16816(acc[0][m], a[m][2 * k2 + 1], bf[2], bf[3]);
           }
+        } else {
+          // gate g of 16 units: the blocks of two warps; a sum past the last source reads zeros behind the gate rows
+#pragma unroll
+          for (int g = 0; g < CT::GR; ++g)
+#pragma unroll
+            for (int h = 0; h < CH; ++h) {
+              uint32_t b0, b1;
+              ldsm_x2_trans(dgs + (g * nwarps + 2 * (part0 + h)) * 128 + (lane & 15) * 16, b0, b1);
+              mma_bf16_16816(acc[h][0], a[0][h * CT::GR + g], b0, b1);
+            }
         }
-        const bool publish = !dead && it < mute_from;
 #pragma unroll
-        for (int m = 0; m < MTW; ++m) {
-          float v[4];
+        for (int h = 0; h < CH; ++h)
 #pragma unroll
-          for (int r = 0; r < 4; ++r) v[r] = CH == 2 ? acc[0][m][r] + acc[CH - 1][m][r] : acc[0][m][r];
-          // rows q / q + 8, columns 2c, 2c + 1 -> even lanes: row q, columns 2c .. 2c + 3; odd lanes: row q + 8, 2c - 2 .. 2c + 1
-          const float x0 = __shfl_xor_sync(0xffffffffu, (c & 1) ? v[0] : v[2], 1);
-          const float x1 = __shfl_xor_sync(0xffffffffu, (c & 1) ? v[1] : v[3], 1);
-          const float4 w = (c & 1) ? make_float4(x0, x1, v[2], v[3]) : make_float4(v[0], v[1], x0, x1);
-          if constexpr (LOCAL) {
-            if (publish)
-              asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(dst_part[m] + nb * part_bytes), "f"(w.x), "f"(w.y),
-                           "f"(w.z), "f"(w.w) : "memory");
-          } else {
-            if (publish && tile0 + 4 * m < n_tiles)
-              st_async_v4_b32(dst_part[m] + nb * part_bytes, __float_as_uint(w.x), __float_as_uint(w.y), __float_as_uint(w.z),
-                              __float_as_uint(w.w), dst_bar[m] + nb * 8);
+          for (int m = 0; m < MTW; ++m) {
+            const float(&v)[4] = acc[h][m];
+            // rows q / q + 8, columns 2c, 2c + 1 -> even lanes: row q, columns 2c .. 2c + 3; odd lanes: row q + 8, 2c - 2 .. 2c + 1
+            const float x0 = __shfl_xor_sync(0xffffffffu, (c & 1) ? v[0] : v[2], 1);
+            const float x1 = __shfl_xor_sync(0xffffffffu, (c & 1) ? v[1] : v[3], 1);
+            const float4 w = (c & 1) ? make_float4(x0, x1, v[2], v[3]) : make_float4(v[0], v[1], x0, x1);
+            if constexpr (LOCAL) {
+              if (publish && part0 + h < sources)
+                asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(dst_part[m] + nb * part_bytes + h * U * (kRegRows * 4)),
+                             "f"(w.x), "f"(w.y), "f"(w.z), "f"(w.w) : "memory");
+            } else {
+              if (publish && tile0 + 4 * m < n_tiles)
+                st_async_v4_b32(dst_part[m] + nb * part_bytes, __float_as_uint(w.x), __float_as_uint(w.y), __float_as_uint(w.z),
+                                __float_as_uint(w.w), dst_bar[m] + nb * 8);
+            }
           }
-        }
-        if constexpr (LOCAL) {
-          __syncwarp();
-          if (lane == 0 && publish) mbar_arrive(smem_u32(&s_part_bar[nb]));
-        }
+      }
+      if constexpr (LOCAL) {
+        __syncwarp();
+        if (lane == 0 && publish) mbar_arrive(smem_u32(&s_part_bar[nb]));
       }
       // this parity's partial sums were complete at the wait above: armed for iteration it + 2
       if (!LOCAL && tid == 0 && !dead && it >= 1 && it + 2 <= T) mbar_arrive_expect_tx(smem_u32(&s_part_bar[it & 1]), part_tx);
       const long long c4 = prof ? clock64() : 0;
       // outputs, while the partial sums of the next step are on their way
+#pragma unroll
+      for (int g = 0; g < CT::GB; ++g)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) dbacc[g][e] += CELL != kGRU ? dgw[g][e] : (g == 0 ? dgr[0][e] : dgw[g > 0 ? g - 1 : 0][e]);  // as cell_backward's gb
 #pragma unroll
       for (int g = 0; g < CT::GR; ++g) reg_stage_16(out + dwx_bytes + g * kRegPlane<2>, off_q, dgp[g]);
       if (own_dwx) {
@@ -413,15 +431,16 @@ frnn_bwd_reg_kernel(const BwdParams p, const float* history, const __grid_consta
       p.err[12] = static_cast<int>(pc[4]);  // mma and scatter
       p.err[13] = static_cast<int>(pc[5]);  // wait alone
     }
-    // bias gradient of the 8 batch rows: the four lanes of a unit in fixed order
+    // bias gradient of the 8 batch rows, added in their order
 #pragma unroll
     for (int g = 0; g < CT::GB; ++g) {
-      float v = dbacc[g];
-      v += __shfl_xor_sync(0xffffffffu, v, 1);
-      v += __shfl_xor_sync(0xffffffffu, v, 2);
+      float v = 0.0f;
+#pragma unroll
+      for (int k = 0; k < kRegRows; ++k) v += __shfl_sync(0xffffffffu, dbacc[g][k & 1], (lane & ~3) + (k >> 1));
       if (c == 0) {
         float* dst = p.db_part + ((static_cast<size_t>(b0 / p.db_rows) * CT::GB + g) * N + n) * D + d;
-        // an entry of 16 rows gets at most two addends on top of the launcher's zeros: the order cannot matter
+        // an entry of 16 rows gets at most two addends on top of the launcher's zeros: the order cannot matter, but the sum may
+        // differ in its last bits from the 16 rows added one by one
         if (p.db_rows == kRegRows) *dst = v;
         else atomicAdd(dst, v);
       }
@@ -447,7 +466,7 @@ int launch_bwd_reg(const BwdParams& p, const void* cache, const float* history, 
   const int out_slot = reg_chunks(U) * reg_round_1k(kRegRows * kRegChunk * (CT::GR * 2 + (own_dwx ? CT::GW * (wx_bf16 ? 2 : 4) : 0)));
   // prefetch depth: 4 steps, 2 where only that lets two CTAs share an SM
   const auto bytes = [&](int st) {
-    return 2 * Cfg::DG_BYTES + 2 * (LOCAL ? 2 : C) * U * kRegRows * 4 + st * stage + (st + 1) * out_slot;
+    return 2 * Cfg::DG_BYTES + 2 * (LOCAL ? Cfg::MAX_SOURCES : C) * U * kRegRows * 4 + st * stage + (st + 1) * out_slot;
   };
   const int nst = bytes(kRegMaxStages) <= 110 * 1024 ? kRegMaxStages : 2;
   const int smem = bytes(nst);

@@ -26,7 +26,7 @@ namespace frnn {
 namespace {
 
 template <int CELL, int KT, bool LOCAL>
-__global__ void __launch_bounds__(LOCAL ? 64 * KT + 32 : 160, reg_min_blocks(CELL, KT, LOCAL))
+__global__ void __launch_bounds__(reg_max_threads(KT, LOCAL), reg_min_blocks(CELL, KT, LOCAL, false))
 frnn_fwd_reg_kernel(const FwdParams p, const __grid_constant__ CUtensorMap wx_map, const __grid_constant__ CUtensorMap hist_map,
                     const __grid_constant__ CUtensorMap cache_map, const __grid_constant__ CUtensorMap hbf_map, const int wx_bf16,
                     const int nst, const int hist_states) {
@@ -218,22 +218,21 @@ frnn_fwd_reg_kernel(const FwdParams p, const __grid_constant__ CUtensorMap wx_ma
       if (t >= 1 && !dead && !mbar_wait_warp<!LOCAL>(smem_u32(&s_hbar[pb]), ((t - 1) >> 1) & 1, limit, abort_flag)) give_up(kErrWaitH, t);
       const long long c2 = prof ? clock64() : 0;
       read_wx();
-      float acc[2][NT][4];  // even and odd k tiles: twice the independent chains
+      // One chain over k per tile, in the order of the tcgen05 kernels: the sums, and with them every output, are the same bits.
+      float acc[NT][4];
 #pragma unroll
-      for (int h = 0; h < 2; ++h)
+      for (int j = 0; j < NT; ++j)
 #pragma unroll
-        for (int j = 0; j < NT; ++j)
-#pragma unroll
-          for (int r = 0; r < 4; ++r) acc[h][j][r] = 0.0f;
+        for (int r = 0; r < 4; ++r) acc[j][r] = 0.0f;
       const uint32_t hb = smem_u32(hbuf) + pb * kHbuf + lane * 16;
 #pragma unroll
       for (int k2 = 0; k2 < KT / 2; ++k2) {
         uint32_t bf[4];
         ldsm_x4_trans(hb + k2 * 512, bf);
 #pragma unroll
-        for (int j = 0; j < NT; ++j) mma_bf16_16816(acc[0][j], a[j][2 * k2], bf[0], bf[1]);
+        for (int j = 0; j < NT; ++j) mma_bf16_16816(acc[j], a[j][2 * k2], bf[0], bf[1]);
 #pragma unroll
-        for (int j = 0; j < NT; ++j) mma_bf16_16816(acc[1][j], a[j][2 * k2 + 1], bf[2], bf[3]);
+        for (int j = 0; j < NT; ++j) mma_bf16_16816(acc[j], a[j][2 * k2 + 1], bf[2], bf[3]);
       }
       const long long c3 = prof ? clock64() : 0;
       float cv[CT::GC][2];
@@ -242,7 +241,7 @@ frnn_fwd_reg_kernel(const FwdParams p, const __grid_constant__ CUtensorMap wx_ma
       for (int e = 0; e < 2; ++e) {
         float ryj[CT::GR], wxj[CT::GW], sj[CT::S], cj[CT::GC];
 #pragma unroll
-        for (int g = 0; g < CT::GR; ++g) ryj[g] = acc[0][g / 2][2 * (g & 1) + e] + acc[1][g / 2][2 * (g & 1) + e];
+        for (int g = 0; g < CT::GR; ++g) ryj[g] = acc[g / 2][2 * (g & 1) + e];
 #pragma unroll
         for (int g = 0; g < CT::GW; ++g) wxj[g] = wx[g][e];
 #pragma unroll
