@@ -16,11 +16,12 @@ constexpr int kRegRows = 8;           // batch rows of a group: the column exten
 constexpr int kRegClusterUnits = 32;  // units of a CTA where a group is a thread-block cluster
 constexpr int kRegNoRoom = -100;      // not taken: more than one wave of clusters, or outputs off the 16-byte grid
 
-// Widths of these kernels. One CTA holds a head of 16, 32 or 48 units whole; other widths run as a cluster of D / 32 CTAs.
+// Widths of these kernels: all multiples of 16 up to 256. One CTA holds a head of 16, 32 or 48 units whole; other widths run as
+// a cluster of ceil(D / 32) CTAs, the last of which has 16 units where D is an odd multiple of 16.
 // At 64 units one CTA's 8 warps share each scheduler two by two and its I/O warp moves two 32-unit tiles per step: LSTM, 8
 // rows, fp32 Wx, 0.85 + 1.19 us per step forward + backward against 0.63 + 0.68 as a cluster of two; Elman, 16 rows x 12
 // heads, 0.76 + 0.81 us.
-inline bool reg_width(int D) { return (D % 32 == 0 && D <= 256) || D == 16 || D == 48; }
+inline bool reg_width(int D) { return D % 16 == 0 && D <= 256; }
 inline bool reg_local(int D) { return D < 64; }
 
 inline int reg_batch_tiles(int B) { return (B + kRegRows - 1) / kRegRows; }

@@ -11,7 +11,8 @@
 // kernels a call takes.
 //   LOCAL: D / 16 row tiles for D / 8 warps. 16 and 32 units: one sum per tile, which half of the warps run; 48 units: three
 //          "sources" of 16 units each, two for the first half of the warps and one for the second.
-//   else:  the sources are the CTAs of the cluster, packets travel by st.async.
+//   else:  the sources are the CTAs of the cluster, packets travel by st.async. HALVES (odd multiples of 16): two sums per
+//          tile, one for each 16 units of the CTA; the last CTA has units, and a sum, in its first half only.
 // The state of step t - 1 stays in registers as the new state of the next iteration, and only the planes that the cell's
 // derivative reads are fetched: an LSTM reads one history plane per step where reading both states at t and t - 1 takes four.
 //
@@ -35,15 +36,15 @@ template <> struct HistPlanes<kSLSTM> { static constexpr int first = 1, count = 
 template <> struct HistPlanes<kGRU> { static constexpr int first = 0, count = 1; };
 template <> struct HistPlanes<kElman> { static constexpr int first = 0, count = 1; };
 
-template <int CELL, int KT, bool LOCAL>
+template <int CELL, int KT, bool LOCAL, bool HALVES>
 struct BwdRegCfg {
   using CT = CellTraits<CELL>;
   static constexpr int MTW = LOCAL ? 1 : (KT + 3) / 4;  // row tiles of a warp
   static constexpr int KTW = 2 * CT::GR;                // k tiles of a warp
-  // Sums of a tile: one over all gate rows of the CTA, except in a 48-unit CTA, where units 0 .. 15, 16 .. 31 and 32 .. 47
-  // have one each and a warp of the first half of the warps runs two of them.
-  static constexpr int CH = LOCAL && KT == 4 ? 2 : 1;
-  static constexpr int MAX_SOURCES = LOCAL ? (KT == 4 ? 3 : 1) : 8;
+  // Sums of a tile: one over all gate rows of the CTA; in a 48-unit CTA one for units 0 .. 15, 16 .. 31 and 32 .. 47 each, of
+  // which a warp of the first half of the warps runs two; with HALVES one for each half of the CTA's units.
+  static constexpr int CH = HALVES || (LOCAL && KT == 4) ? 2 : 1;
+  static constexpr int MAX_SOURCES = LOCAL ? (KT == 4 ? 3 : 1) : 8 * CH;
   static constexpr int DG_BYTES = (CT::GR * (LOCAL ? KT * 16 : 32) * 16 + 511) / 512 * 512;  // two of them: the tiles stay 1 KB aligned
   static constexpr int GCL = CELL == kElman ? 0 : CT::GC;
   static constexpr int HP = HistPlanes<CELL>::first, HS = HistPlanes<CELL>::count;
@@ -51,13 +52,13 @@ struct BwdRegCfg {
   static constexpr int CHUNK = GCL * PLANEC + (HS + CT::S) * PLANE4;  // cache, state of step t - 1, external gradient
 };
 
-template <int CELL, int KT, bool LOCAL>
+template <int CELL, int KT, bool LOCAL, bool HALVES>
 __global__ void __launch_bounds__(reg_max_threads(KT, LOCAL), reg_min_blocks(CELL, KT, LOCAL, true))
 frnn_bwd_reg_kernel(const BwdParams p, const float* history, const __grid_constant__ CUtensorMap cache_map,
                     const __grid_constant__ CUtensorMap hist_map, const __grid_constant__ CUtensorMap init_map,
                     const __grid_constant__ CUtensorMap dhist_map, const __grid_constant__ CUtensorMap dgr_map,
                     const __grid_constant__ CUtensorMap dwx_map, const int wx_bf16, const int own_dwx, const int nst) {
-  using Cfg = BwdRegCfg<CELL, KT, LOCAL>;
+  using Cfg = BwdRegCfg<CELL, KT, LOCAL, HALVES>;
   using CT = CellTraits<CELL>;
   constexpr int S = CT::S, MTW = Cfg::MTW, KTW = Cfg::KTW, CH = Cfg::CH, GCL = Cfg::GCL, HP = Cfg::HP, HS = Cfg::HS;
 
@@ -74,7 +75,7 @@ frnn_bwd_reg_kernel(const BwdParams p, const float* history, const __grid_consta
   const int C = LOCAL ? 1 : p.C;
   const int rank = LOCAL ? 0 : static_cast<int>(blockIdx.x % C), gid = blockIdx.x / C;
   const int n = gid % N, b0 = gid / N * kRegRows;
-  const int sources = LOCAL ? Cfg::MAX_SOURCES : C;
+  const int sources = LOCAL ? Cfg::MAX_SOURCES : (HALVES ? D / 16 : C);
   const int part_bytes = sources * U * kRegRows * 4;  // one parity: [source][unit][8 batch rows] fp32
   const int chunks = (U + kRegChunk - 1) / kRegChunk, stage_bytes = chunks * Cfg::CHUNK;
   uint8_t* const dgbuf = smem;
@@ -102,7 +103,7 @@ frnn_bwd_reg_kernel(const BwdParams p, const float* history, const __grid_consta
     reinterpret_cast<uint4*>(dgbuf)[i] = make_uint4(0u, 0u, 0u, 0u);
   __syncthreads();
   // the packets carry all 8 columns whatever the number of batch rows in use
-  const uint32_t part_tx = static_cast<uint32_t>(part_bytes);
+  const uint32_t part_tx = static_cast<uint32_t>(HALVES ? sources * min(U, D - rank * U) * kRegRows * 4 : part_bytes);
   if (tid == 0 && !LOCAL) {
     mbar_arrive_expect_tx(smem_u32(&s_part_bar[1]), part_tx);              // iteration 1 (the last one if T == 1)
     if (T >= 2) mbar_arrive_expect_tx(smem_u32(&s_part_bar[0]), part_tx);  // iteration 2
@@ -175,7 +176,8 @@ frnn_bwd_reg_kernel(const BwdParams p, const float* history, const __grid_consta
   } else {
     // A fragments of R_slice^T: 8x8 blocks of R are loaded as they lie (gate rows x units p) and transposed in the warp.
     const int n_tiles = D / 16;
-    const int part0 = LOCAL ? warp / n_tiles * Cfg::CH : 0;  // first source of this warp
+    const int part0 = LOCAL ? warp / n_tiles * CH : 0;   // first sum of this warp in the CTA ...
+    const int source0 = LOCAL ? part0 : rank * CH;       // ... and in the group
     const int tile0 = LOCAL ? warp % n_tiles : warp;
     uint32_t a[MTW][KTW][4];
 #pragma unroll
@@ -184,12 +186,12 @@ frnn_bwd_reg_kernel(const BwdParams p, const float* history, const __grid_consta
       for (int kt = 0; kt < KTW; ++kt)
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
-          // block of 8 gate rows: tile kt of the gate-major rows; with CH sums per warp, gate kt % GR of 16 units
+          // block of 8 gate rows: tile kt of the gate-major rows; with two sums per warp, gate kt % GR of 16 units
           const int k8 = CH == 1 ? kt * 2 + (r >> 1) : kt % CT::GR * nwarps + 2 * (part0 + kt / CT::GR) + (r >> 1);
           const int g = k8 * 8 / U, u = k8 * 8 % U + q;
           const int pcol = (tile0 + (LOCAL ? 0 : 4 * m)) * 16 + 8 * (r & 1) + 2 * c;
           uint32_t v = 0u;
-          if (g < CT::GR && pcol < D && part0 + (CH == 1 ? 0 : kt / CT::GR) < sources)
+          if (g < CT::GR && pcol < D && source0 + (CH == 1 ? 0 : kt / CT::GR) < sources)
             v = __ldg(reinterpret_cast<const uint32_t*>(p.R + ((static_cast<size_t>(g) * N + n) * D + rank * U + u) * D + pcol));
           a[m][kt][r] = movmatrix_trans(v);
         }
@@ -197,6 +199,7 @@ frnn_bwd_reg_kernel(const BwdParams p, const float* history, const __grid_consta
     const int ul = warp * kRegUnitsPerWarp + q, d = rank * U + ul;
     const size_t ND = static_cast<size_t>(N) * D, BND = static_cast<size_t>(B) * ND;
     const size_t sBTND = static_cast<size_t>(T) * BND;
+    const bool own = !HALVES || d < D;  // false in two warps of the last CTA, which take part in the products only
     bool act[2];
     float dcar[S][2], dbacc[CT::GB][2], sn[HS][2];
 #pragma unroll
@@ -204,7 +207,7 @@ frnn_bwd_reg_kernel(const BwdParams p, const float* history, const __grid_consta
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
       const size_t b = static_cast<size_t>(b0 + 2 * c + e);
-      act[e] = b < static_cast<size_t>(B);
+      act[e] = own && b < static_cast<size_t>(B);
 #pragma unroll
       for (int k = 0; k < S; ++k) dcar[k][e] = act[e] ? p.d_carry[k * BND + b * ND + static_cast<size_t>(n) * D + d] : 0.0f;
 #pragma unroll
@@ -226,11 +229,11 @@ frnn_bwd_reg_kernel(const BwdParams p, const float* history, const __grid_consta
     for (int m = 0; m < MTW; ++m) {
       const int tile = tile0 + (LOCAL ? 0 : 4 * m);
       if (LOCAL) {
-        dst_part[m] = smem_u32(part) + (part0 * U + tile * 16) * (kRegRows * 4) + row_off;
+        dst_part[m] = smem_u32(part) + (source0 * U + tile * 16) * (kRegRows * 4) + row_off;
         dst_bar[m] = 0u;
       } else {
         const int owner = tile < n_tiles ? tile / 2 : rank;  // 32 units, two tiles
-        dst_part[m] = map_to_cta(smem_u32(part) + (rank * U + (tile & 1) * 16) * (kRegRows * 4) + row_off, owner);
+        dst_part[m] = map_to_cta(smem_u32(part) + (source0 * U + (tile & 1) * 16) * (kRegRows * 4) + row_off, owner);
         dst_bar[m] = map_to_cta(smem_u32(&s_part_bar[0]), owner);
       }
     }
@@ -263,7 +266,7 @@ frnn_bwd_reg_kernel(const BwdParams p, const float* history, const __grid_consta
     if (prof) p.err[20] = static_cast<int>(clock64() - t_entry);
 
     if (!mbar_wait_warp<false>(smem_u32(&s_full[0]), 0, limit, abort_flag)) give_up(kErrWaitWx, 0);
-    constexpr int kSrc = Cfg::MAX_SOURCES;
+    constexpr int kSrc = HALVES ? 8 : Cfg::MAX_SOURCES;  // sources read at once
     long long pc[6] = {0, 0, 0, 0, 0, 0};
     for (int it = 0; it <= T; ++it) {
       if (jitter != 0u) { jitter_stall(jitter, static_cast<uint32_t>(warp), static_cast<uint32_t>(it)); __syncwarp(); }
@@ -292,6 +295,14 @@ frnn_bwd_reg_kernel(const BwdParams p, const float* history, const __grid_consta
         for (int e = 0; e < 2; ++e) ds[k][e] = it < T ? dcar[k][e] + dh[k][e] : dcar[k][e];
 #pragma unroll
       for (int k = 0; k < kSrc; ++k) { ds[0][0] += v[k].x; ds[0][1] += v[k].y; }
+      if (HALVES && it >= 1 && !cut) {
+        const uint8_t* pbuf = part + (it & 1) * part_bytes + ul * (kRegRows * 4) + c * 8;
+#pragma unroll
+        for (int k = 0; k < kSrc; ++k)
+          v[k] = kSrc + k < sources ? *reinterpret_cast<const float2*>(pbuf + (kSrc + k) * U * (kRegRows * 4)) : make_float2(0.0f, 0.0f);
+#pragma unroll
+        for (int k = 0; k < kSrc; ++k) { ds[0][0] += v[k].x; ds[0][1] += v[k].y; }
+      }
       if (clip_on && it >= 1 && it < T) {
         // the gradient carried into h_t from step t + 1 (total minus the external part) is complete here: clip it
 #pragma unroll
@@ -343,7 +354,7 @@ frnn_bwd_reg_kernel(const BwdParams p, const float* history, const __grid_consta
       const long long c3 = prof ? clock64() : 0;
       const int nb = (it + 1) & 1;
       const bool publish = !dead && it < mute_from;
-      if (!LOCAL || part0 < sources) {
+      if (!LOCAL || source0 < sources) {
         float acc[CH][MTW][4];
 #pragma unroll
         for (int h = 0; h < CH; ++h)
@@ -362,15 +373,16 @@ frnn_bwd_reg_kernel(const BwdParams p, const float* history, const __grid_consta
             for (int m = 0; m < MTW; ++m) mma_bf16_16816(acc[0][m], a[m][2 * k2 + 1], bf[2], bf[3]);
           }
         } else {
-          // gate g of 16 units: the blocks of two warps; a sum past the last source reads zeros behind the gate rows
+          // gate g: the blocks of four warps, two for each sum; a sum past the last source is computed and dropped
 #pragma unroll
-          for (int g = 0; g < CT::GR; ++g)
+          for (int g = 0; g < CT::GR; ++g) {
+            uint32_t bf[4];
+            ldsm_x4_trans(dgs + (g * nwarps + 2 * part0) * 128 + lane * 16, bf);
 #pragma unroll
-            for (int h = 0; h < CH; ++h) {
-              uint32_t b0, b1;
-              ldsm_x2_trans(dgs + (g * nwarps + 2 * (part0 + h)) * 128 + (lane & 15) * 16, b0, b1);
-              mma_bf16_16816(acc[h][0], a[0][h * CT::GR + g], b0, b1);
-            }
+            for (int m = 0; m < MTW; ++m) mma_bf16_16816(acc[0][m], a[m][g], bf[0], bf[1]);
+#pragma unroll
+            for (int m = 0; m < MTW; ++m) mma_bf16_16816(acc[CH - 1][m], a[m][CT::GR + g], bf[2], bf[3]);
+          }
         }
 #pragma unroll
         for (int h = 0; h < CH; ++h)
@@ -382,12 +394,12 @@ frnn_bwd_reg_kernel(const BwdParams p, const float* history, const __grid_consta
             const float x1 = __shfl_xor_sync(0xffffffffu, (c & 1) ? v[1] : v[3], 1);
             const float4 w = (c & 1) ? make_float4(x0, x1, v[2], v[3]) : make_float4(v[0], v[1], x0, x1);
             if constexpr (LOCAL) {
-              if (publish && part0 + h < sources)
+              if (publish && source0 + h < sources)
                 asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(dst_part[m] + nb * part_bytes + h * U * (kRegRows * 4)),
                              "f"(w.x), "f"(w.y), "f"(w.z), "f"(w.w) : "memory");
             } else {
-              if (publish && tile0 + 4 * m < n_tiles)
-                st_async_v4_b32(dst_part[m] + nb * part_bytes, __float_as_uint(w.x), __float_as_uint(w.y), __float_as_uint(w.z),
+              if (publish && tile0 + 4 * m < n_tiles && (!HALVES || source0 + h < sources))
+                st_async_v4_b32(dst_part[m] + nb * part_bytes + h * U * (kRegRows * 4), __float_as_uint(w.x), __float_as_uint(w.y), __float_as_uint(w.z),
                                 __float_as_uint(w.w), dst_bar[m] + nb * 8);
             }
           }
@@ -437,7 +449,7 @@ frnn_bwd_reg_kernel(const BwdParams p, const float* history, const __grid_consta
       float v = 0.0f;
 #pragma unroll
       for (int k = 0; k < kRegRows; ++k) v += __shfl_sync(0xffffffffu, dbacc[g][k & 1], (lane & ~3) + (k >> 1));
-      if (c == 0) {
+      if (c == 0 && own) {
         float* dst = p.db_part + ((static_cast<size_t>(b0 / p.db_rows) * CT::GB + g) * N + n) * D + d;
         // an entry of 16 rows gets at most two addends on top of the launcher's zeros: the order cannot matter, but the sum may
         // differ in its last bits from the 16 rows added one by one
@@ -454,19 +466,19 @@ frnn_bwd_reg_kernel(const BwdParams p, const float* history, const __grid_consta
   if (!LOCAL) cluster_sync_all();
 }
 
-template <int CELL, int KT, bool LOCAL>
+template <int CELL, int KT, bool LOCAL, bool HALVES = false>
 int launch_bwd_reg(const BwdParams& p, const void* cache, const float* history, const float* initial,
                    const float* d_history, int wx_bf16, cudaStream_t stream) {
-  using Cfg = BwdRegCfg<CELL, KT, LOCAL>;
+  using Cfg = BwdRegCfg<CELL, KT, LOCAL, HALVES>;
   using CT = CellTraits<CELL>;
-  const int U = LOCAL ? p.D : kRegClusterUnits, C = p.D / U;
+  const int U = LOCAL ? p.D : kRegClusterUnits, C = (p.D + U - 1) / U;
   const int stage = reg_chunks(U) * Cfg::CHUNK;
   // cells whose W-gates are their R-gates may have one bf16 buffer for dWx and dg
   const bool own_dwx = !wx_bf16 || CELL == kGRU || p.dwx != static_cast<void*>(p.dgr);
   const int out_slot = reg_chunks(U) * reg_round_1k(kRegRows * kRegChunk * (CT::GR * 2 + (own_dwx ? CT::GW * (wx_bf16 ? 2 : 4) : 0)));
   // prefetch depth: 4 steps, 2 where only that lets two CTAs share an SM
   const auto bytes = [&](int st) {
-    return 2 * Cfg::DG_BYTES + 2 * (LOCAL ? Cfg::MAX_SOURCES : C) * U * kRegRows * 4 + st * stage + (st + 1) * out_slot;
+    return 2 * Cfg::DG_BYTES + 2 * (LOCAL ? Cfg::MAX_SOURCES : (HALVES ? p.D / 16 : C)) * U * kRegRows * 4 + st * stage + (st + 1) * out_slot;
   };
   const int nst = bytes(kRegMaxStages) <= 110 * 1024 ? kRegMaxStages : 2;
   const int smem = bytes(nst);
@@ -488,7 +500,7 @@ int launch_bwd_reg(const BwdParams& p, const void* cache, const float* history, 
   if (own_dwx &&
       reg_tile_map(&dwx_map, p.dwx, wx_bf16 ? 2 : 4, D, N, B, CT::GW, p.T, uT * CT::GW * nd, nd, CT::GW * nd, CT::GW) != 0)
     return -4;
-  auto kern = frnn_bwd_reg_kernel<CELL, KT, LOCAL>;
+  auto kern = frnn_bwd_reg_kernel<CELL, KT, LOCAL, HALVES>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return static_cast<int>(e);
   BwdParams q = p;
@@ -521,6 +533,20 @@ int launch_bwd_reg(const BwdParams& p, const void* cache, const float* history, 
   return static_cast<int>(e);
 }
 
+template <int CELL, int KT>
+int launch_bwd_reg_cluster(const BwdParams& p, const void* cache, const float* history, const float* initial,
+                           const float* d_history, int wx_bf16, cudaStream_t s) {
+  if (p.D % kRegClusterUnits != 0) {
+    // The odd multiples of 16 begin at 80. The sLSTM at 208 and 240 units needs all 255 registers and is no faster here than
+    // on the tcgen05 kernel: T128 N1, forward and backward, 399 us against 378 at B4 D208 and 488 against 478 at B48 D240.
+    if constexpr (KT > 4 && !(CELL == kSLSTM && KT > 12))
+      return launch_bwd_reg<CELL, KT, false, true>(p, cache, history, initial, d_history, wx_bf16, s);
+    else
+      return kRegNoRoom;
+  }
+  return launch_bwd_reg<CELL, KT, false>(p, cache, history, initial, d_history, wx_bf16, s);
+}
+
 template <int CELL>
 int launch_bwd_reg_cell(const BwdParams& p, const void* cache, const float* history, const float* initial,
                         const float* d_history, int wx_bf16, cudaStream_t s) {
@@ -528,13 +554,13 @@ int launch_bwd_reg_cell(const BwdParams& p, const void* cache, const float* hist
     case 2: return launch_bwd_reg<CELL, 2, true>(p, cache, history, initial, d_history, wx_bf16, s);
     case 4:
       return reg_local(p.D) ? launch_bwd_reg<CELL, 4, true>(p, cache, history, initial, d_history, wx_bf16, s)
-                                  : launch_bwd_reg<CELL, 4, false>(p, cache, history, initial, d_history, wx_bf16, s);
-    case 6: return launch_bwd_reg<CELL, 6, false>(p, cache, history, initial, d_history, wx_bf16, s);
-    case 8: return launch_bwd_reg<CELL, 8, false>(p, cache, history, initial, d_history, wx_bf16, s);
-    case 10: return launch_bwd_reg<CELL, 10, false>(p, cache, history, initial, d_history, wx_bf16, s);
-    case 12: return launch_bwd_reg<CELL, 12, false>(p, cache, history, initial, d_history, wx_bf16, s);
-    case 14: return launch_bwd_reg<CELL, 14, false>(p, cache, history, initial, d_history, wx_bf16, s);
-    case 16: return launch_bwd_reg<CELL, 16, false>(p, cache, history, initial, d_history, wx_bf16, s);
+                            : launch_bwd_reg_cluster<CELL, 4>(p, cache, history, initial, d_history, wx_bf16, s);
+    case 6: return launch_bwd_reg_cluster<CELL, 6>(p, cache, history, initial, d_history, wx_bf16, s);
+    case 8: return launch_bwd_reg_cluster<CELL, 8>(p, cache, history, initial, d_history, wx_bf16, s);
+    case 10: return launch_bwd_reg_cluster<CELL, 10>(p, cache, history, initial, d_history, wx_bf16, s);
+    case 12: return launch_bwd_reg_cluster<CELL, 12>(p, cache, history, initial, d_history, wx_bf16, s);
+    case 14: return launch_bwd_reg_cluster<CELL, 14>(p, cache, history, initial, d_history, wx_bf16, s);
+    case 16: return launch_bwd_reg_cluster<CELL, 16>(p, cache, history, initial, d_history, wx_bf16, s);
     default: return -2;
   }
 }

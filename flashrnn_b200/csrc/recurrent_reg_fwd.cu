@@ -6,7 +6,7 @@
 // for two batch rows: it runs the cell on them in registers and publishes its two values of h_t.
 //   LOCAL: the CTA holds the whole head; h_t goes to the other half of a shared-memory double buffer, one mbarrier
 //          arrival per warp.
-//   else:  a cluster of D / 32 CTAs; a quad of lanes packs the 8 batch rows of a unit into 16 bytes and sends them to
+//   else:  a cluster of ceil(D / 32) CTAs (an odd multiple of 16 leaves two warps of the last one without units); a quad of lanes packs the 8 batch rows of a unit into 16 bytes and sends them to
 //          every CTA of the cluster with st.async on the receiver's mbarrier.
 // One more warp moves data: TMA tiles of Wx in, staged outputs (history, gate cache, bf16 h) out, both under the swizzle
 // that lets 8 units x 4 batch rows be read and written without bank conflicts. The compute warps' own stores of these
@@ -47,6 +47,7 @@ frnn_fwd_reg_kernel(const FwdParams p, const __grid_constant__ CUtensorMap wx_ma
   const int C = LOCAL ? 1 : p.C;
   const int rank = LOCAL ? 0 : static_cast<int>(blockIdx.x % C), gid = blockIdx.x / C;
   const int n = gid % N, b0 = gid / N * kRegRows;
+  const int unit_warps = LOCAL ? nwarps : min(nwarps, (D - rank * U) / kRegUnitsPerWarp);  // warps that own units
   uint8_t* const hbuf = smem;
   uint8_t* const wxs = smem + 2 * kHbuf;
   const int chunks = (U + kRegChunk - 1) / kRegChunk;
@@ -67,7 +68,7 @@ frnn_fwd_reg_kernel(const FwdParams p, const __grid_constant__ CUtensorMap wx_ma
 
   if (tid == 0) {
     for (int i = 0; i < 2; ++i) mbar_init(smem_u32(&s_hbar[i]), (LOCAL ? nwarps : 1) + 1);  // + the I/O warp: Wx has landed
-    for (int i = 0; i < slots; ++i) mbar_init(smem_u32(&s_out_full[i]), nwarps);
+    for (int i = 0; i < slots; ++i) mbar_init(smem_u32(&s_out_full[i]), unit_warps);
     for (int s = 0; s < nst; ++s) mbar_init(smem_u32(&s_wx_full[s]), 1);
     s_gave_up = 0;
     fence_mbar_init();
@@ -143,6 +144,8 @@ frnn_fwd_reg_kernel(const FwdParams p, const __grid_constant__ CUtensorMap wx_ma
       tma_store_wait<0>();
     }
     __syncwarp();
+  } else if (warp >= unit_warps) {
+    cluster_sync_all();
   } else {
     const int ul = warp * kRegUnitsPerWarp + q;  // this thread's unit inside the CTA's slice
     const int d = rank * U + ul;                 // ... and inside the head
@@ -364,7 +367,7 @@ int launch_fwd_reg(const FwdParams& p, const void* wx, int wx_bf16, cudaStream_t
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return static_cast<int>(e);
   FwdParams q = p;
-  q.C = p.D / U;
+  q.C = (p.D + U - 1) / U;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(static_cast<unsigned>(p.N * reg_batch_tiles(p.B) * q.C));
   cfg.blockDim = dim3(static_cast<unsigned>(U / kRegUnitsPerWarp * 32 + 32));

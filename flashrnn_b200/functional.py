@@ -302,11 +302,10 @@ def _run_on_current_device(wx, recurrent, bias, initial, cell: str, zero_normali
         zero_first = bool(torch.all(initial[2] == 0))
     if D > 1792 and D % 256 == 0 and options is None and wx.dtype in (torch.float32, torch.bfloat16):
         return _run_wide(wx, recurrent, bias, initial, cell, zero_first)
-    # The kernels tile the head width in multiples of 16 (from 64 to 256 units the register-resident kernels take
-    # multiples of 32; heads wider than 768: 64, and 128 where only the
+    # The kernels tile the head width in multiples of 16 (heads wider than 768: 64, and 128 where only the
     # column-owning backward fits); the smallest such width that a launch supports is used.
     pad = (-D) % 16
-    for multiple in (32 if 64 < D < 256 else 16, 64, 128):
+    for multiple in (16, 64, 128):
         if _lib.plan(cell, min(wx.shape[0], 8), wx.shape[1], 1, D + (-D) % multiple).supported:
             pad = (-D) % multiple
             break

@@ -13,7 +13,7 @@ CELLS = ("lstm", "slstm", "gru", "elman")
 SHAPES = [(CELLS[(i + j) % 4], (1, 9, 13, 8)[(i + 2 * j) % 4], (7, 1, 6, 3)[(i + j) % 4], 1 + (i + j) % 3, D, 60 + 4 * i + j, j == 0)
           for i, D in enumerate(WIDTHS) for j in range(4)]
 SHAPES += [("lstm", 152, 3, 3, 256, 110, False), ("elman", 1400, 2, 1, 64, 111, False), ("gru", 700, 2, 2, 96, 112, False),
-           ("lstm", 3, 5, 2, 80, 113, False), ("gru", 2, 4, 1, 200, 114, False)]   # widths that are padded to a multiple of 32
+           ("lstm", 3, 5, 2, 80, 113, False), ("gru", 2, 4, 1, 200, 114, False)]   # a half-filled last CTA; a width that is padded to 208
 
 
 @pytest.mark.parametrize("shape", SHAPES, ids=lambda s: f"{s[0]}-B{s[1]}-T{s[2]}-N{s[3]}-D{s[4]}")

@@ -10,10 +10,10 @@ from tests.test_gpu_timeout import _backward, _buffers, _forward
 pytestmark = pytest.mark.gpu
 
 CELLS = ("lstm", "slstm", "gru", "elman")
-WIDTHS = (16, 32, 48, 64, 96, 128, 160, 192, 224, 256)
+WIDTHS = tuple(range(16, 257, 16))   # odd multiples of 16 from 80 on: 16-unit slices there, a half-filled last CTA here
 # every width with every cell; batches: one row, a ragged second group, three groups
 SHAPES = [(CELLS[j], (1, 9, 20)[(i + j) % 3], (1, 14, 33)[(i + 2 * j) % 3], 1 + (i + j) % 2, D) for i, D in enumerate(WIDTHS) for j in range(4)]
-SHAPES += [("lstm", 150, 9, 6, 32), ("elman", 201, 5, 12, 48)]   # 16-row tiles on the tcgen05 side
+SHAPES += [("lstm", 150, 9, 6, 32), ("elman", 201, 5, 12, 48), ("lstm", 40, 6, 6, 112)]   # 16-row tiles on the tcgen05 side
 
 
 @pytest.mark.parametrize("shape", SHAPES, ids=lambda s: f"{s[0]}-B{s[1]}-T{s[2]}-N{s[3]}-D{s[4]}")
@@ -51,3 +51,19 @@ def test_both_kernel_families_agree_bit_for_bit(shape, cuda_device):
             assert ((got.double() - want.double()).abs() <= 2 * 15 * 2.0 ** -24 * 1.01 * rows + 1e-30).all(), shape
         else:
             assert torch.equal(got.view(torch.uint8), want.view(torch.uint8)), (shape, k)
+
+
+@pytest.mark.parametrize("D", [80, 208])
+def test_multiples_of_sixteen_are_not_padded(D, cuda_device):
+    """Results are dense, own their memory, and are those of a prepared sequence (which never pads) bit for bit."""
+    from flashrnn_b200 import PreparedSequence, flashrnn_torch
+    from flashrnn_b200.workloads import make_inputs
+
+    wx, R, b, init = (t.to(cuda_device).contiguous() for t in make_inputs("lstm", 9, 11, 2, D, 78))
+    history, carry = flashrnn_torch(wx.requires_grad_(True), R, b, init, cell="lstm", numerics="fp32_state_bf16_mma")
+    assert history.is_contiguous() and carry.is_contiguous()
+    assert history.untyped_storage().nbytes() == history.numel() * 4
+    seq = PreparedSequence(wx.detach(), R, b, init, "lstm")
+    out, final = seq.run()
+    seq.check()
+    assert torch.equal(out, history) and torch.equal(final, carry)
