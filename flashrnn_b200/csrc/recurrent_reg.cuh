@@ -36,6 +36,10 @@ constexpr int kRegChunk = 32;
 __host__ __device__ inline int reg_round_1k(int bytes) { return (bytes + 1023) & ~1023; }
 inline int reg_chunks(int U) { return (U + kRegChunk - 1) / kRegChunk; }
 constexpr int kRegMaxStages = 4;
+// Dynamic shared memory that every launcher asks for, whatever its call needs: the attribute belongs to the kernel, and a
+// thread that set it to the need of its own call (26 KB for bf16 inference at 256 units) could take it from one that is
+// about to launch (49 KB for fp32 training).
+constexpr int kRegSmemLimit = 220 * 1024;
 // Slots of staged outputs: a warp that stages step t has read the input tile of step t, which the I/O warp fetched after
 // the copies of step t - stages - 1 had read their slot.
 constexpr int kRegMaxSlots = kRegMaxStages + 1;

@@ -482,6 +482,7 @@ int launch_bwd_reg(const BwdParams& p, const void* cache, const float* history, 
   };
   const int nst = bytes(kRegMaxStages) <= 110 * 1024 ? kRegMaxStages : 2;
   const int smem = bytes(nst);
+  if (smem > kRegSmemLimit) return -2;
   const int D = p.D, N = p.N, B = p.B;
   const uint64_t nd = static_cast<uint64_t>(N) * D, uT = p.T, uB = p.B;
   // bulk stores start on 16-byte boundaries; the tcgen05 kernels write these outputs with plain stores
@@ -501,7 +502,7 @@ int launch_bwd_reg(const BwdParams& p, const void* cache, const float* history, 
       reg_tile_map(&dwx_map, p.dwx, wx_bf16 ? 2 : 4, D, N, B, CT::GW, p.T, uT * CT::GW * nd, nd, CT::GW * nd, CT::GW) != 0)
     return -4;
   auto kern = frnn_bwd_reg_kernel<CELL, KT, LOCAL, HALVES>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kRegSmemLimit);
   if (e != cudaSuccess) return static_cast<int>(e);
   BwdParams q = p;
   q.C = C;

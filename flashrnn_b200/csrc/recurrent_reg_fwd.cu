@@ -350,6 +350,7 @@ int launch_fwd_reg(const FwdParams& p, const void* wx, int wx_bf16, cudaStream_t
   const auto bytes = [&](int st) { return 2 * KT * 16 * 16 + st * stage + (st + 1) * out_slot; };
   const int nst = bytes(kRegMaxStages) <= 110 * 1024 ? kRegMaxStages : 2;
   const int smem = bytes(nst);
+  if (smem > kRegSmemLimit) return -2;
   // bulk stores start on 16-byte boundaries; the tcgen05 kernels write these outputs with plain stores
   if (((reinterpret_cast<uintptr_t>(p.history) | reinterpret_cast<uintptr_t>(p.cache) | reinterpret_cast<uintptr_t>(p.hbf)) & 15u) != 0)
     return kRegNoRoom;
@@ -364,7 +365,7 @@ int launch_fwd_reg(const FwdParams& p, const void* wx, int wx_bf16, cudaStream_t
     return -4;
   if (p.hbf != nullptr && reg_tile_map(&hbf_map, p.hbf + nd, 2, p.D, p.N, p.B, 1, p.T, (T + 1) * nd, nd, nd, 1) != 0) return -4;
   auto kern = frnn_fwd_reg_kernel<CELL, KT, LOCAL>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kRegSmemLimit);
   if (e != cudaSuccess) return static_cast<int>(e);
   FwdParams q = p;
   q.C = (p.D + U - 1) / U;
