@@ -142,6 +142,34 @@ int make_tensor_map_strided(CUtensorMap* map, const void* base, int elem_bytes, 
   return r == CUDA_SUCCESS ? 0 : -4;
 }
 
+// The occupancy query takes microseconds; its answer depends on the device, the kernel, its cluster width and its shared
+// memory only and is remembered (kernels x staging layouts x devices; past 1024 entries it is asked again on each call).
+int reg_room(const void* kern, const cudaLaunchConfig_t& cfg, int width, int clusters) {
+  struct Entry { const void* kern; size_t smem; int dev, width, capacity; };
+  static std::mutex mu;
+  static Entry table[1024];
+  static int used = 0;
+  int dev = 0, capacity = -1;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return static_cast<int>(e);
+  if (clusters > 0) {
+    std::lock_guard<std::mutex> lock(mu);
+    for (int i = 0; i < used && capacity < 0; ++i)
+      if (table[i].kern == kern && table[i].smem == cfg.dynamicSmemBytes && table[i].dev == dev && table[i].width == width)
+        capacity = table[i].capacity;
+  }
+  if (capacity >= 0 && clusters > capacity) return kRegNoRoom;
+  e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kRegSmemLimit);
+  if (e != cudaSuccess || clusters == 0) return static_cast<int>(e);
+  if (capacity < 0) {
+    e = cudaOccupancyMaxActiveClusters(&capacity, kern, &cfg);
+    if (e != cudaSuccess) return static_cast<int>(e);
+    std::lock_guard<std::mutex> lock(mu);
+    if (used < 1024) table[used++] = Entry{kern, cfg.dynamicSmemBytes, dev, width, capacity};
+  }
+  return clusters > capacity ? kRegNoRoom : 0;
+}
+
 }  // namespace frnn
 
 using namespace frnn;

@@ -487,23 +487,7 @@ int launch_bwd_reg(const BwdParams& p, const void* cache, const float* history, 
   const uint64_t nd = static_cast<uint64_t>(N) * D, uT = p.T, uB = p.B;
   // bulk stores start on 16-byte boundaries; the tcgen05 kernels write these outputs with plain stores
   if (((reinterpret_cast<uintptr_t>(p.dwx) | reinterpret_cast<uintptr_t>(p.dgr)) & 15u) != 0) return kRegNoRoom;
-  CUtensorMap cache_map, hist_map, init_map, dhist_map, dgr_map, dwx_map;
-  if (reg_tile_map(&hist_map, history, 4, D, N, B, CT::S, p.T, uT * nd, uB * uT * nd, nd, Cfg::HS) != 0 ||
-      reg_tile_map(&dhist_map, d_history, 4, D, N, B, CT::S, p.T, uT * nd, uB * uT * nd, nd, CT::S) != 0 ||
-      reg_tile_map(&init_map, initial, 4, D, N, B, CT::S, 1, nd, uB * nd, nd, Cfg::HS) != 0 ||
-      reg_tile_map(&dgr_map, p.dgr, 2, D, N, B, CT::GR, p.T, uT * CT::GR * nd, nd, CT::GR * nd, CT::GR) != 0)
-    return -4;
-  cache_map = hist_map;  // Elman has no cache: a valid map that is never used
-  if (Cfg::GCL > 0 &&
-      reg_tile_map(&cache_map, cache, CT::CES, D, N, B, CT::GC, p.T, uT * CT::GC * nd, nd, CT::GC * nd, CT::GC) != 0)
-    return -4;
-  dwx_map = dgr_map;
-  if (own_dwx &&
-      reg_tile_map(&dwx_map, p.dwx, wx_bf16 ? 2 : 4, D, N, B, CT::GW, p.T, uT * CT::GW * nd, nd, CT::GW * nd, CT::GW) != 0)
-    return -4;
   auto kern = frnn_bwd_reg_kernel<CELL, KT, LOCAL, HALVES>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kRegSmemLimit);
-  if (e != cudaSuccess) return static_cast<int>(e);
   BwdParams q = p;
   q.C = C;
   cudaLaunchConfig_t cfg = {};
@@ -518,20 +502,30 @@ int launch_bwd_reg(const BwdParams& p, const void* cache, const float* history, 
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = LOCAL ? 0 : 1;
-  if (!LOCAL) {
-    int clusters = 0;
-    e = cudaOccupancyMaxActiveClusters(&clusters, kern, &cfg);
-    if (e != cudaSuccess) return static_cast<int>(e);
-    if (p.N * reg_batch_tiles(p.B) > clusters) return kRegNoRoom;
-  }
+  // whether the call is taken at all comes first: one that is not pays for nothing else
+  const int rc = reg_room(reinterpret_cast<const void*>(kern), cfg, C, LOCAL ? 0 : p.N * reg_batch_tiles(p.B));
+  if (rc != 0) return rc;
+  CUtensorMap cache_map, hist_map, init_map, dhist_map, dgr_map, dwx_map;
+  if (reg_tile_map(&hist_map, history, 4, D, N, B, CT::S, p.T, uT * nd, uB * uT * nd, nd, Cfg::HS) != 0 ||
+      reg_tile_map(&dhist_map, d_history, 4, D, N, B, CT::S, p.T, uT * nd, uB * uT * nd, nd, CT::S) != 0 ||
+      reg_tile_map(&init_map, initial, 4, D, N, B, CT::S, 1, nd, uB * nd, nd, Cfg::HS) != 0 ||
+      reg_tile_map(&dgr_map, p.dgr, 2, D, N, B, CT::GR, p.T, uT * CT::GR * nd, nd, CT::GR * nd, CT::GR) != 0)
+    return -4;
+  cache_map = hist_map;  // Elman has no cache: a valid map that is never used
+  if (Cfg::GCL > 0 &&
+      reg_tile_map(&cache_map, cache, CT::CES, D, N, B, CT::GC, p.T, uT * CT::GC * nd, nd, CT::GC * nd, CT::GC) != 0)
+    return -4;
+  dwx_map = dgr_map;
+  if (own_dwx &&
+      reg_tile_map(&dwx_map, p.dwx, wx_bf16 ? 2 : 4, D, N, B, CT::GW, p.T, uT * CT::GW * nd, nd, CT::GW * nd, CT::GW) != 0)
+    return -4;
   if (p.db_rows != kRegRows) {
     const size_t tiles = static_cast<size_t>((p.B + p.db_rows - 1) / p.db_rows);
-    e = cudaMemsetAsync(p.db_part, 0, tiles * CT::GB * p.N * p.D * sizeof(float), stream);
+    const cudaError_t e = cudaMemsetAsync(p.db_part, 0, tiles * CT::GB * p.N * p.D * sizeof(float), stream);
     if (e != cudaSuccess) return static_cast<int>(e);
   }
-  e = cudaLaunchKernelEx(&cfg, kern, q, history, cache_map, hist_map, init_map, dhist_map, dgr_map, dwx_map, wx_bf16,
-                         own_dwx ? 1 : 0, nst);
-  return static_cast<int>(e);
+  return static_cast<int>(cudaLaunchKernelEx(&cfg, kern, q, history, cache_map, hist_map, init_map, dhist_map, dgr_map, dwx_map,
+                                             wx_bf16, own_dwx ? 1 : 0, nst));
 }
 
 template <int CELL, int KT>

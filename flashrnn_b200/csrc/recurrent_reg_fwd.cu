@@ -354,19 +354,7 @@ int launch_fwd_reg(const FwdParams& p, const void* wx, int wx_bf16, cudaStream_t
   // bulk stores start on 16-byte boundaries; the tcgen05 kernels write these outputs with plain stores
   if (((reinterpret_cast<uintptr_t>(p.history) | reinterpret_cast<uintptr_t>(p.cache) | reinterpret_cast<uintptr_t>(p.hbf)) & 15u) != 0)
     return kRegNoRoom;
-  CUtensorMap map, hist_map, cache_map, hbf_map;
-  const uint64_t nd = static_cast<uint64_t>(p.N) * p.D, T = p.T, Tt = p.T_total;
-  if (reg_tile_map(&map, wx, es, p.D, p.N, p.B, CT::GW, p.T_total, Tt * CT::GW * nd, nd, CT::GW * nd, CT::GW) != 0) return -4;
-  hist_map = cache_map = hbf_map = map;  // valid maps where a stream is not written
-  if (hist_states > 0 &&
-      reg_tile_map(&hist_map, p.history, hes, p.D, p.N, p.B, hist_states, p.T_total, Tt * nd, p.B * Tt * nd, nd, hist_states) != 0)
-    return -4;
-  if (has_cache && reg_tile_map(&cache_map, p.cache, CT::CES, p.D, p.N, p.B, CT::GC, p.T, T * CT::GC * nd, nd, CT::GC * nd, CT::GC) != 0)
-    return -4;
-  if (p.hbf != nullptr && reg_tile_map(&hbf_map, p.hbf + nd, 2, p.D, p.N, p.B, 1, p.T, (T + 1) * nd, nd, nd, 1) != 0) return -4;
   auto kern = frnn_fwd_reg_kernel<CELL, KT, LOCAL>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kRegSmemLimit);
-  if (e != cudaSuccess) return static_cast<int>(e);
   FwdParams q = p;
   q.C = (p.D + U - 1) / U;
   cudaLaunchConfig_t cfg = {};
@@ -381,14 +369,20 @@ int launch_fwd_reg(const FwdParams& p, const void* wx, int wx_bf16, cudaStream_t
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = LOCAL ? 0 : 1;
-  if (!LOCAL) {
-    int clusters = 0;
-    e = cudaOccupancyMaxActiveClusters(&clusters, kern, &cfg);
-    if (e != cudaSuccess) return static_cast<int>(e);
-    if (p.N * reg_batch_tiles(p.B) > clusters) return kRegNoRoom;
-  }
-  e = cudaLaunchKernelEx(&cfg, kern, q, map, hist_map, cache_map, hbf_map, wx_bf16, nst, hist_states);
-  return static_cast<int>(e);
+  // whether the call is taken at all comes first: one that is not pays for nothing else
+  const int rc = reg_room(reinterpret_cast<const void*>(kern), cfg, q.C, LOCAL ? 0 : p.N * reg_batch_tiles(p.B));
+  if (rc != 0) return rc;
+  CUtensorMap map, hist_map, cache_map, hbf_map;
+  const uint64_t nd = static_cast<uint64_t>(p.N) * p.D, T = p.T, Tt = p.T_total;
+  if (reg_tile_map(&map, wx, es, p.D, p.N, p.B, CT::GW, p.T_total, Tt * CT::GW * nd, nd, CT::GW * nd, CT::GW) != 0) return -4;
+  hist_map = cache_map = hbf_map = map;  // valid maps where a stream is not written
+  if (hist_states > 0 &&
+      reg_tile_map(&hist_map, p.history, hes, p.D, p.N, p.B, hist_states, p.T_total, Tt * nd, p.B * Tt * nd, nd, hist_states) != 0)
+    return -4;
+  if (has_cache && reg_tile_map(&cache_map, p.cache, CT::CES, p.D, p.N, p.B, CT::GC, p.T, T * CT::GC * nd, nd, CT::GC * nd, CT::GC) != 0)
+    return -4;
+  if (p.hbf != nullptr && reg_tile_map(&hbf_map, p.hbf + nd, 2, p.D, p.N, p.B, 1, p.T, (T + 1) * nd, nd, nd, 1) != 0) return -4;
+  return static_cast<int>(cudaLaunchKernelEx(&cfg, kern, q, map, hist_map, cache_map, hbf_map, wx_bf16, nst, hist_states));
 }
 
 template <int CELL>
