@@ -40,6 +40,11 @@ constexpr int kRegMaxStages = 4;
 // thread that set it to the need of its own call (26 KB for bf16 inference at 256 units) could take it from one that is
 // about to launch (49 KB for fp32 training).
 constexpr int kRegSmemLimit = 220 * 1024;
+// Steps in flight for a launch that needs so much shared memory with four and with three stages: four, or three where only that
+// lets two CTAs share an SM (heads of 48 units with fp32 Wx). With two, a step's tile was fetched only when the step before had
+// been staged, and the sLSTM backward, whose registers allow one CTA per SM anyway, gained nothing: forward and backward, B64
+// T128 N16 D48 fp32, sLSTM 716 us against 611 now (tcgen05 632), LSTM 589 against 559 (565).
+inline int reg_stages(int bytes4, int bytes3) { return bytes4 > 110 * 1024 && bytes3 <= 110 * 1024 ? 3 : kRegMaxStages; }
 // Slots of staged outputs: a warp that stages step t has read the input tile of step t, which the I/O warp fetched after
 // the copies of step t - stages - 1 had read their slot.
 constexpr int kRegMaxSlots = kRegMaxStages + 1;

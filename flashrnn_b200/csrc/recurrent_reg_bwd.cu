@@ -129,8 +129,8 @@ frnn_bwd_reg_kernel(const BwdParams p, const float* history, const __grid_consta
         }
       };
       for (int it = 0; it < nst && it < T; ++it) fill(it, it);
-      int stage = 0, slot = 0, next = 1 % nst;
-      uint32_t phase = 0, next_phase = 1 / nst;
+      int stage = 0, slot = 0, next = 1;
+      uint32_t phase = 0, next_phase = 0;
       // The barrier of the partial sums of iteration `it` also stands for its tiles: one wait per step on the compute
       // warps' chain, not two.
       auto announce = [&](int it) -> bool {
@@ -145,7 +145,7 @@ frnn_bwd_reg_kernel(const BwdParams p, const float* history, const __grid_consta
         return true;
       };
       bool ok = true;
-      for (int it = 1; it <= 2 && (it < nst || it >= T) && it <= T && ok; ++it) ok = announce(it);
+      for (int it = 1; it <= 2 && it <= T && ok; ++it) ok = announce(it);
       for (int it = 0; it < T && ok; ++it) {
         // released by the CTA's own warps, whose waits have the plain limit: theirs run out first
         if (!mbar_wait_bounded<false, true>(smem_u32(&s_out_full[slot]), phase, 2 * limit, abort_flag)) {
@@ -156,7 +156,7 @@ frnn_bwd_reg_kernel(const BwdParams p, const float* history, const __grid_consta
         // complete (another arrival would overrun its count), and a copy could be on its way into the stage: stop here.
         if (*reinterpret_cast<volatile int*>(&s_gave_up) != 0) break;
         // iteration it + 2 uses the barrier of iteration `it`, which every warp has left
-        if (nst > 2 && it >= 1 && it + 2 <= T) ok = announce(it + 2);
+        if (it >= 1 && it + 2 <= T) ok = announce(it + 2);
         for (int i = 0; i < chunks; ++i) {
           const uint32_t src = smem_u32(outs + slot * out_slot + i * out_chunk);
           const int x = rank * U + i * kRegChunk;
@@ -166,7 +166,6 @@ frnn_bwd_reg_kernel(const BwdParams p, const float* history, const __grid_consta
         tma_store_commit();
         tma_store_wait_read<1>();  // the copies of the previous step have read their slot: see kRegMaxSlots
         if (it + nst < T) fill(it + nst, stage);
-        if (nst <= 2 && it + 2 <= T && (it >= 1 || T > 2)) ok = announce(it + 2);
         if (++stage == nst) stage = 0;
         if (++slot == slots) { slot = 0; phase ^= 1u; }
       }
@@ -476,11 +475,11 @@ int launch_bwd_reg(const BwdParams& p, const void* cache, const float* history, 
   // cells whose W-gates are their R-gates may have one bf16 buffer for dWx and dg
   const bool own_dwx = !wx_bf16 || CELL == kGRU || p.dwx != static_cast<void*>(p.dgr);
   const int out_slot = reg_chunks(U) * reg_round_1k(kRegRows * kRegChunk * (CT::GR * 2 + (own_dwx ? CT::GW * (wx_bf16 ? 2 : 4) : 0)));
-  // prefetch depth: 4 steps, 2 where only that lets two CTAs share an SM
+  // prefetch depth: 4 steps, 3 where only that lets two CTAs share an SM
   const auto bytes = [&](int st) {
     return 2 * Cfg::DG_BYTES + 2 * (LOCAL ? Cfg::MAX_SOURCES : (HALVES ? p.D / 16 : C)) * U * kRegRows * 4 + st * stage + (st + 1) * out_slot;
   };
-  const int nst = bytes(kRegMaxStages) <= 110 * 1024 ? kRegMaxStages : 2;
+  const int nst = reg_stages(bytes(kRegMaxStages), bytes(kRegMaxStages - 1));
   const int smem = bytes(nst);
   if (smem > kRegSmemLimit) return -2;
   const int D = p.D, N = p.N, B = p.B;

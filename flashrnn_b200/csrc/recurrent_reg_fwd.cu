@@ -102,8 +102,8 @@ frnn_fwd_reg_kernel(const FwdParams p, const __grid_constant__ CUtensorMap wx_ma
           tma_load_5d(dst + i * chunk_bytes, &wx_map, bar, rank * U + i * kRegChunk, n, b0, 0, p.t0 + t);
       };
       for (int t = 0; t < nst && t < T; ++t) fill(t, t);
-      int stage = 0, slot = 0, next = 1 % nst;
-      uint32_t phase = 0, next_phase = 1 / nst;
+      int stage = 0, slot = 0, next = 1;
+      uint32_t phase = 0, next_phase = 0;
       // The operand barrier of step t also stands for its Wx tile: one wait per step on the compute warps' chain, not two.
       auto announce = [&](int t) -> bool {
         if (!mbar_wait_bounded<false, true>(smem_u32(&s_wx_full[next]), next_phase & 1, limit, abort_flag)) {
@@ -115,7 +115,7 @@ frnn_fwd_reg_kernel(const FwdParams p, const __grid_constant__ CUtensorMap wx_ma
         return true;
       };
       bool ok = true;
-      for (int t = 1; t <= 2 && t < nst && t < T && ok; ++t) ok = announce(t);
+      for (int t = 1; t <= 2 && t < T && ok; ++t) ok = announce(t);
       for (int t = 0; t < T && ok; ++t) {
         // released by the CTA's own warps, whose waits have the plain limit: theirs run out first
         if (!mbar_wait_bounded<false, true>(smem_u32(&s_out_full[slot]), phase, 2 * limit, abort_flag)) {
@@ -126,7 +126,7 @@ frnn_fwd_reg_kernel(const FwdParams p, const __grid_constant__ CUtensorMap wx_ma
         // complete (another arrival would overrun its count), and a copy could be on its way into the stage: stop here.
         if (*reinterpret_cast<volatile int*>(&s_gave_up) != 0) break;
         // step t + 2 uses the barrier of step t, which every warp has left
-        if (nst > 2 && t >= 1 && t + 2 < T) ok = announce(t + 2);
+        if (t >= 1 && t + 2 < T) ok = announce(t + 2);
         for (int i = 0; i < chunks; ++i) {
           const uint32_t src = smem_u32(outs + slot * out_slot + i * out_chunk);
           const int x = rank * U + i * kRegChunk;
@@ -137,7 +137,6 @@ frnn_fwd_reg_kernel(const FwdParams p, const __grid_constant__ CUtensorMap wx_ma
         tma_store_commit();
         tma_store_wait_read<1>();  // the copies of step t - 1 have read their slot: see kRegMaxSlots
         if (t + nst < T) fill(t + nst, stage);
-        if (nst <= 2 && t + 2 < T) ok = announce(t + 2);
         if (++stage == nst) stage = 0;
         if (++slot == slots) { slot = 0; phase ^= 1u; }
       }
@@ -346,9 +345,9 @@ int launch_fwd_reg(const FwdParams& p, const void* wx, int wx_bf16, cudaStream_t
   const int hes = p.out_bf16 ? 2 : 4;
   const bool has_cache = p.cache != nullptr && CELL != kElman;
   const int out_slot = reg_chunks(U) * reg_round_1k(plane * (hist_states * hes + (has_cache ? CT::GC * CT::CES : 0) + (p.hbf != nullptr ? 2 : 0)));
-  // prefetch depth: 4 steps, 2 where only that lets two CTAs share an SM
+  // prefetch depth: 4 steps, 3 where only that lets two CTAs share an SM
   const auto bytes = [&](int st) { return 2 * KT * 16 * 16 + st * stage + (st + 1) * out_slot; };
-  const int nst = bytes(kRegMaxStages) <= 110 * 1024 ? kRegMaxStages : 2;
+  const int nst = reg_stages(bytes(kRegMaxStages), bytes(kRegMaxStages - 1));
   const int smem = bytes(nst);
   if (smem > kRegSmemLimit) return -2;
   // bulk stores start on 16-byte boundaries; the tcgen05 kernels write these outputs with plain stores
