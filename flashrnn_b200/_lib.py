@@ -77,6 +77,7 @@ class MgPlan(ctypes.Structure):
 SIGNATURES = {
     "frnn_b200_version": (c_int, []),
     "frnn_b200_plan": (c_int, [c_int, c_int, c_int, c_int, c_int, POINTER(Plan)]),
+    "frnn_b200_register_kernels": (c_int, [c_int, c_int, c_int, c_int, c_int]),
     "frnn_b200_forward": (c_int, [c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                                   c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p,
                                   c_void_p]),
@@ -169,6 +170,14 @@ def plan(cell: str, B: int, T: int, N: int, D: int) -> Plan:
         _plans.clear()
     _plans[key] = out
     return out
+
+
+def register_kernels(cell: str, wx_bf16: bool, B: int, N: int, D: int) -> tuple:
+    """(forward, backward): whether a training call of this shape keeps R in registers on the current CUDA device."""
+    rc = load().frnn_b200_register_kernels(CELLS[cell], int(wx_bf16), B, N, D)
+    if rc < 0:
+        raise ValueError(f"frnn_b200_register_kernels failed: {ERROR_TEXT.get(rc, rc)}")
+    return bool(rc & 1), bool(rc & 2)
 
 
 def check(rc: int, what: str) -> None:

@@ -9,9 +9,10 @@
 namespace frnn {
 
 int forward_dispatch(int cell, const FwdParams& p, const void* wx, int wx_bf16, int bv, int unit, cudaStream_t s);
-int forward_reg_dispatch(int cell, const FwdParams& p, const void* wx, int wx_bf16, cudaStream_t s);
+// `ask`: only say whether the call would be taken (kRegTaken or kRegNoRoom)
+int forward_reg_dispatch(int cell, const FwdParams& p, const void* wx, int wx_bf16, cudaStream_t s, bool ask = false);
 int backward_reg_dispatch(int cell, const BwdParams& p, const void* cache, const float* history, const float* initial,
-                          const float* d_history, int wx_bf16, cudaStream_t s);
+                          const float* d_history, int wx_bf16, cudaStream_t s, bool ask = false);
 int forward_ksplit_dispatch(int cell, const FwdParams& p, const void* wx, int wx_bf16, int bv, int ksplit, cudaStream_t s,
                             int* capacity_only);
 int forward_ksplit_capacity(int cell, int bv, int ksplit, int D);
@@ -292,6 +293,26 @@ extern "C" int frnn_b200_plan(int cell, int B, int T, int N, int D, frnn_b200_pl
     out->supported = 0;
   }
   return 0;
+}
+
+extern "C" int frnn_b200_register_kernels(int cell, int wx_bf16, int B, int N, int D) {
+  frnn_b200_plan_t plan;
+  const int rc = frnn_b200_plan(cell, B, 1, N, D, &plan);
+  if (rc != 0) return rc;
+  if (!plan.supported) return -2;
+  if (!reg_width(D)) return 0;
+  FwdParams f{};
+  f.B = B; f.T = 1; f.T_total = 1; f.N = N; f.D = D;
+  f.cache = reinterpret_cast<void*>(16);  // a training call: cache and bf16 h are staged; never dereferenced
+  f.hbf = reinterpret_cast<__nv_bfloat16*>(16);
+  BwdParams b{};
+  b.B = B; b.T = 1; b.N = N; b.D = D;
+  b.db_rows = plan.batch_tile;
+  const int fwd = forward_reg_dispatch(cell, f, nullptr, wx_bf16, nullptr, true);
+  const int bwd = backward_reg_dispatch(cell, b, nullptr, nullptr, nullptr, nullptr, wx_bf16, nullptr, true);
+  for (const int v : {fwd, bwd})
+    if (v != kRegTaken && v != kRegNoRoom) return v > 0 ? -1000 - v : v;
+  return (fwd == kRegTaken ? 1 : 0) | (bwd == kRegTaken ? 2 : 0);
 }
 
 namespace {

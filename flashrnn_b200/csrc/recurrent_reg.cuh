@@ -71,6 +71,8 @@ constexpr int reg_min_blocks(int cell, int kt, bool local, bool backward) {
 // Threads of a CTA: a warp per 8 units (4 in a cluster; up to 32 units with two k tiles, 48 with four) and the I/O warp.
 constexpr int reg_max_threads(int kt, bool local) { return local && kt > 2 ? 7 * 32 : 5 * 32; }
 
+constexpr int kRegTaken = -101;       // answer to a question: the call would run here
+
 // 0 if the current device holds `clusters` clusters of `width` CTAs of the launch at once (0 clusters: no such condition),
 // kRegNoRoom if it does not, else a cudaError_t. Raises the kernel's shared-memory limit; the capacity is remembered.
 int reg_room(const void* kern, const cudaLaunchConfig_t& cfg, int width, int clusters);

@@ -467,7 +467,7 @@ frnn_bwd_reg_kernel(const BwdParams p, const float* history, const __grid_consta
 
 template <int CELL, int KT, bool LOCAL, bool HALVES = false>
 int launch_bwd_reg(const BwdParams& p, const void* cache, const float* history, const float* initial,
-                   const float* d_history, int wx_bf16, cudaStream_t stream) {
+                   const float* d_history, int wx_bf16, cudaStream_t stream, bool ask) {
   using Cfg = BwdRegCfg<CELL, KT, LOCAL, HALVES>;
   using CT = CellTraits<CELL>;
   const int U = LOCAL ? p.D : kRegClusterUnits, C = (p.D + U - 1) / U;
@@ -503,7 +503,7 @@ int launch_bwd_reg(const BwdParams& p, const void* cache, const float* history, 
   cfg.numAttrs = LOCAL ? 0 : 1;
   // whether the call is taken at all comes first: one that is not pays for nothing else
   const int rc = reg_room(reinterpret_cast<const void*>(kern), cfg, C, LOCAL ? 0 : p.N * reg_batch_tiles(p.B));
-  if (rc != 0) return rc;
+  if (rc != 0 || ask) return rc != 0 ? rc : kRegTaken;
   CUtensorMap cache_map, hist_map, init_map, dhist_map, dgr_map, dwx_map;
   if (reg_tile_map(&hist_map, history, 4, D, N, B, CT::S, p.T, uT * nd, uB * uT * nd, nd, Cfg::HS) != 0 ||
       reg_tile_map(&dhist_map, d_history, 4, D, N, B, CT::S, p.T, uT * nd, uB * uT * nd, nd, CT::S) != 0 ||
@@ -529,32 +529,32 @@ int launch_bwd_reg(const BwdParams& p, const void* cache, const float* history, 
 
 template <int CELL, int KT>
 int launch_bwd_reg_cluster(const BwdParams& p, const void* cache, const float* history, const float* initial,
-                           const float* d_history, int wx_bf16, cudaStream_t s) {
+                           const float* d_history, int wx_bf16, cudaStream_t s, bool ask) {
   if (p.D % kRegClusterUnits != 0) {
     // The odd multiples of 16 begin at 80. The sLSTM at 208 and 240 units needs all 255 registers and is no faster here than
     // on the tcgen05 kernel: T128 N1, forward and backward, 399 us against 378 at B4 D208 and 488 against 478 at B48 D240.
     if constexpr (KT > 4 && !(CELL == kSLSTM && KT > 12))
-      return launch_bwd_reg<CELL, KT, false, true>(p, cache, history, initial, d_history, wx_bf16, s);
+      return launch_bwd_reg<CELL, KT, false, true>(p, cache, history, initial, d_history, wx_bf16, s, ask);
     else
       return kRegNoRoom;
   }
-  return launch_bwd_reg<CELL, KT, false>(p, cache, history, initial, d_history, wx_bf16, s);
+  return launch_bwd_reg<CELL, KT, false>(p, cache, history, initial, d_history, wx_bf16, s, ask);
 }
 
 template <int CELL>
 int launch_bwd_reg_cell(const BwdParams& p, const void* cache, const float* history, const float* initial,
-                        const float* d_history, int wx_bf16, cudaStream_t s) {
+                        const float* d_history, int wx_bf16, cudaStream_t s, bool ask) {
   switch (reg_k_tiles(p.D)) {
-    case 2: return launch_bwd_reg<CELL, 2, true>(p, cache, history, initial, d_history, wx_bf16, s);
+    case 2: return launch_bwd_reg<CELL, 2, true>(p, cache, history, initial, d_history, wx_bf16, s, ask);
     case 4:
-      return reg_local(p.D) ? launch_bwd_reg<CELL, 4, true>(p, cache, history, initial, d_history, wx_bf16, s)
-                            : launch_bwd_reg_cluster<CELL, 4>(p, cache, history, initial, d_history, wx_bf16, s);
-    case 6: return launch_bwd_reg_cluster<CELL, 6>(p, cache, history, initial, d_history, wx_bf16, s);
-    case 8: return launch_bwd_reg_cluster<CELL, 8>(p, cache, history, initial, d_history, wx_bf16, s);
-    case 10: return launch_bwd_reg_cluster<CELL, 10>(p, cache, history, initial, d_history, wx_bf16, s);
-    case 12: return launch_bwd_reg_cluster<CELL, 12>(p, cache, history, initial, d_history, wx_bf16, s);
-    case 14: return launch_bwd_reg_cluster<CELL, 14>(p, cache, history, initial, d_history, wx_bf16, s);
-    case 16: return launch_bwd_reg_cluster<CELL, 16>(p, cache, history, initial, d_history, wx_bf16, s);
+      return reg_local(p.D) ? launch_bwd_reg<CELL, 4, true>(p, cache, history, initial, d_history, wx_bf16, s, ask)
+                            : launch_bwd_reg_cluster<CELL, 4>(p, cache, history, initial, d_history, wx_bf16, s, ask);
+    case 6: return launch_bwd_reg_cluster<CELL, 6>(p, cache, history, initial, d_history, wx_bf16, s, ask);
+    case 8: return launch_bwd_reg_cluster<CELL, 8>(p, cache, history, initial, d_history, wx_bf16, s, ask);
+    case 10: return launch_bwd_reg_cluster<CELL, 10>(p, cache, history, initial, d_history, wx_bf16, s, ask);
+    case 12: return launch_bwd_reg_cluster<CELL, 12>(p, cache, history, initial, d_history, wx_bf16, s, ask);
+    case 14: return launch_bwd_reg_cluster<CELL, 14>(p, cache, history, initial, d_history, wx_bf16, s, ask);
+    case 16: return launch_bwd_reg_cluster<CELL, 16>(p, cache, history, initial, d_history, wx_bf16, s, ask);
     default: return -2;
   }
 }
@@ -562,12 +562,12 @@ int launch_bwd_reg_cell(const BwdParams& p, const void* cache, const float* hist
 }  // namespace
 
 int backward_reg_dispatch(int cell, const BwdParams& p, const void* cache, const float* history, const float* initial,
-                          const float* d_history, int wx_bf16, cudaStream_t s) {
+                          const float* d_history, int wx_bf16, cudaStream_t s, bool ask) {
   switch (cell) {
-    case kLSTM: return launch_bwd_reg_cell<kLSTM>(p, cache, history, initial, d_history, wx_bf16, s);
-    case kSLSTM: return launch_bwd_reg_cell<kSLSTM>(p, cache, history, initial, d_history, wx_bf16, s);
-    case kGRU: return launch_bwd_reg_cell<kGRU>(p, cache, history, initial, d_history, wx_bf16, s);
-    case kElman: return launch_bwd_reg_cell<kElman>(p, cache, history, initial, d_history, wx_bf16, s);
+    case kLSTM: return launch_bwd_reg_cell<kLSTM>(p, cache, history, initial, d_history, wx_bf16, s, ask);
+    case kSLSTM: return launch_bwd_reg_cell<kSLSTM>(p, cache, history, initial, d_history, wx_bf16, s, ask);
+    case kGRU: return launch_bwd_reg_cell<kGRU>(p, cache, history, initial, d_history, wx_bf16, s, ask);
+    case kElman: return launch_bwd_reg_cell<kElman>(p, cache, history, initial, d_history, wx_bf16, s, ask);
     default: return -1;
   }
 }

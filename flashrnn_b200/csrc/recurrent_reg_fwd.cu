@@ -336,7 +336,7 @@ frnn_fwd_reg_kernel(const FwdParams p, const __grid_constant__ CUtensorMap wx_ma
 }
 
 template <int CELL, int KT, bool LOCAL>
-int launch_fwd_reg(const FwdParams& p, const void* wx, int wx_bf16, cudaStream_t stream) {
+int launch_fwd_reg(const FwdParams& p, const void* wx, int wx_bf16, cudaStream_t stream, bool ask) {
   using CT = CellTraits<CELL>;
   const int U = LOCAL ? p.D : kRegClusterUnits, es = wx_bf16 ? 2 : 4;
   const int plane = kRegRows * kRegChunk;
@@ -370,7 +370,7 @@ int launch_fwd_reg(const FwdParams& p, const void* wx, int wx_bf16, cudaStream_t
   cfg.numAttrs = LOCAL ? 0 : 1;
   // whether the call is taken at all comes first: one that is not pays for nothing else
   const int rc = reg_room(reinterpret_cast<const void*>(kern), cfg, q.C, LOCAL ? 0 : p.N * reg_batch_tiles(p.B));
-  if (rc != 0) return rc;
+  if (rc != 0 || ask) return rc != 0 ? rc : kRegTaken;
   CUtensorMap map, hist_map, cache_map, hbf_map;
   const uint64_t nd = static_cast<uint64_t>(p.N) * p.D, T = p.T, Tt = p.T_total;
   if (reg_tile_map(&map, wx, es, p.D, p.N, p.B, CT::GW, p.T_total, Tt * CT::GW * nd, nd, CT::GW * nd, CT::GW) != 0) return -4;
@@ -385,30 +385,30 @@ int launch_fwd_reg(const FwdParams& p, const void* wx, int wx_bf16, cudaStream_t
 }
 
 template <int CELL>
-int launch_fwd_reg_cell(const FwdParams& p, const void* wx, int wx_bf16, cudaStream_t s) {
+int launch_fwd_reg_cell(const FwdParams& p, const void* wx, int wx_bf16, cudaStream_t s, bool ask) {
   switch (reg_k_tiles(p.D)) {
-    case 2: return launch_fwd_reg<CELL, 2, true>(p, wx, wx_bf16, s);
+    case 2: return launch_fwd_reg<CELL, 2, true>(p, wx, wx_bf16, s, ask);
     case 4:
-      return reg_local(p.D) ? launch_fwd_reg<CELL, 4, true>(p, wx, wx_bf16, s)
-                                  : launch_fwd_reg<CELL, 4, false>(p, wx, wx_bf16, s);
-    case 6: return launch_fwd_reg<CELL, 6, false>(p, wx, wx_bf16, s);
-    case 8: return launch_fwd_reg<CELL, 8, false>(p, wx, wx_bf16, s);
-    case 10: return launch_fwd_reg<CELL, 10, false>(p, wx, wx_bf16, s);
-    case 12: return launch_fwd_reg<CELL, 12, false>(p, wx, wx_bf16, s);
-    case 14: return launch_fwd_reg<CELL, 14, false>(p, wx, wx_bf16, s);
-    case 16: return launch_fwd_reg<CELL, 16, false>(p, wx, wx_bf16, s);
+      return reg_local(p.D) ? launch_fwd_reg<CELL, 4, true>(p, wx, wx_bf16, s, ask)
+                                  : launch_fwd_reg<CELL, 4, false>(p, wx, wx_bf16, s, ask);
+    case 6: return launch_fwd_reg<CELL, 6, false>(p, wx, wx_bf16, s, ask);
+    case 8: return launch_fwd_reg<CELL, 8, false>(p, wx, wx_bf16, s, ask);
+    case 10: return launch_fwd_reg<CELL, 10, false>(p, wx, wx_bf16, s, ask);
+    case 12: return launch_fwd_reg<CELL, 12, false>(p, wx, wx_bf16, s, ask);
+    case 14: return launch_fwd_reg<CELL, 14, false>(p, wx, wx_bf16, s, ask);
+    case 16: return launch_fwd_reg<CELL, 16, false>(p, wx, wx_bf16, s, ask);
     default: return -2;
   }
 }
 
 }  // namespace
 
-int forward_reg_dispatch(int cell, const FwdParams& p, const void* wx, int wx_bf16, cudaStream_t s) {
+int forward_reg_dispatch(int cell, const FwdParams& p, const void* wx, int wx_bf16, cudaStream_t s, bool ask) {
   switch (cell) {
-    case kLSTM: return launch_fwd_reg_cell<kLSTM>(p, wx, wx_bf16, s);
-    case kSLSTM: return launch_fwd_reg_cell<kSLSTM>(p, wx, wx_bf16, s);
-    case kGRU: return launch_fwd_reg_cell<kGRU>(p, wx, wx_bf16, s);
-    case kElman: return launch_fwd_reg_cell<kElman>(p, wx, wx_bf16, s);
+    case kLSTM: return launch_fwd_reg_cell<kLSTM>(p, wx, wx_bf16, s, ask);
+    case kSLSTM: return launch_fwd_reg_cell<kSLSTM>(p, wx, wx_bf16, s, ask);
+    case kGRU: return launch_fwd_reg_cell<kGRU>(p, wx, wx_bf16, s, ask);
+    case kElman: return launch_fwd_reg_cell<kElman>(p, wx, wx_bf16, s, ask);
     default: return -1;
   }
 }

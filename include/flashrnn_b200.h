@@ -78,6 +78,12 @@ int frnn_b200_version(void);
  * (flashrnn/flashrnn/flashrnn.py:383-677, cuda_init_parametric.py). D must be a multiple of 16. */
 int frnn_b200_plan(int cell, int B, int T, int N, int D, frnn_b200_plan_t* out);
 
+/* Which kernels a training call of this shape takes on the current device: bit 0 is set if the forward pass, bit 1 if the
+ * backward pass keeps R in the registers of its warps (D <= 256, as many groups of 8 batch rows as run at once); where a
+ * bit is clear the kernels that frnn_b200_plan describes run, as they do for outputs that are not 16-byte aligned. Both
+ * give the same results (db of 16-row batch tiles: up to rounding). Negative: a code as above, or -1000 - cudaError_t. */
+int frnn_b200_register_kernels(int cell, int wx_bf16, int B, int N, int D);
+
 /* Forward recurrence over T steps (flashrnn/flashrnn/fused/flashrnn.cc:69-145 forward();
  * arithmetic of flashrnn/flashrnn2/reference.py:72-114 with fp32 state and bf16 R / h operands).
  *   wx        : Wx, fp32 (wx_bf16 = 0) or bf16 (wx_bf16 = 1)

@@ -49,6 +49,17 @@ def test_plan_describes_the_headline_workload():
     assert not _lib.plan("lstm", 8, 8, 1, 40).supported       # the ABI wants D % 16 == 0 (Python pads)
 
 
+def test_kernel_query_without_a_device():
+    """Widths that only one kernel family covers are answered from the shape; the rest needs the device's capacity."""
+    for cell in _lib.CELLS:
+        assert _lib.register_kernels(cell, True, 8, 2, 384) == (False, False)
+    lib = _lib.load()
+    assert lib.frnn_b200_register_kernels(9, 0, 8, 1, 64) == -1 and lib.frnn_b200_register_kernels(0, 0, 8, 1, 40) == -2
+    if not torch.cuda.is_available():
+        with pytest.raises(ValueError, match="register_kernels failed: -1"):
+            _lib.register_kernels("lstm", True, 8, 3, 256)
+
+
 def test_argument_checks_mirror_the_reference():
     wx, R, b, init = make_inputs("lstm", 2, 3, 2, 16, 0)
     with pytest.raises(ValueError, match="unsupported cell"):

@@ -126,9 +126,9 @@ TILE16 = [
     ("lstm", 256, 32, 4, 128, 61),    # one GPU's share of N32 D128 B256 with the heads split over 8 GPUs
     ("slstm", 200, 12, 4, 128, 62),   # ragged last tile (200 = 12 * 16 + 8)
     ("gru", 160, 10, 2, 256, 63),
-    ("elman", 112, 9, 12, 64, 64),
+    ("elman", 232, 5, 12, 64, 64),
     ("lstm", 48, 4, 4, 512, 65),      # 16-CTA clusters asking for all 512 tensor-memory columns, 192 CTAs: two waves
-    ("lstm", 70, 6, 8, 48, 66),       # 16-unit slices
+    ("lstm", 200, 6, 6, 112, 66),     # 16-unit slices
 ]
 
 
@@ -140,6 +140,8 @@ def test_sixteen_row_tiles_on_the_cluster_path(shape, cuda_device):
     cell, B, T, N, D, seed = shape
     plan = _lib.plan(cell, B, T, N, D)
     assert plan.supported and plan.batch_tile == 16 and plan.fwd_batch_tile == 16 and plan.exchange == 0
+    for wx_bf16 in (False, True):   # and the plan is what runs: not the kernels with R in registers
+        assert _lib.register_kernels(cell, wx_bf16, B, N, D) == (False, False)
     wx, R, b, init = make_inputs(cell, B, T, N, D, seed, cell == "slstm")
     S = port.SIZES[cell][3]
     gen = torch.Generator().manual_seed(seed + 500)
