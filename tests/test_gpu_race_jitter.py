@@ -1,5 +1,5 @@
 """Race verification by delay injection: with err[6] = seed the kernels stall, in a quarter of the steps and for up
-to 8 us, the epilogue warps or the tensor-core warp of pseudo-randomly chosen CTAs, so that the CTAs of a group (and
+to 8 us, the epilogue warps, the tensor-core warp or the I/O warp of pseudo-randomly chosen CTAs, so that the CTAs of a group (and
 the warp roles inside a CTA) drift against each other at every hand-off of the exchange protocols (operand pushes,
 partial sums, staged stores, slot reuse). Every result must stay bit-identical to the undisturbed run. The hook is
 compiled into the fp32-Wx instantiations of the kernels (the exchange code is the same for both Wx types).
@@ -14,8 +14,12 @@ from tests.test_gpu_timeout import _backward, _buffers, _forward
 
 pytestmark = pytest.mark.gpu
 
-# every exchange path: thread-block cluster (8- and 16-row tiles, 16-unit slices), global memory with one CTA per
+# every exchange path: R in registers (clusters, a half-filled last CTA, one CTA per head, two staged tiles per CTA with three
+# and four stages), thread-block cluster of tcgen05 kernels (8- and 16-row tiles, 16-unit slices), global memory with one CTA per
 # unit slice, K split inside clusters + global publication (forward and backward), and the 1-D backward over global memory
+REGISTER = [("slstm", 9, 24, 2, 48), ("lstm", 9, 24, 2, 48), ("gru", 5, 33, 3, 32), ("elman", 3, 40, 2, 16), ("lstm", 9, 24, 2, 80),
+            ("gru", 8, 24, 1, 240)]
+TCGEN05 = [("lstm", 200, 8, 6, 112)]
 SHAPES = [
     ("lstm", 8, 40, 3, 256), ("gru", 5, 33, 2, 128), ("slstm", 16, 24, 4, 128), ("elman", 9, 30, 1, 512),
     ("lstm", 200, 16, 4, 128), ("lstm", 24, 20, 2, 48),
@@ -25,13 +29,15 @@ OUTPUTS_FWD = ("hist", "carry", "cache", "hbf")
 OUTPUTS_BWD = ("dwx", "dgr", "dinit", "dbp")
 
 
-@pytest.mark.parametrize("shape", SHAPES, ids=lambda s: f"{s[0]}-B{s[1]}-T{s[2]}-N{s[3]}-D{s[4]}")
+@pytest.mark.parametrize("shape", SHAPES + REGISTER + TCGEN05, ids=lambda s: f"{s[0]}-B{s[1]}-T{s[2]}-N{s[3]}-D{s[4]}")
 def test_results_do_not_depend_on_injected_delays(shape, cuda_device):
     from flashrnn_b200 import _lib
 
     lib = _lib.load()
     cell, B, T, N, D = shape
     assert _lib.plan(cell, B, T, N, D).supported
+    if shape in REGISTER or shape in TCGEN05:
+        assert _lib.register_kernels(cell, False, B, N, D) == (shape in REGISTER,) * 2
     t = _buffers(_lib, cell, B, T, N, D, cuda_device)
     t["dH"] = torch.randn(t["hist"].shape, generator=torch.Generator().manual_seed(3)).to(cuda_device)
     err = torch.zeros(32, dtype=torch.int32, device=cuda_device)

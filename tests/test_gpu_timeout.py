@@ -41,15 +41,16 @@ def _backward(lib, _lib, cell, B, T, N, D, t, err, limit_ms):
                                   limit_ms, err.data_ptr(), torch.cuda.current_stream().cuda_stream)
 
 
-# one shape that exchanges inside a thread-block cluster, one that exchanges through global memory
-@pytest.mark.parametrize("shape", [("lstm", 8, 24, 2, 128), ("lstm", 4, 12, 1, 576), ("lstm", 4, 12, 1, 768),
-                                   ("lstm", 64, 12, 1, 768)],
-                         ids=["cluster", "global", "global-ksplit", "global-1d"])
+# R in registers as a cluster and as one CTA, clusters of the tcgen05 kernels, and three ways through global memory
+@pytest.mark.parametrize("shape", [("lstm", 8, 24, 2, 128), ("lstm", 8, 24, 2, 48), ("lstm", 8, 24, 1, 512), ("lstm", 4, 12, 1, 576),
+                                   ("lstm", 4, 12, 1, 768), ("lstm", 64, 12, 1, 768)],
+                         ids=["registers-cluster", "registers-one-cta", "tcgen05-cluster", "global", "global-ksplit", "global-1d"])
 def test_stalled_exchange_is_reported_and_context_survives(shape, cuda_device):
     from flashrnn_b200 import _lib
 
     lib = _lib.load()
     cell, B, T, N, D = shape
+    assert _lib.register_kernels(cell, False, B, N, D) == (D <= 128,) * 2
     t = _buffers(_lib, cell, B, T, N, D, cuda_device)
     err = torch.zeros(32, dtype=torch.int32, device=cuda_device)
     assert _forward(lib, _lib, cell, B, T, N, D, t, err, 0) == 0
