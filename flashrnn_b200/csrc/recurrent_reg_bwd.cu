@@ -57,7 +57,8 @@ __global__ void __launch_bounds__(reg_max_threads(KT, LOCAL), reg_min_blocks(CEL
 frnn_bwd_reg_kernel(const BwdParams p, const float* history, const __grid_constant__ CUtensorMap cache_map,
                     const __grid_constant__ CUtensorMap hist_map, const __grid_constant__ CUtensorMap init_map,
                     const __grid_constant__ CUtensorMap dhist_map, const __grid_constant__ CUtensorMap dgr_map,
-                    const __grid_constant__ CUtensorMap dwx_map, const int wx_bf16, const int own_dwx, const int nst) {
+                    const __grid_constant__ CUtensorMap dwx_map, const int wx_bf16, const int own_dwx, const int stages_in_flight) {
+  const int nst = LOCAL && KT > 2 ? stages_in_flight : kRegMaxStages;  // three only in a 48-unit CTA
   using Cfg = BwdRegCfg<CELL, KT, LOCAL, HALVES>;
   using CT = CellTraits<CELL>;
   constexpr int S = CT::S, MTW = Cfg::MTW, KTW = Cfg::KTW, CH = Cfg::CH, GCL = Cfg::GCL, HP = Cfg::HP, HS = Cfg::HS;
@@ -421,10 +422,6 @@ frnn_bwd_reg_kernel(const BwdParams p, const float* history, const __grid_consta
       const long long c4 = prof ? clock64() : 0;
       // outputs, while the partial sums of the next step are on their way
 #pragma unroll
-      for (int g = 0; g < CT::GB; ++g)
-#pragma unroll
-        for (int e = 0; e < 2; ++e) dbacc[g][e] += CELL != kGRU ? dgw[g][e] : (g == 0 ? dgr[0][e] : dgw[g > 0 ? g - 1 : 0][e]);  // as cell_backward's gb
-#pragma unroll
       for (int g = 0; g < CT::GR; ++g) reg_stage_16(out + dwx_bytes + g * kRegPlane<2>, off_q, dgp[g]);
       if (own_dwx) {
 #pragma unroll
@@ -436,6 +433,10 @@ frnn_bwd_reg_kernel(const BwdParams p, const float* history, const __grid_consta
       fence_proxy_async_smem();
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_u32(&s_out_full[slot]));
+#pragma unroll
+      for (int g = 0; g < CT::GB; ++g)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) dbacc[g][e] += CELL != kGRU ? dgw[g][e] : (g == 0 ? dgr[0][e] : dgw[g > 0 ? g - 1 : 0][e]);  // as cell_backward's gb
       out += out_slot;
       if (++slot == slots) { slot = 0; out = my_out; }
       const long long c5 = prof ? clock64() : 0;
@@ -488,7 +489,7 @@ int launch_bwd_reg(const BwdParams& p, const void* cache, const float* history, 
   const auto bytes = [&](int st) {
     return 2 * Cfg::DG_BYTES + 2 * (LOCAL ? Cfg::MAX_SOURCES : (HALVES ? p.D / 16 : C)) * U * kRegRows * 4 + st * stage + (st + 1) * out_slot;
   };
-  const int nst = reg_stages(bytes(kRegMaxStages), bytes(kRegMaxStages - 1));
+  const int nst = LOCAL && KT > 2 ? reg_stages(bytes(kRegMaxStages), bytes(kRegMaxStages - 1)) : kRegMaxStages;
   const int smem = bytes(nst);
   if (smem > kRegSmemLimit) return -2;
   const int D = p.D, N = p.N, B = p.B;

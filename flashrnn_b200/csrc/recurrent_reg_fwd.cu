@@ -29,7 +29,8 @@ template <int CELL, int KT, bool LOCAL>
 __global__ void __launch_bounds__(reg_max_threads(KT, LOCAL), reg_min_blocks(CELL, KT, LOCAL, false))
 frnn_fwd_reg_kernel(const FwdParams p, const __grid_constant__ CUtensorMap wx_map, const __grid_constant__ CUtensorMap hist_map,
                     const __grid_constant__ CUtensorMap cache_map, const __grid_constant__ CUtensorMap hbf_map, const int wx_bf16,
-                    const int nst, const int hist_states) {
+                    const int stages_in_flight, const int hist_states) {
+  const int nst = LOCAL && KT > 2 ? stages_in_flight : kRegMaxStages;  // three only in a 48-unit CTA
   using CT = CellTraits<CELL>;
   constexpr int NT = (CT::GR + 1) / 2;  // 16-row tiles: gates 2j and 2j + 1 of the warp's units
   constexpr int kHbuf = KT * 16 * 16;   // bytes of one operand buffer: [k][8 batch rows] bf16
@@ -356,7 +357,7 @@ int launch_fwd_reg(const FwdParams& p, const void* wx, int wx_bf16, cudaStream_t
   const int out_slot = reg_chunks(U) * reg_round_1k(plane * (hist_states * hes + (has_cache ? CT::GC * CT::CES : 0) + (p.hbf != nullptr ? 2 : 0)));
   // prefetch depth: 4 steps, 3 where only that lets two CTAs share an SM
   const auto bytes = [&](int st) { return 2 * KT * 16 * 16 + st * stage + (st + 1) * out_slot; };
-  const int nst = reg_stages(bytes(kRegMaxStages), bytes(kRegMaxStages - 1));
+  const int nst = LOCAL && KT > 2 ? reg_stages(bytes(kRegMaxStages), bytes(kRegMaxStages - 1)) : kRegMaxStages;
   const int smem = bytes(nst);
   if (smem > kRegSmemLimit) return -2;
   // bulk stores start on 16-byte boundaries; the tcgen05 kernels write these outputs with plain stores
