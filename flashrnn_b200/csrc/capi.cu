@@ -145,30 +145,42 @@ int make_tensor_map_strided(CUtensorMap* map, const void* base, int elem_bytes, 
 
 // The occupancy query takes microseconds; its answer depends on the device, the kernel, its cluster width and its shared
 // memory only and is remembered (kernels x staging layouts x devices; past 1024 entries it is asked again on each call).
-int reg_room(const void* kern, const cudaLaunchConfig_t& cfg, int width, int clusters) {
+int reg_room(const void* kern, const cudaLaunchConfig_t& cfg, int width, int N, int B, int D) {
   struct Entry { const void* kern; size_t smem; int dev, width, capacity; };
   static std::mutex mu;
   static Entry table[1024];
   static int used = 0;
+  const long long groups = static_cast<long long>(N) * reg_batch_tiles(B), groups16 = static_cast<long long>(N) * ((B + 15) / 16);
+  const auto taken = [&](int capacity) {
+    if (groups <= capacity) return true;
+    if (width > 1 || capacity < 1) return false;
+    const long long rivals = 2ll * sm_count() / (D % 32 == 0 ? D / 32 : D / 16);  // 16-row tcgen05 groups that run at once
+    return 3 * ((groups + capacity - 1) / capacity) <= 4 * ((groups16 + rivals - 1) / rivals);
+  };
   int dev = 0, capacity = -1;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return static_cast<int>(e);
-  if (clusters > 0) {
+  {
     std::lock_guard<std::mutex> lock(mu);
     for (int i = 0; i < used && capacity < 0; ++i)
       if (table[i].kern == kern && table[i].smem == cfg.dynamicSmemBytes && table[i].dev == dev && table[i].width == width)
         capacity = table[i].capacity;
   }
-  if (capacity >= 0 && clusters > capacity) return kRegNoRoom;
+  if (capacity >= 0 && !taken(capacity)) return kRegNoRoom;
   e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kRegSmemLimit);
-  if (e != cudaSuccess || clusters == 0) return static_cast<int>(e);
+  if (e != cudaSuccess) return static_cast<int>(e);
   if (capacity < 0) {
-    e = cudaOccupancyMaxActiveClusters(&capacity, kern, &cfg);
+    if (width > 1) {
+      e = cudaOccupancyMaxActiveClusters(&capacity, kern, &cfg);
+    } else {
+      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&capacity, kern, static_cast<int>(cfg.blockDim.x), cfg.dynamicSmemBytes);
+      capacity *= sm_count();
+    }
     if (e != cudaSuccess) return static_cast<int>(e);
     std::lock_guard<std::mutex> lock(mu);
     if (used < 1024) table[used++] = Entry{kern, cfg.dynamicSmemBytes, dev, width, capacity};
   }
-  return clusters > capacity ? kRegNoRoom : 0;
+  return taken(capacity) ? 0 : kRegNoRoom;
 }
 
 }  // namespace frnn
@@ -355,8 +367,7 @@ int forward_common(int cell, const void* wx, int wx_bf16, const void* r_bf16, co
     if (me != cudaSuccess) return static_cast<int>(me);
     p.xg_data = static_cast<uint8_t*>(xchg);
   }
-  // Narrow heads: R in registers, as long as all groups run at once. A second wave would double the time, where the
-  // tcgen05 kernels can take 16 batch rows per group (LSTM B256 N4 D128: 1.66 us per step in two waves against 1.27).
+  // narrow heads: R in registers where reg_room has it so, else the kernels of the plan; the results are the same
   if (reg_width(D)) {
     const int reg_rc = forward_reg_dispatch(cell, p, wx, wx_bf16, static_cast<cudaStream_t>(stream));
     if (reg_rc != kRegNoRoom) return reg_rc;
@@ -449,7 +460,7 @@ extern "C" int frnn_b200_backward_ex(int cell, const void* cache, const float* h
     p.xg_data = static_cast<uint8_t*>(xchg);
   }
   p.db_rows = plan.batch_tile;
-  if (reg_width(D)) {  // as in the forward pass (LSTM B256 N4 D128: 2.13 us per step in two waves against 1.64)
+  if (reg_width(D)) {
     const int reg_rc = backward_reg_dispatch(cell, p, cache, history, initial, d_history, wx_bf16, static_cast<cudaStream_t>(stream));
     if (reg_rc != kRegNoRoom) return reg_rc;
   }

@@ -73,9 +73,16 @@ constexpr int reg_max_threads(int kt, bool local) { return local && kt > 2 ? 7 *
 
 constexpr int kRegTaken = -101;       // answer to a question: the call would run here
 
-// 0 if the current device holds `clusters` clusters of `width` CTAs of the launch at once (0 clusters: no such condition),
-// kRegNoRoom if it does not, else a cudaError_t. Raises the kernel's shared-memory limit; the capacity is remembered.
-int reg_room(const void* kern, const cudaLaunchConfig_t& cfg, int width, int clusters);
+// 0 if a launch of N heads and B batch rows is taken, in clusters of `width` CTAs or (1) as plain CTAs, kRegNoRoom if not, else
+// a cudaError_t. Raises the kernel's shared-memory limit; the capacity it asks the driver for is remembered.
+//   Clusters: all groups run at once. A second wave would double the time, where the tcgen05 kernels can take 16 batch rows
+//     per group (LSTM B256 N4 D128: 1.66 us per step in two waves against 1.27 forward, 2.13 against 1.64 backward).
+//   Plain CTAs (16, 32, 48 units): several share an SM and need no tensor memory, so they pay in waves too; a wave takes about three
+//     quarters of one of 16-row tcgen05 groups, of which an SM holds two. Forward and backward, T128, us, against those: LSTM B256
+//     N24 D32 569 / 793, GRU 533 / 709, sLSTM 761 / 1063; LSTM B256 N48 D16 625 / 910, B256 N16 D48 1636 / 1928. The other side
+//     is the sLSTM with 16 units and fp32 Wx (11 KB a stage, two CTAs per SM): backward B96 N48, two waves against one, 453 / 269,
+//     B400, nine against five, 1645 / 1202.
+int reg_room(const void* kern, const cudaLaunchConfig_t& cfg, int width, int N, int B, int D);
 
 #ifdef __CUDACC__
 template <int ES> constexpr int kRegPlane = kRegRows * kRegChunk * ES;  // bytes of a staged plane

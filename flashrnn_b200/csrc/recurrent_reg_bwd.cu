@@ -512,7 +512,7 @@ int launch_bwd_reg(const BwdParams& p, const void* cache, const float* history, 
   cfg.attrs = attr;
   cfg.numAttrs = LOCAL ? 0 : 1;
   // whether the call is taken at all comes first: one that is not pays for nothing else
-  const int rc = reg_room(reinterpret_cast<const void*>(kern), cfg, C, LOCAL ? 0 : p.N * reg_batch_tiles(p.B));
+  const int rc = reg_room(reinterpret_cast<const void*>(kern), cfg, C, p.N, p.B, p.D);
   if (rc != 0 || ask) return rc != 0 ? rc : kRegTaken;
   CUtensorMap cache_map, hist_map, init_map, dhist_map, dgr_map, dwx_map;
   if (reg_tile_map(&hist_map, history, 4, D, N, B, CT::S, p.T, uT * nd, uB * uT * nd, nd, Cfg::HS) != 0 ||

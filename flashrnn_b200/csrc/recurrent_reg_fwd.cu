@@ -379,7 +379,7 @@ int launch_fwd_reg(const FwdParams& p, const void* wx, int wx_bf16, cudaStream_t
   cfg.attrs = attr;
   cfg.numAttrs = LOCAL ? 0 : 1;
   // whether the call is taken at all comes first: one that is not pays for nothing else
-  const int rc = reg_room(reinterpret_cast<const void*>(kern), cfg, q.C, LOCAL ? 0 : p.N * reg_batch_tiles(p.B));
+  const int rc = reg_room(reinterpret_cast<const void*>(kern), cfg, q.C, p.N, p.B, p.D);
   if (rc != 0 || ask) return rc != 0 ? rc : kRegTaken;
   CUtensorMap map, hist_map, cache_map, hbf_map;
   const uint64_t nd = static_cast<uint64_t>(p.N) * p.D, T = p.T, Tt = p.T_total;

@@ -79,7 +79,7 @@ int frnn_b200_version(void);
 int frnn_b200_plan(int cell, int B, int T, int N, int D, frnn_b200_plan_t* out);
 
 /* Which kernels a training call of this shape takes on the current device: bit 0 is set if the forward pass, bit 1 if the
- * backward pass keeps R in the registers of its warps (D <= 256, as many groups of 8 batch rows as run at once); where a
+ * backward pass keeps R in the registers of its warps (D <= 256, as long as its groups of 8 batch rows do not need too many waves); where a
  * bit is clear the kernels that frnn_b200_plan describes run, as they do for outputs that are not 16-byte aligned. Both
  * give the same results (db of 16-row batch tiles: up to rounding). Negative: a code as above, or -1000 - cudaError_t. */
 int frnn_b200_register_kernels(int cell, int wx_bf16, int B, int N, int D);

@@ -13,7 +13,7 @@ CELLS = ("lstm", "slstm", "gru", "elman")
 WIDTHS = tuple(range(16, 257, 16))   # odd multiples of 16 from 80 on: 16-unit slices there, a half-filled last CTA here
 # every width with every cell; batches: one row, a ragged second group, three groups
 SHAPES = [(CELLS[j], (1, 9, 20)[(i + j) % 3], (1, 14, 33)[(i + 2 * j) % 3], 1 + (i + j) % 2, D) for i, D in enumerate(WIDTHS) for j in range(4)]
-SHAPES += [("lstm", 150, 9, 6, 32), ("elman", 201, 5, 12, 48), ("lstm", 40, 6, 6, 112)]   # 16-row tiles on the tcgen05 side
+SHAPES += [("lstm", 150, 9, 6, 32), ("elman", 201, 5, 12, 48), ("lstm", 40, 6, 6, 112), ("slstm", 72, 5, 48, 16)]   # 16-row tiles on the tcgen05 side
 
 
 @pytest.mark.parametrize("shape", SHAPES, ids=lambda s: f"{s[0]}-B{s[1]}-T{s[2]}-N{s[3]}-D{s[4]}")
@@ -23,6 +23,8 @@ def test_both_kernel_families_agree_bit_for_bit(shape, cuda_device):
     lib = _lib.load()
     cell, B, T, N, D = shape
     plan = _lib.plan(cell, B, T, N, D)
+    no_backward = cell == "slstm" and (D in (208, 240) or (D == 16 and B > 40))   # the backward stays on tcgen05 either way
+    assert _lib.register_kernels(cell, False, B, N, D) == (True, not no_backward)
     t = _buffers(_lib, cell, B, T, N, D, cuda_device)
     g = torch.Generator().manual_seed(5)
     t["dH"] = torch.randn(t["hist"].shape, generator=g).to(cuda_device)
