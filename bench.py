@@ -46,7 +46,7 @@ REFERENCE_BUDGET_S = 150.0                      # wall-clock budget of the refer
 # dram__bytes_read.sum + dram__bytes_write.sum per launch on this workload. NOT measured by this run: quoted from
 # the ncu capture summarised in the profile below (bench.py cannot run ncu on itself); re-capture when a kernel changes.
 NCU_TRAFFIC_PROFILE = "profiles/recurrence_kernels_cfg2_lstm_bf16_B8_T1024_N3_D256.md"
-NCU_TRAFFIC_BYTES = {"fwd": 52.0e6 + 62.5e6, "bwd": 152.7e6 + 32.9e6, "wgrad": 63.0e6 + 2.1e6}
+NCU_TRAFFIC_BYTES = {"fwd": 52.0e6 + 61.8e6, "bwd": 127.5e6 + 28.4e6, "wgrad": 63.0e6 + 1.6e6}
 
 
 def _peaks():
@@ -425,7 +425,7 @@ def main():
                       "note": "the same step as eager launches through flashrnn(...) + autograd"},
             "gpu_launches": args.steps * 5,
             "kernels_ms": breakdown,
-            "roofline": {"bound": "tensor", "kernel": f"frnn_{dom}_kernel", "achieved": achieved, "peak": bf16_peak,
+            "roofline": {"bound": "tensor", "kernel": breakdown["kernels"][dom], "achieved": achieved, "peak": bf16_peak,
                          "unit": "TFLOP/s", "frac": achieved / bf16_peak, "peak_source": peak_kind,
                          "traffic": NCU_TRAFFIC_BYTES[dom],
                          "traffic_source": f"quoted from the committed ncu summary {NCU_TRAFFIC_PROFILE}, not measured by this run",
@@ -642,8 +642,7 @@ def kernel_breakdown(_lib, dev, d_wx, d_R, d_b, d_init, flush, reps):
     d_history = torch.zeros_like(history)
     d_history[0] = 1.0
     d_carry = torch.zeros_like(carry)
-    dwx = torch.empty_like(d_wx)
-    dgr = torch.empty(plan.dgr_bytes // 2, dtype=bf, device=dev)
+    dwx = dgr = torch.empty_like(d_wx)   # one buffer, as the public call passes it (bf16 Wx, W-gates == R-gates)
     d_initial = torch.empty_like(carry)
     db_part = torch.empty(plan.dbpart_bytes // 4, dtype=f32, device=dev)
     dR = torch.empty((GR, N, D, D), dtype=f32, device=dev)
@@ -684,13 +683,17 @@ def kernel_breakdown(_lib, dev, d_wx, d_R, d_b, d_init, flush, reps):
         out[name] = total / reps
     if int(err[0].item()) != 0:
         raise RuntimeError(f"device-side error {err.tolist()}")
-    # in-kernel phase timers of CTA 0 (SM cycles per step)
-    # err[8..15] are the epilogue warps' phases, err[16..18] the MMA warp's (see the kernels' `prof` blocks)
+    # in-kernel phase timers of CTA 0 (SM cycles per step): word of the error array -> phase
+    in_registers = dict(zip(("fwd", "bwd"), _lib.register_kernels(CELL, True, B, N, D)))
     names = {
-        "fwd": ("wx_stage_wait", "mma_wait", "tmem_read", "epilogue_barrier", "cell", "push_h", "state_stores",
-                "commit_to_epilogue"),
-        "bwd": ("stage_wait_and_read", "partial_wait_and_sum", "cell", "stores_and_first_tile_wait", "scatter",
-                "partial_wait_only", "stage_wait_only", None),
+        "fwd": {16: "operand_wait", 17: "wx_read_and_mma", 12: "cell", 13: "push_h", 14: "staging"},
+        "bwd": {13: "wait_only", 9: "wait_and_partial_sum", 10: "cell_and_barrier", 12: "mma_and_scatter", 11: "staging", 15: "step"},
+    }
+    tcgen05_names = {   # err[8..15] are the epilogue warps' phases, err[16..18] the MMA warp's
+        "fwd": {8: "wx_stage_wait", 9: "mma_wait", 10: "tmem_read", 11: "epilogue_barrier", 12: "cell", 13: "push_h",
+                14: "state_stores", 15: "commit_to_epilogue", 16: "mma_warp_wait", 17: "mma_warp_issue", 18: "push_to_mma_wake"},
+        "bwd": {8: "stage_wait_and_read", 9: "partial_wait_and_sum", 10: "cell", 11: "stores_and_first_tile_wait", 12: "scatter",
+                13: "partial_wait_only", 14: "stage_wait_only", 16: "mma_warp_wait", 17: "mma_warp_issue"},
     }
     for name, fn in (("fwd", fwd), ("bwd", bwd)):
         err.zero_()
@@ -698,11 +701,10 @@ def kernel_breakdown(_lib, dev, d_wx, d_R, d_b, d_init, flush, reps):
         fn()
         torch.cuda.synchronize()
         v = err.tolist()
-        phases = {k: round(v[8 + i] / T, 1) for i, k in enumerate(names[name]) if k is not None}
-        phases.update({"mma_warp_wait": round(v[16] / T, 1), "mma_warp_issue": round(v[17] / T, 1)})
-        if name == "fwd":
-            phases["push_to_mma_wake"] = round(v[18] / T, 1)
-        out[name + "_phase_cycles_per_step"] = phases
+        chosen = names if in_registers[name] else tcgen05_names
+        out[name + "_phase_cycles_per_step"] = {k: round(v[word] / T, 1) for word, k in chosen[name].items()}
+    out["kernels"] = {k: f"frnn_{k}_reg_kernel" if taken else f"frnn_{k}_kernel" for k, taken in in_registers.items()}
+    out["kernels"]["wgrad"] = "wgrad_tma_kernel"
     err.zero_()
     return out
 

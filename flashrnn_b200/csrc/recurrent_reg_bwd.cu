@@ -20,9 +20,9 @@
 // sums of a parity are overwritten only after the CTA barrier of the step that read them; a TMA stage is refilled by the I/O
 // warp after every warp has staged its outputs of the step that used it.
 //
-// Bound: the serial chain of a step. LSTM B8 N3 D256, 1562 cycles = wait and reads 576 + cell and barrier 138 + mma and
-// scatter 717 + staging 123; 0.93 us per step against 1.32 of the tcgen05 kernel; GRU B16 N24 D32 0.68 against 1.02; Elman B16
-// N12 D64 0.50 against 0.84; sLSTM B16 N4 D128 1.07 against 1.33.
+// Bound: the serial chain of a step. LSTM B8 N3 D256, 1513 cycles at 1845 MHz (see recurrent_reg_fwd.cu) = wait and reads 628 (the
+// wait alone 173) + cell and barrier 137 + mma and scatter 612 + staging 127; 0.88 us per step of the call against 1.32 of the
+// tcgen05 kernel; GRU B16 N24 D32 0.71 against 1.02; Elman B16 N12 D64 0.49 against 0.84; sLSTM B16 N4 D128 1.01 against 1.33.
 #include "recurrent_reg.cuh"
 
 namespace frnn {

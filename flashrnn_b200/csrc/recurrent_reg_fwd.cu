@@ -15,10 +15,11 @@
 // A group cannot overtake itself: a half of the operand double buffer is written again only after every warp has published
 // the step in between, and a warp publishes after its own reads of that half.
 //
-// Bound: the serial chain of a step, mostly instruction issue of one warp per scheduler: at LSTM B8 N3 D256, 1331 cycles =
-// operand wait 150 + Wx read and 32 mma 471 + cell 161 + publication 221 + staging of the outputs 318. Per step there, against
-// the tcgen05 kernel: 0.80 us against 1.29; GRU B16 N24 D32 0.63 against 0.68; Elman B16 N12 D64 0.52 against 0.66. A wait of
-// its own for the Wx tile cost 150 cycles more (D256: 0.85 us).
+// Bound: the serial chain of a step, mostly instruction issue and mma latency of one warp per scheduler: at LSTM B8 N3 D256, 1326
+// cycles = operand wait 149 + Wx read and 32 mma 522 + cell 136 + publication 195 + staging of the outputs 324. The SM runs these at
+// 1845 MHz (clock64 against globaltimer; the driver shows 1965), 0.71 us; the rest of the call's 0.79 us per step is the prologue
+// (16 k cycles) and the launch. Per step there, against the tcgen05 kernel: 0.79 us against 1.30; GRU B16 N24 D32 0.58 against 0.68;
+// Elman B16 N12 D64 0.52 against 0.66. A wait of its own for the Wx tile cost 150 cycles more (D256: 0.85 us).
 #include "recurrent_reg.cuh"
 
 namespace frnn {

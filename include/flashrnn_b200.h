@@ -16,7 +16,10 @@
  * flashrnn/flashrnn2/hybrid_fw2d.cu:85-89,366-373): if the caller sets err[3] = 1, CTA 0 adds up
  * SM clock cycles per phase over all steps into err[8..12] (epilogue warp: input wait, operand /
  * tensor-core wait, accumulator read, epilogue sync, cell + stores + exchange) and err[16..17]
- * (MMA warp: operand wait, issue).
+ * (MMA warp: operand wait, issue). Kernels with R in registers (frnn_b200_register_kernels) use
+ * forward err[16] operand wait, [17] Wx read and products, [12] cell, [13] publication, [14] staging;
+ * backward err[9] wait and partial sums (wait alone: [13]), [10] cell, [12] products and scatter,
+ * [11] staging, [15] the whole step.
  * Test hook for the failure path: with err[4] = 1 the CTAs stop publishing their per-step exchange
  * data from step err[5] on, so the next bounded wait (limit = wait_limit_ms) runs out and the call
  * reports err[0] = 101 (forward) / 106 or 107 (backward) and returns normally.
