@@ -14,7 +14,7 @@ namespace frnn {
 constexpr int kRegUnitsPerWarp = 8;
 constexpr int kRegRows = 8;           // batch rows of a group: the column extent of one mma
 constexpr int kRegClusterUnits = 32;  // units of a CTA where a group is a thread-block cluster
-constexpr int kRegNoRoom = -100;      // not taken: more than one wave of clusters, or outputs off the 16-byte grid
+constexpr int kRegNoRoom = -100;      // not taken: too many waves, or outputs off the 16-byte grid
 
 // Widths of these kernels: all multiples of 16 up to 256. One CTA holds a head of 16, 32 or 48 units whole; other widths run as
 // a cluster of ceil(D / 32) CTAs, the last of which has 16 units where D is an odd multiple of 16.
