@@ -78,6 +78,7 @@ SIGNATURES = {
     "frnn_b200_version": (c_int, []),
     "frnn_b200_plan": (c_int, [c_int, c_int, c_int, c_int, c_int, POINTER(Plan)]),
     "frnn_b200_register_kernels": (c_int, [c_int, c_int, c_int, c_int, c_int]),
+    "frnn_b200_register_rows": (c_int, [c_int, c_int, c_int, c_int, c_int]),
     "frnn_b200_forward": (c_int, [c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                                   c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p,
                                   c_void_p]),
@@ -178,6 +179,15 @@ def register_kernels(cell: str, wx_bf16: bool, B: int, N: int, D: int) -> tuple:
     if rc < 0:
         raise ValueError(f"frnn_b200_register_kernels failed: {ERROR_TEXT.get(rc, rc)}")
     return bool(rc & 1), bool(rc & 2)
+
+
+def register_rows(cell: str, wx_bf16: bool, B: int, N: int, D: int) -> tuple:
+    """(forward, backward): batch rows of a group of the kernels with R in registers that a training call of this shape takes
+    on the current CUDA device, 0 where it takes the kernels of the plan."""
+    rc = load().frnn_b200_register_rows(CELLS[cell], int(wx_bf16), B, N, D)
+    if rc < 0:
+        raise ValueError(f"frnn_b200_register_rows failed: {ERROR_TEXT.get(rc, rc)}")
+    return rc & 0xff, rc >> 8
 
 
 def check(rc: int, what: str) -> None:

@@ -9,10 +9,12 @@
 namespace frnn {
 
 int forward_dispatch(int cell, const FwdParams& p, const void* wx, int wx_bf16, int bv, int unit, cudaStream_t s);
-// `ask`: only say whether the call would be taken (kRegTaken or kRegNoRoom)
-int forward_reg_dispatch(int cell, const FwdParams& p, const void* wx, int wx_bf16, cudaStream_t s, bool ask = false);
-int backward_reg_dispatch(int cell, const BwdParams& p, const void* cache, const float* history, const float* initial,
-                          const float* d_history, int wx_bf16, cudaStream_t s, bool ask = false);
+// Register-resident kernels, groups of `rows` (8 or 16) batch rows. `ask`: only say whether the call would be taken (kRegTaken
+// or kRegNoRoom).
+template <int CELL> int launch_fwd_reg_cell(const FwdParams& p, const void* wx, int wx_bf16, cudaStream_t s, int rows, bool ask);
+template <int CELL>
+int launch_bwd_reg_cell(const BwdParams& p, const void* cache, const float* history, const float* initial, const float* d_history,
+                        int wx_bf16, cudaStream_t s, int rows, bool ask);
 int forward_ksplit_dispatch(int cell, const FwdParams& p, const void* wx, int wx_bf16, int bv, int ksplit, cudaStream_t s,
                             int* capacity_only);
 int forward_ksplit_capacity(int cell, int bv, int ksplit, int D);
@@ -138,24 +140,24 @@ int make_tensor_map_strided(CUtensorMap* map, const void* base, int elem_bytes, 
   const CUtensorMapDataType dt = elem_bytes == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
   const CUresult r = fn(map, dt, static_cast<cuuint32_t>(rank), const_cast<void*>(base), gdims, gstrides, gbox, estr,
                         CU_TENSOR_MAP_INTERLEAVE_NONE,
-                        swizzle_bytes == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
+                        swizzle_bytes == 128 ? CU_TENSOR_MAP_SWIZZLE_128B
+                            : (swizzle_bytes == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B),
                         CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS ? 0 : -4;
 }
 
 // The occupancy query takes microseconds; its answer depends on the device, the kernel, its cluster width and its shared
 // memory only and is remembered (kernels x staging layouts x devices; past 1024 entries it is asked again on each call).
-int reg_room(const void* kern, const cudaLaunchConfig_t& cfg, int width, int N, int B, int D) {
+int reg_room(const void* kern, const cudaLaunchConfig_t& cfg, int width, long long groups, long long rival_groups, int D) {
   struct Entry { const void* kern; size_t smem; int dev, width, capacity; };
   static std::mutex mu;
   static Entry table[1024];
   static int used = 0;
-  const long long groups = static_cast<long long>(N) * reg_batch_tiles(B), groups16 = static_cast<long long>(N) * ((B + 15) / 16);
   const auto taken = [&](int capacity) {
     if (groups <= capacity) return true;
-    if (width > 1 || capacity < 1) return false;
+    if (rival_groups <= 0 || capacity < 1) return false;
     const long long rivals = 2ll * sm_count() / (D % 32 == 0 ? D / 32 : D / 16);  // 16-row tcgen05 groups that run at once
-    return 3 * ((groups + capacity - 1) / capacity) <= 4 * ((groups16 + rivals - 1) / rivals);
+    return 3 * ((groups + capacity - 1) / capacity) <= 4 * ((rival_groups + rivals - 1) / rivals);
   };
   int dev = 0, capacity = -1;
   cudaError_t e = cudaGetDevice(&dev);
@@ -168,6 +170,7 @@ int reg_room(const void* kern, const cudaLaunchConfig_t& cfg, int width, int N, 
   }
   if (capacity >= 0 && !taken(capacity)) return kRegNoRoom;
   e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kRegSmemLimit);
+  if (e == cudaSuccess && width > 8) e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   if (e != cudaSuccess) return static_cast<int>(e);
   if (capacity < 0) {
     if (width > 1) {
@@ -181,6 +184,27 @@ int reg_room(const void* kern, const cudaLaunchConfig_t& cfg, int width, int N, 
     if (used < 1024) table[used++] = Entry{kern, cfg.dynamicSmemBytes, dev, width, capacity};
   }
   return taken(capacity) ? 0 : kRegNoRoom;
+}
+
+int forward_reg_dispatch(int cell, const FwdParams& p, const void* wx, int wx_bf16, cudaStream_t s, int rows, bool ask) {
+  switch (cell) {
+    case kLSTM: return launch_fwd_reg_cell<kLSTM>(p, wx, wx_bf16, s, rows, ask);
+    case kSLSTM: return launch_fwd_reg_cell<kSLSTM>(p, wx, wx_bf16, s, rows, ask);
+    case kGRU: return launch_fwd_reg_cell<kGRU>(p, wx, wx_bf16, s, rows, ask);
+    case kElman: return launch_fwd_reg_cell<kElman>(p, wx, wx_bf16, s, rows, ask);
+    default: return -1;
+  }
+}
+
+int backward_reg_dispatch(int cell, const BwdParams& p, const void* cache, const float* history, const float* initial,
+                          const float* d_history, int wx_bf16, cudaStream_t s, int rows, bool ask) {
+  switch (cell) {
+    case kLSTM: return launch_bwd_reg_cell<kLSTM>(p, cache, history, initial, d_history, wx_bf16, s, rows, ask);
+    case kSLSTM: return launch_bwd_reg_cell<kSLSTM>(p, cache, history, initial, d_history, wx_bf16, s, rows, ask);
+    case kGRU: return launch_bwd_reg_cell<kGRU>(p, cache, history, initial, d_history, wx_bf16, s, rows, ask);
+    case kElman: return launch_bwd_reg_cell<kElman>(p, cache, history, initial, d_history, wx_bf16, s, rows, ask);
+    default: return -1;
+  }
 }
 
 }  // namespace frnn
@@ -307,7 +331,7 @@ extern "C" int frnn_b200_plan(int cell, int B, int T, int N, int D, frnn_b200_pl
   return 0;
 }
 
-extern "C" int frnn_b200_register_kernels(int cell, int wx_bf16, int B, int N, int D) {
+extern "C" int frnn_b200_register_rows(int cell, int wx_bf16, int B, int N, int D) {
   frnn_b200_plan_t plan;
   const int rc = frnn_b200_plan(cell, B, 1, N, D, &plan);
   if (rc != 0) return rc;
@@ -320,11 +344,30 @@ extern "C" int frnn_b200_register_kernels(int cell, int wx_bf16, int B, int N, i
   BwdParams b{};
   b.B = B; b.T = 1; b.N = N; b.D = D;
   b.db_rows = plan.batch_tile;
-  const int fwd = forward_reg_dispatch(cell, f, nullptr, wx_bf16, nullptr, true);
-  const int bwd = backward_reg_dispatch(cell, b, nullptr, nullptr, nullptr, nullptr, wx_bf16, nullptr, true);
-  for (const int v : {fwd, bwd})
-    if (v != kRegTaken && v != kRegNoRoom) return v > 0 ? -1000 - v : v;
-  return (fwd == kRegTaken ? 1 : 0) | (bwd == kRegTaken ? 2 : 0);
+  int answer = 0;
+  for (int pass = 0; pass < 2; ++pass) {
+    for (int rows = kRegRows; rows <= 2 * kRegRows; rows += kRegRows) {
+      const int v = pass == 0 ? forward_reg_dispatch(cell, f, nullptr, wx_bf16, nullptr, rows, true)
+                              : backward_reg_dispatch(cell, b, nullptr, nullptr, nullptr, nullptr, wx_bf16, nullptr, rows, true);
+      if (v != kRegTaken && v != kRegNoRoom) return v > 0 ? -1000 - v : v;
+      if (v == kRegTaken) {
+        answer |= rows << (8 * pass);
+        break;
+      }
+    }
+  }
+  return answer;
+}
+
+extern "C" int frnn_b200_register_kernels(int cell, int wx_bf16, int B, int N, int D) {
+  if (D > 256) {  // answered from the shape
+    frnn_b200_plan_t plan;
+    const int rc = frnn_b200_plan(cell, B, 1, N, D, &plan);
+    return rc != 0 ? rc : (plan.supported ? 0 : -2);
+  }
+  const int rows = frnn_b200_register_rows(cell, wx_bf16, B, N, D);
+  if (rows < 0) return rows;
+  return ((rows & 0xff) == kRegRows ? 1 : 0) | (rows >> 8 == kRegRows ? 2 : 0);
 }
 
 namespace {
@@ -368,8 +411,8 @@ int forward_common(int cell, const void* wx, int wx_bf16, const void* r_bf16, co
     p.xg_data = static_cast<uint8_t*>(xchg);
   }
   // narrow heads: R in registers where reg_room has it so, else the kernels of the plan; the results are the same
-  if (reg_width(D)) {
-    const int reg_rc = forward_reg_dispatch(cell, p, wx, wx_bf16, static_cast<cudaStream_t>(stream));
+  for (int rows = kRegRows; rows <= 2 * kRegRows && reg_width(D); rows += kRegRows) {
+    const int reg_rc = forward_reg_dispatch(cell, p, wx, wx_bf16, static_cast<cudaStream_t>(stream), rows, false);
     if (reg_rc != kRegNoRoom) return reg_rc;
   }
   if (plan.fwd_ksplit)
@@ -460,8 +503,8 @@ extern "C" int frnn_b200_backward_ex(int cell, const void* cache, const float* h
     p.xg_data = static_cast<uint8_t*>(xchg);
   }
   p.db_rows = plan.batch_tile;
-  if (reg_width(D)) {
-    const int reg_rc = backward_reg_dispatch(cell, p, cache, history, initial, d_history, wx_bf16, static_cast<cudaStream_t>(stream));
+  for (int rows = kRegRows; rows <= 2 * kRegRows && reg_width(D); rows += kRegRows) {
+    const int reg_rc = backward_reg_dispatch(cell, p, cache, history, initial, d_history, wx_bf16, static_cast<cudaStream_t>(stream), rows, false);
     if (reg_rc != kRegNoRoom) return reg_rc;
   }
   if (plan.bwd_ksplit)

@@ -1,0 +1,6 @@
+// Instantiations of recurrent_reg_fwd.cuh for one cell.
+#include "recurrent_reg_fwd.cuh"
+
+namespace frnn {
+template int launch_fwd_reg_cell<kLSTM>(const FwdParams&, const void*, int, cudaStream_t, int, bool);
+}  // namespace frnn
