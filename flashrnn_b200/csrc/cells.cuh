@@ -161,15 +161,17 @@ __device__ __forceinline__ void cell_backward(const float* cache, const float* s
     const float d_ig = dc * tz + dpre;
     const float d_fg = dc * c_p + dpre * n_p;
     const float d_z = dc * ig * (1.0f - tz * tz);
-    float d_i = d_ig * ig;
-    float d_logf = d_fg * fg;
-    const float dm = slstm_v1 ? 0.0f : ds[3] - d_i - d_logf;
+    // Products that are used more than once: whether the compiler contracts one into a following sum depends on the code around
+    // it, and a step must not round differently in two instantiations.
+    float d_i = __fmul_rn(d_ig, ig);
+    float d_logf = __fmul_rn(d_fg, fg);
+    const float dm = slstm_v1 ? 0.0f : __fadd_rn(__fadd_rn(ds[3], -d_i), -d_logf);
     if (slstm_take_i) {
       d_i = __fmaf_rn(d_ig, ig, dm);
     } else if (i > logf) {
       d_i = __fmaf_rn(d_ig, ig, dm);
     } else if (i < logf) {
-      d_logf += dm;
+      d_logf = __fadd_rn(d_logf, dm);
     } else {
       d_i += 0.5f * dm;
       d_logf += 0.5f * dm;

@@ -39,12 +39,14 @@ __host__ __device__ constexpr int reg_round_1k(int bytes) { return (bytes + 1023
 // thread that set it to the need of its own call (26 KB for bf16 inference at 256 units) could take it from one that is
 // about to launch (49 KB for fp32 training).
 constexpr int kRegSmemLimit = 220 * 1024;
-// Tiles travel several steps at a time: a transfer is 4 steps of every plane, or 2 where 4 would not let as many CTAs share an SM as
-// the registers do, and two of them are in flight in either direction. A warp waits for its input and reports its output once
+// Tiles travel several steps at a time: a transfer is 4 steps of every plane, or fewer where 4 would not let as many CTAs share an SM
+// as the registers do, and two of them are in flight in either direction. A warp waits for its input and reports its output once
 // per transfer: waiting, fences, arrivals and the bookkeeping around them are instructions on the chain of a step.
 constexpr int kRegSlots = 2;
 inline int reg_transfer_steps(int fixed_bytes, int step_bytes, int blocks) {
-  return fixed_bytes + kRegSlots * 4 * step_bytes <= 224 * 1024 / blocks ? 4 : 2;
+  int steps = 4;
+  while (steps > 1 && fixed_bytes + kRegSlots * steps * step_bytes > 224 * 1024 / blocks) --steps;
+  return steps;
 }
 // Tensor map with the dimensions (unit of the head, head, batch row, plane, step). A box that reaches past the head, the
 // batch or the steps is filled with zeros on the way in and cut off on the way out.
