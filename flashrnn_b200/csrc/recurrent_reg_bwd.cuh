@@ -237,20 +237,13 @@ frnn_bwd_reg_kernel(const BwdParams p, const float* history, const float* initia
     constexpr int compute_threads = nwarps * 32;
     const bool v1 = p.slstm_v1 != 0, zero_first = p.slstm_zero_first != 0, cut = p.cut_recurrent != 0, clip_on = p.grad_clip > 0.0f;
     const float grad_clip = p.grad_clip;
-    // where this lane's packets of a tile go: the row q or q + 8 of the tile, four batch rows
-    const uint32_t row_off = static_cast<uint32_t>((q + 8 * (c & 1)) * kUnit + (c >> 1) * 16);
-    uint32_t dst_part[MTW], dst_bar[MTW];
+    // where this lane's words of a tile go: the rows q and q + 8 of the tile, batch rows 2c and 2c + 1
+    const uint32_t row_off = smem_u32(part) + static_cast<uint32_t>(source0 * kPartSource + ((tile0 & 1) * 16 + q) * kUnit + c * 8);
+    uint32_t owner_delta[MTW];  // shared memory of the CTA that owns the tile's units: 32 of them, two tiles
 #pragma unroll
     for (int m = 0; m < MTW; ++m) {
       const int tile = tile0 + nwarps * m;
-      if (LOCAL) {
-        dst_part[m] = smem_u32(part) + source0 * kPartSource + tile * 16 * kUnit + row_off;
-        dst_bar[m] = 0u;
-      } else {
-        const int owner = tile < n_tiles ? tile / 2 : rank;  // 32 units, two tiles
-        dst_part[m] = map_to_cta(smem_u32(part) + source0 * kPartSource + (tile & 1) * 16 * kUnit + row_off, owner);
-        dst_bar[m] = map_to_cta(smem_u32(&s_part_bar[0]), owner);
-      }
+      owner_delta[m] = LOCAL ? static_cast<uint32_t>(tile / 2 * 32 * kUnit) : map_to_cta(smem_u32(smem), tile < n_tiles ? tile / 2 : rank) - smem_u32(smem);
     }
 
     bool dead = false;  // warp-uniform: after a failed wait the warp walks on without waiting
@@ -437,18 +430,18 @@ frnn_bwd_reg_kernel(const BwdParams p, const float* history, const float* initia
 #pragma unroll
                   for (int m = 0; m < MTW; ++m) {
                     const float(&v)[4] = acc[e][h][m];
-                    // rows q / q + 8, columns 2c, 2c + 1 -> even lanes: row q, columns 2c .. 2c + 3; odd lanes: row q + 8, 2c - 2 .. 2c + 1
-                    const float x0 = __shfl_xor_sync(0xffffffffu, (c & 1) ? v[0] : v[2], 1);
-                    const float x1 = __shfl_xor_sync(0xffffffffu, (c & 1) ? v[1] : v[3], 1);
-                    const float4 w = (c & 1) ? make_float4(x0, x1, v[2], v[3]) : make_float4(v[0], v[1], x0, x1);
-                    const uint32_t dst = dst_part[m] + nb * part_bytes + h * kPartSource + (e0 + e) * kPartTile;
+                    const uint32_t dst = row_off + owner_delta[m] + nb * part_bytes + h * kPartSource + (e0 + e) * kPartTile;
                     if constexpr (LOCAL) {
-                      if (publish)
-                        asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(dst), "f"(w.x), "f"(w.y), "f"(w.z), "f"(w.w) : "memory");
+                      if (publish) {
+                        asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(dst), "f"(v[0]), "f"(v[1]) : "memory");
+                        asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(dst + 8 * kUnit), "f"(v[2]), "f"(v[3]) : "memory");
+                      }
                     } else {
-                      if (publish && tile0 + nwarps * m < n_tiles && (!HALVES || source0 + h < sources))
-                        st_async_v4_b32(dst, __float_as_uint(w.x), __float_as_uint(w.y), __float_as_uint(w.z), __float_as_uint(w.w),
-                                        dst_bar[m] + nb * 8);
+                      const uint32_t bar = smem_u32(&s_part_bar[nb]) + owner_delta[m];
+                      if (publish && tile0 + nwarps * m < n_tiles && (!HALVES || source0 + h < sources)) {
+                        st_async_v2_b32(dst, __float_as_uint(v[0]), __float_as_uint(v[1]), bar);
+                        st_async_v2_b32(dst + 8 * kUnit, __float_as_uint(v[2]), __float_as_uint(v[3]), bar);
+                      }
                     }
                   }
             }

@@ -32,26 +32,28 @@ namespace {
 
 enum : int { kRegAny = 0, kRegTrain = 1, kRegPlain = 2 };
 
-template <int CELL, int KT, bool LOCAL, int UC, int NB>
+template <int CELL, int KT, bool LOCAL, int NB>
 struct FwdRegCfg {
   static constexpr int UPW = CELL == kElman ? 8 : 4;         // units of a warp: one 16-row tile holds all gates of four
   static constexpr int IT = UPW / 4, NI = NB * IT;           // items (unit, batch row) of a thread, per column tile and in all
   static constexpr int ROWS = NB * kRegRows;
-  static constexpr int CHUNK = !LOCAL && UC == 16 ? 16 : kRegChunk;
-  static constexpr int MAX_C = LOCAL ? 1 : (UC == 16 ? KT : KT / 2);
-  static constexpr int THREADS = (UC / UPW + 1) * 32;
+  static constexpr int U = LOCAL ? KT * 16 : 32;             // units of a CTA
+  static constexpr int MAX_C = LOCAL ? 1 : KT / 2;
+  static constexpr int THREADS = (U / UPW + 1) * 32;
+  // h_t goes to a peer as the words of two batch rows, or (GATHER) as packets of eight that a quad of lanes puts together
+  static constexpr bool GATHER = UPW == 8 && MAX_C > 4;
   // CTAs per SM the register budget is cut for
-  static constexpr int MIN_BLOCKS = LOCAL ? (KT <= 2 ? 4 : (CELL == kSLSTM ? 1 : 2)) : (UC == 16 ? 2 : (KT <= 8 || CELL == kElman ? 2 : 1));
+  static constexpr int MIN_BLOCKS = LOCAL ? (KT <= 2 ? 4 : (CELL == kSLSTM ? 1 : 2)) : (KT <= 8 || CELL == kElman ? 2 : 1);
 };
 
-template <int CELL, int KT, bool LOCAL, int UC, int NB>
-__global__ void __launch_bounds__(FwdRegCfg<CELL, KT, LOCAL, UC, NB>::THREADS, FwdRegCfg<CELL, KT, LOCAL, UC, NB>::MIN_BLOCKS)
+template <int CELL, int KT, bool LOCAL, int NB>
+__global__ void __launch_bounds__(FwdRegCfg<CELL, KT, LOCAL, NB>::THREADS, FwdRegCfg<CELL, KT, LOCAL, NB>::MIN_BLOCKS)
 frnn_fwd_reg_kernel(const FwdParams p, const __grid_constant__ CUtensorMap wx_map, const __grid_constant__ CUtensorMap hist_map,
                     const __grid_constant__ CUtensorMap cache_map, const __grid_constant__ CUtensorMap hbf_map, const int wx_bf16,
                     const int ring_steps, const int hist_states) {
-  using Cfg = FwdRegCfg<CELL, KT, LOCAL, UC, NB>;
+  using Cfg = FwdRegCfg<CELL, KT, LOCAL, NB>;
   using CT = CellTraits<CELL>;
-  constexpr int UPW = Cfg::UPW, IT = Cfg::IT, NI = Cfg::NI, CHUNK = Cfg::CHUNK, ROWS = Cfg::ROWS, U = UC, nwarps = UC / UPW;
+  constexpr int UPW = Cfg::UPW, IT = Cfg::IT, NI = Cfg::NI, CHUNK = kRegChunk, ROWS = Cfg::ROWS, U = Cfg::U, nwarps = U / UPW;
   constexpr int kPlane2 = ROWS * CHUNK * 2, kPlane4 = ROWS * CHUNK * 4, kPlaneC = ROWS * CHUNK * CT::CES;
   constexpr int kHalf = KT * 16 * 16;    // bytes of one column tile of the operand: [k][8 batch rows] bf16
   constexpr int kHbuf = NB * kHalf;      // ... of one operand buffer
@@ -216,17 +218,15 @@ frnn_fwd_reg_kernel(const FwdParams p, const __grid_constant__ CUtensorMap wx_ma
       *reinterpret_cast<volatile int*>(&s_gave_up) = 1;
     };
 
-    // A packet is 8 batch rows of one unit, 16 bytes. SENDERS lanes hold it: the quads q and q + 4 where there is one column tile and
-    // each has half of the unit's rows, else one quad.
-    constexpr int SENDERS = UPW == 4 && NB == 1 ? 8 : 4, NS = LOCAL ? 1 : (Cfg::MAX_C + SENDERS - 1) / SENDERS;
-    const int sender = SENDERS == 8 ? hi * 4 + c : c;
+    // Peers of a lane. Words: a lane of a unit's first quad and the one 16 above it hold the same word of the first column tile and
+    // share the peers; with two column tiles each has a word of its own for every peer. Packets: the quad shares the peers.
+    constexpr int SENDERS = Cfg::GATHER ? 4 : (UPW == 4 && NB == 1 ? 2 : 1), NS = (Cfg::MAX_C + SENDERS - 1) / SENDERS;
+    const int sender = Cfg::GATHER ? c : (SENDERS == 2 ? hi : 0);
     uint32_t peer_delta[NS];
-#pragma unroll
-    for (int i = 0; i < NS; ++i) peer_delta[i] = 0u;
     if (!LOCAL) {
 #pragma unroll
       for (int i = 0; i < NS; ++i)
-        if (SENDERS * i + sender < C) peer_delta[i] = map_to_cta(smem_u32(smem), SENDERS * i + sender) - smem_u32(smem);
+        peer_delta[i] = SENDERS * i + sender < C ? map_to_cta(smem_u32(smem), SENDERS * i + sender) - smem_u32(smem) : 0u;
       cluster_sync_all();
     }
     if (prof) p.err[20] = static_cast<int>(clock64() - t_entry);
@@ -342,8 +342,7 @@ frnn_fwd_reg_kernel(const FwdParams p, const __grid_constant__ CUtensorMap wx_ma
               for (int i = 0; i < NI; ++i) sts_u16(hslot + i / IT * kHalf + (item_row(i) & 7) * 2, bf16_bits(st[0][i]));
             }
           } else {
-            constexpr int PK = UPW == 8 ? NB : 1;  // packets of this lane's unit that its quad has
-            uint32_t pk[PK][4];
+            constexpr int PK = UPW == 8 ? NB : 1;  // words of this lane
 #pragma unroll
             for (int j = 0; j < PK; ++j) {
               uint32_t w;
@@ -354,16 +353,18 @@ frnn_fwd_reg_kernel(const FwdParams p, const __grid_constant__ CUtensorMap wx_ma
                 const float other = __shfl_xor_sync(0xffffffffu, NB == 2 && !hi ? st[0][NB - 1] : st[0][0], 16);
                 w = pack_bf16x2(hi ? other : mine, hi ? mine : other);
               }
-              gather_quad(w, lane, pk[j]);
-            }
-            if (publish && !dead) {
-              const uint32_t bar = smem_u32(&s_hbar[(t + 1) & 1]);
+              uint32_t pk[4];
+              if constexpr (Cfg::GATHER) gather_quad(w, lane, pk);
+              if (publish && !dead) {
+                const uint32_t bar = smem_u32(&s_hbar[(t + 1) & 1]);
+                const uint32_t dst = hslot + (UPW == 8 ? j : (NB == 2 ? hi : 0)) * kHalf + (Cfg::GATHER ? 0 : c * 4);
 #pragma unroll
-              for (int j = 0; j < PK; ++j) {
-                const uint32_t dst = hslot + (UPW == 8 ? j : (NB == 2 ? hi : 0)) * kHalf;
-#pragma unroll
-                for (int i = 0; i < NS; ++i)
-                  if (SENDERS * i + sender < C) st_async_v4_b32(dst + peer_delta[i], pk[j][0], pk[j][1], pk[j][2], pk[j][3], bar + peer_delta[i]);
+                for (int i = 0; i < NS; ++i) {
+                  if (SENDERS * i + sender < C) {
+                    if constexpr (Cfg::GATHER) st_async_v4_b32(dst + peer_delta[i], pk[0], pk[1], pk[2], pk[3], bar + peer_delta[i]);
+                    else st_async_b32(dst + peer_delta[i], w, bar + peer_delta[i]);
+                  }
+                }
               }
             }
           }
@@ -439,11 +440,11 @@ frnn_fwd_reg_kernel(const FwdParams p, const __grid_constant__ CUtensorMap wx_ma
 }
 
 // Runs the call, or (ask) only says whether it would: kRegTaken / kRegNoRoom.
-template <int CELL, int KT, bool LOCAL, int UC, int NB>
+template <int CELL, int KT, bool LOCAL, int NB>
 int launch_fwd_reg(const FwdParams& p, const void* wx, int wx_bf16, cudaStream_t stream, bool ask, long long rival_groups = 0) {
-  using Cfg = FwdRegCfg<CELL, KT, LOCAL, UC, NB>;
+  using Cfg = FwdRegCfg<CELL, KT, LOCAL, NB>;
   using CT = CellTraits<CELL>;
-  constexpr int U = UC, ROWS = Cfg::ROWS, CHUNK = Cfg::CHUNK, plane = ROWS * CHUNK, chunks = (U + CHUNK - 1) / CHUNK;
+  constexpr int U = Cfg::U, ROWS = Cfg::ROWS, CHUNK = kRegChunk, plane = ROWS * CHUNK, chunks = (U + CHUNK - 1) / CHUNK;
   const int es = wx_bf16 ? 2 : 4;
   const int stage = chunks * CT::GW * plane * es;
   const int hist_states = p.output_mode == 0 ? CT::S : (p.output_mode == 1 ? 1 : 0);
@@ -457,7 +458,7 @@ int launch_fwd_reg(const FwdParams& p, const void* wx, int wx_bf16, cudaStream_t
   // bulk stores start on 16-byte boundaries; the tcgen05 kernels write these outputs with plain stores
   if (((reinterpret_cast<uintptr_t>(p.history) | reinterpret_cast<uintptr_t>(p.cache) | reinterpret_cast<uintptr_t>(p.hbf)) & 15u) != 0)
     return kRegNoRoom;
-  auto kern = frnn_fwd_reg_kernel<CELL, KT, LOCAL, UC, NB>;
+  auto kern = frnn_fwd_reg_kernel<CELL, KT, LOCAL, NB>;
   FwdParams q = p;
   q.C = (p.D + U - 1) / U;
   const long long groups = static_cast<long long>(p.N) * reg_batch_tiles(p.B, ROWS);
@@ -490,25 +491,11 @@ int launch_fwd_reg(const FwdParams& p, const void* wx, int wx_bf16, cudaStream_t
   return static_cast<int>(cudaLaunchKernelEx(&cfg, kern, q, map, hist_map, cache_map, hbf_map, wx_bf16, steps, hist_states));
 }
 
-template <int CELL, int KT>
-int launch_fwd_reg_cluster(const FwdParams& p, const void* wx, int wx_bf16, cudaStream_t s, int rows, bool ask) {
-  if (rows == kRegRows) {
-    if constexpr (CELL != kElman && KT <= 16) {
-      if (!ask) {
-        const int rc = launch_fwd_reg<CELL, KT, false, 16, 1>(p, wx, wx_bf16, s, ask);
-        if (rc != kRegNoRoom) return rc;
-      }
-    }
-    return launch_fwd_reg<CELL, KT, false, 32, 1>(p, wx, wx_bf16, s, ask);
-  }
-  return launch_fwd_reg<CELL, KT, false, 32, 2>(p, wx, wx_bf16, s, ask);
-}
-
-template <int CELL, int KT>
-int launch_fwd_reg_local(const FwdParams& p, const void* wx, int wx_bf16, cudaStream_t s, int rows, bool ask) {
-  const long long rivals = static_cast<long long>(p.N) * reg_batch_tiles(p.B, 16);
-  if (rows == kRegRows) return launch_fwd_reg<CELL, KT, true, KT * 16, 1>(p, wx, wx_bf16, s, ask, rivals);
-  return launch_fwd_reg<CELL, KT, true, KT * 16, 2>(p, wx, wx_bf16, s, ask, rivals);
+template <int CELL, int KT, bool LOCAL>
+int launch_fwd_reg_rows(const FwdParams& p, const void* wx, int wx_bf16, cudaStream_t s, int rows, bool ask) {
+  const long long rivals = LOCAL ? static_cast<long long>(p.N) * reg_batch_tiles(p.B, 16) : 0;
+  if (rows == kRegRows) return launch_fwd_reg<CELL, KT, LOCAL, 1>(p, wx, wx_bf16, s, ask, rivals);
+  return launch_fwd_reg<CELL, KT, LOCAL, 2>(p, wx, wx_bf16, s, ask, rivals);
 }
 
 }  // namespace
@@ -516,20 +503,20 @@ int launch_fwd_reg_local(const FwdParams& p, const void* wx, int wx_bf16, cudaSt
 template <int CELL>
 int launch_fwd_reg_cell(const FwdParams& p, const void* wx, int wx_bf16, cudaStream_t s, int rows, bool ask) {
   switch (reg_k_tiles(p.D)) {
-    case 1: return launch_fwd_reg_local<CELL, 1>(p, wx, wx_bf16, s, rows, ask);
-    case 2: return launch_fwd_reg_local<CELL, 2>(p, wx, wx_bf16, s, rows, ask);
-    case 3: return launch_fwd_reg_local<CELL, 3>(p, wx, wx_bf16, s, rows, ask);
-    case 4: return launch_fwd_reg_cluster<CELL, 4>(p, wx, wx_bf16, s, rows, ask);
-    case 6: return launch_fwd_reg_cluster<CELL, 6>(p, wx, wx_bf16, s, rows, ask);
-    case 8: return launch_fwd_reg_cluster<CELL, 8>(p, wx, wx_bf16, s, rows, ask);
+    case 1: return launch_fwd_reg_rows<CELL, 1, true>(p, wx, wx_bf16, s, rows, ask);
+    case 2: return launch_fwd_reg_rows<CELL, 2, true>(p, wx, wx_bf16, s, rows, ask);
+    case 3: return launch_fwd_reg_rows<CELL, 3, true>(p, wx, wx_bf16, s, rows, ask);
+    case 4: return launch_fwd_reg_rows<CELL, 4, false>(p, wx, wx_bf16, s, rows, ask);
+    case 6: return launch_fwd_reg_rows<CELL, 6, false>(p, wx, wx_bf16, s, rows, ask);
+    case 8: return launch_fwd_reg_rows<CELL, 8, false>(p, wx, wx_bf16, s, rows, ask);
     case 10:
-    case 12: return launch_fwd_reg_cluster<CELL, 12>(p, wx, wx_bf16, s, rows, ask);
+    case 12: return launch_fwd_reg_rows<CELL, 12, false>(p, wx, wx_bf16, s, rows, ask);
     case 14:
-    case 16: return launch_fwd_reg_cluster<CELL, 16>(p, wx, wx_bf16, s, rows, ask);
+    case 16: return launch_fwd_reg_rows<CELL, 16, false>(p, wx, wx_bf16, s, rows, ask);
     case 20:
-    case 24: return launch_fwd_reg_cluster<CELL, 24>(p, wx, wx_bf16, s, rows, ask);
+    case 24: return launch_fwd_reg_rows<CELL, 24, false>(p, wx, wx_bf16, s, rows, ask);
     case 28:
-    case 32: return launch_fwd_reg_cluster<CELL, 32>(p, wx, wx_bf16, s, rows, ask);
+    case 32: return launch_fwd_reg_rows<CELL, 32, false>(p, wx, wx_bf16, s, rows, ask);
     default: return -2;
   }
 }
