@@ -9,7 +9,7 @@
 namespace frnn {
 
 int forward_dispatch(int cell, const FwdParams& p, const void* wx, int wx_bf16, int bv, int unit, cudaStream_t s);
-// Register-resident kernels, groups of `rows` (8 or 16) batch rows. `ask`: only say whether the call would be taken (kRegTaken
+// Register-resident kernels, groups of `rows` (8, 16 or 24) batch rows. `ask`: only say whether the call would be taken (kRegTaken
 // or kRegNoRoom).
 template <int CELL> int launch_fwd_reg_cell(const FwdParams& p, const void* wx, int wx_bf16, cudaStream_t s, int rows, bool ask);
 template <int CELL>
@@ -346,7 +346,7 @@ extern "C" int frnn_b200_register_rows(int cell, int wx_bf16, int B, int N, int 
   b.db_rows = plan.batch_tile;
   int answer = 0;
   for (int pass = 0; pass < 2; ++pass) {
-    for (int rows = kRegRows; rows <= 2 * kRegRows; rows += kRegRows) {
+    for (int rows = kRegRows; rows <= kRegMaxRows; rows += kRegRows) {
       const int v = pass == 0 ? forward_reg_dispatch(cell, f, nullptr, wx_bf16, nullptr, rows, true)
                               : backward_reg_dispatch(cell, b, nullptr, nullptr, nullptr, nullptr, wx_bf16, nullptr, rows, true);
       if (v != kRegTaken && v != kRegNoRoom) return v > 0 ? -1000 - v : v;
@@ -411,7 +411,7 @@ int forward_common(int cell, const void* wx, int wx_bf16, const void* r_bf16, co
     p.xg_data = static_cast<uint8_t*>(xchg);
   }
   // narrow heads: R in registers where reg_room has it so, else the kernels of the plan; the results are the same
-  for (int rows = kRegRows; rows <= 2 * kRegRows && reg_width(D); rows += kRegRows) {
+  for (int rows = kRegRows; rows <= kRegMaxRows && reg_width(D); rows += kRegRows) {
     const int reg_rc = forward_reg_dispatch(cell, p, wx, wx_bf16, static_cast<cudaStream_t>(stream), rows, false);
     if (reg_rc != kRegNoRoom) return reg_rc;
   }
@@ -503,7 +503,7 @@ extern "C" int frnn_b200_backward_ex(int cell, const void* cache, const float* h
     p.xg_data = static_cast<uint8_t*>(xchg);
   }
   p.db_rows = plan.batch_tile;
-  for (int rows = kRegRows; rows <= 2 * kRegRows && reg_width(D); rows += kRegRows) {
+  for (int rows = kRegRows; rows <= kRegMaxRows && reg_width(D); rows += kRegRows) {
     const int reg_rc = backward_reg_dispatch(cell, p, cache, history, initial, d_history, wx_bf16, static_cast<cudaStream_t>(stream), rows, false);
     if (reg_rc != kRegNoRoom) return reg_rc;
   }

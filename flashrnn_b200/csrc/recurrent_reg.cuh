@@ -11,7 +11,8 @@
 
 namespace frnn {
 
-constexpr int kRegRows = 8;           // batch rows of one column tile of an mma; a group has one or two of them
+constexpr int kRegRows = 8;           // batch rows of one column tile of an mma; a group has one, two or (clusters of 6 CTAs and more) three
+constexpr int kRegMaxRows = 24;
 constexpr int kRegNoRoom = -100;      // not taken: too many waves, or outputs off the 16-byte grid
 constexpr int kRegTaken = -101;       // answer to a question: the call would run here
 
@@ -44,10 +45,12 @@ constexpr int kRegSmemLimit = 220 * 1024;
 // per transfer: waiting, fences, arrivals and the bookkeeping around them are instructions on the chain of a step.
 constexpr int kRegSlots = 2;
 inline int reg_transfer_steps(int fixed_bytes, int step_bytes, int blocks) {
+  const int limit = blocks == 1 ? kRegSmemLimit - 2 * kRegSlots * 1024 : 224 * 1024 / blocks;  // less what rounding adds
   int steps = 4;
-  while (steps > 1 && fixed_bytes + kRegSlots * steps * step_bytes > 224 * 1024 / blocks) --steps;
+  while (steps > 1 && fixed_bytes + kRegSlots * steps * step_bytes > limit) --steps;
   return steps;
 }
+
 // Tensor map with the dimensions (unit of the head, head, batch row, plane, step). A box that reaches past the head, the
 // batch or the steps is filled with zeros on the way in and cut off on the way out.
 inline int reg_tile_map(CUtensorMap* map, const void* base, int es, int D, int N, int B, int planes, int steps,

@@ -59,7 +59,7 @@ struct BwdRegCfg {
   // dg is double-buffered; what follows it starts at a multiple of 1 KB
   static constexpr int DG_ALL = reg_round_1k(2 * NB * DG_BYTES);
   // CTAs per SM the register budget is cut for
-  static constexpr int MIN_BLOCKS = LOCAL ? (KT <= 2 ? (CELL == kLSTM || CELL == kSLSTM ? 2 : 3) : (CELL == kSLSTM ? 1 : 2))
+  static constexpr int MIN_BLOCKS = LOCAL ? (KT <= 2 ? (NB > 1 || CELL == kLSTM || CELL == kSLSTM ? 2 : 3) : (CELL == kSLSTM ? 1 : 2))
                                           : (KT <= 8 || CELL == kElman ? 2 : 1);
 };
 
@@ -505,15 +505,15 @@ frnn_bwd_reg_kernel(const BwdParams p, const float* history, const float* initia
       float v = 0.0f;
 #pragma unroll
       for (int e = 0; e < NB; ++e) {
-        if (e > 0 && p.db_rows == kRegRows) v = 0.0f;
+        if (e > 0 && (NB == 3 || p.db_rows == kRegRows)) v = 0.0f;
 #pragma unroll
         for (int k = 0; k < kRegRows; ++k) v += __shfl_sync(0xffffffffu, dbacc[g][e], (k & 1) * 16 + (lane & 12) + (k >> 1));
         const int b = b0 + e * kRegRows;
         if (c == 0 && hi == 0 && own && b < B) {
           float* dst = p.db_part + ((static_cast<size_t>(b / p.db_rows) * CT::GB + g) * N + n) * D + d;
-          // One group of 8 rows per half of a 16-row entry: at most two addends on top of the launcher's zeros, so the order cannot
-          // matter, but the sum may differ in its last bits from the 16 rows added one by one.
-          if (NB == 1 && p.db_rows != kRegRows) atomicAdd(dst, v);
+          // The halves of a 16-row entry may come from two groups: at most two addends on top of the launcher's zeros, so the order
+          // cannot matter, but the sum may differ in its last bits from the 16 rows added one by one.
+          if (NB != 2 && p.db_rows != kRegRows) atomicAdd(dst, v);
           else *dst = v;
         }
       }
@@ -577,7 +577,7 @@ int launch_bwd_reg(const BwdParams& p, const void* cache, const float* history, 
   if (Cfg::GCL > 0 && map(&cache_map, cache, CT::CES, CT::GC, p.T, uT * CT::GC * nd, nd, CT::GC * nd, CT::GC) != 0) return -4;
   dwx_map = dgr_map;
   if (own_dwx && map(&dwx_map, p.dwx, wx_bf16 ? 2 : 4, CT::GW, p.T, uT * CT::GW * nd, nd, CT::GW * nd, CT::GW) != 0) return -4;
-  if (NB == 1 && p.db_rows != kRegRows) {
+  if (NB != 2 && p.db_rows != kRegRows) {
     const size_t tiles = static_cast<size_t>((p.B + p.db_rows - 1) / p.db_rows);
     const cudaError_t e = cudaMemsetAsync(p.db_part, 0, tiles * CT::GB * p.N * p.D * sizeof(float), stream);
     if (e != cudaSuccess) return static_cast<int>(e);
@@ -601,7 +601,20 @@ int launch_bwd_reg_rows(const BwdRegCall& v) {
   const long long rivals = LOCAL ? static_cast<long long>(v.p.N) * reg_batch_tiles(v.p.B, 16) : 0;
   if (v.rows == kRegRows)
     return launch_bwd_reg<CELL, KT, LOCAL, HALVES, 1>(v.p, v.cache, v.history, v.initial, v.d_history, v.wx_bf16, v.stream, v.ask, rivals);
-  return launch_bwd_reg<CELL, KT, LOCAL, HALVES, 2>(v.p, v.cache, v.history, v.initial, v.d_history, v.wx_bf16, v.stream, v.ask, rivals);
+  // Where registers run out (the sLSTM from 288 units on and with two sums a tile, four gates beyond 384 units), or the tcgen05 kernel's
+  // clusters of 9 still run two to an SM, more rows per group are no faster than that kernel. T48 N1 - 4, us, against it: 16 rows sLSTM B64
+  // D320 127 / 157, D288 126 / 120, D448 322 / 253, B256 D112 177 / 168; 24 rows LSTM B64 D384 162 / 245, B256 D288 160 / 149, B56
+  // D512 (T64) 400 / 354; GRU B256 D288 95 / 131.
+  constexpr bool tight = CELL == kLSTM || CELL == kSLSTM;
+  if (v.rows == 2 * kRegRows) {
+    if ((CELL == kSLSTM && (HALVES || KT == 32 || v.p.D == 288))) return kRegNoRoom;
+    return launch_bwd_reg<CELL, KT, LOCAL, HALVES, 2>(v.p, v.cache, v.history, v.initial, v.d_history, v.wx_bf16, v.stream, v.ask, rivals);
+  }
+  if constexpr (KT >= 16 && !HALVES && !(tight && KT == 32)) {
+    if (tight && v.p.D == 288) return kRegNoRoom;
+    return launch_bwd_reg<CELL, KT, LOCAL, HALVES, 3>(v.p, v.cache, v.history, v.initial, v.d_history, v.wx_bf16, v.stream, v.ask);
+  }
+  return kRegNoRoom;
 }
 
 template <int CELL, int KT>

@@ -218,10 +218,10 @@ frnn_fwd_reg_kernel(const FwdParams p, const __grid_constant__ CUtensorMap wx_ma
       *reinterpret_cast<volatile int*>(&s_gave_up) = 1;
     };
 
-    // Peers of a lane. Words: a lane of a unit's first quad and the one 16 above it hold the same word of the first column tile and
-    // share the peers; with two column tiles each has a word of its own for every peer. Packets: the quad shares the peers.
-    constexpr int SENDERS = Cfg::GATHER ? 4 : (UPW == 4 && NB == 1 ? 2 : 1), NS = (Cfg::MAX_C + SENDERS - 1) / SENDERS;
-    const int sender = Cfg::GATHER ? c : (SENDERS == 2 ? hi : 0);
+    // Peers of a lane. Words: lanes 16 apart hold the two rows of a word between them; of two column tiles each packs one and sends it
+    // to every peer, of a single one both pack the same word and share the peers. Packets: the quad shares the peers.
+    constexpr int SENDERS = Cfg::GATHER ? 4 : 1, NS = (Cfg::MAX_C + SENDERS - 1) / SENDERS;
+    const int sender = Cfg::GATHER ? c : 0;
     uint32_t peer_delta[NS];
     if (!LOCAL) {
 #pragma unroll
@@ -342,27 +342,42 @@ frnn_fwd_reg_kernel(const FwdParams p, const __grid_constant__ CUtensorMap wx_ma
               for (int i = 0; i < NI; ++i) sts_u16(hslot + i / IT * kHalf + (item_row(i) & 7) * 2, bf16_bits(st[0][i]));
             }
           } else {
-            constexpr int PK = UPW == 8 ? NB : 1;  // words of this lane
+            const uint32_t bar = smem_u32(&s_hbar[(t + 1) & 1]);
+            if constexpr (UPW == 8) {
 #pragma unroll
-            for (int j = 0; j < PK; ++j) {
-              uint32_t w;
-              if constexpr (UPW == 8) {
-                w = pack_bf16x2(st[0][2 * j], st[0][2 * j + 1]);
-              } else {  // lanes 16 apart have the rows 2c and 2c + 1; with two tiles lanes 0 - 15 pack the first, 16 - 31 the second
-                const float mine = NB == 2 && hi ? st[0][NB - 1] : st[0][0];
-                const float other = __shfl_xor_sync(0xffffffffu, NB == 2 && !hi ? st[0][NB - 1] : st[0][0], 16);
-                w = pack_bf16x2(hi ? other : mine, hi ? mine : other);
-              }
-              uint32_t pk[4];
-              if constexpr (Cfg::GATHER) gather_quad(w, lane, pk);
-              if (publish && !dead) {
-                const uint32_t bar = smem_u32(&s_hbar[(t + 1) & 1]);
-                const uint32_t dst = hslot + (UPW == 8 ? j : (NB == 2 ? hi : 0)) * kHalf + (Cfg::GATHER ? 0 : c * 4);
+              for (int j = 0; j < NB; ++j) {
+                const uint32_t w = pack_bf16x2(st[0][2 * j], st[0][2 * j + 1]), dst = hslot + j * kHalf;
+                uint32_t pk[4];
+                if constexpr (Cfg::GATHER) gather_quad(w, lane, pk);
+                if (publish && !dead) {
 #pragma unroll
-                for (int i = 0; i < NS; ++i) {
-                  if (SENDERS * i + sender < C) {
+                  for (int i = 0; i < NS; ++i) {
+                    if (SENDERS * i + sender >= C) continue;
                     if constexpr (Cfg::GATHER) st_async_v4_b32(dst + peer_delta[i], pk[0], pk[1], pk[2], pk[3], bar + peer_delta[i]);
-                    else st_async_b32(dst + peer_delta[i], w, bar + peer_delta[i]);
+                    else st_async_b32(dst + c * 4 + peer_delta[i], w, bar + peer_delta[i]);
+                  }
+                }
+              }
+            } else {
+#pragma unroll
+              for (int j = 0; j < NB; j += 2) {
+                const bool two = j + 1 < NB;
+                const float mine = two && hi ? st[0][two ? j + 1 : j] : st[0][j];
+                const float other = __shfl_xor_sync(0xffffffffu, two && !hi ? st[0][two ? j + 1 : j] : st[0][j], 16);
+                const uint32_t w = pack_bf16x2(hi ? other : mine, hi ? mine : other);
+                if (publish && !dead) {
+                  if (two) {
+                    const uint32_t dst = hslot + (j + hi) * kHalf + c * 4;
+#pragma unroll
+                    for (int i = 0; i < NS; ++i)
+                      if (i < C) st_async_b32(dst + peer_delta[i], w, bar + peer_delta[i]);
+                  } else {
+                    const uint32_t dst = hslot + j * kHalf + c * 4;
+#pragma unroll
+                    for (int i = 0; i < NS; i += 2) {
+                      const uint32_t delta = hi ? peer_delta[i + 1 < NS ? i + 1 : i] : peer_delta[i];
+                      if (i + hi < C) st_async_b32(dst + delta, w, bar + delta);
+                    }
                   }
                 }
               }
@@ -495,7 +510,15 @@ template <int CELL, int KT, bool LOCAL>
 int launch_fwd_reg_rows(const FwdParams& p, const void* wx, int wx_bf16, cudaStream_t s, int rows, bool ask) {
   const long long rivals = LOCAL ? static_cast<long long>(p.N) * reg_batch_tiles(p.B, 16) : 0;
   if (rows == kRegRows) return launch_fwd_reg<CELL, KT, LOCAL, 1>(p, wx, wx_bf16, s, ask, rivals);
-  return launch_fwd_reg<CELL, KT, LOCAL, 2>(p, wx, wx_bf16, s, ask, rivals);
+  // More rows per group: 13 to 14 cycles of a scheduler per mma and column tile, while a tcgen05.mma costs the same for 16 rows as for 8
+  // and its kernel has two CTAs of up to 448 units on an SM. T48 N1 - 4, us, against that kernel: 16 rows LSTM B64 D448 105 / 102, D512
+  // 120 / 222; 24 rows B96 D256 344 / 411 (T256), B256 D288 108 / 99, B64 D384 116 / 108. The Elman cell has half the tiles: D512 153 / 327.
+  if (rows == 2 * kRegRows) {
+    if (CELL != kElman && p.D > 384 && p.D <= 448) return kRegNoRoom;
+    return launch_fwd_reg<CELL, KT, LOCAL, 2>(p, wx, wx_bf16, s, ask, rivals);
+  }
+  if constexpr (KT == 12 || KT == 16 || (CELL == kElman && KT > 16)) return launch_fwd_reg<CELL, KT, LOCAL, 3>(p, wx, wx_bf16, s, ask);
+  return kRegNoRoom;
 }
 
 }  // namespace

@@ -87,7 +87,7 @@ int frnn_b200_plan(int cell, int B, int T, int N, int D, frnn_b200_plan_t* out);
  * give the same results (db of 16-row batch tiles: up to rounding). Negative: a code as above, or -1000 - cudaError_t. */
 int frnn_b200_register_kernels(int cell, int wx_bf16, int B, int N, int D);
 
-/* The same for groups of 8 or 16 batch rows and D <= 512: bits 0-7 the rows of a forward, bits 8-15 of a backward group (8 or 16);
+/* The same for groups of 8, 16 or 24 batch rows and D <= 512: bits 0-7 the rows of a forward, bits 8-15 of a backward group;
  * 0 where the kernels that frnn_b200_plan describes run. Negative: as above. */
 int frnn_b200_register_rows(int cell, int wx_bf16, int B, int N, int D);
 
