@@ -19,7 +19,7 @@ PKG = Path(__file__).resolve().parent
 CSRC = PKG / "csrc"
 LIB_DIR = PKG / "lib"
 LIB_PATH = LIB_DIR / "libflashrnn_b200.so"
-SOURCES = ("capi.cu", "capi_mg.cu", *(f"recurrent_reg_{d}_{c}.cu" for d in ("bwd", "fwd") for c in ("slstm", "lstm", "gru", "elman")),
+SOURCES = ("capi.cu", "capi_mg.cu", *(f"recurrent_{k}_{c}.cu" for k in ("reg_bwd", "reg_fwd", "wide_bwd", "wide_fwd") for c in ("slstm", "lstm", "gru", "elman")),
            "recurrent_fwd.cu", "recurrent_fwd_ksplit.cu", "recurrent_bwd.cu", "recurrent_bwd_ksplit.cu",
            "recurrent_mg_fwd.cu", "recurrent_mg_bwd.cu", "wgrad.cu", "input_proj.cu")
 NVCC_FLAGS = (

@@ -15,6 +15,8 @@ template <int CELL> int launch_fwd_reg_cell(const FwdParams& p, const void* wx, 
 template <int CELL>
 int launch_bwd_reg_cell(const BwdParams& p, const void* cache, const float* history, const float* initial, const float* d_history,
                         int wx_bf16, cudaStream_t s, int rows, bool ask);
+// The same for wide heads, with the groups and the split of the plan: launched, or kRegNoRoom.
+template <int CELL> int launch_fwd_wide_cell(const FwdParams& p, const void* wx, int wx_bf16, int rows, int ksplit, cudaStream_t s);
 int forward_ksplit_dispatch(int cell, const FwdParams& p, const void* wx, int wx_bf16, int bv, int ksplit, cudaStream_t s,
                             int* capacity_only);
 int forward_ksplit_capacity(int cell, int bv, int ksplit, int D);
@@ -141,7 +143,8 @@ int make_tensor_map_strided(CUtensorMap* map, const void* base, int elem_bytes, 
   const CUresult r = fn(map, dt, static_cast<cuuint32_t>(rank), const_cast<void*>(base), gdims, gstrides, gbox, estr,
                         CU_TENSOR_MAP_INTERLEAVE_NONE,
                         swizzle_bytes == 128 ? CU_TENSOR_MAP_SWIZZLE_128B
-                            : (swizzle_bytes == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B),
+                            : (swizzle_bytes == 64 ? CU_TENSOR_MAP_SWIZZLE_64B
+                                                    : (swizzle_bytes == 32 ? CU_TENSOR_MAP_SWIZZLE_32B : CU_TENSOR_MAP_SWIZZLE_NONE)),
                         CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS ? 0 : -4;
 }
@@ -192,6 +195,16 @@ int forward_reg_dispatch(int cell, const FwdParams& p, const void* wx, int wx_bf
     case kSLSTM: return launch_fwd_reg_cell<kSLSTM>(p, wx, wx_bf16, s, rows, ask);
     case kGRU: return launch_fwd_reg_cell<kGRU>(p, wx, wx_bf16, s, rows, ask);
     case kElman: return launch_fwd_reg_cell<kElman>(p, wx, wx_bf16, s, rows, ask);
+    default: return -1;
+  }
+}
+
+int forward_wide_dispatch(int cell, const FwdParams& p, const void* wx, int wx_bf16, int rows, int ksplit, cudaStream_t s) {
+  switch (cell) {
+    case kLSTM: return launch_fwd_wide_cell<kLSTM>(p, wx, wx_bf16, rows, ksplit, s);
+    case kSLSTM: return launch_fwd_wide_cell<kSLSTM>(p, wx, wx_bf16, rows, ksplit, s);
+    case kGRU: return launch_fwd_wide_cell<kGRU>(p, wx, wx_bf16, rows, ksplit, s);
+    case kElman: return launch_fwd_wide_cell<kElman>(p, wx, wx_bf16, rows, ksplit, s);
     default: return -1;
   }
 }
@@ -311,8 +324,14 @@ extern "C" int frnn_b200_plan(int cell, int B, int T, int N, int D, frnn_b200_pl
     out->supported = fwd_ok && bwd_ok;
     const int64_t fwd_groups = static_cast<int64_t>(N) * ((B + out->fwd_batch_tile - 1) / out->fwd_batch_tile);
     const int64_t bwd_groups = static_cast<int64_t>(N) * out->n_btiles;
-    const int64_t fwd_b = 4ll * bt * D * 2;  // four operand slots
-    const int64_t bwd_b = out->bwd_ksplit ? 4ll * bt * c.gr * D * 2                                        // four slots of dG
+    // four operand slots of 16 rows (tensor-memory kernels) or one of the group's rows per step, up to kWideSlots (registers)
+    const int64_t slots = wide_slots(T);
+    const auto operand = [&](int ksplit, int tile, int64_t k) {
+      const int64_t four = 4ll * bt * k * 2, wide = ksplit ? slots * tile * k * 2 : 0;
+      return four > wide ? four : wide;
+    };
+    const int64_t fwd_b = operand(out->fwd_ksplit, out->fwd_batch_tile, D);
+    const int64_t bwd_b = out->bwd_ksplit ? operand(out->bwd_ksplit, out->batch_tile, static_cast<int64_t>(c.gr) * D)
                                           : 2ll * out->cluster * out->cluster * out->unit * out->batch_tile * 4;  // two slots of partial dh
     out->xchg_bytes = fwd_groups * fwd_b > bwd_groups * bwd_b ? fwd_groups * fwd_b : bwd_groups * bwd_b;
   }
@@ -405,10 +424,15 @@ int forward_common(int cell, const void* wx, int wx_bf16, const void* r_bf16, co
   p.wait_limit_ns = (wait_limit_ms > 0 ? static_cast<unsigned long long>(wait_limit_ms) : 2000ull) * 1000000ull;
   if (plan.exchange) {
     if (!xchg) return -5;
-    // every exchange word starts as "not yet written" (all ones)
-    const cudaError_t me = cudaMemsetAsync(xchg, 0xff, static_cast<size_t>(plan.xchg_bytes), static_cast<cudaStream_t>(stream));
-    if (me != cudaSuccess) return static_cast<int>(me);
     p.xg_data = static_cast<uint8_t*>(xchg);
+    if (plan.fwd_ksplit) {
+      const int rc_wide = forward_wide_dispatch(cell, p, wx, wx_bf16, plan.fwd_batch_tile, plan.fwd_ksplit, static_cast<cudaStream_t>(stream));
+      if (rc_wide != kRegNoRoom) return rc_wide;
+    }
+    // every exchange word starts as "not yet written" (all ones): four slots of 16 rows per group
+    const size_t bytes = static_cast<size_t>(N) * ((B + plan.fwd_batch_tile - 1) / plan.fwd_batch_tile) * 4 * 16 * D * 2;
+    const cudaError_t me = cudaMemsetAsync(xchg, 0xff, bytes, static_cast<cudaStream_t>(stream));
+    if (me != cudaSuccess) return static_cast<int>(me);
   }
   // narrow heads: R in registers where reg_room has it so, else the kernels of the plan; the results are the same
   for (int rows = kRegRows; rows <= kRegMaxRows && reg_width(D); rows += kRegRows) {

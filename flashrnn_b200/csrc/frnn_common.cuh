@@ -229,7 +229,7 @@ inline uint32_t tmem_cols_pow2(int needed, uint32_t minimum) {
 int make_tensor_map(CUtensorMap* map, const void* base, int elem_bytes, int rank, const uint64_t* dims,
                     const uint32_t* box, bool swizzle128 = false, const uint64_t* stride_dims = nullptr);
 // The same with the byte strides of dimensions 1 .. rank - 1 given (any order of dimensions) and a swizzle span of 32, 64
-// or 128 bytes, which the inner extent of the box fills.
+// or 128 bytes (16: none), which the inner extent of the box fills.
 int make_tensor_map_strided(CUtensorMap* map, const void* base, int elem_bytes, int rank, const uint64_t* dims,
                             const uint64_t* strides, const uint32_t* box, int swizzle_bytes);
 

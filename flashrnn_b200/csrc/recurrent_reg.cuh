@@ -51,6 +51,13 @@ inline int reg_transfer_steps(int fixed_bytes, int step_bytes, int blocks) {
   return steps;
 }
 
+// Modes of the forward's step loops: any outputs and hooks, the outputs of a training call, a whole fp32 history alone.
+enum : int { kRegAny = 0, kRegTrain = 1, kRegPlain = 2 };
+
+// Wide heads (recurrent_wide_*.cuh): slots of the exchange in global memory, steps between two fences.
+constexpr int kWideSlots = 64, kWideFence = 8;
+inline int wide_slots(int T) { return T < kWideSlots ? T : kWideSlots; }
+
 // Tensor map with the dimensions (unit of the head, head, batch row, plane, step). A box that reaches past the head, the
 // batch or the steps is filled with zeros on the way in and cut off on the way out.
 inline int reg_tile_map(CUtensorMap* map, const void* base, int es, int D, int N, int B, int planes, int steps,
@@ -78,11 +85,11 @@ __device__ __forceinline__ void reg_report(int* err, int code, int detail) {
 }
 
 // Byte offset of (batch row, unit of the chunk) in a plane of the staged tiles: rows of CHUNK * ES bytes, 16-byte blocks
-// permuted as the TMA swizzle of that span does.
+// permuted as the TMA swizzle of that span does (none at 16 bytes).
 template <int ES, int CHUNK>
 __device__ __forceinline__ uint32_t reg_tile_offset(int row, int unit) {
   constexpr int span = CHUNK * ES;
-  const int x = span == 128 ? row & 7 : (span == 64 ? (row >> 1) & 3 : (row >> 2) & 1);
+  const int x = span == 128 ? row & 7 : (span == 64 ? (row >> 1) & 3 : (span == 32 ? (row >> 2) & 1 : 0));
   return static_cast<uint32_t>(row * span) + (static_cast<uint32_t>(unit * ES) ^ static_cast<uint32_t>(x << 4));
 }
 __device__ __forceinline__ float lds_f32(uint32_t a) { float v; asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(a)); return v; }

@@ -30,8 +30,6 @@ namespace frnn {
 
 namespace {
 
-enum : int { kRegAny = 0, kRegTrain = 1, kRegPlain = 2 };
-
 template <int CELL, int KT, bool LOCAL, int NB>
 struct FwdRegCfg {
   static constexpr int UPW = CELL == kElman ? 8 : 4;         // units of a warp: one 16-row tile holds all gates of four

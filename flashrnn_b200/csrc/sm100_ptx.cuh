@@ -477,6 +477,9 @@ __device__ __forceinline__ void st_relaxed_gpu_v4(void* p, uint4 v) {
   asm volatile("st.relaxed.gpu.global.v4.u32 [%0], {%1, %2, %3, %4};" ::"l"(p), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w)
                : "memory");
 }
+__device__ __forceinline__ void st_relaxed_gpu_u32(void* p, uint32_t v) {
+  asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
 __device__ __forceinline__ void fence_acq_rel_gpu() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
 constexpr uint32_t kXgFill = 0xffffffffu;  // "not yet written" pattern of an exchange word
 __device__ __forceinline__ bool xg_arrived(const uint4& v) {
