@@ -16,6 +16,9 @@ template <int CELL>
 int launch_bwd_reg_cell(const BwdParams& p, const void* cache, const float* history, const float* initial, const float* d_history,
                         int wx_bf16, cudaStream_t s, int rows, bool ask);
 // The same for wide heads, with the groups and the split of the plan: launched, or kRegNoRoom.
+template <int CELL>
+int launch_bwd_wide_cell(const BwdParams& p, const void* cache, const float* history, const float* initial, const float* d_history,
+                         int wx_bf16, int rows, int ksplit, cudaStream_t s);
 template <int CELL> int launch_fwd_wide_cell(const FwdParams& p, const void* wx, int wx_bf16, int rows, int ksplit, cudaStream_t s);
 int forward_ksplit_dispatch(int cell, const FwdParams& p, const void* wx, int wx_bf16, int bv, int ksplit, cudaStream_t s,
                             int* capacity_only);
@@ -205,6 +208,17 @@ int forward_wide_dispatch(int cell, const FwdParams& p, const void* wx, int wx_b
     case kSLSTM: return launch_fwd_wide_cell<kSLSTM>(p, wx, wx_bf16, rows, ksplit, s);
     case kGRU: return launch_fwd_wide_cell<kGRU>(p, wx, wx_bf16, rows, ksplit, s);
     case kElman: return launch_fwd_wide_cell<kElman>(p, wx, wx_bf16, rows, ksplit, s);
+    default: return -1;
+  }
+}
+
+int backward_wide_dispatch(int cell, const BwdParams& p, const void* cache, const float* history, const float* initial,
+                           const float* d_history, int wx_bf16, int rows, int ksplit, cudaStream_t s) {
+  switch (cell) {
+    case kLSTM: return launch_bwd_wide_cell<kLSTM>(p, cache, history, initial, d_history, wx_bf16, rows, ksplit, s);
+    case kSLSTM: return launch_bwd_wide_cell<kSLSTM>(p, cache, history, initial, d_history, wx_bf16, rows, ksplit, s);
+    case kGRU: return launch_bwd_wide_cell<kGRU>(p, cache, history, initial, d_history, wx_bf16, rows, ksplit, s);
+    case kElman: return launch_bwd_wide_cell<kElman>(p, cache, history, initial, d_history, wx_bf16, rows, ksplit, s);
     default: return -1;
   }
 }
@@ -522,9 +536,18 @@ extern "C" int frnn_b200_backward_ex(int cell, const void* cache, const float* h
   p.wait_limit_ns = (wait_limit_ms > 0 ? static_cast<unsigned long long>(wait_limit_ms) : 2000ull) * 1000000ull;
   if (plan.exchange) {
     if (!xchg) return -5;
-    const cudaError_t me = cudaMemsetAsync(xchg, 0xff, static_cast<size_t>(plan.xchg_bytes), static_cast<cudaStream_t>(stream));
-    if (me != cudaSuccess) return static_cast<int>(me);
     p.xg_data = static_cast<uint8_t*>(xchg);
+    const size_t groups = static_cast<size_t>(N) * plan.n_btiles;
+    if (plan.bwd_ksplit) {
+      const int rc_wide = backward_wide_dispatch(cell, p, cache, history, initial, d_history, wx_bf16, plan.batch_tile, plan.bwd_ksplit,
+                                                 static_cast<cudaStream_t>(stream));
+      if (rc_wide != kRegNoRoom) return rc_wide;
+    }
+    // every exchange word starts as "not yet written": four slots of 16 rows of dG, or two of the partial dh of a group
+    const size_t bytes = plan.bwd_ksplit ? groups * 4 * 16 * plan.gates_r * D * 2
+                                         : groups * 2 * plan.cluster * plan.cluster * plan.unit * plan.batch_tile * 4;
+    const cudaError_t me = cudaMemsetAsync(xchg, 0xff, bytes, static_cast<cudaStream_t>(stream));
+    if (me != cudaSuccess) return static_cast<int>(me);
   }
   p.db_rows = plan.batch_tile;
   for (int rows = kRegRows; rows <= kRegMaxRows && reg_width(D); rows += kRegRows) {

@@ -1,0 +1,6 @@
+// Instantiations of recurrent_wide_bwd.cuh for one cell.
+#include "recurrent_wide_bwd.cuh"
+
+namespace frnn {
+template int launch_bwd_wide_cell<kElman>(const BwdParams&, const void*, const float*, const float*, const float*, int, int, int, cudaStream_t);
+}  // namespace frnn
