@@ -192,7 +192,7 @@ frnn_bwd_wide_kernel(const BwdParams p, const float* history, const float* initi
       in_at[i] = static_cast<uint32_t>(ul / CHUNK * in_chunk);
       out_at[i] = static_cast<uint32_t>(ul / CHUNK * out_chunk);
       part_src[i] = smem_u32(part) + static_cast<uint32_t>(tile * Cfg::PART_TILE + ul * 32 + row * 4);
-      word_at[i] = static_cast<uint32_t>(tile * K + d) * 16 + c * 4;
+      word_at[i] = static_cast<uint32_t>(tile * K + d + (CT::GR > 1 ? hi * D : 0)) * 16 + c * 4;  // of the gate that the lane publishes
     }
     const bool v1 = p.slstm_v1 != 0, zero_first = p.slstm_zero_first != 0, cut = p.cut_recurrent != 0, clip_on = p.grad_clip > 0.0f;
     const float grad_clip = p.grad_clip;
@@ -266,8 +266,6 @@ frnn_bwd_wide_kernel(const BwdParams p, const float* history, const float* initi
             if (it >= 1) {
               wait_parts(it);
               if (!(any && cut)) add_parts(it, ds[0]);
-              // this parity's partial sums were complete at the wait: armed for iteration it + 2
-              if (tid == 0 && !dead && it + 2 <= T) mbar_arrive_expect_tx(smem_u32(&s_part_bar[it & 1]), Cfg::PART);
             }
             if (any && clip_on && it >= 1) {
               // the gradient carried into h_t from step t + 1 (total minus the external part) is complete here: clip it
@@ -302,18 +300,22 @@ frnn_bwd_wide_kernel(const BwdParams p, const float* history, const float* initi
               for (int g = 0; g < CT::GW; ++g) gw[g] = !drop || act[i] ? gw[g] : 0.0f;
 #pragma unroll
               for (int k = 0; k < HS; ++k) sn[k][i] = sp[k][i];
-              // Words of dG_t: the lanes 16 apart have the rows 2c and 2c + 1 and take every other gate's word; the one that does not
-              // store a word refills its place in a later slot.
+              // Words of dG_t, two gates at a time: the lanes 16 apart have the rows 2c and 2c + 1 and a gate's word each.
               uint32_t dgp[CT::GR];
 #pragma unroll
-              for (int g = 0; g < CT::GR; ++g) {
-                dgp[g] = bf16_bits(gr[g]);
-                const uint32_t other = __shfl_xor_sync(0xffffffffu, dgp[g], 16);
-                const uint32_t w = xg_clean(hi ? other | dgp[g] << 16 : dgp[g] | other << 16);
-                if (publish && !dead) {
-                  if ((g & 1) == hi) st_relaxed_gpu_u32(xg_now + word_at[i] + static_cast<size_t>(g) * D * 16, w);
-                  else if (refill) st_relaxed_gpu_u32(xg_ahead + word_at[i] + static_cast<size_t>(g) * D * 16, kXgFill);
-                }
+              for (int g = 0; g < CT::GR; ++g) dgp[g] = bf16_bits(gr[g]);
+#pragma unroll
+              for (int g = 0; g < CT::GR; g += 2) {
+                const bool two = g + 1 < CT::GR;
+                const uint32_t second = dgp[two ? g + 1 : g], other = __shfl_xor_sync(0xffffffffu, hi ? dgp[g] : second, 16);
+                const uint32_t w = xg_clean(hi ? other | second << 16 : dgp[g] | other << 16);
+                const size_t at = word_at[i] + static_cast<size_t>(g * D) * 16;
+                if (publish && !dead && (two || !hi)) st_relaxed_gpu_u32(xg_now + at, w);
+              }
+              if (publish && !dead && refill) {
+#pragma unroll
+                for (int g = 0; g < CT::GR; g += 2)
+                  if (g + 1 < CT::GR || !hi) st_relaxed_gpu_u32(xg_ahead + word_at[i] + static_cast<size_t>(g * D) * 16, kXgFill);
               }
               // outputs and bias sums, while dG_t is on its way
 #pragma unroll
@@ -329,6 +331,8 @@ frnn_bwd_wide_kernel(const BwdParams p, const float* history, const float* initi
 #pragma unroll
               for (int g = 0; g < CT::GB; ++g) dbacc[g][i] += CELL != kGRU ? gw[g] : (g == 0 ? gr[0] : gw[g > 0 ? g - 1 : 0]);  // as cell_backward's gb
             }
+            // this parity's partial sums were complete at the wait: armed for iteration it + 2
+            if (tid == 0 && !dead && it >= 1 && it + 2 <= T) mbar_arrive_expect_tx(smem_u32(&s_part_bar[it & 1]), Cfg::PART);
             c3 = clock();
           }
           // this CTA's chunk of dG_t -> operand buffer of this parity
