@@ -148,17 +148,18 @@ def load() -> ctypes.CDLL:
 _plans: dict = {}
 
 
-def plan(cell: str, B: int, T: int, N: int, D: int) -> Plan:
-    """Launch plan of a shape on the CURRENT CUDA device (the plan depends on its SM count). Remembered per
-    (device, shape): the host path asks several times per call."""
-    dev = -1
-    try:
-        import torch
+def plan(cell: str, B: int, T: int, N: int, D: int, device: int = None) -> Plan:
+    """Launch plan of a shape on the CURRENT CUDA device (the plan depends on its SM count), whose index a caller that knows
+    it gives. Remembered per (device, shape): the host path asks several times per call."""
+    dev = -1 if device is None else device
+    if device is None:
+        try:
+            import torch
 
-        if torch.cuda.is_available():
-            dev = torch.cuda.current_device()
-    except ImportError:  # the binding itself does not need torch
-        pass
+            if torch.cuda.is_available():
+                dev = torch.cuda.current_device()
+        except ImportError:  # the binding itself does not need torch
+            pass
     key = (dev, cell, B, T, N, D)
     hit = _plans.get(key)
     if hit is not None:

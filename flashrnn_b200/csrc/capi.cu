@@ -174,18 +174,18 @@ int reg_room(const void* kern, const cudaLaunchConfig_t& cfg, int width, long lo
       if (table[i].kern == kern && table[i].smem == cfg.dynamicSmemBytes && table[i].dev == dev && table[i].width == width)
         capacity = table[i].capacity;
   }
-  if (capacity >= 0 && !taken(capacity)) return kRegNoRoom;
+  if (capacity >= 0) return taken(capacity) ? 0 : kRegNoRoom;  // its attributes were set before the entry was made
   e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kRegSmemLimit);
   if (e == cudaSuccess && width > 8) e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   if (e != cudaSuccess) return static_cast<int>(e);
-  if (capacity < 0) {
-    if (width > 1) {
-      e = cudaOccupancyMaxActiveClusters(&capacity, kern, &cfg);
-    } else {
-      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&capacity, kern, static_cast<int>(cfg.blockDim.x), cfg.dynamicSmemBytes);
-      capacity *= sm_count();
-    }
-    if (e != cudaSuccess) return static_cast<int>(e);
+  if (width > 1) {
+    e = cudaOccupancyMaxActiveClusters(&capacity, kern, &cfg);
+  } else {
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&capacity, kern, static_cast<int>(cfg.blockDim.x), cfg.dynamicSmemBytes);
+    capacity *= sm_count();
+  }
+  if (e != cudaSuccess) return static_cast<int>(e);
+  {
     std::lock_guard<std::mutex> lock(mu);
     if (used < 1024) table[used++] = Entry{kern, cfg.dynamicSmemBytes, dev, width, capacity};
   }

@@ -15,6 +15,7 @@ stays connected to autograd.
 from __future__ import annotations
 
 from dataclasses import dataclass
+import threading
 import time
 from typing import Optional
 
@@ -35,16 +36,66 @@ def _ptr(t: Optional[torch.Tensor]):
     return None if t is None else t.data_ptr()
 
 
-def _stream(device) -> int:
-    return torch.cuda.current_stream(device).cuda_stream
+def _stream(device: torch.device) -> int:
+    return torch._C._cuda_getCurrentRawStream(device.index)
 
 
-def _raise_device_error(err: torch.Tensor, what: str) -> None:
-    code, step, cta = (int(v) for v in err[:3].tolist())
-    if code != 0:
-        raise RuntimeError(
-            f"{what}: device-side wait ran out (code {code}: {_lib.ERROR_TEXT.get(code, '?')}, step {step}, CTA {cta})"
-        )
+def _raise_device_error(err: torch.Tensor, what) -> None:
+    """``err`` is one launch's word (``what`` its name) or a block of them, a row each (``what``: the names)."""
+    rows, names = ([err.tolist()], [what]) if err.ndim == 1 else (err.tolist(), what)
+    for row, name in zip(rows, names):
+        code, step, cta = row[:3]
+        if code != 0:
+            raise RuntimeError(
+                f"{name}: device-side wait ran out (code {code}: {_lib.ERROR_TEXT.get(code, '?')}, step {step}, CTA {cta})"
+            )
+
+
+class _ErrorBlock:
+    """Error words of the eager launches of one thread on one stream, zeroed together, read back together.
+
+    A fill, a new event and a device-to-host copy per launch were a third of the host time of a short call (about 30 of 95 us).
+    A block is filled by its thread only, which records the block's event behind every launch. Any thread may close the words
+    tracked so far (under the lock, without touching the stream, which could be capturing by then): they go to the queue with
+    that event and the block gets a new one. A word that is handed out but not tracked yet, i.e. whose launch another thread
+    is just making, stays for the next time."""
+
+    SIZE = 64
+
+    def __init__(self, device, stream):
+        self.stream, self.event = stream, torch.cuda.Event()
+        self.words = torch.zeros((self.SIZE, 32), dtype=torch.int32, device=device)
+        self.names = []      # of the words tracked, in order
+        self.closed = 0      # words that are in the queue
+        self.given = 0
+
+    def close(self) -> None:
+        if len(self.names) > self.closed:
+            _pending_errors.append((self.event, self.words[self.closed:len(self.names)], self.names[self.closed:]))
+            self.closed, self.event = len(self.names), torch.cuda.Event()
+
+
+_blocks: dict = {}            # (thread, device, raw stream) -> the block its next launch takes a word from
+_blocks_lock = threading.Lock()
+
+
+def _error_word(device: torch.device) -> torch.Tensor:
+    """32 zeroed words for a launch of this thread on the device's current stream; goes to ``_track`` after the launch."""
+    if _capturing():
+        return torch.zeros(32, dtype=torch.int32, device=device)   # zeroed by every replay
+    key = (threading.get_ident(), device.index, _stream(device))
+    with _blocks_lock:
+        block = _blocks.get(key)
+        if block is None or block.given == block.SIZE:
+            if block is not None:
+                block.close()
+            block = _blocks[key] = _ErrorBlock(device, torch.cuda.current_stream(device))
+        if len(block.names) < block.given:        # a launch that was refused after it had taken its word: it is free again
+            block.given = len(block.names)
+        word = block.words[block.given]
+        block.given += 1
+    word._frnn_block = block
+    return word
 
 
 _captured_errors: list = []   # error words of launches recorded into CUDA graphs: (err, what), newest last
@@ -69,6 +120,12 @@ def _track(err: torch.Tensor, what: str) -> None:
         _captured_errors.append((err, what))
         del _captured_errors[:-256]
         return
+    block = getattr(err, "_frnn_block", None)
+    if block is not None:
+        with _blocks_lock:
+            block.event.record(block.stream)
+            block.names.append(what)
+        return
     ev = torch.cuda.Event()
     ev.record(torch.cuda.current_stream(err.device))
     _pending_errors.append((ev, err, what))
@@ -87,6 +144,11 @@ def poll_errors(block: bool = False) -> None:
         if now - _last_poll < 0.02:
             return
         _last_poll = now
+    with _blocks_lock:
+        for key, block in list(_blocks.items()):
+            block.close()
+            if block.closed == block.given:       # nothing on the way: blocks of finished threads and old streams go
+                del _blocks[key]
     keep = []
     while _pending_errors:
         ev, err, what = _pending_errors.pop(0)
@@ -109,12 +171,7 @@ class _Recurrence(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, wx, recurrent, bias, initial, cell: str, zero_first: bool, options=None):
-        # the C ABI plans for and launches on the current device: make the tensors' device current
-        with torch.cuda.device(wx.device):
-            return _Recurrence._forward(ctx, wx, recurrent, bias, initial, cell, zero_first, options)
-
-    @staticmethod
-    def _forward(ctx, wx, recurrent, bias, initial, cell: str, zero_first: bool, options):
+        # the C ABI plans for and launches on the current device, which _run has made that of the tensors
         lib = _lib.load()
         poll_errors()
         B, T, _, N, D = wx.shape
@@ -124,7 +181,7 @@ class _Recurrence(torch.autograd.Function):
         r_bf = recurrent.detach().to(torch.bfloat16).contiguous()
         b32 = bias.detach().to(torch.float32).contiguous()
         init32 = initial.detach().to(torch.float32).contiguous()
-        plan = _lib.plan(cell, B, T, N, D)
+        plan = _lib.plan(cell, B, T, N, D, dev.index)
         if not plan.supported:
             raise ValueError(
                 f"flashrnn_b200: cell={cell} D={D} is outside the sm_100a kernel family "
@@ -140,7 +197,7 @@ class _Recurrence(torch.autograd.Function):
                 cache = torch.empty(plan.cache_bytes, dtype=torch.uint8, device=dev)
             hbf = torch.empty(plan.hbf_bytes // 2, dtype=torch.bfloat16, device=dev)
         xchg = torch.empty(plan.xchg_bytes, dtype=torch.uint8, device=dev) if plan.xchg_bytes else None
-        err = torch.zeros(32, dtype=torch.int32, device=dev)
+        err = _error_word(dev)
         rc = lib.frnn_b200_forward_ex(
             _lib.CELLS[cell], wx_c.data_ptr(), int(wx_c.dtype == torch.bfloat16), r_bf.data_ptr(), b32.data_ptr(),
             init32.data_ptr(), history.data_ptr(), carry.data_ptr(), _ptr(cache), _ptr(hbf), _ptr(xchg), B, T, N, D,
@@ -192,7 +249,7 @@ class _Recurrence(torch.autograd.Function):
         if plan.wgrad_work_bytes:
             work = torch.empty(plan.wgrad_work_bytes // 4, dtype=torch.float32, device=dev)
         xchg = torch.empty(plan.xchg_bytes, dtype=torch.uint8, device=dev) if plan.xchg_bytes else None
-        err = torch.zeros(32, dtype=torch.int32, device=dev)
+        err = _error_word(dev)
         stream = _stream(dev)
         rc = lib.frnn_b200_backward_ex(
             _lib.CELLS[cell], _ptr(cache) if cache.numel() else None, history.data_ptr(), init32.data_ptr(),
@@ -302,6 +359,8 @@ def _run_on_current_device(wx, recurrent, bias, initial, cell: str, zero_normali
         zero_first = bool(torch.all(initial[2] == 0))
     if D > 1792 and D % 256 == 0 and options is None and wx.dtype in (torch.float32, torch.bfloat16):
         return _run_wide(wx, recurrent, bias, initial, cell, zero_first)
+    if D % 16 == 0 and _lib.plan(cell, wx.shape[0], wx.shape[1], wx.shape[3], D, wx.device.index).supported:
+        return _Recurrence.apply(wx, recurrent, bias, initial, cell, zero_first, options)   # as it is, in one launch
     # The kernels tile the head width in multiples of 16 (heads wider than 768: 64, and 128 where only the
     # column-owning backward fits); the smallest such width that a launch supports is used.
     pad = (-D) % 16
@@ -404,6 +463,8 @@ def flashrnn_torch(wx, recurrent, bias, initial, *, cell: str = "lstm", numerics
         raise ValueError("bias gate count does not match cell")
     if initial.shape != (S, batch, 1, heads, width):
         raise ValueError("initial state must have layout [S,B,1,N,D]")
+    if not torch.is_autocast_enabled("cuda"):
+        return _run(wx, recurrent, bias, initial, cell, zero_normalizer)
     with torch.autocast("cuda", enabled=False):
         return _run(wx, recurrent, bias, initial, cell, zero_normalizer)
 
@@ -467,6 +528,9 @@ def flashrnn(Wx, R, b, states=None, function: str = "lstm", config: Optional[Fla
         states = torch.zeros((S, B, 1, N, D), dtype=torch.float32, device=Wx.device)
     elif states.shape != (S, B, 1, N, D):
         raise ValueError("states must have layout [S,B,1,N,D]")
+    if not torch.is_autocast_enabled("cuda"):
+        return _run(Wx.to(_DTYPES[dtype]), R, b.to(torch.float32), states.to(torch.float32), function,
+                    zero_normalizer, options)
     with torch.autocast("cuda", enabled=False):
         return _run(Wx.to(_DTYPES[dtype]), R, b.to(torch.float32), states.to(torch.float32), function,
                     zero_normalizer, options)

@@ -17,7 +17,7 @@ from typing import Optional
 import torch
 
 from . import _lib
-from .functional import SIZES, FlashRNNConfig, _track, flashrnn, poll_errors
+from .functional import SIZES, FlashRNNConfig, _error_word, _track, flashrnn, poll_errors
 
 
 class _Projection(torch.autograd.Function):
@@ -33,7 +33,7 @@ class _Projection(torch.autograd.Function):
             w16 = weight.detach().to(torch.bfloat16).contiguous()
             b32 = None if bias is None else bias.detach().to(torch.float32).contiguous()
             out = torch.empty((B, T, J), dtype=out_dtype, device=dev)
-            err = torch.zeros(32, dtype=torch.int32, device=dev)
+            err = _error_word(dev)
             rc = lib.frnn_b200_input_projection(
                 x16.data_ptr(), w16.data_ptr(), None if b32 is None else b32.data_ptr(), out.data_ptr(),
                 int(out_dtype == torch.bfloat16), B, T, J, I, err.data_ptr(), torch.cuda.current_stream(dev).cuda_stream)
@@ -68,6 +68,8 @@ def input_projection(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch
         raise ValueError("the projection kernel needs I % 8 == 0 and G*N*D % 64 == 0")
     if out_dtype not in (torch.bfloat16, torch.float32):
         raise ValueError("out_dtype must be bfloat16 or float32")
+    if not torch.is_autocast_enabled("cuda"):
+        return _Projection.apply(x, weight, bias, out_dtype)
     with torch.autocast("cuda", enabled=False):
         return _Projection.apply(x, weight, bias, out_dtype)
 
