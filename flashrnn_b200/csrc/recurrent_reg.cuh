@@ -98,6 +98,69 @@ __device__ __forceinline__ void sts_f32(uint32_t a, float v) { asm volatile("st.
 __device__ __forceinline__ void sts_u16(uint32_t a, uint32_t v) { asm volatile("st.shared.u16 [%0], %1;" ::"r"(a), "h"(static_cast<uint16_t>(v)) : "memory"); }
 __device__ __forceinline__ uint32_t bf16_bits(float v) { return static_cast<uint32_t>(__bfloat16_as_ushort(__float2bfloat16_rn(v))); }
 
+// The first of two operand buffers [column tile][k][8 batch rows] from the initial states (row 0 of the head, `row` floats from batch row
+// to batch row), the second one zero. A word is two batch rows of one k; neighbouring threads take neighbouring k.
+template <int NB, int KT>
+__device__ __forceinline__ void reg_fill_operand(uint8_t* buf, const float* initial, size_t row, int b0, int B, int K, int tid, int threads) {
+  constexpr int kWords = NB * KT * 64;
+#pragma unroll 4
+  for (int i = tid; i < kWords; i += threads) {
+    const int k = i % (KT * 16), pair = i / (KT * 16), b = b0 + 2 * pair;  // pair: column tile * 4 + rows of it / 2
+    const float* const src = initial + static_cast<size_t>(b) * row + k;
+    const float lo = k < K && b < B ? __ldg(src) : 0.0f, hi = k < K && b + 1 < B ? __ldg(src + row) : 0.0f;
+    reinterpret_cast<uint32_t*>(buf)[(pair >> 2) * (KT * 64) + k * 4 + (pair & 3)] = pack_bf16x2(lo, hi);
+  }
+  for (int i = tid; i < kWords / 4; i += threads) reinterpret_cast<uint4*>(buf + kWords * 4)[i] = make_uint4(0u, 0u, 0u, 0u);
+}
+
+// A fragments of a 16-row tile, K k of which count. Row r of the tile is `base` + (r / UPW) * gate + (r % UPW) * stride (elements) while
+// its gate r / UPW < GR, else zeros. Rows on the 16-byte grid come 64 k at a time through 2 KB of the warp's own shared memory:
+// 4 loads, 4 stores and an ldmatrix per k tile, where word by word a thread has four loads per k tile, all of them
+// unrolled. Prologue in cycles, word by word / this: LSTM D256 N3 13.0 k / 10.5 k, D128 N4 9.0 k / 5.8 k, D768 8.9 k / 6.5 k; LSTM B4 T16
+// N1 D768 38.2 us / 37.4.
+constexpr int kRegScratch = 2048;
+template <int KT, int UPW, int GR>
+__device__ __forceinline__ void reg_load_rows(const __nv_bfloat16* base, size_t gate, size_t stride, int K, uint32_t scratch, int lane,
+                                              bool aligned, uint32_t (&a)[KT][4]) {
+  if (aligned) {
+    constexpr int CHUNKS = (KT + 3) / 4;
+    const int r0 = lane >> 3, col = lane & 7;  // this lane's piece: rows r0 + 4 j, 8 k
+    uint4 v[CHUNKS][4];
+#pragma unroll
+    for (int m = 0; m < CHUNKS; ++m)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int g = 4 * j / UPW, u = UPW == 4 ? r0 : r0 + 4 * (j & 1);
+        v[m][j] = g < GR && m * 64 + col * 8 < K ? __ldg(reinterpret_cast<const uint4*>(base + g * gate + u * stride + m * 64 + col * 8))
+                                                 : make_uint4(0u, 0u, 0u, 0u);
+      }
+#pragma unroll
+    for (int m = 0; m < CHUNKS; ++m) {
+      __syncwarp();
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int r = r0 + 4 * j;
+        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(scratch + r * 128 + ((col ^ (r & 7)) << 4)), "r"(v[m][j].x), "r"(v[m][j].y),
+                     "r"(v[m][j].z), "r"(v[m][j].w) : "memory");
+      }
+      __syncwarp();
+      const int r = ((lane >> 3) & 1) * 8 + (lane & 7);
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (4 * m + i < KT) ldsm_x4(scratch + r * 128 + (((2 * i + (lane >> 4)) ^ (r & 7)) << 4), a[4 * m + i]);
+    }
+  } else {
+    const int q = lane >> 2, c = lane & 3;
+#pragma unroll
+    for (int kt = 0; kt < KT; ++kt)
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        const int row = q + 8 * (r & 1), g = row / UPW, k = kt * 16 + 8 * (r >> 1) + 2 * c;
+        a[kt][r] = g < GR && k < K ? __ldg(reinterpret_cast<const uint32_t*>(base + g * gate + row % UPW * stride + k)) : 0u;
+      }
+  }
+}
+
 // Four neighbouring lanes hold one 16-byte packet, a word each: afterwards every lane holds all of it.
 __device__ __forceinline__ void gather_quad(uint32_t a, int lane, uint32_t (&pk)[4]) {
   const uint32_t b1 = __shfl_xor_sync(0xffffffffu, a, 1);

@@ -22,6 +22,7 @@
 // Elman B16 N12 D64 0.52 against 0.66. A wait of its own for the Wx tile cost 150 cycles more (D256: 0.85 us).
 #pragma once
 
+#include <algorithm>
 #include <type_traits>
 
 #include "recurrent_reg.cuh"
@@ -98,16 +99,8 @@ frnn_fwd_reg_kernel(const FwdParams p, const __grid_constant__ CUtensorMap wx_ma
     fence_mbar_init();
     tma_prefetch_desc(&wx_map);
   }
-  // operand buffer 0 = round_bf16(initial h), zero for rows past the batch and k past the head
-  for (int i = tid; i < 2 * kHbuf / 4; i += blockDim.x) {
-    const int half = i / (kHalf / 4) % NB, k = i % (kHalf / 4) >> 2, b = b0 + half * 8 + 2 * (i & 3);
-    uint32_t v = 0u;
-    if (k < D) {
-      const float* src = p.initial + (static_cast<size_t>(b) * N + n) * D + k;
-      v = pack_bf16x2(b < B ? src[0] : 0.0f, b + 1 < B ? src[static_cast<size_t>(N) * D] : 0.0f);
-    }
-    reinterpret_cast<uint32_t*>(hbuf)[i] = v;
-  }
+  // operand buffer 0 = round_bf16(initial h), zero for rows past the batch and k past the head; buffer 1 zero
+  reg_fill_operand<NB, KT>(hbuf, p.initial + static_cast<size_t>(n) * D, static_cast<size_t>(N) * D, b0, B, D, tid, blockDim.x);
   __syncthreads();
   const uint32_t h_tx = static_cast<uint32_t>(D) * ROWS * 2u;
   if (tid == 0 && !LOCAL) {
@@ -174,14 +167,9 @@ frnn_fwd_reg_kernel(const FwdParams p, const __grid_constant__ CUtensorMap wx_ma
     const int d = rank * U + ul;     // ... and inside the head
     auto item_row = [&](int i) { return i / IT * 8 + 2 * c + (UPW == 4 ? hi : i % IT); };
     uint32_t a[KT][4];
-#pragma unroll
-    for (int kt = 0; kt < KT; ++kt)
-#pragma unroll
-      for (int r = 0; r < 4; ++r) {
-        const int g = UPW == 4 ? 2 * (r & 1) + hi : r & 1, k = kt * 16 + 8 * (r >> 1) + 2 * c;
-        a[kt][r] = (g < CT::GR && k < D)
-            ? __ldg(reinterpret_cast<const uint32_t*>(p.R + ((static_cast<size_t>(g) * N + n) * D + d) * D + k)) : 0u;
-      }
+    // The I/O warp of a cluster asks for the first tiles after the cluster has met: the ring is scratch until then.
+    reg_load_rows<KT, UPW, CT::GR>(p.R + (static_cast<size_t>(n) * D + rank * U + warp * UPW) * D, static_cast<size_t>(N) * D * D, D, D,
+                                   smem_u32(wxs) + warp * kRegScratch, lane, !LOCAL && (reinterpret_cast<uintptr_t>(p.R) & 15u) == 0, a);
 
     const size_t ND = static_cast<size_t>(N) * D;
     bool act[NI];
@@ -466,7 +454,8 @@ int launch_fwd_reg(const FwdParams& p, const void* wx, int wx_bf16, cudaStream_t
   const int out_step = plane * (hist_states * hes + (has_cache ? CT::GC * CT::CES : 0) + (p.hbf != nullptr ? 2 : 0));
   constexpr int fixed = reg_round_1k(2 * NB * KT * 16 * 16);
   const int steps = reg_transfer_steps(fixed, stage + chunks * out_step, Cfg::MIN_BLOCKS);
-  const int smem = fixed + reg_round_1k(kRegSlots * steps * stage) + kRegSlots * chunks * reg_round_1k(steps * out_step);
+  const int ring = reg_round_1k(kRegSlots * steps * stage) + kRegSlots * chunks * reg_round_1k(steps * out_step);
+  const int smem = fixed + std::max(ring, LOCAL ? 0 : (Cfg::THREADS / 32 - 1) * kRegScratch);
   if (smem > kRegSmemLimit) return kRegNoRoom;
   // bulk stores start on 16-byte boundaries; the tcgen05 kernels write these outputs with plain stores
   if (((reinterpret_cast<uintptr_t>(p.history) | reinterpret_cast<uintptr_t>(p.cache) | reinterpret_cast<uintptr_t>(p.hbf)) & 15u) != 0)

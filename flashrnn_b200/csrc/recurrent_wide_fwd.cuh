@@ -18,6 +18,7 @@
 // Bound: the serial chain of a step. FIGURES
 #pragma once
 
+#include <algorithm>
 #include <type_traits>
 
 #include "recurrent_reg.cuh"
@@ -92,16 +93,8 @@ frnn_fwd_wide_kernel(const FwdParams p, const __grid_constant__ CUtensorMap wx_m
     fence_mbar_init();
     tma_prefetch_desc(&wx_map);
   }
-  // operand buffer 0 = round_bf16(initial h) of the chunk, zero for rows past the batch and k past the chunk (there in both buffers)
-  for (int i = tid; i < 2 * Cfg::HBUF / 4; i += blockDim.x) {
-    const int half = i / (Cfg::HALF / 4) % NB, k = i % (Cfg::HALF / 4) >> 2, b = b0 + half * 8 + 2 * (i & 3);
-    uint32_t v = 0u;
-    if (k < Kc) {
-      const float* src = p.initial + (static_cast<size_t>(b) * N + n) * D + ks * Kc + k;
-      v = pack_bf16x2(b < B ? src[0] : 0.0f, b + 1 < B ? src[static_cast<size_t>(N) * D] : 0.0f);
-    }
-    reinterpret_cast<uint32_t*>(hbuf)[i] = v;
-  }
+  // operand buffer 0 = round_bf16(initial h) of the chunk, zero for rows past the batch and k past the chunk; buffer 1 zero
+  reg_fill_operand<NB, KT>(hbuf, p.initial + static_cast<size_t>(n) * D + ks * Kc, static_cast<size_t>(N) * D, b0, B, Kc, tid, blockDim.x);
   __syncthreads();
   if (tid == 0) {
     mbar_arrive_expect_tx(smem_u32(&s_part_bar[0]), Cfg::PART);
@@ -150,14 +143,9 @@ frnn_fwd_wide_kernel(const FwdParams p, const __grid_constant__ CUtensorMap wx_m
     __syncwarp();
   } else {
     uint32_t a[KT][4];
-#pragma unroll
-    for (int kt = 0; kt < KT; ++kt)
-#pragma unroll
-      for (int r = 0; r < 4; ++r) {
-        const int g = 2 * (r & 1) + hi, k = kt * 16 + 8 * (r >> 1) + 2 * c;
-        a[kt][r] = (g < CT::GR && k < Kc)
-            ? __ldg(reinterpret_cast<const uint32_t*>(p.R + ((static_cast<size_t>(g) * N + n) * D + rt * 32 + warp * 4 + uq) * D + ks * Kc + k)) : 0u;
-      }
+    // the ring is scratch until the cluster has met
+    reg_load_rows<KT, 4, CT::GR>(p.R + (static_cast<size_t>(n) * D + rt * 32 + warp * 4) * D + ks * Kc, static_cast<size_t>(N) * D * D, D, Kc,
+                                 smem_u32(wxs) + warp * kRegScratch, lane, (reinterpret_cast<uintptr_t>(p.R) & 15u) == 0, a);
 
     // the item of a thread of an owner warp: one unit of one batch row
     const size_t ND = static_cast<size_t>(N) * D;
@@ -386,8 +374,9 @@ int launch_fwd_wide(const FwdParams& p, const void* wx, int wx_bf16, cudaStream_
   const int hist_states = p.output_mode == 0 ? CT::S : (p.output_mode == 1 ? 1 : 0);
   const bool has_cache = p.cache != nullptr && CELL != kElman;
   constexpr int steps = 4;
-  const int smem = Cfg::FIXED + kRegSlots * (reg_round_1k(steps * CT::GW * plane * es) + reg_round_1k(steps * plane * hist_states * hes) +
+  const int ring = kRegSlots * (reg_round_1k(steps * CT::GW * plane * es) + reg_round_1k(steps * plane * hist_states * hes) +
                                              reg_round_1k(has_cache ? steps * plane * CT::GC * CT::CES : 0) + (p.hbf != nullptr ? reg_round_1k(steps * plane * 2) : 0));
+  const int smem = Cfg::FIXED + std::max(ring, 8 * kRegScratch);
   if (smem > kRegSmemLimit) return kRegNoRoom;
   if (((reinterpret_cast<uintptr_t>(p.history) | reinterpret_cast<uintptr_t>(p.cache) | reinterpret_cast<uintptr_t>(p.hbf)) & 15u) != 0)
     return kRegNoRoom;  // bulk stores start on 16-byte boundaries

@@ -14,7 +14,6 @@ namespace frnn {
 
 namespace {
 
-constexpr int kThreads = 128;
 constexpr int kKC = 64;  // (b,t) rows per shared-memory chunk
 
 struct WgradParams {
@@ -27,133 +26,21 @@ struct WgradParams {
   int ksplit;
   int chunks_per_split;
   int pack;     // heads that share one 64-wide TMA box (narrow heads, D = 16 or 32), else 1
-  // Row window (TMA kernel, pack == 1): the contraction produces only the rows o in [m_off, m_off + Dm) of every
+  int npt;      // tiles of NP columns that cover D
+  // Row window (pack == 1): the contraction produces only the rows o in [m_off, m_off + Dm) of every
   // gate (a rank's units of a row-sharded head) and writes them as [GR][N][out_rows][D] starting at `out`.
-  // Dm = out_rows = D and m_off = 0 describe the whole matrix.
+  // Dm is a multiple of 64; rows o >= out_rows are not stored. Dm = D rounded up, out_rows = D and m_off = 0 describe the
+  // whole matrix.
   int Dm, m_off, out_rows;
 };
 
-// Both operands are MN-major (the contraction index is the slow one in memory). Un-swizzled
-// canonical tiles: 8(k) x 8(mn) core matrices of 128 bytes, k-groups 128 B apart, mn-groups
-// 1024 B apart.
-__global__ void __launch_bounds__(kThreads, 1) wgrad_kernel(const WgradParams p) {
-  extern __shared__ __align__(1024) uint8_t smem[];
-  __shared__ __align__(8) uint64_t s_bar;
-  __shared__ uint32_t s_tmem_base;
-  const int tid = threadIdx.x, warp = tid >> 5;
-  const int D = p.D, N = p.N, T = p.T, GR = p.GR, NP = p.NP;
-  const int npt = D / NP;
-  const int mtile = blockIdx.x / npt, ptile = blockIdx.x % npt;
-  const int n = blockIdx.y, split = blockIdx.z;
-  const int m0 = mtile * 128, p0 = ptile * NP;
-  const int M = GR * D;
-  const long long K = static_cast<long long>(p.B) * T;
-  uint8_t* const sA = smem;               // 16 mn-groups * 1024
-  uint8_t* const sB = smem + 16 * 1024;   // NP/8 mn-groups * 1024
-  uint32_t tmem_cols = 32;
-  while (tmem_cols < static_cast<uint32_t>(NP)) tmem_cols <<= 1;
-
-  if (tid == 0) {
-    mbar_init(smem_u32(&s_bar), 1);
-    fence_mbar_init();
-  }
-  if (warp == 0) {
-    tmem_alloc(smem_u32(&s_tmem_base), tmem_cols);
-    tmem_relinquish_alloc();
-  }
-  tc_fence_before_sync();
-  __syncthreads();
-  tc_fence_after_sync();
-  const uint32_t tbase = s_tmem_base;
-  const uint32_t idesc = umma_idesc_bf16(128, NP, true, true);
-  const int c_begin = split * p.chunks_per_split;
-  const long long total_chunks = (K + kKC - 1) / kKC;
-  int c_end = c_begin + p.chunks_per_split;
-  if (c_end > total_chunks) c_end = static_cast<int>(total_chunks);
-  bool ok = true;
-  int issued = 0;
-  for (int c = c_begin; c < c_end; ++c) {
-    const long long k0 = static_cast<long long>(c) * kKC;
-    // A chunk: dg^T [128 m x 64 k]
-    for (int v = tid; v < kKC * 16; v += kThreads) {
-      const int k = v >> 4, mg = v & 15;
-      const int m = m0 + mg * 8;
-      const long long kt = k0 + k;
-      uint4 val = make_uint4(0u, 0u, 0u, 0u);
-      if (m < M && kt < K) {
-        const int g = m / D, o = m % D;
-        val = __ldg(reinterpret_cast<const uint4*>(p.dgr + ((kt * GR + g) * N + n) * D + o));
-      }
-      *reinterpret_cast<uint4*>(sA + mg * 1024 + (k >> 3) * 128 + (k & 7) * 16) = val;
-    }
-    // B chunk: round_bf16(h_{t-1}) [NP p x 64 k]
-    const int pgs = NP / 8;
-    for (int v = tid; v < kKC * pgs; v += kThreads) {
-      const int k = v / pgs, pg = v % pgs;
-      const long long kt = k0 + k;
-      uint4 val = make_uint4(0u, 0u, 0u, 0u);
-      if (kt < K) {
-        const long long b = kt / T, t = kt % T;
-        val = __ldg(reinterpret_cast<const uint4*>(p.hbf + ((b * (T + 1) + t) * N + n) * D + p0 + pg * 8));
-      }
-      *reinterpret_cast<uint4*>(sB + pg * 1024 + (k >> 3) * 128 + (k & 7) * 16) = val;
-    }
-    fence_proxy_async_smem();
-    __syncthreads();
-    if (tid == 0) {
-      tc_fence_after_sync();
-      for (int kk = 0; kk < kKC / 16; ++kk) {
-        const uint64_t ad = umma_smem_desc(smem_u32(sA) + kk * 256, 128, 1024);
-        const uint64_t bd = umma_smem_desc(smem_u32(sB) + kk * 256, 128, 1024);
-        umma_bf16_ss(tbase, ad, bd, idesc, (issued > 0 || kk > 0) ? 1u : 0u);
-      }
-      umma_commit(smem_u32(&s_bar));
-    }
-    ok = mbar_wait_bounded<false, true>(smem_u32(&s_bar), issued & 1, 2000000000ull, p.err);
-    ++issued;
-    if (!ok) break;
-  }
-  if (!ok && tid == 0) {
-    atomicCAS(p.err, 0, kErrWaitMma);
-    // the chunk whose commit was not seen may still be on the tensor core: wait for it once more (no abort
-    // flag: the commit completes by itself) before the tensor memory is released below
-    mbar_wait_bounded<false, true>(smem_u32(&s_bar), (issued - 1) & 1, 2000000000ull, nullptr);
-  }
-  tc_fence_after_sync();
-  // epilogue: accumulator rows -> global (row = (g, o), contiguous along p)
-  {
-    const int m = m0 + tid;
-    float* dst = nullptr;
-    if (m < M) {
-      const int g = m / D, o = m % D;
-      dst = p.out + static_cast<size_t>(split) * GR * N * D * D + ((static_cast<size_t>(g) * N + n) * D + o) * D + p0;
-    }
-    for (int c8 = 0; c8 < NP; c8 += 8) {
-      uint32_t r[8];
-      if (issued > 0 && ok) {
-        tmem_ld_x8(tmem_addr(tbase, 32 * warp, c8), r);
-        tmem_ld_wait();
-      } else {
-#pragma unroll
-        for (int q = 0; q < 8; ++q) r[q] = 0u;
-      }
-      if (dst != nullptr) {
-        *reinterpret_cast<float4*>(dst + c8) = make_float4(__uint_as_float(r[0]), __uint_as_float(r[1]), __uint_as_float(r[2]), __uint_as_float(r[3]));
-        *reinterpret_cast<float4*>(dst + c8 + 4) = make_float4(__uint_as_float(r[4]), __uint_as_float(r[5]), __uint_as_float(r[6]), __uint_as_float(r[7]));
-      }
-    }
-  }
-  tc_fence_before_sync();
-  __syncthreads();
-  if (warp == 0) tmem_dealloc(tbase, tmem_cols);
-}
-
-// ---------------------------------------------------------------------------------------------
-// Pipelined variant for D % 64 == 0: operands arrive by TMA (128-byte swizzle, 64 x 64 boxes)
-// through a 4-stage ring; warp 0 = TMA producer, warp 1 = UMMA issuer, warps 2-5 = epilogue.
-// A stage holds 64 (b,t) rows: A = dg^T [128 m x 64 k] as two boxes, B = h~ [NP p x 64 k] as
-// NP/64 boxes. A chunk never straddles a batch row; rows past T read as zeros on the dg side.
-// ---------------------------------------------------------------------------------------------
+// Operands arrive by TMA (128-byte swizzle, 64 x 64 boxes) through a 4-stage ring; warp 0 = TMA producer, warp 1 = UMMA
+// issuer, warps 2-5 = epilogue. A stage holds 64 (b,t) rows: A = dg^T [128 m x 64 k] as two boxes, B = h~ [NP p x 64 k] as
+// NP/64 boxes. A chunk never straddles a batch row; rows past T read as zeros on the dg side. A width that is no multiple of
+// 64 is rounded up to whole boxes: what they reach past a head is filled with zeros and not stored.
+// Us with the reductions, against the plain-load kernel that such widths (and 320, 448, 640, whose equal tiles were no whole boxes)
+// had, one chunk at a time: GRU B13 T333 N2 D208 22.9 / 55.6, LSTM B16 T256 N16 D48 20.0 / 76.0, B32 T512 N2 D320 66 / 1079, B96
+// T256 N8 D176 91 / 1705, B8 T1024 N1 D640 58 / 851.
 constexpr int kTmaThreads = 192;
 constexpr int kTmaStages = 4;
 
@@ -167,7 +54,7 @@ wgrad_tma_kernel(const WgradParams p, const __grid_constant__ CUtensorMap dgr_ma
   __shared__ uint32_t s_tmem_base;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int D = p.D, T = p.T, GR = p.GR, NP = p.NP;
-  const int npt = p.pack > 1 ? 1 : D / NP;
+  const int npt = p.npt;
   const int mtile = blockIdx.x / npt, ptile = blockIdx.x % npt;
   const int n = blockIdx.y, split = blockIdx.z;
   const int m0 = mtile * 128, p0 = ptile * NP;
@@ -272,12 +159,12 @@ wgrad_tma_kernel(const WgradParams p, const __grid_constant__ CUtensorMap dgr_ma
     tc_fence_after_sync();
     if (pack == 1) {
       float* dst = nullptr;
-      if (m < M) {
+      if (m < M && m % Dm < p.out_rows) {
         const int g = m / Dm, o = m % Dm;
         dst = p.out + static_cast<size_t>(split) * GR * p.N * p.out_rows * D +
               ((static_cast<size_t>(g) * p.N + n) * p.out_rows + o) * D + p0;
       }
-      for (int c8 = 0; c8 < NP; c8 += 8) {
+      for (int c8 = 0; c8 < NP && p0 + c8 < D; c8 += 8) {
         uint32_t r[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
         if (have) {
           tmem_ld_x8(tmem_addr(tbase, 32 * q, c8), r);
@@ -346,24 +233,19 @@ __global__ void reduce_parts_strided_kernel(const float* __restrict__ parts, flo
 
 }  // namespace
 
-// The TMA kernel needs whole 64-element boxes along both output dimensions; heads of 16 or 32
-// units are packed 4 or 2 to a box.
-static bool wgrad_uses_tma(int D, int np) { return D % 64 == 0 && np % 64 == 0; }
+// Heads of 16 or 32 units are packed 4 or 2 to a box of 64.
 static int wgrad_pack(int D) { return (D == 16 || D == 32) ? 64 / D : 1; }
 
 int wgrad_plan(int gr, int B, int T, int N, int D, int* np_out, int* ksplit_out, int* cps_out) {
-  // column tiles: the fewest equal parts of D that are at most 256 wide and a multiple of 16
   if (D % 16 != 0) return -2;
-  int npt = (D + 255) / 256;
-  while (D % npt != 0 || (D / npt) % 16 != 0) ++npt;
   const int pack = wgrad_pack(D);
-  const int np = pack > 1 ? 64 : D / npt;
-  const int mtiles = pack > 1 ? (gr + 1) / 2 : (gr * D + 127) / 128;
+  // column tiles: the fewest of at most 256 columns, whole boxes of 64 each
+  const int boxes = (D + 63) / 64, npt = (boxes + 3) / 4;
+  const int np = pack > 1 ? 64 : (boxes + npt - 1) / npt * 64;
+  const int mtiles = pack > 1 ? (gr + 1) / 2 : (gr * boxes * 64 + 127) / 128;
   const long long tiles = pack > 1 ? static_cast<long long>(mtiles) * ((N + pack - 1) / pack)
                                    : static_cast<long long>(mtiles) * npt * N;
-  const long long chunks = (pack > 1 || wgrad_uses_tma(D, np))
-                               ? static_cast<long long>(B) * ((T + kKC - 1) / kKC)   // per batch row
-                               : (static_cast<long long>(B) * T + kKC - 1) / kKC;
+  const long long chunks = static_cast<long long>(B) * ((T + kKC - 1) / kKC);   // per batch row
   long long ks = 148 / tiles;
   if (ks < 1) ks = 1;
   if (ks > 32) ks = 32;
@@ -387,11 +269,12 @@ int wgrad_launch(int gr, int gb, const __nv_bfloat16* dgr, const __nv_bfloat16* 
   p.err = err;
   p.B = B; p.T = T; p.N = N; p.D = D; p.GR = gr;
   p.NP = np; p.ksplit = ksplit; p.chunks_per_split = cps;
-  p.Dm = D; p.m_off = 0; p.out_rows = D;
-  const int pack = wgrad_pack(D);
+  const int pack = wgrad_pack(D), boxes = (D + 63) / 64;
+  p.Dm = boxes * 64; p.m_off = 0; p.out_rows = D;
   p.pack = pack;
-  const int mtiles = pack > 1 ? (gr + 1) / 2 : (gr * D + 127) / 128;
-  dim3 grid(static_cast<unsigned>(pack > 1 ? mtiles : mtiles * (D / np)),
+  p.npt = pack > 1 ? 1 : (D + np - 1) / np;
+  const int mtiles = pack > 1 ? (gr + 1) / 2 : (gr * boxes * 64 + 127) / 128;
+  dim3 grid(static_cast<unsigned>(mtiles * p.npt),
             static_cast<unsigned>(pack > 1 ? (N + pack - 1) / pack : N), static_cast<unsigned>(ksplit));
   cudaError_t e;
   if (pack > 1) {
@@ -407,7 +290,7 @@ int wgrad_launch(int gr, int gb, const __nv_bfloat16* dgr, const __nv_bfloat16* 
     e = cudaFuncSetAttribute(wgrad_tma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return static_cast<int>(e);
     wgrad_tma_kernel<<<grid, kTmaThreads, smem, s>>>(p, dgr_map, hbf_map);
-  } else if (wgrad_uses_tma(D, np)) {
+  } else {
     CUtensorMap dgr_map, hbf_map;
     const uint64_t ddims[5] = {static_cast<uint64_t>(D), static_cast<uint64_t>(N), static_cast<uint64_t>(gr),
                                static_cast<uint64_t>(T), static_cast<uint64_t>(B)};
@@ -421,11 +304,6 @@ int wgrad_launch(int gr, int gb, const __nv_bfloat16* dgr, const __nv_bfloat16* 
     e = cudaFuncSetAttribute(wgrad_tma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return static_cast<int>(e);
     wgrad_tma_kernel<<<grid, kTmaThreads, smem, s>>>(p, dgr_map, hbf_map);
-  } else {
-    const int smem = 16 * 1024 + (np / 8) * 1024;
-    e = cudaFuncSetAttribute(wgrad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return static_cast<int>(e);
-    wgrad_kernel<<<grid, kThreads, smem, s>>>(p);
   }
   e = cudaGetLastError();
   if (e != cudaSuccess) return static_cast<int>(e);
@@ -452,6 +330,7 @@ int wgrad_launch_rows(int gr, int gb, const __nv_bfloat16* dgr, const __nv_bfloa
   p.dgr = dgr; p.hbf = hbf; p.out = dR; p.err = err;
   p.B = B; p.T = T; p.N = 1; p.D = D; p.GR = gr;
   p.NP = 256; p.ksplit = 1;
+  p.npt = D / 256;
   p.chunks_per_split = B * ((T + kKC - 1) / kKC);
   p.pack = 1;
   p.Dm = Dm; p.m_off = m_off; p.out_rows = out_rows;
