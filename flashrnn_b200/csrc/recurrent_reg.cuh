@@ -1,10 +1,15 @@
-// Shape rules and device helpers of the register-resident recurrence kernels (recurrent_reg_fwd.cu, recurrent_reg_bwd.cu).
+// Shape rules and device helpers of the register-resident recurrence kernels (recurrent_reg_fwd.cuh, recurrent_reg_bwd.cuh).
 //
 // A step of a narrow head is a product of a [GR*U x D] slice of R with a [D x 8] operand: 8 batch rows, one warp-level
 // m16n8k16 column tile. tcgen05.mma spends about 79 cycles per 128x16x16 instruction whatever the 8 columns need, and its
 // result comes back through tensor memory and shared memory (commit, tcgen05.ld, gate buffer, barrier). Here the slice of
 // R lives in the registers of the warps as mma.sync fragments for the whole sequence, the accumulators of a unit's gates
 // land in the registers of the thread that runs the cell, and nothing but the operand itself passes through shared memory.
+//
+// A warp has 4 units (a 16-row tile holds their four gates), so that a thread has one item (unit, batch row) per column tile and an SM
+// sub-partition two warps: a lone warp issues an instruction every 4.5 cycles, and of 8 units per warp the cell, the staging and the
+// publication were twice as many instructions on the chain of a step (LSTM B8 N3 D256, us per step forward / backward: 0.80 / 0.89
+// against 0.64 / 0.66).
 #pragma once
 
 #include "frnn_common.cuh"
@@ -17,11 +22,10 @@ constexpr int kRegNoRoom = -100;      // not taken: too many waves, or outputs o
 constexpr int kRegTaken = -101;       // answer to a question: the call would run here
 
 // Widths of these kernels: all multiples of 16 up to 256, multiples of 32 up to 512. One CTA holds a head of 16, 32 or 48 units
-// whole; other widths run as a cluster of CTAs with 32 units (the forward also with 16), the last of which has 16 units where D is
-// an odd multiple of 16.
-// At 64 units one CTA's warps share the schedulers and its I/O warp moves two 32-unit tiles per step: LSTM, 8
-// rows, fp32 Wx, 0.85 + 1.19 us per step forward + backward against 0.63 + 0.68 as a cluster of two; Elman, 16 rows x 12
-// heads, 0.76 + 0.81 us.
+// whole; other widths run as a cluster of CTAs with 32 units, the last of which has 16 units where D is an odd multiple of 16.
+// At 64 units one CTA's warps would share the schedulers and its I/O warp move two 32-unit tiles per step: with 8 units per warp, LSTM, 8
+// rows, fp32 Wx, 0.85 + 1.19 us per step forward + backward against 0.63 + 0.68 as a cluster of two. CTAs of 16 units (clusters of
+// 16 at 256) were no faster either: forward 0.68 against 0.67.
 inline bool reg_width(int D) { return D % 16 == 0 && (D <= 256 || (D % 32 == 0 && D <= 512)); }
 inline bool reg_local(int D) { return D < 64; }
 
@@ -30,7 +34,7 @@ inline int reg_batch_tiles(int B, int rows) { return (B + rows - 1) / rows; }
 // time), multiples of 4 from 288 units on (fewer instantiations; the tiles past the head are zero).
 inline int reg_k_tiles(int D) { return reg_local(D) ? D / 16 : (D <= 256 ? (D + 31) / 32 * 2 : (D + 63) / 64 * 4); }
 
-// Staged tiles (Wx, cache, states, gradients): per chunk of units of the CTA (32, or 16 in a CTA of 16 units) and per plane (gate or
+// Staged tiles (Wx, cache, states, gradients): per chunk of 32 units of the CTA (wide heads: the units it owns) and per plane (gate or
 // state) the batch rows of the group, rows of 32, 64 or 128 bytes under the TMA swizzle of that span. The threads of a warp
 // read 4 units of 8 rows at once: un-swizzled these rows would share their banks.
 constexpr int kRegChunk = 32;

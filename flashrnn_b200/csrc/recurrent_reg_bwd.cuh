@@ -1,7 +1,7 @@
 // Reverse-time recurrence of narrow heads with R in the register file (see recurrent_reg.cuh).
 //
-// Groups, CTAs and the unit each thread owns are those of recurrent_reg_fwd.cu. Per step t a thread
-//   1. adds up the partial dh_t of its unit and two batch rows (fixed order), the external gradient and the pointwise
+// Groups, CTAs and the items of a thread are those of recurrent_reg_fwd.cuh (4 units a warp for every cell). Per step t a thread
+//   1. adds up the partial dh_t of its items (fixed order), the external gradient and the pointwise
 //      carry, runs the cell backward and writes round_bf16(dg_t) to shared memory for ldmatrix (one CTA barrier),
 //   2. multiplies with its warp's fragments of R_slice^T [D x GR*U] (rows = units p of h_{t-1}, k = gate rows of this CTA),
 //   3. hands the accumulators to the owners of those units: two lanes swap halves so that each packet is 4 batch rows of
@@ -9,8 +9,8 @@
 // The sums of step 2 run over the same gate rows in the same order as in the tcgen05 kernels, whose CTAs own 32 units (16
 // where the width is not a multiple of 32), and step 1 adds them in the same order: every gradient is the same bits, whichever
 // kernels a call takes.
-//   LOCAL: D / 16 row tiles for D / 8 warps. 16 and 32 units: one sum per tile, which half of the warps run; 48 units: three
-//          "sources" of 16 units each, two for the first half of the warps and one for the second.
+//   LOCAL: D / 16 row tiles for D / 4 warps. 16 and 32 units: one sum per tile, which the first warps run; 48 units: three
+//          "sources" of 16 units each, a warp for each of the nine (tile, sum) pairs.
 //   else:  the sources are the CTAs of the cluster, packets travel by st.async. HALVES (odd multiples of 16): two sums per
 //          tile, one for each 16 units of the CTA; the last CTA has units, and a sum, in its first half only.
 // The state of step t - 1 stays in registers as the new state of the next iteration, and only the planes that the cell's
@@ -20,9 +20,12 @@
 // sums of a parity are overwritten only after the CTA barrier of the step that read them; a TMA stage is refilled by the I/O
 // warp after every warp has staged its outputs of the step that used it.
 //
-// Bound: the serial chain of a step. LSTM B8 N3 D256, 1513 cycles at 1845 MHz (see recurrent_reg_fwd.cu) = wait and reads 628 (the
-// wait alone 173) + cell and barrier 137 + mma and scatter 612 + staging 127; 0.88 us per step of the call against 1.32 of the
-// tcgen05 kernel; GRU B16 N24 D32 0.71 against 1.02; Elman B16 N12 D64 0.49 against 0.84; sLSTM B16 N4 D128 1.01 against 1.33.
+// Bound: the serial chain of a step, as in recurrent_reg_fwd.cuh. LSTM B8 N3 D256, cycles: tiles read, partial sums
+// awaited (316) and added 526, cell 83, staging 64, mma and scatter 442; the prologue is 9.5 k.
+// us per step before (8 units a warp, a transfer per step) and now: LSTM B8 N3 D256 0.89 / 0.66; LSTM B16 N4 D128 0.78 / 0.58; sLSTM
+// there 1.03 / 0.90 (its derivative is the longest); LSTM B8 N1 D64 fp32 0.70 / 0.62; GRU B16 N24 D32 0.71 / 0.46; Elman B16 N12 D64 0.49 /
+// 0.35. Against the tcgen05 kernels, which had these before: LSTM B256 N4 D128 (16 rows) 1.68 / 1.38; B8 N1 D384 1.61 / 0.85, D512 1.84 /
+// 1.45; B64 N3 D256 (24 rows) 1.77 / 1.06.
 #pragma once
 
 #include <type_traits>

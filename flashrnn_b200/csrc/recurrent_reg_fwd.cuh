@@ -1,25 +1,30 @@
 // Forward recurrence of narrow heads with R in the register file (see recurrent_reg.cuh).
 //
-// A group is one (head, 8 batch rows). Warp w of a CTA owns 8 hidden units and all of their gates: its rows of R are
-// m16n8k16 A fragments, two gates of the 8 units per 16-row tile, loaded once. Per step a warp reads the operand
-// round_bf16(h_{t-1}) with ldmatrix, multiplies, and each thread then holds the pre-activations of all gates of ONE unit
-// for two batch rows: it runs the cell on them in registers and publishes its two values of h_t.
-//   LOCAL: the CTA holds the whole head; h_t goes to the other half of a shared-memory double buffer, one mbarrier
-//          arrival per warp.
-//   else:  a cluster of ceil(D / 32) CTAs (an odd multiple of 16 leaves two warps of the last one without units); a quad of lanes packs the 8 batch rows of a unit into 16 bytes and sends them to
-//          every CTA of the cluster with st.async on the receiver's mbarrier.
+// A group is one (head, 8, 16 or 24 batch rows: NB column tiles). Warp w of a CTA owns 4 hidden units (Elman: 8) and all of their
+// gates: its rows of R are m16n8k16 A fragments, the four gates of 4 units per 16-row tile, loaded once. Per step a warp reads the
+// operand round_bf16(h_{t-1}) with ldmatrix, multiplies, and two lanes swap halves, so that each thread holds the pre-activations of
+// all gates of ONE item (unit, batch row) per column tile: it runs the cell on them in registers and publishes its value of h_t.
+//   LOCAL: the CTA holds the whole head; h_t goes to the other half of a shared-memory double buffer, one CTA barrier a step.
+//   else:  a cluster of ceil(D / 32) CTAs (an odd multiple of 16 leaves four warps of the last one without units); the word of two
+//          batch rows of a unit goes to every CTA of the cluster with st.async on the receiver's mbarrier, half of the peers from
+//          either lane of the pair. Packets of 16 bytes, put together by a quad of lanes, were 3 to 8 % slower on every cell but the
+//          Elman with more than four peers (GATHER).
 // One more warp moves data: TMA tiles of Wx in, staged outputs (history, gate cache, bf16 h) out, both under the swizzle
-// that lets 8 units x 4 batch rows be read and written without bank conflicts. The compute warps' own stores of these
-// outputs cost 800 cycles per step in address arithmetic and partial-line stores, their own TMA issue about as much.
+// that lets units x batch rows be read and written without bank conflicts, several steps per transfer (reg_transfer_steps). The
+// compute warps' own stores of these outputs cost 800 cycles per step in address arithmetic and partial-line stores, their own
+// TMA issue about as much. The loop over the steps is compiled for the outputs that the call has (kRegTrain, kRegPlain, kRegAny):
+// flags and offsets at run time were 5 to 25 % of a step.
 //
 // A group cannot overtake itself: a half of the operand double buffer is written again only after every warp has published
 // the step in between, and a warp publishes after its own reads of that half.
 //
-// Bound: the serial chain of a step, mostly instruction issue and mma latency of one warp per scheduler: at LSTM B8 N3 D256, 1326
-// cycles = operand wait 149 + Wx read and 32 mma 522 + cell 136 + publication 195 + staging of the outputs 324. The SM runs these at
-// 1845 MHz (clock64 against globaltimer; the driver shows 1965), 0.71 us; the rest of the call's 0.79 us per step is the prologue
-// (16 k cycles) and the launch. Per step there, against the tcgen05 kernel: 0.79 us against 1.30; GRU B16 N24 D32 0.58 against 0.68;
-// Elman B16 N12 D64 0.52 against 0.66. A wait of its own for the Wx tile cost 150 cycles more (D256: 0.85 us).
+// Bound: the serial chain of a step: instruction issue (4.5 cycles for each instruction of a lone warp), mma latency (24 cycles a
+// dependent pair, 13 to 14.5 of a scheduler each), DSMEM flight (400), one successful mbarrier wait (150 to 180). LSTM B8 N3 D256, cycles: Wx read
+// and operand wait 268, ldmatrix and mma 433, cell 107, publication 242, staging 201; the prologue is 10 k.
+// us per step before (8 units a warp, packets, a transfer per step) and now, kernel and prologue: LSTM B8 N3 D256 0.80 / 0.64; LSTM
+// B16 N4 D128 0.71 / 0.50; sLSTM there 0.85 / 0.59; LSTM B8 N1 D64 fp32 0.64 / 0.42; GRU B16 N24 D32 0.58 / 0.30; Elman B16 N12 D64
+// 0.53 / 0.34. Against the tcgen05 kernels, which had these before: LSTM B256 N4 D128 (16 rows) 1.30 / 1.03; B8 N1 D384 1.68 / 0.78,
+// D512 2.07 / 1.10; B64 N3 D256 (24 rows) 1.47 / 0.97.
 #pragma once
 
 #include <algorithm>

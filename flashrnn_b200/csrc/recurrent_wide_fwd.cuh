@@ -15,7 +15,10 @@
 // latest, that one before the data of the step after it, whose reader fences by step t + 2 * kWideFence + 1, long before it polls the
 // refilled slot at step t + kWideSlots / 2. So no reader can take old data of a slot for new.
 //
-// Bound: the serial chain of a step. FIGURES
+// Bound: the serial chain of a step, two hops of it: LSTM B16 N1 D768 (KS = 2), cycles: h_t of the other CTAs polled 1075, ldmatrix, mma
+// and partial gates sent 755, wait for the partial gates and their sum 583, cell and publication 227, staging 224. us per step of the
+// tensor-memory kernel and here: there 2.31 / 1.73, B4 (KS = 4) 2.12 / 1.62; D1024 B8 2.35 / 1.71. What went: tcgen05.mma, its commit and
+// tcgen05.ld (950 cycles against 300 of mma.sync), a fence per step (now one in kWideFence), scattered output stores.
 #pragma once
 
 #include <algorithm>
@@ -424,6 +427,8 @@ int launch_fwd_wide_k(const FwdParams& p, const void* wx, int wx_bf16, cudaStrea
   }
   if (kt <= 24) return launch_fwd_wide<CELL, KS, NB, 24>(p, wx, wx_bf16, s);
   if (kt <= 28) return launch_fwd_wide<CELL, KS, NB, 28>(p, wx, wx_bf16, s);
+  // 128 of the 168 registers (nine warps) are fragments, some of the rest are spilled: still LSTM B16 N1 D1024 2.65 / 2.06 us per step
+  if (kt <= 32) return launch_fwd_wide<CELL, KS, NB, 32>(p, wx, wx_bf16, s);
   return kRegNoRoom;
 }
 
