@@ -40,15 +40,13 @@ def _stream(device: torch.device) -> int:
     return torch._C._cuda_getCurrentRawStream(device.index)
 
 
-def _raise_device_error(err: torch.Tensor, what) -> None:
-    """``err`` is one launch's word (``what`` its name) or a block of them, a row each (``what``: the names)."""
-    rows, names = ([err.tolist()], [what]) if err.ndim == 1 else (err.tolist(), what)
-    for row, name in zip(rows, names):
-        code, step, cta = row[:3]
-        if code != 0:
-            raise RuntimeError(
-                f"{name}: device-side wait ran out (code {code}: {_lib.ERROR_TEXT.get(code, '?')}, step {step}, CTA {cta})"
-            )
+def _raise_device_error(row, what: str) -> None:
+    """``row``: the words of a launch, on the host."""
+    code, step, cta = row[:3]
+    if code != 0:
+        raise RuntimeError(
+            f"{what}: device-side wait ran out (code {code}: {_lib.ERROR_TEXT.get(code, '?')}, step {step}, CTA {cta})"
+        )
 
 
 class _ErrorBlock:
@@ -150,20 +148,27 @@ def poll_errors(block: bool = False) -> None:
             if block.closed == block.given:       # nothing on the way: blocks of finished threads and old streams go
                 del _blocks[key]
     keep = []
-    while _pending_errors:
-        ev, err, what = _pending_errors.pop(0)
-        if block:
-            ev.synchronize()
-        if ev.query():
-            _raise_device_error(err, what)
-        else:
-            keep.append((ev, err, what))
-    _pending_errors.extend(keep)
+    try:
+        while _pending_errors:
+            ev, err, what = _pending_errors.pop(0)
+            if block:
+                ev.synchronize()
+            if not ev.query():
+                keep.append((ev, err, what))
+                continue
+            # the word of one launch, or a block of them with a row each: the rows behind one that raises wait for the next look
+            rows, names = ([err.tolist()], [what]) if err.ndim == 1 else (err.tolist(), what)
+            for i, (row, name) in enumerate(zip(rows, names)):
+                if row[0] != 0 and i + 1 < len(rows):
+                    keep.append((ev, err[i + 1:], what[i + 1:]))
+                _raise_device_error(row, name)
+    finally:
+        _pending_errors.extend(keep)
     if block and _captured_errors:
         for device in {err.device for err, _ in _captured_errors}:
             torch.cuda.synchronize(device)
         for err, what in _captured_errors:
-            _raise_device_error(err, what + " (in a replayed CUDA graph)")
+            _raise_device_error(err.tolist(), what + " (in a replayed CUDA graph)")
 
 
 class _Recurrence(torch.autograd.Function):

@@ -151,3 +151,37 @@ def test_error_polling_on_the_host(monkeypatch):
     monkeypatch.setattr(torch.cuda, "synchronize", lambda device=None: None)
     with pytest.raises(RuntimeError, match="captured launch.*replayed CUDA graph"):
         F.poll_errors(block=True)
+
+
+def test_every_failed_launch_is_reported(monkeypatch):
+    """One look raises the first error it finds; the words behind it, in the same block and in other entries, finished or not, are
+    there for the next one."""
+    from flashrnn_b200 import functional as F
+
+    class _Event:
+        done = True
+        def synchronize(self): self.done = True
+        def query(self): return self.done
+
+    running = _Event()
+    running.done = False
+    words = torch.zeros((5, 32), dtype=torch.int32)
+    words[1, :3] = torch.tensor([101, 7, 3])
+    words[4, :3] = torch.tensor([106, 2, 9])
+    alone = torch.tensor([103, 1, 1] + [0] * 29, dtype=torch.int32)
+    monkeypatch.setattr(F, "_captured_errors", [])
+    monkeypatch.setattr(F, "_blocks", {})
+    monkeypatch.setattr(F, "_last_poll", 0.0)
+    monkeypatch.setattr(F, "_pending_errors", [(running, torch.zeros(32, dtype=torch.int32), "running"),
+                                               (_Event(), words, [f"launch {i}" for i in range(5)]), (_Event(), alone, "alone")])
+    with pytest.raises(RuntimeError, match="launch 1: .*code 101.*step 7, CTA 3"):
+        F.poll_errors()
+    assert "running" in [what for _, _, what in F._pending_errors]
+    reports = []
+    for _ in range(2):
+        with pytest.raises(RuntimeError) as e:
+            F.poll_errors(block=True)
+        reports.append(str(e.value))
+    assert sorted(r.split(":")[0] for r in reports) == ["alone", "launch 4"], reports
+    F.poll_errors(block=True)
+    assert F._pending_errors == []
