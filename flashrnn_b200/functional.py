@@ -268,8 +268,8 @@ class _Recurrence(torch.autograd.Function):
             _lib.CELLS[cell], dgr.data_ptr(), hbf.data_ptr(), db_part.data_ptr(), dR.data_ptr(), db.data_ptr(),
             _ptr(work), B, T, N, D, err.data_ptr(), stream,
         )
+        _track(err, "frnn_b200_backward")   # the first launch has the word, whether the second was accepted or not
         _lib.check(rc, "frnn_b200_wgrad")
-        _track(err, "frnn_b200_backward")
         need = ctx.needs_input_grad
         return (
             dwx if need[0] else None,

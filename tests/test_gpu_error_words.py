@@ -80,3 +80,31 @@ def test_threads_and_streams_have_blocks_of_their_own(cuda_device):
     assert not errors and len({w.data_ptr() for w in words}) == 200
     with pytest.raises(RuntimeError, match="c30: .*code 103"):
         F.poll_errors(block=True)
+
+
+def test_word_of_a_backward_whose_contraction_was_refused(cuda_device, monkeypatch):
+    """The recurrence runs with the word, so no later launch may get it, and what it reports is found."""
+    from flashrnn_b200 import _lib, flashrnn_torch
+    from flashrnn_b200 import functional as F
+    from flashrnn_b200.workloads import make_inputs
+
+    lib = _lib.load()
+
+    class Refuses:
+        def __getattr__(self, name):
+            return (lambda *args: -2) if name == "frnn_b200_wgrad" else getattr(lib, name)
+
+    given, inner = [], F._error_word
+    monkeypatch.setattr(F, "_error_word", lambda device: given.append(inner(device)) or given[-1])
+    wx, R, b, init = (t.to(cuda_device).requires_grad_(True) for t in make_inputs("lstm", 2, 3, 1, 64, 5))
+    history, _ = flashrnn_torch(wx, R, b, init, cell="lstm", numerics="fp32_state_bf16_mma")
+    monkeypatch.setattr(_lib, "load", Refuses)
+    with pytest.raises(RuntimeError, match="frnn_b200_wgrad failed"):
+        F._Recurrence._backward(history.grad_fn, torch.ones_like(history), None)
+    assert len(given) == 2                             # forward, backward
+    later = inner(torch.device("cuda", torch.cuda.current_device()))
+    assert later.data_ptr() not in [w.data_ptr() for w in given]
+    F._track(later, "later")
+    given[1][0] = 106
+    with pytest.raises(RuntimeError, match="frnn_b200_backward: .*code 106"):
+        F.poll_errors(block=True)
