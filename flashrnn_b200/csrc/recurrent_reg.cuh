@@ -153,6 +153,9 @@ __device__ __forceinline__ void reg_load_rows(const __nv_bfloat16* base, size_t 
       for (int i = 0; i < 4; ++i)
         if (4 * m + i < KT) ldsm_x4(scratch + r * 128 + (((2 * i + (lane >> 4)) ^ (r & 7)) << 4), a[4 * m + i]);
     }
+    // TMA writes these bytes next: ordinary accesses and those of the async proxy are ordered by a proxy fence, which the caller's
+    // cluster barrier alone is not.
+    fence_proxy_async_smem();
   } else {
     const int q = lane >> 2, c = lane & 3;
 #pragma unroll
