@@ -338,10 +338,10 @@ extern "C" int frnn_b200_plan(int cell, int B, int T, int N, int D, frnn_b200_pl
     out->supported = fwd_ok && bwd_ok;
     const int64_t fwd_groups = static_cast<int64_t>(N) * ((B + out->fwd_batch_tile - 1) / out->fwd_batch_tile);
     const int64_t bwd_groups = static_cast<int64_t>(N) * out->n_btiles;
-    // four operand slots of 16 rows (tensor-memory kernels) or one of the group's rows per step, up to kWideSlots (registers)
-    const int64_t slots = wide_slots(T);
+    // Four operand slots of 16 rows (tensor-memory kernels) or kWideSlots of the group's rows (registers). Whatever T is: a caller that
+    // runs a sequence in pieces sizes the scratch once.
     const auto operand = [&](int ksplit, int tile, int64_t k) {
-      const int64_t four = 4ll * bt * k * 2, wide = ksplit ? slots * tile * k * 2 : 0;
+      const int64_t four = 4ll * bt * k * 2, wide = ksplit ? static_cast<int64_t>(kWideSlots) * tile * k * 2 : 0;
       return four > wide ? four : wide;
     };
     const int64_t fwd_b = operand(out->fwd_ksplit, out->fwd_batch_tile, D);

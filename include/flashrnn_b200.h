@@ -60,7 +60,8 @@ typedef struct frnn_b200_plan {
   int exchange;          /* 0: CTAs of a group exchange through cluster shared memory;
                             1: group wider than a cluster (D > 512): through global memory;
                             2: as 1, with 16-unit slices in the backward (768 < D)           */
-  int64_t xchg_bytes;    /* scratch for exchange >= 1 (forward and backward), else 0      */
+  int64_t xchg_bytes;    /* scratch for exchange >= 1 (forward and backward), else 0; does
+                            not depend on T                                               */
   int fwd_ksplit;        /* 0, or 2/4: the forward splits the contraction of a 32-unit row
                             tile over this many CTAs (a cluster) and exchanges h through
                             global memory                                                  */

@@ -185,3 +185,10 @@ def test_every_failed_launch_is_reported(monkeypatch):
     assert sorted(r.split(":")[0] for r in reports) == ["alone", "launch 4"], reports
     F.poll_errors(block=True)
     assert F._pending_errors == []
+
+
+@pytest.mark.parametrize("cell,B,N,D", [("lstm", 1, 1, 576), ("lstm", 16, 1, 768), ("slstm", 9, 1, 1024), ("gru", 8, 1, 1280), ("elman", 30, 2, 640)])
+def test_exchange_scratch_does_not_depend_on_the_length(cell, B, N, D):
+    """A caller that runs a sequence in pieces sizes the scratch from the plan of any of them: it has to do for the longest."""
+    sizes = {_lib.plan(cell, B, T, N, D).xchg_bytes for T in (1, 5, 64, 65, 1000)}
+    assert len(sizes) == 1 and sizes.pop() > 0
