@@ -277,15 +277,18 @@ int wgrad_launch(int gr, int gb, const __nv_bfloat16* dgr, const __nv_bfloat16* 
   dim3 grid(static_cast<unsigned>(mtiles * p.npt),
             static_cast<unsigned>(pack > 1 ? (N + pack - 1) / pack : N), static_cast<unsigned>(ksplit));
   cudaError_t e;
+  // The maps of h end at T: slot T of a batch row, h_T, belongs to no product. A last chunk would multiply it with the zeros that stand
+  // for the steps past T, which is no zero where h_T is not finite.
   if (pack > 1) {
     CUtensorMap dgr_map, hbf_map;
     const uint64_t ddims[4] = {static_cast<uint64_t>(N) * D, static_cast<uint64_t>(gr), static_cast<uint64_t>(T),
                                static_cast<uint64_t>(B)};
     const uint32_t dbox[4] = {64u, 1u, static_cast<uint32_t>(kKC), 1u};
-    const uint64_t hdims[3] = {static_cast<uint64_t>(N) * D, static_cast<uint64_t>(T + 1), static_cast<uint64_t>(B)};
+    const uint64_t hdims[3] = {static_cast<uint64_t>(N) * D, static_cast<uint64_t>(T), static_cast<uint64_t>(B)};
+    const uint64_t hstride[3] = {static_cast<uint64_t>(N) * D, static_cast<uint64_t>(T + 1), static_cast<uint64_t>(B)};
     const uint32_t hbox[3] = {64u, static_cast<uint32_t>(kKC), 1u};
     if (make_tensor_map(&dgr_map, dgr, 2, 4, ddims, dbox, true) != 0) return -4;
-    if (make_tensor_map(&hbf_map, hbf, 2, 3, hdims, hbox, true) != 0) return -4;
+    if (make_tensor_map(&hbf_map, hbf, 2, 3, hdims, hbox, true, hstride) != 0) return -4;
     const int smem = kTmaStages * (16384 + 64 * 128) + 1024;
     e = cudaFuncSetAttribute(wgrad_tma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return static_cast<int>(e);
@@ -295,11 +298,11 @@ int wgrad_launch(int gr, int gb, const __nv_bfloat16* dgr, const __nv_bfloat16* 
     const uint64_t ddims[5] = {static_cast<uint64_t>(D), static_cast<uint64_t>(N), static_cast<uint64_t>(gr),
                                static_cast<uint64_t>(T), static_cast<uint64_t>(B)};
     const uint32_t dbox[5] = {64u, 1u, 1u, static_cast<uint32_t>(kKC), 1u};
-    const uint64_t hdims[4] = {static_cast<uint64_t>(D), static_cast<uint64_t>(N), static_cast<uint64_t>(T + 1),
-                               static_cast<uint64_t>(B)};
+    const uint64_t hdims[4] = {static_cast<uint64_t>(D), static_cast<uint64_t>(N), static_cast<uint64_t>(T), static_cast<uint64_t>(B)};
+    const uint64_t hstride[4] = {static_cast<uint64_t>(D), static_cast<uint64_t>(N), static_cast<uint64_t>(T + 1), static_cast<uint64_t>(B)};
     const uint32_t hbox[4] = {64u, 1u, static_cast<uint32_t>(kKC), 1u};
     if (make_tensor_map(&dgr_map, dgr, 2, 5, ddims, dbox, true) != 0) return -4;
-    if (make_tensor_map(&hbf_map, hbf, 2, 4, hdims, hbox, true) != 0) return -4;
+    if (make_tensor_map(&hbf_map, hbf, 2, 4, hdims, hbox, true, hstride) != 0) return -4;
     const int smem = kTmaStages * (16384 + np * 128) + 1024;
     e = cudaFuncSetAttribute(wgrad_tma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return static_cast<int>(e);
