@@ -258,10 +258,9 @@ int wgrad_plan(int gr, int B, int T, int N, int D, int* np_out, int* ksplit_out,
   return 0;
 }
 
-int wgrad_launch(int gr, int gb, const __nv_bfloat16* dgr, const __nv_bfloat16* hbf, const float* db_part, int n_btiles,
-                 float* dR, float* db, float* work, int* err, int B, int T, int N, int D, cudaStream_t s) {
-  int np, ksplit, cps;
-  if (wgrad_plan(gr, B, T, N, D, &np, &ksplit, &cps) != 0) return -2;
+static int wgrad_launch_split(int gr, int gb, const __nv_bfloat16* dgr, const __nv_bfloat16* hbf, const float* db_part, int n_btiles,
+                              float* dR, float* db, float* work, int* err, int B, int T, int N, int D, int np, int ksplit, int cps,
+                              cudaStream_t s) {
   if (ksplit > 1 && work == nullptr) return -5;
   WgradParams p{};
   p.dgr = dgr; p.hbf = hbf;
@@ -319,6 +318,13 @@ int wgrad_launch(int gr, int gb, const __nv_bfloat16* dgr, const __nv_bfloat16* 
   const long long nb = static_cast<long long>(gb) * N * D;
   reduce_parts_kernel<<<static_cast<unsigned>((nb / 4 + 255) / 256), 256, 0, s>>>(db_part, db, nb, n_btiles);
   return static_cast<int>(cudaGetLastError());
+}
+
+int wgrad_launch(int gr, int gb, const __nv_bfloat16* dgr, const __nv_bfloat16* hbf, const float* db_part, int n_btiles,
+                 float* dR, float* db, float* work, int* err, int B, int T, int N, int D, cudaStream_t s) {
+  int np, ksplit, cps;
+  if (wgrad_plan(gr, B, T, N, D, &np, &ksplit, &cps) != 0) return -2;
+  return wgrad_launch_split(gr, gb, dgr, hbf, db_part, n_btiles, dR, db, work, err, B, T, N, D, np, ksplit, cps, s);
 }
 
 // Row-sharded wide head (one head, N = 1): dR[g, o, p] for the rows o in [m_off, m_off + Dm) only, from this
@@ -404,12 +410,19 @@ int wgrad_launch_static(int gr, int gb, const __nv_bfloat16* dgr, const __nv_bfl
                         int n_btiles, float* dR, float* db, int* err, int B, int T, int N, int D, cudaStream_t s) {
   int np, ksplit, cps;
   if (wgrad_plan(gr, B, T, N, D, &np, &ksplit, &cps) != 0) return -2;
-  const size_t need = ksplit > 1 ? static_cast<size_t>(ksplit) * gr * N * D * D * sizeof(float) : 0;
-  if (need > kStaticWorkBytes) return -6;
+  const size_t part = static_cast<size_t>(gr) * N * D * D * sizeof(float);
+  if (ksplit > 1 && ksplit * part > kStaticWorkBytes) {
+    // Widths of whole 256-column tiles are refused, as plan.wgrad_work_bytes tells their caller. The tiles of other widths are rounded up,
+    // hence fewer, and may split further than the array has room for (LSTM D736: 72 tiles, two parts, 17.3 MB): less far then.
+    if (D % 256 == 0) return -6;
+    const int chunks = B * ((T + kKC - 1) / kKC), room = static_cast<int>(kStaticWorkBytes / part), parts = room < 1 ? 1 : room;
+    cps = (chunks + parts - 1) / parts;
+    ksplit = (chunks + cps - 1) / cps;
+  }
   float* work = nullptr;
   const int rc = static_work_address(&work);
   if (rc != 0) return rc;
-  return wgrad_launch(gr, gb, dgr, hbf, db_part, n_btiles, dR, db, work, err, B, T, N, D, s);
+  return wgrad_launch_split(gr, gb, dgr, hbf, db_part, n_btiles, dR, db, work, err, B, T, N, D, np, ksplit, cps, s);
 }
 
 }  // namespace frnn

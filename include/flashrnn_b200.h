@@ -189,8 +189,8 @@ int frnn_b200_wgrad(int cell, const void* dgr, const void* hbf, const float* db_
  * memory budget fixed at start-up, or thin plugins that only ever see input and output pointers.
  * This entry point has no counterpart in the reference. The split-K partial tiles go to a fixed
  * 16 MiB array inside the library image (each GPU that loads the library holds it until the
- * process exits); the call returns -6 when plan.wgrad_work_bytes exceeds that. It allocates
- * nothing. The first call on a device looks up the array's device address (a one-time set-up
+ * process exits). Where plan.wgrad_work_bytes exceeds that the call returns -6 if D is a multiple
+ * of 256, and uses fewer, larger partial sums else. It allocates nothing. The first call on a device looks up the array's device address (a one-time set-up
  * that should happen before any stream capture starts). All calls on a device share the array:
  * calls that overlap on the GPU race with each other; consecutive calls on one stream are safe,
  * and no clearing is needed because every partial tile is rewritten before it is reduced. */

@@ -192,3 +192,20 @@ def test_exchange_scratch_does_not_depend_on_the_length(cell, B, N, D):
     """A caller that runs a sequence in pieces sizes the scratch from the plan of any of them: it has to do for the longest."""
     sizes = {_lib.plan(cell, B, T, N, D).xchg_bytes for T in (1, 5, 64, 65, 1000)}
     assert len(sizes) == 1 and sizes.pop() > 0
+
+
+@pytest.mark.skipif(torch.cuda.is_available(), reason="the call is made with pointers to nothing")
+def test_allocation_free_contraction_refuses_whole_tiles_only():
+    """-6 comes before any CUDA call; every other width gets as far as the missing device."""
+    lib = _lib.load()
+
+    def refused(cell, B, T, N, D):
+        return lib.frnn_b200_wgrad_noalloc(_lib.CELLS[cell], 16, 16, 16, 16, 16, B, T, N, D, 16, None) == -6
+
+    for cell in ("lstm", "slstm", "gru", "elman"):
+        for D in range(16, 1793, 16):
+            for N in (1, 2, 3, 4, 6, 9):
+                plan = _lib.plan(cell, 8, 300, N, D)
+                if plan.supported:
+                    assert refused(cell, 8, 300, N, D) == (D % 256 == 0 and plan.wgrad_work_bytes > 16 << 20), (cell, N, D)
+    assert refused("lstm", 8, 1024, 3, 256) and not refused("lstm", 8, 300, 1, 736) and not refused("elman", 8, 300, 1, 1472)

@@ -101,3 +101,28 @@ def test_noalloc_rejects_oversized_problem(cuda_device):
     rc = lib.frnn_b200_wgrad_noalloc(_lib.CELLS[cell], one.data_ptr(), one.data_ptr(), one.data_ptr(), one.data_ptr(),
                                      one.data_ptr(), B, T, N, D, one.data_ptr(), 0)
     assert rc == -6
+
+
+@pytest.mark.parametrize("cell,N,D", [("lstm", 1, 736), ("elman", 4, 736), ("elman", 1, 1472)])
+def test_noalloc_splits_less_where_the_partial_sums_do_not_fit(cell, N, D, cuda_device):
+    """Widths whose column tiles are rounded up: the regular call splits further than 16 MiB hold, this one as far as they do."""
+    from flashrnn_b200 import _lib
+
+    lib, B, T = _lib.load(), 9, 67
+    plan = _lib.plan(cell, B, T, N, D)
+    assert plan.wgrad_work_bytes > 16 * 1024 * 1024
+    g = torch.Generator().manual_seed(D)
+    gr, gb = plan.gates_r, plan.gates_b
+    dgr = torch.randn((B, T, gr, N, D), generator=g).to(cuda_device).bfloat16()
+    hbf = torch.randn((B, T + 1, N, D), generator=g).to(cuda_device).bfloat16()
+    db_part = torch.randn((plan.n_btiles, gb, N, D), generator=g).to(cuda_device)
+    dR, db = torch.full((gr, N, D, D), float("nan"), device=cuda_device), torch.empty((gb, N, D), device=cuda_device)
+    err = torch.zeros(32, dtype=torch.int32, device=cuda_device)
+    rc = lib.frnn_b200_wgrad_noalloc(_lib.CELLS[cell], dgr.data_ptr(), hbf.data_ptr(), db_part.data_ptr(), dR.data_ptr(), db.data_ptr(),
+                                     B, T, N, D, err.data_ptr(), torch.cuda.current_stream(cuda_device).cuda_stream)
+    torch.cuda.synchronize()
+    assert rc == 0 and err[0].item() == 0
+    ref = torch.einsum("btgno,btnp->gnop", dgr.double(), hbf[:, :T].double())
+    mag = torch.einsum("btgno,btnp->gnop", dgr.double().abs(), hbf[:, :T].double().abs())
+    # fp32 sums of exact products of bf16 values: one rounding per term of a partial sum of at most `mag`
+    assert ((dR.double() - ref).abs() <= B * T * 2.0 ** -23 * mag).all()
