@@ -175,7 +175,8 @@ def plan(cell: str, B: int, T: int, N: int, D: int, device: int = None) -> Plan:
 
 
 def register_kernels(cell: str, wx_bf16: bool, B: int, N: int, D: int) -> tuple:
-    """(forward, backward): whether a training call of this shape keeps R in registers on the current CUDA device."""
+    """(forward, backward): whether a training call of this shape, of at most 256 units, keeps R in registers in groups of 8 batch
+    rows on the current CUDA device. ``register_rows`` answers for every width and group."""
     rc = load().frnn_b200_register_kernels(CELLS[cell], int(wx_bf16), B, N, D)
     if rc < 0:
         raise ValueError(f"frnn_b200_register_kernels failed: {ERROR_TEXT.get(rc, rc)}")
@@ -183,8 +184,8 @@ def register_kernels(cell: str, wx_bf16: bool, B: int, N: int, D: int) -> tuple:
 
 
 def register_rows(cell: str, wx_bf16: bool, B: int, N: int, D: int) -> tuple:
-    """(forward, backward): batch rows of a group of the kernels with R in registers that a training call of this shape takes
-    on the current CUDA device, 0 where it takes the kernels of the plan."""
+    """(forward, backward): batch rows of a group of the kernels with R in registers that a training call of this shape, of any
+    width, takes on the current CUDA device, 0 where it takes the tensor-memory kernels of the plan."""
     rc = load().frnn_b200_register_rows(CELLS[cell], int(wx_bf16), B, N, D)
     if rc < 0:
         raise ValueError(f"frnn_b200_register_rows failed: {ERROR_TEXT.get(rc, rc)}")

@@ -15,11 +15,12 @@ template <int CELL> int launch_fwd_reg_cell(const FwdParams& p, const void* wx, 
 template <int CELL>
 int launch_bwd_reg_cell(const BwdParams& p, const void* cache, const float* history, const float* initial, const float* d_history,
                         int wx_bf16, cudaStream_t s, int rows, bool ask);
-// The same for wide heads, with the groups and the split of the plan: launched, or kRegNoRoom.
+// The same for wide heads, with the groups and the split of the plan.
 template <int CELL>
 int launch_bwd_wide_cell(const BwdParams& p, const void* cache, const float* history, const float* initial, const float* d_history,
-                         int wx_bf16, int rows, int ksplit, cudaStream_t s);
-template <int CELL> int launch_fwd_wide_cell(const FwdParams& p, const void* wx, int wx_bf16, int rows, int ksplit, cudaStream_t s);
+                         int wx_bf16, int rows, int ksplit, cudaStream_t s, bool ask);
+template <int CELL>
+int launch_fwd_wide_cell(const FwdParams& p, const void* wx, int wx_bf16, int rows, int ksplit, cudaStream_t s, bool ask);
 int forward_ksplit_dispatch(int cell, const FwdParams& p, const void* wx, int wx_bf16, int bv, int ksplit, cudaStream_t s,
                             int* capacity_only);
 int forward_ksplit_capacity(int cell, int bv, int ksplit, int D);
@@ -202,23 +203,23 @@ int forward_reg_dispatch(int cell, const FwdParams& p, const void* wx, int wx_bf
   }
 }
 
-int forward_wide_dispatch(int cell, const FwdParams& p, const void* wx, int wx_bf16, int rows, int ksplit, cudaStream_t s) {
+int forward_wide_dispatch(int cell, const FwdParams& p, const void* wx, int wx_bf16, int rows, int ksplit, cudaStream_t s, bool ask) {
   switch (cell) {
-    case kLSTM: return launch_fwd_wide_cell<kLSTM>(p, wx, wx_bf16, rows, ksplit, s);
-    case kSLSTM: return launch_fwd_wide_cell<kSLSTM>(p, wx, wx_bf16, rows, ksplit, s);
-    case kGRU: return launch_fwd_wide_cell<kGRU>(p, wx, wx_bf16, rows, ksplit, s);
-    case kElman: return launch_fwd_wide_cell<kElman>(p, wx, wx_bf16, rows, ksplit, s);
+    case kLSTM: return launch_fwd_wide_cell<kLSTM>(p, wx, wx_bf16, rows, ksplit, s, ask);
+    case kSLSTM: return launch_fwd_wide_cell<kSLSTM>(p, wx, wx_bf16, rows, ksplit, s, ask);
+    case kGRU: return launch_fwd_wide_cell<kGRU>(p, wx, wx_bf16, rows, ksplit, s, ask);
+    case kElman: return launch_fwd_wide_cell<kElman>(p, wx, wx_bf16, rows, ksplit, s, ask);
     default: return -1;
   }
 }
 
 int backward_wide_dispatch(int cell, const BwdParams& p, const void* cache, const float* history, const float* initial,
-                           const float* d_history, int wx_bf16, int rows, int ksplit, cudaStream_t s) {
+                           const float* d_history, int wx_bf16, int rows, int ksplit, cudaStream_t s, bool ask) {
   switch (cell) {
-    case kLSTM: return launch_bwd_wide_cell<kLSTM>(p, cache, history, initial, d_history, wx_bf16, rows, ksplit, s);
-    case kSLSTM: return launch_bwd_wide_cell<kSLSTM>(p, cache, history, initial, d_history, wx_bf16, rows, ksplit, s);
-    case kGRU: return launch_bwd_wide_cell<kGRU>(p, cache, history, initial, d_history, wx_bf16, rows, ksplit, s);
-    case kElman: return launch_bwd_wide_cell<kElman>(p, cache, history, initial, d_history, wx_bf16, rows, ksplit, s);
+    case kLSTM: return launch_bwd_wide_cell<kLSTM>(p, cache, history, initial, d_history, wx_bf16, rows, ksplit, s, ask);
+    case kSLSTM: return launch_bwd_wide_cell<kSLSTM>(p, cache, history, initial, d_history, wx_bf16, rows, ksplit, s, ask);
+    case kGRU: return launch_bwd_wide_cell<kGRU>(p, cache, history, initial, d_history, wx_bf16, rows, ksplit, s, ask);
+    case kElman: return launch_bwd_wide_cell<kElman>(p, cache, history, initial, d_history, wx_bf16, rows, ksplit, s, ask);
     default: return -1;
   }
 }
@@ -369,7 +370,6 @@ extern "C" int frnn_b200_register_rows(int cell, int wx_bf16, int B, int N, int 
   const int rc = frnn_b200_plan(cell, B, 1, N, D, &plan);
   if (rc != 0) return rc;
   if (!plan.supported) return -2;
-  if (!reg_width(D)) return 0;
   FwdParams f{};
   f.B = B; f.T = 1; f.T_total = 1; f.N = N; f.D = D;
   f.cache = reinterpret_cast<void*>(16);  // a training call: cache and bf16 h are staged; never dereferenced
@@ -379,9 +379,15 @@ extern "C" int frnn_b200_register_rows(int cell, int wx_bf16, int B, int N, int 
   b.db_rows = plan.batch_tile;
   int answer = 0;
   for (int pass = 0; pass < 2; ++pass) {
+    const int ksplit = pass == 0 ? plan.fwd_ksplit : plan.bwd_ksplit, tile = pass == 0 ? plan.fwd_batch_tile : plan.batch_tile;
     for (int rows = kRegRows; rows <= kRegMaxRows; rows += kRegRows) {
-      const int v = pass == 0 ? forward_reg_dispatch(cell, f, nullptr, wx_bf16, nullptr, rows, true)
-                              : backward_reg_dispatch(cell, b, nullptr, nullptr, nullptr, nullptr, wx_bf16, nullptr, rows, true);
+      int v = kRegNoRoom;
+      if (reg_width(D))
+        v = pass == 0 ? forward_reg_dispatch(cell, f, nullptr, wx_bf16, nullptr, rows, true)
+                      : backward_reg_dispatch(cell, b, nullptr, nullptr, nullptr, nullptr, wx_bf16, nullptr, rows, true);
+      else if (ksplit != 0 && rows == tile)
+        v = pass == 0 ? forward_wide_dispatch(cell, f, nullptr, wx_bf16, rows, ksplit, nullptr, true)
+                      : backward_wide_dispatch(cell, b, nullptr, nullptr, nullptr, nullptr, wx_bf16, rows, ksplit, nullptr, true);
       if (v != kRegTaken && v != kRegNoRoom) return v > 0 ? -1000 - v : v;
       if (v == kRegTaken) {
         answer |= rows << (8 * pass);
@@ -440,7 +446,8 @@ int forward_common(int cell, const void* wx, int wx_bf16, const void* r_bf16, co
     if (!xchg) return -5;
     p.xg_data = static_cast<uint8_t*>(xchg);
     if (plan.fwd_ksplit) {
-      const int rc_wide = forward_wide_dispatch(cell, p, wx, wx_bf16, plan.fwd_batch_tile, plan.fwd_ksplit, static_cast<cudaStream_t>(stream));
+      const int rc_wide = forward_wide_dispatch(cell, p, wx, wx_bf16, plan.fwd_batch_tile, plan.fwd_ksplit, static_cast<cudaStream_t>(stream),
+                                                false);
       if (rc_wide != kRegNoRoom) return rc_wide;
     }
     // every exchange word starts as "not yet written" (all ones): four slots of 16 rows per group
@@ -540,7 +547,7 @@ extern "C" int frnn_b200_backward_ex(int cell, const void* cache, const float* h
     const size_t groups = static_cast<size_t>(N) * plan.n_btiles;
     if (plan.bwd_ksplit) {
       const int rc_wide = backward_wide_dispatch(cell, p, cache, history, initial, d_history, wx_bf16, plan.batch_tile, plan.bwd_ksplit,
-                                                 static_cast<cudaStream_t>(stream));
+                                                 static_cast<cudaStream_t>(stream), false);
       if (rc_wide != kRegNoRoom) return rc_wide;
     }
     // every exchange word starts as "not yet written": four slots of 16 rows of dG, or two of the partial dh of a group

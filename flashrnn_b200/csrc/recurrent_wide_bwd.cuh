@@ -464,7 +464,7 @@ frnn_bwd_wide_kernel(const BwdParams p, const float* history, const float* initi
 
 template <int CELL, int KS, int NB, int KT>
 int launch_bwd_wide(const BwdParams& p, const void* cache, const float* history, const float* initial, const float* d_history,
-                    int wx_bf16, cudaStream_t stream) {
+                    int wx_bf16, cudaStream_t stream, bool ask) {
   using Cfg = BwdWideCfg<CELL, KS, NB, KT>;
   using CT = CellTraits<CELL>;
   const bool own_dwx = !wx_bf16 || CELL == kGRU || p.dwx != static_cast<void*>(p.dgr);
@@ -496,7 +496,7 @@ int launch_bwd_wide(const BwdParams& p, const void* cache, const float* history,
   cfg.attrs = attr;
   cfg.numAttrs = 2;
   const int rc = reg_room(reinterpret_cast<const void*>(kern), cfg, KS, clusters, 0, D);
-  if (rc != 0) return rc;
+  if (rc != 0 || ask) return rc != 0 ? rc : kRegTaken;
   CUtensorMap cache_map, hist_map, dhist_map, dgr_map, dwx_map;
   const uint64_t nd = static_cast<uint64_t>(N) * D, uT = p.T, uB = p.B;
   const auto map = [&](CUtensorMap* m, const void* base, int es, int planes, uint64_t bs, uint64_t ps, uint64_t ss, int box_planes) {
@@ -523,6 +523,7 @@ struct BwdWideCall {
   const float *history, *initial, *d_history;
   int wx_bf16;
   cudaStream_t stream;
+  bool ask;
 };
 
 template <int CELL, int KS, int NB>
@@ -531,7 +532,7 @@ int launch_bwd_wide_k(const BwdWideCall& v) {
   if (kc % 16 != 0) return kRegNoRoom;
   const int kt = kc / 16;
   const auto go = [&](auto bound) {
-    return launch_bwd_wide<CELL, KS, NB, decltype(bound)::value>(v.p, v.cache, v.history, v.initial, v.d_history, v.wx_bf16, v.stream);
+    return launch_bwd_wide<CELL, KS, NB, decltype(bound)::value>(v.p, v.cache, v.history, v.initial, v.d_history, v.wx_bf16, v.stream, v.ask);
   };
   if (kt <= 12) return go(std::integral_constant<int, 12>{});
   if (kt <= 18) return go(std::integral_constant<int, 18>{});
@@ -546,11 +547,11 @@ int launch_bwd_wide_k(const BwdWideCall& v) {
 }  // namespace
 
 // The call of a plan with `ksplit` CTAs per tile of 128 units and `rows` batch rows per group, or kRegNoRoom (its fragments do not fit
-// the registers, outputs off the 16-byte grid, clusters that do not fit). Fills the exchange slots itself.
+// the registers, outputs off the 16-byte grid, clusters that do not fit). Fills the exchange slots itself. `ask`: only say whether (kRegTaken).
 template <int CELL>
 int launch_bwd_wide_cell(const BwdParams& p, const void* cache, const float* history, const float* initial, const float* d_history,
-                         int wx_bf16, int rows, int ksplit, cudaStream_t s) {
-  const BwdWideCall v{p, cache, history, initial, d_history, wx_bf16, s};
+                         int wx_bf16, int rows, int ksplit, cudaStream_t s, bool ask) {
+  const BwdWideCall v{p, cache, history, initial, d_history, wx_bf16, s, ask};
   if (ksplit == 8) return rows == 8 ? launch_bwd_wide_k<CELL, 8, 1>(v) : launch_bwd_wide_k<CELL, 8, 2>(v);
   if constexpr (CELL == kElman) {  // the other cells' chunks are wider than the registers hold
     if (ksplit == 4) return rows == 8 ? launch_bwd_wide_k<CELL, 4, 1>(v) : launch_bwd_wide_k<CELL, 4, 2>(v);

@@ -2,5 +2,5 @@
 #include "recurrent_wide_bwd.cuh"
 
 namespace frnn {
-template int launch_bwd_wide_cell<kElman>(const BwdParams&, const void*, const float*, const float*, const float*, int, int, int, cudaStream_t);
+template int launch_bwd_wide_cell<kElman>(const BwdParams&, const void*, const float*, const float*, const float*, int, int, int, cudaStream_t, bool);
 }  // namespace frnn

@@ -1,4 +1,4 @@
-// Forward recurrence of heads of 576 to 1792 units with R in the register file (see recurrent_reg.cuh, recurrent_reg_fwd.cuh).
+// Forward recurrence of heads of 576 to 1024 units with R in the register file (see recurrent_reg.cuh, recurrent_reg_fwd.cuh).
 //
 // The decomposition is that of recurrent_fwd_ksplit.cu: a group (head, 8 or 16 batch rows) is D/32 row tiles of 32 units times KS
 // chunks of the contraction, the KS CTAs of a tile are a cluster. Warp w of a CTA has the fragments of units 4w .. 4w + 3 of the
@@ -369,7 +369,7 @@ frnn_fwd_wide_kernel(const FwdParams p, const __grid_constant__ CUtensorMap wx_m
 }
 
 template <int CELL, int KS, int NB, int KT>
-int launch_fwd_wide(const FwdParams& p, const void* wx, int wx_bf16, cudaStream_t stream) {
+int launch_fwd_wide(const FwdParams& p, const void* wx, int wx_bf16, cudaStream_t stream, bool ask) {
   using Cfg = FwdWideCfg<CELL, KS, NB, KT>;
   using CT = CellTraits<CELL>;
   constexpr int plane = Cfg::ROWS * Cfg::CHUNK;
@@ -400,7 +400,7 @@ int launch_fwd_wide(const FwdParams& p, const void* wx, int wx_bf16, cudaStream_
   cfg.attrs = attr;
   cfg.numAttrs = 2;
   const int rc = reg_room(reinterpret_cast<const void*>(kern), cfg, KS, clusters, 0, p.D);
-  if (rc != 0) return rc;
+  if (rc != 0 || ask) return rc != 0 ? rc : kRegTaken;
   CUtensorMap map, hist_map, cache_map, hbf_map;
   const uint64_t nd = static_cast<uint64_t>(p.N) * p.D, T = p.T, Tt = p.T_total;
   const int end = p.t0 + p.T;  // steps past the call's own are neither read nor written
@@ -419,27 +419,28 @@ int launch_fwd_wide(const FwdParams& p, const void* wx, int wx_bf16, cudaStream_
 }
 
 template <int CELL, int KS, int NB>
-int launch_fwd_wide_k(const FwdParams& p, const void* wx, int wx_bf16, cudaStream_t s) {
+int launch_fwd_wide_k(const FwdParams& p, const void* wx, int wx_bf16, cudaStream_t s, bool ask) {
   const int kt = (p.D / KS + 15) / 16;
-  if constexpr (KS == 4) {
-    if (kt <= 12) return launch_fwd_wide<CELL, KS, NB, 12>(p, wx, wx_bf16, s);
-    if (kt <= 16) return launch_fwd_wide<CELL, KS, NB, 16>(p, wx, wx_bf16, s);
+  if constexpr (KS == 4) {  // D / 8 CTAs a group, all of them resident: 1056 units at most
+    if (kt <= 12) return launch_fwd_wide<CELL, KS, NB, 12>(p, wx, wx_bf16, s, ask);
+    if (kt <= 16) return launch_fwd_wide<CELL, KS, NB, 16>(p, wx, wx_bf16, s, ask);
+  } else {
+    if (kt <= 24) return launch_fwd_wide<CELL, KS, NB, 24>(p, wx, wx_bf16, s, ask);
+    if (kt <= 28) return launch_fwd_wide<CELL, KS, NB, 28>(p, wx, wx_bf16, s, ask);
+    // 128 of the 168 registers (nine warps) are fragments, some of the rest are spilled: still LSTM B16 N1 D1024 2.65 / 2.06 us per step
+    if (kt <= 32) return launch_fwd_wide<CELL, KS, NB, 32>(p, wx, wx_bf16, s, ask);
   }
-  if (kt <= 24) return launch_fwd_wide<CELL, KS, NB, 24>(p, wx, wx_bf16, s);
-  if (kt <= 28) return launch_fwd_wide<CELL, KS, NB, 28>(p, wx, wx_bf16, s);
-  // 128 of the 168 registers (nine warps) are fragments, some of the rest are spilled: still LSTM B16 N1 D1024 2.65 / 2.06 us per step
-  if (kt <= 32) return launch_fwd_wide<CELL, KS, NB, 32>(p, wx, wx_bf16, s);
   return kRegNoRoom;
 }
 
 }  // namespace
 
 // The call of a plan with `ksplit` CTAs per row tile and `rows` batch rows per group, or kRegNoRoom (its fragments do not fit the
-// registers, outputs off the 16-byte grid, clusters that do not fit). Fills the exchange slots itself.
+// registers, outputs off the 16-byte grid, clusters that do not fit). Fills the exchange slots itself. `ask`: only say whether (kRegTaken).
 template <int CELL>
-int launch_fwd_wide_cell(const FwdParams& p, const void* wx, int wx_bf16, int rows, int ksplit, cudaStream_t s) {
-  if (ksplit == 2) return rows == 8 ? launch_fwd_wide_k<CELL, 2, 1>(p, wx, wx_bf16, s) : launch_fwd_wide_k<CELL, 2, 2>(p, wx, wx_bf16, s);
-  if (ksplit == 4) return rows == 8 ? launch_fwd_wide_k<CELL, 4, 1>(p, wx, wx_bf16, s) : launch_fwd_wide_k<CELL, 4, 2>(p, wx, wx_bf16, s);
+int launch_fwd_wide_cell(const FwdParams& p, const void* wx, int wx_bf16, int rows, int ksplit, cudaStream_t s, bool ask) {
+  if (ksplit == 2) return rows == 8 ? launch_fwd_wide_k<CELL, 2, 1>(p, wx, wx_bf16, s, ask) : launch_fwd_wide_k<CELL, 2, 2>(p, wx, wx_bf16, s, ask);
+  if (ksplit == 4 && rows == 8) return launch_fwd_wide_k<CELL, 4, 1>(p, wx, wx_bf16, s, ask);  // where 16 rows fit so, 8 rows with ksplit 2 do
   return kRegNoRoom;
 }
 

@@ -2,5 +2,5 @@
 #include "recurrent_wide_fwd.cuh"
 
 namespace frnn {
-template int launch_fwd_wide_cell<kElman>(const FwdParams&, const void*, int, int, int, cudaStream_t);
+template int launch_fwd_wide_cell<kElman>(const FwdParams&, const void*, int, int, int, cudaStream_t, bool);
 }  // namespace frnn

@@ -16,7 +16,7 @@
  * flashrnn/flashrnn2/hybrid_fw2d.cu:85-89,366-373): if the caller sets err[3] = 1, CTA 0 adds up
  * SM clock cycles per phase over all steps into err[8..12] (epilogue warp: input wait, operand /
  * tensor-core wait, accumulator read, epilogue sync, cell + stores + exchange) and err[16..17]
- * (MMA warp: operand wait, issue). Kernels with R in registers (frnn_b200_register_kernels) use
+ * (MMA warp: operand wait, issue). Kernels with R in registers (frnn_b200_register_rows) use
  * forward err[16] operand wait, [17] Wx read and products, [12] cell, [13] publication, [14] staging;
  * backward err[9] wait and partial sums (wait alone: [13]), [10] cell, [12] products and scatter,
  * [11] staging, [15] the whole step.
@@ -82,14 +82,16 @@ int frnn_b200_version(void);
  * (flashrnn/flashrnn/flashrnn.py:383-677, cuda_init_parametric.py). D must be a multiple of 16. */
 int frnn_b200_plan(int cell, int B, int T, int N, int D, frnn_b200_plan_t* out);
 
-/* Which kernels a training call of this shape takes on the current device: bit 0 is set if the forward pass, bit 1 if the
- * backward pass keeps R in the registers of its warps (D <= 256, as long as its groups of 8 batch rows do not need too many waves); where a
- * bit is clear the kernels that frnn_b200_plan describes run, as they do for outputs that are not 16-byte aligned. Both
- * give the same results (db of 16-row batch tiles: up to rounding). Negative: a code as above, or -1000 - cudaError_t. */
+/* Whether a training call of at most 256 units takes the kernels with R in the registers of their warps, in groups of 8 batch
+ * rows, on the current device: bit 0 the forward, bit 1 the backward pass. 0 says nothing about wider groups and heads
+ * (always 0 beyond 256 units, answered without a device). Negative: a code as above, or -1000 - cudaError_t. */
 int frnn_b200_register_kernels(int cell, int wx_bf16, int B, int N, int D);
 
-/* The same for groups of 8, 16 or 24 batch rows and D <= 512: bits 0-7 the rows of a forward, bits 8-15 of a backward group;
- * 0 where the kernels that frnn_b200_plan describes run. Negative: as above. */
+/* Which kernels a training call takes on the current device, at any width: bits 0-7 the batch rows (8, 16 or 24) of a forward
+ * group, bits 8-15 of a backward group, of the kernels with R in registers (up to 512 units: a group is one CTA or one cluster;
+ * wider: clusters that exchange through global memory, with the split of frnn_b200_plan); 0 where the tensor-memory kernels
+ * that frnn_b200_plan describes run, as they do for outputs that are not 16-byte aligned. Both give the same results (db of
+ * 16-row batch tiles: up to rounding). Negative: as above. */
 int frnn_b200_register_rows(int cell, int wx_bf16, int B, int N, int D);
 
 /* Forward recurrence over T steps (flashrnn/flashrnn/fused/flashrnn.cc:69-145 forward();
