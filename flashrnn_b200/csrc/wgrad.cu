@@ -14,7 +14,18 @@ namespace frnn {
 
 namespace {
 
-constexpr int kKC = 64;  // (b,t) rows per shared-memory chunk
+constexpr int kKC = 64;  // (b,t) rows per shared-memory chunk: `tb` steps of kKC / tb batch rows
+
+// Steps of a chunk: 64, or the power of two that holds a shorter sequence.
+int chunk_steps(int T) {
+  int tb = kKC;
+  while (tb > 1 && tb / 2 >= T) tb /= 2;
+  return tb;
+}
+long long chunk_count(int B, int T) {
+  const int tb = chunk_steps(T), bb = kKC / tb;
+  return static_cast<long long>((B + bb - 1) / bb) * ((T + tb - 1) / tb);
+}
 
 struct WgradParams {
   const __nv_bfloat16* dgr;  // [B*T][GR][N][D]
@@ -27,6 +38,7 @@ struct WgradParams {
   int chunks_per_split;
   int pack;     // heads that share one 64-wide TMA box (narrow heads, D = 16 or 32), else 1
   int npt;      // tiles of NP columns that cover D
+  int tb;       // steps of a chunk
   // Row window (pack == 1): the contraction produces only the rows o in [m_off, m_off + Dm) of every
   // gate (a rank's units of a row-sharded head) and writes them as [GR][N][out_rows][D] starting at `out`.
   // Dm is a multiple of 64; rows o >= out_rows are not stored. Dm = D rounded up, out_rows = D and m_off = 0 describe the
@@ -36,8 +48,9 @@ struct WgradParams {
 
 // Operands arrive by TMA (128-byte swizzle, 64 x 64 boxes) through a 4-stage ring; warp 0 = TMA producer, warp 1 = UMMA
 // issuer, warps 2-5 = epilogue. A stage holds 64 (b,t) rows: A = dg^T [128 m x 64 k] as two boxes, B = h~ [NP p x 64 k] as
-// NP/64 boxes. A chunk never straddles a batch row; rows past T read as zeros on the dg side. A width that is no multiple of
-// 64 is rounded up to whole boxes: what they reach past a head is filled with zeros and not stored.
+// NP/64 boxes. A chunk is 64 steps of a batch row, or several batch rows of a sequence of up to 32 steps; rows past B or T read as
+// zeros. A width that is no multiple of 64 is rounded up to whole boxes: what they reach past a head is filled with zeros and
+// not stored.
 // Us with the reductions, against the plain-load kernel that such widths (and 320, 448, 640, whose equal tiles were no whole boxes)
 // had, one chunk at a time: GRU B13 T333 N2 D208 22.9 / 55.6, LSTM B16 T256 N16 D48 20.0 / 76.0, B32 T512 N2 D320 66 / 1079, B96
 // T256 N8 D176 91 / 1705, B8 T1024 N1 D640 58 / 851.
@@ -64,8 +77,9 @@ wgrad_tma_kernel(const WgradParams p, const __grid_constant__ CUtensorMap dgr_ma
   // tile holds pack x pack head blocks per gate of which only the diagonal ones are kept;
   // blockIdx.x = gate pair, blockIdx.y = head group.
   const int pack = p.pack;
-  const int cpb = (T + kKC - 1) / kKC;  // chunks per batch row
-  const int total_chunks = p.B * cpb;
+  const int tb = p.tb, bb = kKC / tb;   // steps and batch rows of a chunk
+  const int cpb = (T + tb - 1) / tb;    // chunks per bb batch rows
+  const int total_chunks = (p.B + bb - 1) / bb * cpb;
   const int c_begin = split * p.chunks_per_split;
   const int c_end = min(c_begin + p.chunks_per_split, total_chunks);
   const int n_chunks = max(c_end - c_begin, 0);
@@ -104,7 +118,7 @@ wgrad_tma_kernel(const WgradParams p, const __grid_constant__ CUtensorMap dgr_ma
           atomicCAS(p.err, 0, kErrWaitEmpty);
           break;
         }
-        const int b = c / cpb, t0 = (c % cpb) * kKC;
+        const int b = c / cpb * bb, t0 = c % cpb * tb;
         const uint32_t bar = smem_u32(&s_full[s]);
         const uint32_t sa = base + s * stage_bytes, sb = sa + 16384u;
         mbar_arrive_expect_tx(bar, stage_bytes);
@@ -245,7 +259,7 @@ int wgrad_plan(int gr, int B, int T, int N, int D, int* np_out, int* ksplit_out,
   const int mtiles = pack > 1 ? (gr + 1) / 2 : (gr * boxes * 64 + 127) / 128;
   const long long tiles = pack > 1 ? static_cast<long long>(mtiles) * ((N + pack - 1) / pack)
                                    : static_cast<long long>(mtiles) * npt * N;
-  const long long chunks = static_cast<long long>(B) * ((T + kKC - 1) / kKC);   // per batch row
+  const long long chunks = chunk_count(B, T);
   long long ks = 148 / tiles;
   if (ks < 1) ks = 1;
   if (ks > 32) ks = 32;
@@ -271,6 +285,8 @@ static int wgrad_launch_split(int gr, int gb, const __nv_bfloat16* dgr, const __
   const int pack = wgrad_pack(D), boxes = (D + 63) / 64;
   p.Dm = boxes * 64; p.m_off = 0; p.out_rows = D;
   p.pack = pack;
+  p.tb = chunk_steps(T);
+  const uint32_t tb = static_cast<uint32_t>(p.tb), bb = static_cast<uint32_t>(kKC) / tb;
   p.npt = pack > 1 ? 1 : (D + np - 1) / np;
   const int mtiles = pack > 1 ? (gr + 1) / 2 : (gr * boxes * 64 + 127) / 128;
   dim3 grid(static_cast<unsigned>(mtiles * p.npt),
@@ -282,10 +298,10 @@ static int wgrad_launch_split(int gr, int gb, const __nv_bfloat16* dgr, const __
     CUtensorMap dgr_map, hbf_map;
     const uint64_t ddims[4] = {static_cast<uint64_t>(N) * D, static_cast<uint64_t>(gr), static_cast<uint64_t>(T),
                                static_cast<uint64_t>(B)};
-    const uint32_t dbox[4] = {64u, 1u, static_cast<uint32_t>(kKC), 1u};
+    const uint32_t dbox[4] = {64u, 1u, tb, bb};
     const uint64_t hdims[3] = {static_cast<uint64_t>(N) * D, static_cast<uint64_t>(T), static_cast<uint64_t>(B)};
     const uint64_t hstride[3] = {static_cast<uint64_t>(N) * D, static_cast<uint64_t>(T + 1), static_cast<uint64_t>(B)};
-    const uint32_t hbox[3] = {64u, static_cast<uint32_t>(kKC), 1u};
+    const uint32_t hbox[3] = {64u, tb, bb};
     if (make_tensor_map(&dgr_map, dgr, 2, 4, ddims, dbox, true) != 0) return -4;
     if (make_tensor_map(&hbf_map, hbf, 2, 3, hdims, hbox, true, hstride) != 0) return -4;
     const int smem = kTmaStages * (16384 + 64 * 128) + 1024;
@@ -296,10 +312,10 @@ static int wgrad_launch_split(int gr, int gb, const __nv_bfloat16* dgr, const __
     CUtensorMap dgr_map, hbf_map;
     const uint64_t ddims[5] = {static_cast<uint64_t>(D), static_cast<uint64_t>(N), static_cast<uint64_t>(gr),
                                static_cast<uint64_t>(T), static_cast<uint64_t>(B)};
-    const uint32_t dbox[5] = {64u, 1u, 1u, static_cast<uint32_t>(kKC), 1u};
+    const uint32_t dbox[5] = {64u, 1u, 1u, tb, bb};
     const uint64_t hdims[4] = {static_cast<uint64_t>(D), static_cast<uint64_t>(N), static_cast<uint64_t>(T), static_cast<uint64_t>(B)};
     const uint64_t hstride[4] = {static_cast<uint64_t>(D), static_cast<uint64_t>(N), static_cast<uint64_t>(T + 1), static_cast<uint64_t>(B)};
-    const uint32_t hbox[4] = {64u, 1u, static_cast<uint32_t>(kKC), 1u};
+    const uint32_t hbox[4] = {64u, 1u, tb, bb};
     if (make_tensor_map(&dgr_map, dgr, 2, 5, ddims, dbox, true) != 0) return -4;
     if (make_tensor_map(&hbf_map, hbf, 2, 4, hdims, hbox, true, hstride) != 0) return -4;
     const int smem = kTmaStages * (16384 + np * 128) + 1024;
@@ -340,6 +356,7 @@ int wgrad_launch_rows(int gr, int gb, const __nv_bfloat16* dgr, const __nv_bfloa
   p.B = B; p.T = T; p.N = 1; p.D = D; p.GR = gr;
   p.NP = 256; p.ksplit = 1;
   p.npt = D / 256;
+  p.tb = kKC;
   p.chunks_per_split = B * ((T + kKC - 1) / kKC);
   p.pack = 1;
   p.Dm = Dm; p.m_off = m_off; p.out_rows = out_rows;
@@ -415,7 +432,7 @@ int wgrad_launch_static(int gr, int gb, const __nv_bfloat16* dgr, const __nv_bfl
     // Widths of whole 256-column tiles are refused, as plan.wgrad_work_bytes tells their caller. The tiles of other widths are rounded up,
     // hence fewer, and may split further than the array has room for (LSTM D736: 72 tiles, two parts, 17.3 MB): less far then.
     if (D % 256 == 0) return -6;
-    const int chunks = B * ((T + kKC - 1) / kKC), room = static_cast<int>(kStaticWorkBytes / part), parts = room < 1 ? 1 : room;
+    const int chunks = static_cast<int>(chunk_count(B, T)), room = static_cast<int>(kStaticWorkBytes / part), parts = room < 1 ? 1 : room;
     cps = (chunks + parts - 1) / parts;
     ksplit = (chunks + cps - 1) / cps;
   }

@@ -1,5 +1,5 @@
-"""dR contraction of widths that are no multiple of 64 (boxes that reach past a head, several column tiles) and of widths that no equal
-whole-box tiles divide (320, 448, 640): against an fp64 einsum of the same bf16 operands."""
+"""dR contraction of widths that are no multiple of 64 (boxes that reach past a head, several column tiles), of widths that no equal
+whole-box tiles divide (320, 448, 640) and of sequences shorter than a chunk: against an fp64 einsum of the same bf16 operands."""
 
 import pytest
 import torch
@@ -8,6 +8,8 @@ pytestmark = pytest.mark.gpu
 
 CASES = [("gru", 3, 70, 2, 80), ("lstm", 2, 33, 3, 48), ("elman", 5, 64, 1, 112), ("gru", 13, 100, 2, 208), ("lstm", 1, 1, 1, 240),
          ("slstm", 2, 65, 2, 176), ("lstm", 4, 40, 1, 320), ("elman", 3, 129, 2, 448), ("gru", 2, 63, 1, 640), ("lstm", 2, 64, 1, 704)]
+# several batch rows to a chunk: a ragged last one, steps past the sequence, packed heads, every number of rows
+CASES += [("lstm", 70, 1, 2, 80), ("gru", 33, 3, 1, 208), ("elman", 9, 32, 5, 32), ("lstm", 130, 2, 3, 64), ("slstm", 19, 7, 3, 16), ("gru", 5, 9, 1, 320)]
 
 
 @pytest.mark.parametrize("case", CASES, ids=lambda c: f"{c[0]}-B{c[1]}-T{c[2]}-N{c[3]}-D{c[4]}")
