@@ -68,6 +68,8 @@ __device__ __forceinline__ float logsigmoid_f(float x) {
 // forward: st holds the previous state on entry and the new state on return.
 // ry = R*round_bf16(h_prev) for the GR recurrent gates, wx = this step's input gates.
 // cache receives what cell_backward needs (nothing useful for Elman).
+// A sum of two products is written as what is rounded first and what is fused, here and below: the compiler's choice depends on the code
+// around it, and a step must not round differently in two instantiations.
 // ---------------------------------------------------------------------------------------------
 template <int CELL>
 __device__ __forceinline__ void cell_forward(const float* ry, const float* wx, const float* b,
@@ -77,7 +79,7 @@ __device__ __forceinline__ void cell_forward(const float* ry, const float* wx, c
     const float sf = sigmoid_f((wx[1] + ry[1]) + b[1]);
     const float tz = tanh_f((wx[2] + ry[2]) + b[2]);
     const float so = sigmoid_f((wx[3] + ry[3]) + b[3]);
-    const float c = sf * st[1] + si * tz;
+    const float c = __fmaf_rn(si, tz, __fmul_rn(sf, st[1]));
     st[0] = so * tanh_f(c);
     st[1] = c;
     cache[0] = si; cache[1] = sf; cache[2] = tz; cache[3] = so;
@@ -90,7 +92,7 @@ __device__ __forceinline__ void cell_forward(const float* ry, const float* wx, c
     const float m = slstm_take_i ? i : fmaxf(i, logf);
     const float ig = __expf(i - m);
     const float fg = __expf(logf - m);
-    const float c = fg * st[1] + ig * tanh_p(z);
+    const float c = __fmaf_rn(fg, st[1], __fmul_rn(ig, tanh_p(z)));
     const float n = fmaxf(fg * st[2] + ig, 1.0f);
     st[0] = sigmoid_p(o) * c * rcp_fast(n);  // rcp.approx: 1 ulp, against a dozen instructions for the IEEE quotient
     st[1] = c; st[2] = n; st[3] = m;
@@ -100,7 +102,7 @@ __device__ __forceinline__ void cell_forward(const float* ry, const float* wx, c
     const float r = sigmoid_f((wx[0] + ry[1]) + b[1]);
     const float u = sigmoid_f((wx[1] + ry[2]) + b[2]);
     const float v = tanh_f((wx[2] + b[3]) + r * cand);
-    st[0] = u * st[0] + (1.0f - u) * v;
+    st[0] = __fmaf_rn(u, st[0], __fmul_rn(1.0f - u, v));
     // the cache holds fp16 values: keep an (absurdly) large candidate finite there
     cache[0] = fminf(fmaxf(cand, -60000.0f), 60000.0f); cache[1] = r; cache[2] = u; cache[3] = v;
   } else {
@@ -159,10 +161,9 @@ __device__ __forceinline__ void cell_backward(const float* cache, const float* s
     const float mask = slstm_v1 ? 1.0f : (pre_n > 1.0f ? 1.0f : (pre_n == 1.0f ? 0.5f : 0.0f));
     const float dpre = dn * mask;
     const float d_ig = dc * tz + dpre;
-    const float d_fg = dc * c_p + dpre * n_p;
+    const float d_fg = __fmaf_rn(dc, c_p, __fmul_rn(dpre, n_p));
     const float d_z = dc * ig * (1.0f - tz * tz);
-    // Products that are used more than once: whether the compiler contracts one into a following sum depends on the code around
-    // it, and a step must not round differently in two instantiations.
+    // products that are used more than once
     float d_i = __fmul_rn(d_ig, ig);
     float d_logf = __fmul_rn(d_fg, fg);
     const float dm = slstm_v1 ? 0.0f : __fadd_rn(__fadd_rn(ds[3], -d_i), -d_logf);

@@ -17,6 +17,7 @@ CASES = [
     (("elman", 16, 130, 1, 768), (2, 8), (8, 8)), (("lstm", 8, 66, 1, 1024), (4, 8), (8, 8)), (("lstm", 13, 7, 1, 1024), (2, 8), (8, 16)),
     (("slstm", 32, 5, 1, 1024), (2, 0), (16, 0)), (("slstm", 9, 4, 1, 960), (2, 0), (8, 0)), (("elman", 13, 67, 1, 1024), (2, 4), (8, 8)),
     (("elman", 9, 70, 1, 1536), (2, 4), (0, 8)), (("elman", 7, 5, 1, 1792), (2, 8), (0, 8)), (("slstm", 32, 70, 1, 896), (2, 4), (16, 0)),
+    (("gru", 22, 16, 1, 1024), (2, 4), (16, 0)), (("gru", 30, 64, 1, 832), (2, 0), (16, 0)), (("gru", 30, 70, 1, 768), (2, 4), (16, 0)),
     (("elman", 30, 130, 1, 768), (2, 4), (16, 8)), (("elman", 64, 66, 1, 768), (0, 2), (0, 8)), (("gru", 16, 66, 1, 1280), (2, 8), (0, 16)),
 ]
 OUT = {"forward": ("hist", "carry", "cache", "hbf"), "backward": ("dwx", "dgr", "dinit", "dbp")}
