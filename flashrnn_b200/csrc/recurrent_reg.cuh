@@ -55,8 +55,9 @@ inline int reg_transfer_steps(int fixed_bytes, int step_bytes, int blocks) {
   return steps;
 }
 
-// Modes of the forward's step loops: any outputs and hooks, the outputs of a training call, a whole fp32 history alone.
-enum : int { kRegAny = 0, kRegTrain = 1, kRegPlain = 2 };
+// Modes of the step loops. Forward: any outputs and the hooks, any outputs, those of a training call, the same with h clipped, a whole fp32
+// history alone, fp32 hidden states alone, bf16 snapshots alone, nothing but the carry. Backward: options and hooks, options, neither.
+enum : int { kRegHooks = 0, kRegAny, kRegTrain, kRegClipped, kRegPlain, kRegHidden, kRegNarrow, kRegLast };
 
 // Wide heads (recurrent_wide_*.cuh): slots of the exchange in global memory, steps between two fences.
 constexpr int kWideSlots = 64, kWideFence = 8;

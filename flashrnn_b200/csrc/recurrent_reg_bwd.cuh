@@ -276,15 +276,15 @@ frnn_bwd_reg_kernel(const BwdParams p, const float* history, const float* initia
       }
     };
     // The steps, compiled without the options and hooks of a call and with them: their flags are a good part of a step's instructions.
-    auto run = [&](auto any_tag) {
-      constexpr bool any = decltype(any_tag)::value;
+    auto run = [&](auto mode_tag) {
+      constexpr bool hook = decltype(mode_tag)::value == kRegHooks, any = decltype(mode_tag)::value != kRegPlain;
       long long pc[6] = {0, 0, 0, 0, 0, 0};
-      auto clock = [&]() -> long long { return any && prof ? clock64() : 0; };
+      auto clock = [&]() -> long long { return hook && prof ? clock64() : 0; };
       // what a silenced iteration leaves out is waited for on a barrier that nobody arrives at (one CTA) or that stays incomplete
       auto wait_parts = [&](int it) {
         if constexpr (LOCAL) {
           asm volatile("bar.sync 2, %0;" ::"n"(compute_threads) : "memory");
-          if (any && it > mute_from && !dead && !mbar_wait_warp<false>(smem_u32(&s_part_bar[0]), 0, limit, abort_flag)) give_up(kErrWaitPart, it);
+          if (hook && it > mute_from && !dead && !mbar_wait_warp<false>(smem_u32(&s_part_bar[0]), 0, limit, abort_flag)) give_up(kErrWaitPart, it);
         } else {
           if (!dead && !mbar_wait_warp<true>(smem_u32(&s_part_bar[it & 1]), ((it - 1) >> 1) & 1, limit, abort_flag)) give_up(kErrWaitPart, it);
         }
@@ -301,7 +301,7 @@ frnn_bwd_reg_kernel(const BwdParams p, const float* history, const float* initia
         uint32_t out_w = out + first * dwx_bytes;
         uint32_t out_g = out + ring_steps * dwx_bytes + first * (CT::GR * kPlane2) + off2;
         for (int t = t0 + first; t >= t0; --t, ++it) {
-          if (any && jitter != 0u) { jitter_stall(jitter, static_cast<uint32_t>(warp), static_cast<uint32_t>(it)); __syncwarp(); }
+          if (hook && jitter != 0u) { jitter_stall(jitter, static_cast<uint32_t>(warp), static_cast<uint32_t>(it)); __syncwarp(); }
           const long long c1 = clock();
           float cache[CT::GC][NB], sp[HS][NB], dh[S][NB], ds[S][NB];
 #pragma unroll
@@ -386,7 +386,7 @@ frnn_bwd_reg_kernel(const BwdParams p, const float* history, const float* initia
           asm volatile("bar.sync 1, %0;" ::"n"(compute_threads) : "memory");
           const long long c3 = clock();
           const int nb = (it + 1) & 1;
-          const bool publish = !dead && !(any && it >= mute_from);
+          const bool publish = !dead && !(hook && it >= mute_from);
           if (has_pair) {
             // Two column tiles: side by side where a warp has one row tile, else one after the other.
             constexpr int NP = MTW * CH == 1 ? NB : 1;
@@ -473,7 +473,7 @@ frnn_bwd_reg_kernel(const BwdParams p, const float* history, const float* initia
 #pragma unroll
             for (int e = 0; e < NB; ++e) dbacc[g][e] += CELL != kGRU ? dgw[g][e] : (g == 0 ? dgr[0][e] : dgw[g > 0 ? g - 1 : 0][e]);  // as cell_backward's gb
           const long long c5 = clock();
-          if (any && prof) {
+          if (hook && prof) {
             pc[0] += c5 - c1; pc[1] += c2 - c1; pc[2] += c3 - c2; pc[3] += c5 - c4; pc[4] += c4 - c3; pc[5] += cw - c1;
           }
         }
@@ -484,7 +484,7 @@ frnn_bwd_reg_kernel(const BwdParams p, const float* history, const float* initia
       }
       wait_parts(T);
       if (!(any && cut)) add_parts(T, dcar[0]);
-      if (any && prof) {  // the slots of the tcgen05 kernels' phase timers that have a counterpart here
+      if (hook && prof) {  // the slots of the tcgen05 kernels' phase timers that have a counterpart here
         p.err[15] = static_cast<int>(pc[0]);  // the whole step
         p.err[9] = static_cast<int>(pc[1]);   // tiles read, wait for the partial sums, their sum
         p.err[10] = static_cast<int>(pc[2]);  // cell, dg to shared memory, CTA barrier
@@ -493,8 +493,9 @@ frnn_bwd_reg_kernel(const BwdParams p, const float* history, const float* initia
         p.err[13] = static_cast<int>(pc[5]);  // tiles read, wait
       }
     };
-    if (hooks || cut || clip_on || v1) run(std::true_type{});
-    else run(std::false_type{});
+    if (hooks) run(std::integral_constant<int, kRegHooks>{});
+    else if (cut || clip_on || v1) run(std::integral_constant<int, kRegAny>{});
+    else run(std::integral_constant<int, kRegPlain>{});
 #pragma unroll
     for (int e = 0; e < NB; ++e)
       if (act[e]) {

@@ -226,12 +226,13 @@ frnn_fwd_reg_kernel(const FwdParams p, const __grid_constant__ CUtensorMap wx_ma
     // hooks): the flags of a call cost a fifth of a step's instructions.
     auto run = [&](auto mode_tag) {
       constexpr int MODE = decltype(mode_tag)::value;
-      const bool any = MODE == kRegAny, save = any ? has_cache : MODE == kRegTrain && CELL != kElman, keep_h = any ? has_hbf : MODE == kRegTrain;
-      const bool narrow = any && out_bf16, clipped = any && clip_on;
-      const int states = any ? hist_states : CT::S;
-      const int hist_step = any ? hist_bytes : CT::S * kPlane4, cache_step = any ? cache_bytes : (save ? CT::GC * kPlaneC : 0);
+      constexpr bool hook = MODE == kRegHooks, any = hook || MODE == kRegAny, train = MODE == kRegTrain || MODE == kRegClipped;
+      const bool save = any ? has_cache : train && CELL != kElman, keep_h = any ? has_hbf : train;
+      const bool narrow = any ? out_bf16 : MODE == kRegNarrow, clipped = any ? clip_on : MODE == kRegClipped;
+      const int states = any || MODE == kRegNarrow ? hist_states : (MODE == kRegHidden ? 1 : (MODE == kRegLast ? 0 : CT::S));
+      const int hist_step = any || MODE == kRegNarrow ? hist_bytes : states * kPlane4, cache_step = any ? cache_bytes : (save ? CT::GC * kPlaneC : 0);
       long long pc[6] = {0, 0, 0, 0, 0, 0};
-      auto clock = [&]() -> long long { return any && prof ? clock64() : 0; };
+      auto clock = [&]() -> long long { return hook && prof ? clock64() : 0; };
       uint32_t hb = smem_u32(hbuf), hb_next = hb + kHbuf;  // operand of this step, of the next
       int slot = 0;
       uint32_t in_phase = 0;
@@ -241,7 +242,7 @@ frnn_fwd_reg_kernel(const FwdParams p, const __grid_constant__ CUtensorMap wx_ma
         uint32_t in = my_chunk + slot * stage_bytes, out_h = my_out + slot * out_slot;
         uint32_t out_c = out_h + ring_steps * hist_step, out_b = out_c + ring_steps * cache_step;
         for (int t = t0; t < t_end; ++t) {
-          if (any && jitter != 0u) { jitter_stall(jitter, static_cast<uint32_t>(warp), static_cast<uint32_t>(t)); __syncwarp(); }
+          if (hook && jitter != 0u) { jitter_stall(jitter, static_cast<uint32_t>(warp), static_cast<uint32_t>(t)); __syncwarp(); }
           const long long c1 = clock();
           float wx[CT::GW][NI];
           if (wx_bf16) {
@@ -259,7 +260,7 @@ frnn_fwd_reg_kernel(const FwdParams p, const __grid_constant__ CUtensorMap wx_ma
           if constexpr (LOCAL) {
             // h of every warp; what a silenced step leaves out is waited for on a barrier that nobody arrives at
             if (t >= 1) asm volatile("bar.sync 1, %0;" ::"n"(nwarps * 32) : "memory");
-            if (any && t > mute_from && !dead && !mbar_wait_warp<false>(smem_u32(&s_hbar[0]), 0, limit, abort_flag)) give_up(kErrWaitH, t);
+            if (hook && t > mute_from && !dead && !mbar_wait_warp<false>(smem_u32(&s_hbar[0]), 0, limit, abort_flag)) give_up(kErrWaitH, t);
           } else {
             if (t >= 1 && !dead && !mbar_wait_warp<true>(smem_u32(&s_hbar[t & 1]), ((t - 1) >> 1) & 1, limit, abort_flag)) give_up(kErrWaitH, t);
           }
@@ -325,7 +326,7 @@ frnn_fwd_reg_kernel(const FwdParams p, const __grid_constant__ CUtensorMap wx_ma
             for (int k = 0; k < CT::GC; ++k) cv[k][i] = cj[k];
           }
           const long long c4 = clock();
-          const bool publish = t + 1 < T && !(any && (dead || t >= mute_from));
+          const bool publish = t + 1 < T && !(hook && (dead || t >= mute_from));
           const uint32_t hslot = hb_next + (rank * U + warp * UPW + uq) * 16;
           if constexpr (LOCAL) {
             if (publish) {
@@ -403,7 +404,7 @@ frnn_fwd_reg_kernel(const FwdParams p, const __grid_constant__ CUtensorMap wx_ma
           hb = hb_next;
           hb_next = swap;
           const long long c6 = clock();
-          if (any && prof) {
+          if (hook && prof) {
             pc[1] += c2 - c1; pc[2] += c3 - c2; pc[3] += c4 - c3; pc[4] += c5 - c4; pc[5] += c6 - c5;
           }
         }
@@ -412,7 +413,7 @@ frnn_fwd_reg_kernel(const FwdParams p, const __grid_constant__ CUtensorMap wx_ma
         if (lane == 0) mbar_arrive(smem_u32(&s_out_full[slot]));
         if (++slot == kRegSlots) { slot = 0; in_phase ^= 1u; }
       }
-      if (any && prof) {  // the slots of the tcgen05 kernels' phase timers that have a counterpart here
+      if (hook && prof) {  // the slots of the tcgen05 kernels' phase timers that have a counterpart here
         p.err[12] = static_cast<int>(pc[3]);   // accumulators -> h_t
         p.err[13] = static_cast<int>(pc[4]);   // publication
         p.err[14] = static_cast<int>(pc[5]);   // outputs staged
@@ -420,10 +421,16 @@ frnn_fwd_reg_kernel(const FwdParams p, const __grid_constant__ CUtensorMap wx_ma
         p.err[17] = static_cast<int>(pc[2]);   // ldmatrix, mma
       }
     };
-    if (hooks || hist_states != CT::S || out_bf16 || clip_on) run(std::integral_constant<int, kRegAny>{});
-    else if (has_hbf && (has_cache || CELL == kElman)) run(std::integral_constant<int, kRegTrain>{});
-    else if (!has_hbf && !has_cache) run(std::integral_constant<int, kRegPlain>{});
-    else run(std::integral_constant<int, kRegAny>{});
+    const bool alone = !has_cache && !has_hbf, whole = hist_states == CT::S && !out_bf16;
+    if (hooks) run(std::integral_constant<int, kRegHooks>{});
+    else if (whole && has_hbf && (has_cache || CELL == kElman)) {
+      if (clip_on) run(std::integral_constant<int, kRegClipped>{});
+      else run(std::integral_constant<int, kRegTrain>{});
+    } else if (clip_on || !alone) run(std::integral_constant<int, kRegAny>{});
+    else if (hist_states == 0) run(std::integral_constant<int, kRegLast>{});
+    else if (out_bf16) run(std::integral_constant<int, kRegNarrow>{});
+    else if (whole) run(std::integral_constant<int, kRegPlain>{});
+    else run(std::integral_constant<int, kRegHidden>{});
 #pragma unroll
     for (int i = 0; i < NI; ++i) {
       if (!act[i]) continue;

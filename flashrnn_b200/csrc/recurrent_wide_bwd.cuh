@@ -224,10 +224,10 @@ frnn_bwd_wide_kernel(const BwdParams p, const float* history, const float* initi
       }
     };
     // The steps, compiled without the options and hooks of a call and with them.
-    auto run = [&](auto any_tag) {
-      constexpr bool any = decltype(any_tag)::value;
+    auto run = [&](auto mode_tag) {
+      constexpr bool hook = decltype(mode_tag)::value == kRegHooks, any = decltype(mode_tag)::value != kRegPlain;
       long long pc[6] = {0, 0, 0, 0, 0, 0};
-      auto clock = [&]() -> long long { return any && prof ? clock64() : 0; };
+      auto clock = [&]() -> long long { return hook && prof ? clock64() : 0; };
       auto wait_parts = [&](int it) {
         if (!dead && !mbar_wait_warp<true>(smem_u32(&s_part_bar[it & 1]), ((it - 1) >> 1) & 1, limit, abort_flag)) give_up(kErrWaitPart, it);
       };
@@ -238,7 +238,7 @@ frnn_bwd_wide_kernel(const BwdParams p, const float* history, const float* initi
         const int first = T - 1 - it - t0;  // step of the transfer it begins with, counting down
         const uint32_t in = smem_u32(stages) + slot * stage_bytes, out = smem_u32(outs) + slot * out_slot;
         for (int t = t0 + first; t >= t0; --t, ++it) {
-          if (any && jitter != 0u) { jitter_stall(jitter, static_cast<uint32_t>(warp), static_cast<uint32_t>(it)); __syncwarp(); }
+          if (hook && jitter != 0u) { jitter_stall(jitter, static_cast<uint32_t>(warp), static_cast<uint32_t>(it)); __syncwarp(); }
           const long long c1 = clock();
           long long c2 = c1, c3 = c1;
           if (owner) {
@@ -276,7 +276,7 @@ frnn_bwd_wide_kernel(const BwdParams p, const float* history, const float* initi
             }
             c2 = clock();
             const bool take_i = CELL == kSLSTM && t == 0 && zero_first;
-            const bool publish = !(any && (dead || it >= mute_from));
+            const bool publish = !(hook && (dead || it >= mute_from));
             uint8_t* const xg_now = xg + static_cast<size_t>(it % kWideSlots) * slot_bytes;
             uint8_t* const xg_ahead = xg + static_cast<size_t>((it + kWideSlots / 2) % kWideSlots) * slot_bytes;
             const bool refill = it + kWideSlots / 2 < T && it + kWideSlots / 2 >= xg_slots;
@@ -404,7 +404,7 @@ frnn_bwd_wide_kernel(const BwdParams p, const float* history, const float* initi
             }
           }
           const long long c5 = clock();
-          if (any && prof) {
+          if (hook && prof) {
             pc[0] += c5 - c1; pc[1] += c2 - c1; pc[2] += c3 - c2; pc[3] += c4 - c3; pc[4] += c5 - c4;
           }
         }
@@ -419,7 +419,7 @@ frnn_bwd_wide_kernel(const BwdParams p, const float* history, const float* initi
         wait_parts(T);
         if (!(any && cut)) add_parts(T, dcar[0]);
       }
-      if (any && prof) {
+      if (hook && prof) {
         p.err[15] = static_cast<int>(pc[0]);  // the whole step
         p.err[9] = static_cast<int>(pc[1]);   // tiles read, wait for the partial sums, their sum
         p.err[10] = static_cast<int>(pc[2]);  // cell, publication, outputs staged
@@ -427,8 +427,9 @@ frnn_bwd_wide_kernel(const BwdParams p, const float* history, const float* initi
         p.err[12] = static_cast<int>(pc[4]);  // mma and scatter
       }
     };
-    if (hooks || cut || clip_on || v1) run(std::true_type{});
-    else run(std::false_type{});
+    if (hooks) run(std::integral_constant<int, kRegHooks>{});
+    else if (cut || clip_on || v1) run(std::integral_constant<int, kRegAny>{});
+    else run(std::integral_constant<int, kRegPlain>{});
     // bias gradient of the batch rows of the group, added in their order: through the buffers of the partial sums, which the last wait
     // of every owner warp left
     asm volatile("bar.sync 1, 256;" ::: "memory");

@@ -189,12 +189,13 @@ frnn_fwd_wide_kernel(const FwdParams p, const __grid_constant__ CUtensorMap wx_m
     // hooks): see recurrent_reg_fwd.cuh.
     auto run = [&](auto mode_tag) {
       constexpr int MODE = decltype(mode_tag)::value;
-      const bool any = MODE == kRegAny, save = any ? has_cache : MODE == kRegTrain && CELL != kElman, keep_h = any ? has_hbf : MODE == kRegTrain;
-      const bool narrow = any && out_bf16, clipped = any && clip_on;
-      const int states = any ? hist_states : CT::S;
-      const int hist_step = any ? hist_bytes : CT::S * kPlane4, cache_step = any ? cache_bytes : (save ? CT::GC * kPlaneC : 0);
+      constexpr bool hook = MODE == kRegHooks, any = hook || MODE == kRegAny, train = MODE == kRegTrain || MODE == kRegClipped;
+      const bool save = any ? has_cache : train && CELL != kElman, keep_h = any ? has_hbf : train;
+      const bool narrow = any ? out_bf16 : MODE == kRegNarrow, clipped = any ? clip_on : MODE == kRegClipped;
+      const int states = any || MODE == kRegNarrow ? hist_states : (MODE == kRegHidden ? 1 : (MODE == kRegLast ? 0 : CT::S));
+      const int hist_step = any || MODE == kRegNarrow ? hist_bytes : states * kPlane4, cache_step = any ? cache_bytes : (save ? CT::GC * kPlaneC : 0);
       long long pc[6] = {0, 0, 0, 0, 0, 0};
-      auto clock = [&]() -> long long { return any && prof ? clock64() : 0; };
+      auto clock = [&]() -> long long { return hook && prof ? clock64() : 0; };
       int slot = 0;
       uint32_t in_phase = 0;
       for (int t0 = 0; t0 < T; t0 += ring_steps) {
@@ -203,7 +204,7 @@ frnn_fwd_wide_kernel(const FwdParams p, const __grid_constant__ CUtensorMap wx_m
         uint32_t in = smem_u32(wxs) + slot * stage_bytes, out_h = smem_u32(outs) + slot * out_slot;
         uint32_t out_c = out_h + region_c, out_b = out_h + region_b;
         for (int t = t0; t < t_end; ++t) {
-          if (any && jitter != 0u) { jitter_stall(jitter, static_cast<uint32_t>(warp), static_cast<uint32_t>(t)); __syncwarp(); }
+          if (hook && jitter != 0u) { jitter_stall(jitter, static_cast<uint32_t>(warp), static_cast<uint32_t>(t)); __syncwarp(); }
           const int pb = t & 1;
           const long long c1 = clock();
           const uint32_t hb = smem_u32(hbuf) + pb * Cfg::HBUF + lane * 16;
@@ -259,7 +260,7 @@ frnn_fwd_wide_kernel(const FwdParams p, const __grid_constant__ CUtensorMap wx_m
             cell_forward<CELL>(ry, wx, bias, st, cv, take_i);
             if (clipped) st[0] = fminf(fmaxf(st[0], -clip), clip);
             const float mine = act ? st[0] : 0.0f, other = __shfl_xor_sync(0xffffffffu, mine, 16);
-            const bool publish = t + 1 < T && !(any && (dead || t >= mute_from));
+            const bool publish = t + 1 < T && !(hook && (dead || t >= mute_from));
             if (publish && !dead) {
               const uint32_t w = hi ? kXgFill : xg_clean(pack_bf16x2(mine, other));
               const int ahead = t + 1 + (hi ? kWideSlots / 2 : 0);
@@ -327,7 +328,7 @@ frnn_fwd_wide_kernel(const FwdParams p, const __grid_constant__ CUtensorMap wx_m
             asm volatile("bar.sync 1, 256;" ::: "memory");
           }
           const long long c6 = clock();
-          if (any && prof) {
+          if (hook && prof) {
             pc[1] += c6 - c5; pc[2] += c2 - c1; pc[3] += c4 - c3; pc[4] += c3 - c2; pc[5] += c5 - c4;
           }
         }
@@ -338,7 +339,7 @@ frnn_fwd_wide_kernel(const FwdParams p, const __grid_constant__ CUtensorMap wx_m
         }
         if (++slot == kRegSlots) { slot = 0; in_phase ^= 1u; }
       }
-      if (any && prof) {  // the slots of the tcgen05 kernels' phase timers that have a counterpart here
+      if (hook && prof) {  // the slots of the tcgen05 kernels' phase timers that have a counterpart here
         p.err[11] = static_cast<int>(pc[4]);   // wait for the partial gates, their sum
         p.err[12] = static_cast<int>(pc[3]);   // cell, publication
         p.err[14] = static_cast<int>(pc[5]);   // outputs staged
@@ -346,10 +347,16 @@ frnn_fwd_wide_kernel(const FwdParams p, const __grid_constant__ CUtensorMap wx_m
         p.err[17] = static_cast<int>(pc[2]);   // ldmatrix, mma, partial gates sent
       }
     };
-    if (hooks || hist_states != CT::S || out_bf16 || clip_on) run(std::integral_constant<int, kRegAny>{});
-    else if (has_hbf && (has_cache || CELL == kElman)) run(std::integral_constant<int, kRegTrain>{});
-    else if (!has_hbf && !has_cache) run(std::integral_constant<int, kRegPlain>{});
-    else run(std::integral_constant<int, kRegAny>{});
+    const bool alone = !has_cache && !has_hbf, whole = hist_states == CT::S && !out_bf16;
+    if (hooks) run(std::integral_constant<int, kRegHooks>{});
+    else if (whole && has_hbf && (has_cache || CELL == kElman)) {
+      if (clip_on) run(std::integral_constant<int, kRegClipped>{});
+      else run(std::integral_constant<int, kRegTrain>{});
+    } else if (clip_on || !alone) run(std::integral_constant<int, kRegAny>{});
+    else if (hist_states == 0) run(std::integral_constant<int, kRegLast>{});
+    else if (out_bf16) run(std::integral_constant<int, kRegNarrow>{});
+    else if (whole) run(std::integral_constant<int, kRegPlain>{});
+    else run(std::integral_constant<int, kRegHidden>{});
     if (act) {
 #pragma unroll
       for (int k = 0; k < CT::S; ++k) p.carry[static_cast<size_t>(k) * B * ND + item] = st[k];
