@@ -41,6 +41,31 @@ int input_proj_launch(const void* x, const void* w, const float* bias, void* out
 int wgrad_launch_static(int gr, int gb, const __nv_bfloat16* dgr, const __nv_bfloat16* hbf, const float* db_part,
                         int n_btiles, float* dR, float* db, int* err, int B, int T, int N, int D, cudaStream_t s);
 
+cudaError_t raise_limits(const void* kern, int bytes, bool wide) {
+  struct Entry { const void* kern; int dev, bytes; bool wide; };
+  static std::mutex mu;
+  static Entry table[1024];
+  static int used = 0;
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  std::lock_guard<std::mutex> lock(mu);  // until the attribute is set: two raises must not pass each other
+  Entry* at = nullptr;
+  for (int i = 0; i < used && at == nullptr; ++i)
+    if (table[i].kern == kern && table[i].dev == dev) at = &table[i];
+  const int had = at != nullptr ? at->bytes : 0;
+  const bool had_wide = at != nullptr && at->wide;
+  if (had < bytes) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  if (e == cudaSuccess && wide && !had_wide) e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  if (e != cudaSuccess) return e;
+  if (at == nullptr && used < 1024) at = &(table[used++] = Entry{kern, dev, 0, false});
+  if (at != nullptr) {
+    at->bytes = had < bytes ? bytes : had;
+    at->wide = had_wide || wide;
+  }
+  return e;
+}
+
 namespace {
 
 using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,

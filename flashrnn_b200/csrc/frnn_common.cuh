@@ -188,6 +188,10 @@ __host__ __device__ __forceinline__ uint32_t kmajor_offset(int rows, int row, in
   return static_cast<uint32_t>((k >> 3) * (rows * 16) + (row >> 3) * 128 + (row & 7) * 16 + (k & 7) * 2);
 }
 
+// Host: dynamic shared memory of a kernel, clusters of more than 8 CTAs. These limits belong to the kernel, whose calls need different ones:
+// they are only ever raised, so that no thread takes them from one that is about to launch.
+cudaError_t raise_limits(const void* kern, int bytes, bool wide);
+
 // Host: keep the CTAs that can share one SM within the SM's 512 tensor-memory columns.
 // tcgen05.alloc has no time limit: a CTA whose request does not fit waits until a co-resident CTA
 // frees its columns. CTAs of one launch wait on one another (cluster barriers, exchange), so a CTA
@@ -195,12 +199,12 @@ __host__ __device__ __forceinline__ uint32_t kmajor_offset(int rows, int row, in
 // The launchers therefore ask the occupancy calculator how many CTAs of the kernel fit one SM with
 // the chosen shared-memory size and, where that many would ask for more than 512 columns together,
 // enlarge the dynamic shared memory until no more than 512 / tmem_cols CTAs fit. Returns 0, a
-// cudaError_t, or -3 when the budget cannot be met. Sets the kernel's dynamic shared-memory limit.
+// cudaError_t, or -3 when the budget cannot be met. Raises the kernel's dynamic shared-memory limit.
 template <typename Kern>
-inline int fit_tmem_budget(Kern kern, int threads, uint32_t tmem_cols, int* smem) {
+inline int fit_tmem_budget(Kern kern, int threads, uint32_t tmem_cols, int* smem, bool wide = false) {
   const int allowed = tmem_cols >= 512u ? 1 : static_cast<int>(512u / tmem_cols);
   for (int attempt = 0; attempt < 2; ++attempt) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, *smem);
+    cudaError_t e = raise_limits(reinterpret_cast<const void*>(kern), *smem, wide);
     if (e != cudaSuccess) return static_cast<int>(e);
     int blocks = 0;
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, kern, threads, static_cast<size_t>(*smem));

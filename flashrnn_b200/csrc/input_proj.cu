@@ -253,7 +253,9 @@ int input_proj_launch(const void* x, const void* w, const float* bias, void* out
   const uint32_t obox[2] = {out_bf16 ? 64u : 32u, 32u};
   if (make_tensor_map(&out_map, out, out_bf16 ? 2 : 4, 2, odims, obox, true) != 0) return -4;
   const int smem = kProjStages * (16384 + np * 128) + 4 * 8192 + 1024;  // ring + two staging buffers per epilogue warp
-  cudaError_t e = cudaFuncSetAttribute(input_proj_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  // the limit of the widest tile, whichever this call has: see kTmaSmemLimit in wgrad.cu
+  cudaError_t e = cudaFuncSetAttribute(input_proj_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       kProjStages * (16384 + 256 * 128) + 4 * 8192 + 1024);
   if (e != cudaSuccess) return static_cast<int>(e);
   int dev = 0, sms = 0;
   e = cudaGetDevice(&dev);

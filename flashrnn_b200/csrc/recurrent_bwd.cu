@@ -634,13 +634,9 @@ int launch_bwd(const BwdParams& p, const void* cache, const float* history, cons
   }
   auto kern = frnn_bwd_kernel<CELL, BV, U, WX_BF16, XG, OPTS>;
   const int fit = fit_tmem_budget(
-      kern, kBwdThreads, tmem_cols_pow2(((MTB * Cfg::BT + 31) / 32 * 32) + MTB * (Cfg::ROWS / 2), 32u), &smem);
+      kern, kBwdThreads, tmem_cols_pow2(((MTB * Cfg::BT + 31) / 32 * 32) + MTB * (Cfg::ROWS / 2), 32u), &smem, p.C > 8 && !XG);
   if (fit != 0) return fit;
   cudaError_t e = cudaSuccess;
-  if (p.C > 8 && !XG) {
-    e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    if (e != cudaSuccess) return static_cast<int>(e);
-  }
   const int n_btiles = (p.B + BV - 1) / BV;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(static_cast<unsigned>(p.N * n_btiles * p.C));

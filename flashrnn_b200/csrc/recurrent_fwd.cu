@@ -518,13 +518,9 @@ int launch_fwd_ext(const FwdParams& p, const void* wx, cudaStream_t stream) {
   const uint32_t box[5] = {static_cast<uint32_t>(U), 1u, static_cast<uint32_t>(CT::GW), 1u, static_cast<uint32_t>(p.wx_box_b)};
   if (make_tensor_map(&map, wx, Cfg::WX_ES, 5, dims, box) != 0) return -4;
   auto kern = frnn_fwd_kernel<CELL, BV, U, WX_BF16, XG, EXT>;
-  const int fit = fit_tmem_budget(kern, kFwdThreads, tmem_cols_pow2(Cfg::A_COL0 + Cfg::MT * (p.D / 2), 32u), &smem);
+  const int fit = fit_tmem_budget(kern, kFwdThreads, tmem_cols_pow2(Cfg::A_COL0 + Cfg::MT * (p.D / 2), 32u), &smem, p.C > 8 && !XG);
   if (fit != 0) return fit;
   cudaError_t e = cudaSuccess;
-  if (p.C > 8 && !XG) {
-    e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    if (e != cudaSuccess) return static_cast<int>(e);
-  }
   const int n_btiles = (p.B + BV - 1) / BV;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(static_cast<unsigned>(p.N * n_btiles * p.C));

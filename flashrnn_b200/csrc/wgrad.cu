@@ -56,6 +56,9 @@ struct WgradParams {
 // T256 N8 D176 91 / 1705, B8 T1024 N1 D640 58 / 851.
 constexpr int kTmaThreads = 192;
 constexpr int kTmaStages = 4;
+// Every launch asks for the limit of the widest tile: the attribute belongs to the kernel, and a thread with narrower tiles would take it from
+// one that is about to launch.
+constexpr int kTmaSmemLimit = kTmaStages * (16384 + 256 * 128) + 1024;
 
 __global__ void __launch_bounds__(kTmaThreads, 1)
 wgrad_tma_kernel(const WgradParams p, const __grid_constant__ CUtensorMap dgr_map,
@@ -305,7 +308,7 @@ static int wgrad_launch_split(int gr, int gb, const __nv_bfloat16* dgr, const __
     if (make_tensor_map(&dgr_map, dgr, 2, 4, ddims, dbox, true) != 0) return -4;
     if (make_tensor_map(&hbf_map, hbf, 2, 3, hdims, hbox, true, hstride) != 0) return -4;
     const int smem = kTmaStages * (16384 + 64 * 128) + 1024;
-    e = cudaFuncSetAttribute(wgrad_tma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    e = cudaFuncSetAttribute(wgrad_tma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTmaSmemLimit);
     if (e != cudaSuccess) return static_cast<int>(e);
     wgrad_tma_kernel<<<grid, kTmaThreads, smem, s>>>(p, dgr_map, hbf_map);
   } else {
@@ -319,7 +322,7 @@ static int wgrad_launch_split(int gr, int gb, const __nv_bfloat16* dgr, const __
     if (make_tensor_map(&dgr_map, dgr, 2, 5, ddims, dbox, true) != 0) return -4;
     if (make_tensor_map(&hbf_map, hbf, 2, 4, hdims, hbox, true, hstride) != 0) return -4;
     const int smem = kTmaStages * (16384 + np * 128) + 1024;
-    e = cudaFuncSetAttribute(wgrad_tma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    e = cudaFuncSetAttribute(wgrad_tma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTmaSmemLimit);
     if (e != cudaSuccess) return static_cast<int>(e);
     wgrad_tma_kernel<<<grid, kTmaThreads, smem, s>>>(p, dgr_map, hbf_map);
   }
@@ -370,7 +373,7 @@ int wgrad_launch_rows(int gr, int gb, const __nv_bfloat16* dgr, const __nv_bfloa
   if (make_tensor_map(&dgr_map, dgr, 2, 5, ddims, dbox, true) != 0) return -4;
   if (make_tensor_map(&hbf_map, hbf, 2, 4, hdims, hbox, true, hstride) != 0) return -4;
   const int smem = kTmaStages * (16384 + 256 * 128) + 1024;
-  cudaError_t e = cudaFuncSetAttribute(wgrad_tma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  cudaError_t e = cudaFuncSetAttribute(wgrad_tma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTmaSmemLimit);
   if (e != cudaSuccess) return static_cast<int>(e);
   dim3 grid(static_cast<unsigned>((gr * Dm / 128) * (D / 256)), 1u, 1u);
   wgrad_tma_kernel<<<grid, kTmaThreads, smem, s>>>(p, dgr_map, hbf_map);
