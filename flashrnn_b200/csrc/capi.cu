@@ -8,7 +8,8 @@
 
 namespace frnn {
 
-int forward_dispatch(int cell, const FwdParams& p, const void* wx, int wx_bf16, int bv, int unit, cudaStream_t s);
+// `at_once`: only say how many groups run at once
+int forward_dispatch(int cell, const FwdParams& p, const void* wx, int wx_bf16, int bv, int unit, cudaStream_t s, int* at_once = nullptr);
 // Register-resident kernels, groups of `rows` (8, 16 or 24) batch rows. `ask`: only say whether the call would be taken (kRegTaken
 // or kRegNoRoom).
 template <int CELL> int launch_fwd_reg_cell(const FwdParams& p, const void* wx, int wx_bf16, cudaStream_t s, int rows, bool ask);
@@ -30,7 +31,7 @@ int backward_ksplit_dispatch(int cell, const BwdParams& p, const void* cache, co
                              const float* d_history, int wx_bf16, int bv, int ksplit, cudaStream_t s, int* capacity_only);
 int backward_ksplit_capacity(int cell, int bv, int ksplit, int D);
 int backward_dispatch(int cell, const BwdParams& p, const void* cache, const float* history, const float* initial,
-                      const float* d_history, int wx_bf16, int bv, int unit, cudaStream_t s);
+                      const float* d_history, int wx_bf16, int bv, int unit, cudaStream_t s, int* at_once = nullptr);
 int wgrad_plan(int gr, int B, int T, int N, int D, int* np_out, int* ksplit_out, int* cps_out);
 int wgrad_launch(int gr, int gb, const __nv_bfloat16* dgr, const __nv_bfloat16* hbf, const float* db_part, int n_btiles,
                  float* dR, float* db, float* work, int* err, int B, int T, int N, int D, cudaStream_t s);
@@ -66,6 +67,17 @@ cudaError_t raise_limits(const void* kern, int bytes, bool wide) {
   return e;
 }
 
+// SMs of the current device (148 on a B200; also the answer when no device is visible).
+int sm_count() {
+  int dev = 0, n = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+      n <= 0) {
+    cudaGetLastError();
+    return 148;
+  }
+  return n;
+}
+
 namespace {
 
 using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -83,17 +95,6 @@ EncodeTiledFn encode_tiled_fn() {
       fn = reinterpret_cast<EncodeTiledFn>(sym);
   });
   return fn;
-}
-
-// SMs of the current device (148 on a B200; also the answer when no device is visible).
-int sm_count() {
-  int dev = 0, n = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-      n <= 0) {
-    cudaGetLastError();
-    return 148;
-  }
-  return n;
 }
 
 // CTAs of the clustered backward launch that the device can hold at once, remembered per shape
@@ -180,42 +181,74 @@ int make_tensor_map_strided(CUtensorMap* map, const void* base, int elem_bytes, 
 
 // The occupancy query takes microseconds; its answer depends on the device, the kernel, its cluster width and its shared
 // memory only and is remembered (kernels x staging layouts x devices; past 1024 entries it is asked again on each call).
-int reg_room(const void* kern, const cudaLaunchConfig_t& cfg, int width, long long groups, long long rival_groups, int D) {
+int reg_capacity(const void* kern, const cudaLaunchConfig_t& cfg, int width) {
   struct Entry { const void* kern; size_t smem; int dev, width, capacity; };
   static std::mutex mu;
   static Entry table[1024];
   static int used = 0;
-  const auto taken = [&](int capacity) {
-    if (groups <= capacity) return true;
-    if (rival_groups <= 0 || capacity < 1) return false;
-    const long long rivals = 2ll * sm_count() / (D % 32 == 0 ? D / 32 : D / 16);  // 16-row tcgen05 groups that run at once
-    return 3 * ((groups + capacity - 1) / capacity) <= 4 * ((rival_groups + rivals - 1) / rivals);
-  };
   int dev = 0, capacity = -1;
   cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return static_cast<int>(e);
+  if (e != cudaSuccess) return -static_cast<int>(e);
   {
     std::lock_guard<std::mutex> lock(mu);
     for (int i = 0; i < used && capacity < 0; ++i)
       if (table[i].kern == kern && table[i].smem == cfg.dynamicSmemBytes && table[i].dev == dev && table[i].width == width)
         capacity = table[i].capacity;
   }
-  if (capacity >= 0) return taken(capacity) ? 0 : kRegNoRoom;  // its attributes were set before the entry was made
+  if (capacity >= 0) return capacity;  // its attributes were set before the entry was made
   e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kRegSmemLimit);
   if (e == cudaSuccess && width > 8) e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-  if (e != cudaSuccess) return static_cast<int>(e);
+  if (e != cudaSuccess) return -static_cast<int>(e);
   if (width > 1) {
     e = cudaOccupancyMaxActiveClusters(&capacity, kern, &cfg);
   } else {
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&capacity, kern, static_cast<int>(cfg.blockDim.x), cfg.dynamicSmemBytes);
     capacity *= sm_count();
   }
-  if (e != cudaSuccess) return static_cast<int>(e);
+  if (e != cudaSuccess) return -static_cast<int>(e);
+  std::lock_guard<std::mutex> lock(mu);
+  if (used < 1024) table[used++] = Entry{kern, cfg.dynamicSmemBytes, dev, width, capacity};
+  return capacity;
+}
+
+int reg_room(const void* kern, const cudaLaunchConfig_t& cfg, int width, long long groups, long long rival_groups, int D) {
+  const int capacity = reg_capacity(kern, cfg, width);
+  if (capacity < 0) return -capacity;
+  if (groups <= capacity) return 0;
+  if (rival_groups <= 0 || capacity < 1) return kRegNoRoom;
+  const long long rivals = 2ll * sm_count() / (D % 32 == 0 ? D / 32 : D / 16);  // 16-row tcgen05 groups that run at once
+  return 3 * ((groups + capacity - 1) / capacity) <= 4 * ((rival_groups + rivals - 1) / rivals) ? 0 : kRegNoRoom;
+}
+
+RegRival reg_rival(bool backward, int cell, int wx_bf16, int N, int B, int D) {
+  struct Entry { int dev, kind, D, at_once; };
+  static std::mutex mu;
+  static Entry table[512];
+  static int used = 0;
+  frnn_b200_plan_t plan;
+  if (frnn_b200_plan(cell, B, 1, N, D, &plan) != 0 || !plan.supported || plan.exchange != 0) return {0, 0};
+  const int rows = backward ? plan.batch_tile : plan.fwd_batch_tile;
+  const int kind = (backward ? 1 : 0) | (wx_bf16 ? 2 : 0) | (rows == 16 ? 4 : 0) | cell << 3;
+  int dev = 0, at_once = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return {0, 0};
   {
     std::lock_guard<std::mutex> lock(mu);
-    if (used < 1024) table[used++] = Entry{kern, cfg.dynamicSmemBytes, dev, width, capacity};
+    for (int i = 0; i < used && at_once == 0; ++i)
+      if (table[i].dev == dev && table[i].kind == kind && table[i].D == D) at_once = table[i].at_once;
   }
-  return taken(capacity) ? 0 : kRegNoRoom;
+  if (at_once == 0) {
+    FwdParams f{};
+    f.B = B; f.T = 1; f.T_total = 1; f.N = N; f.D = D; f.C = plan.cluster; f.wx_box_b = rows; f.fwd_clip = INFINITY;
+    BwdParams b{};
+    b.B = B; b.T = 1; b.N = N; b.D = D; b.C = plan.cluster; b.box_b = rows;
+    const int rc = backward ? backward_dispatch(cell, b, nullptr, nullptr, nullptr, nullptr, wx_bf16, rows, plan.unit, nullptr, &at_once)
+                            : forward_dispatch(cell, f, nullptr, wx_bf16, rows, plan.unit, nullptr, &at_once);
+    if (rc != 0 || at_once < 1) return {0, 0};
+    std::lock_guard<std::mutex> lock(mu);
+    if (used < 512) table[used++] = Entry{dev, kind, D, at_once};
+  }
+  const long long groups = static_cast<long long>(N) * reg_batch_tiles(B, rows);
+  return {rows, static_cast<int>((groups + at_once - 1) / at_once)};
 }
 
 int forward_reg_dispatch(int cell, const FwdParams& p, const void* wx, int wx_bf16, cudaStream_t s, int rows, bool ask) {

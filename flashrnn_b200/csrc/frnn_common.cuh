@@ -227,6 +227,8 @@ inline uint32_t tmem_cols_pow2(int needed, uint32_t minimum) {
   return c;
 }
 
+int sm_count();  // of the current device
+
 // Host: build a tiled tensor map (no swizzle, no interleave). dims/box innermost first.
 // `stride_dims` (optional): extents the strides are computed from when the described tensor is a window of a
 // larger dense array (e.g. the first T of T + 1 time slots).

@@ -603,7 +603,7 @@ frnn_bwd_kernel(const BwdParams p, const __grid_constant__ CUtensorMap cache_map
 
 template <int CELL, int BV, int U, bool WX_BF16, bool XG, bool OPTS>
 int launch_bwd(const BwdParams& p, const void* cache, const float* history, const float* initial,
-               const float* d_history, cudaStream_t stream) {
+               const float* d_history, cudaStream_t stream, int* at_once) {
   using Cfg = BwdCfg<CELL, BV, U, WX_BF16>;
   using CT = typename Cfg::CT;
   const int part_bytes = p.C * BV * U * 4;
@@ -617,14 +617,14 @@ int launch_bwd(const BwdParams& p, const void* cache, const float* history, cons
   const uint64_t uD = p.D, uN = p.N, uT = p.T, uB = p.B;
   const uint32_t ub = static_cast<uint32_t>(p.box_b);
   CUtensorMap cache_map, hist_map, init_map, dhist_map;
-  {
+  if (at_once == nullptr) {
     const uint64_t dims[5] = {uD, uN, static_cast<uint64_t>(Cfg::GCL > 0 ? Cfg::GCL : 1), uT, uB};
     const uint32_t box[5] = {U, 1u, static_cast<uint32_t>(Cfg::GCL > 0 ? Cfg::GCL : 1), 1u, ub};
     // Elman has no cache: describe the history instead so that the (unused) map is valid.
     const void* base = Cfg::GCL > 0 ? static_cast<const void*>(cache) : static_cast<const void*>(history);
     if (make_tensor_map(&cache_map, base, Cfg::GCL > 0 ? CT::CES : 4, 5, dims, box) != 0) return -4;
   }
-  {
+  if (at_once == nullptr) {
     const uint64_t dims[5] = {uD, uN, uT, uB, static_cast<uint64_t>(CT::S)};
     const uint32_t box[5] = {U, 1u, 1u, ub, static_cast<uint32_t>(CT::S)};
     if (make_tensor_map(&hist_map, history, 4, 5, dims, box) != 0) return -4;
@@ -656,6 +656,12 @@ int launch_bwd(const BwdParams& p, const void* cache, const float* history, cons
   }
   cfg.attrs = attr;
   cfg.numAttrs = 1;
+  if (at_once != nullptr) {  // asked only how many groups run at once
+    if (p.C > 1) return static_cast<int>(cudaOccupancyMaxActiveClusters(at_once, kern, &cfg));
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(at_once, kern, static_cast<int>(cfg.blockDim.x), cfg.dynamicSmemBytes);
+    *at_once *= sm_count();
+    return static_cast<int>(e);
+  }
   if (!XG && p.C > 1) {
     // a cluster that cannot be placed (too many CTAs or too much shared memory per GPC) is reported, not launched
     int max_clusters = 0;
@@ -669,40 +675,40 @@ int launch_bwd(const BwdParams& p, const void* cache, const float* history, cons
 
 template <int CELL, int BV, int U>
 int launch_bwd_dt(const BwdParams& p, const void* cache, const float* history, const float* initial,
-                  const float* d_history, int wx_bf16, cudaStream_t s) {
+                  const float* d_history, int wx_bf16, cudaStream_t s, int* at_once) {
   const bool opts = p.grad_clip > 0.0f || p.cut_recurrent != 0 || p.slstm_v1 != 0;
   if (p.xg_data != nullptr) {  // groups wider than a cluster exchange through global memory
     if (opts)
-      return wx_bf16 ? launch_bwd<CELL, BV, U, true, true, true>(p, cache, history, initial, d_history, s)
-                     : launch_bwd<CELL, BV, U, false, true, true>(p, cache, history, initial, d_history, s);
-    return wx_bf16 ? launch_bwd<CELL, BV, U, true, true, false>(p, cache, history, initial, d_history, s)
-                   : launch_bwd<CELL, BV, U, false, true, false>(p, cache, history, initial, d_history, s);
+      return wx_bf16 ? launch_bwd<CELL, BV, U, true, true, true>(p, cache, history, initial, d_history, s, at_once)
+                     : launch_bwd<CELL, BV, U, false, true, true>(p, cache, history, initial, d_history, s, at_once);
+    return wx_bf16 ? launch_bwd<CELL, BV, U, true, true, false>(p, cache, history, initial, d_history, s, at_once)
+                   : launch_bwd<CELL, BV, U, false, true, false>(p, cache, history, initial, d_history, s, at_once);
   }
   if (opts)
-    return wx_bf16 ? launch_bwd<CELL, BV, U, true, false, true>(p, cache, history, initial, d_history, s)
-                   : launch_bwd<CELL, BV, U, false, false, true>(p, cache, history, initial, d_history, s);
-  return wx_bf16 ? launch_bwd<CELL, BV, U, true, false, false>(p, cache, history, initial, d_history, s)
-                 : launch_bwd<CELL, BV, U, false, false, false>(p, cache, history, initial, d_history, s);
+    return wx_bf16 ? launch_bwd<CELL, BV, U, true, false, true>(p, cache, history, initial, d_history, s, at_once)
+                   : launch_bwd<CELL, BV, U, false, false, true>(p, cache, history, initial, d_history, s, at_once);
+  return wx_bf16 ? launch_bwd<CELL, BV, U, true, false, false>(p, cache, history, initial, d_history, s, at_once)
+                 : launch_bwd<CELL, BV, U, false, false, false>(p, cache, history, initial, d_history, s, at_once);
 }
 template <int CELL>
 int launch_bwd_cell(const BwdParams& p, const void* cache, const float* history, const float* initial,
-                    const float* d_history, int wx_bf16, int bv, int unit, cudaStream_t s) {
-  if (bv == 8 && unit == 32) return launch_bwd_dt<CELL, 8, 32>(p, cache, history, initial, d_history, wx_bf16, s);
-  if (bv == 16 && unit == 32) return launch_bwd_dt<CELL, 16, 32>(p, cache, history, initial, d_history, wx_bf16, s);
-  if (bv == 8 && unit == 16) return launch_bwd_dt<CELL, 8, 16>(p, cache, history, initial, d_history, wx_bf16, s);
-  if (bv == 16 && unit == 16) return launch_bwd_dt<CELL, 16, 16>(p, cache, history, initial, d_history, wx_bf16, s);
+                    const float* d_history, int wx_bf16, int bv, int unit, cudaStream_t s, int* at_once) {
+  if (bv == 8 && unit == 32) return launch_bwd_dt<CELL, 8, 32>(p, cache, history, initial, d_history, wx_bf16, s, at_once);
+  if (bv == 16 && unit == 32) return launch_bwd_dt<CELL, 16, 32>(p, cache, history, initial, d_history, wx_bf16, s, at_once);
+  if (bv == 8 && unit == 16) return launch_bwd_dt<CELL, 8, 16>(p, cache, history, initial, d_history, wx_bf16, s, at_once);
+  if (bv == 16 && unit == 16) return launch_bwd_dt<CELL, 16, 16>(p, cache, history, initial, d_history, wx_bf16, s, at_once);
   return -2;
 }
 
 }  // namespace
 
 int backward_dispatch(int cell, const BwdParams& p, const void* cache, const float* history, const float* initial,
-                      const float* d_history, int wx_bf16, int bv, int unit, cudaStream_t s) {
+                      const float* d_history, int wx_bf16, int bv, int unit, cudaStream_t s, int* at_once) {
   switch (cell) {
-    case kLSTM: return launch_bwd_cell<kLSTM>(p, cache, history, initial, d_history, wx_bf16, bv, unit, s);
-    case kSLSTM: return launch_bwd_cell<kSLSTM>(p, cache, history, initial, d_history, wx_bf16, bv, unit, s);
-    case kGRU: return launch_bwd_cell<kGRU>(p, cache, history, initial, d_history, wx_bf16, bv, unit, s);
-    case kElman: return launch_bwd_cell<kElman>(p, cache, history, initial, d_history, wx_bf16, bv, unit, s);
+    case kLSTM: return launch_bwd_cell<kLSTM>(p, cache, history, initial, d_history, wx_bf16, bv, unit, s, at_once);
+    case kSLSTM: return launch_bwd_cell<kSLSTM>(p, cache, history, initial, d_history, wx_bf16, bv, unit, s, at_once);
+    case kGRU: return launch_bwd_cell<kGRU>(p, cache, history, initial, d_history, wx_bf16, bv, unit, s, at_once);
+    case kElman: return launch_bwd_cell<kElman>(p, cache, history, initial, d_history, wx_bf16, bv, unit, s, at_once);
     default: return -1;
   }
 }

@@ -506,7 +506,7 @@ frnn_fwd_kernel(const FwdParams p, const __grid_constant__ CUtensorMap wx_map) {
 }
 
 template <int CELL, int BV, int U, bool WX_BF16, bool XG, bool EXT>
-int launch_fwd_ext(const FwdParams& p, const void* wx, cudaStream_t stream) {
+int launch_fwd_ext(const FwdParams& p, const void* wx, cudaStream_t stream, int* at_once) {
   using Cfg = FwdCfg<CELL, BV, U, WX_BF16>;
   using CT = typename Cfg::CT;
   const int hbuf_bytes = Cfg::BT * p.D * 2;
@@ -516,7 +516,7 @@ int launch_fwd_ext(const FwdParams& p, const void* wx, cudaStream_t stream) {
   const uint64_t dims[5] = {static_cast<uint64_t>(p.D), static_cast<uint64_t>(p.N), static_cast<uint64_t>(CT::GW),
                             static_cast<uint64_t>(p.T_total), static_cast<uint64_t>(p.B)};
   const uint32_t box[5] = {static_cast<uint32_t>(U), 1u, static_cast<uint32_t>(CT::GW), 1u, static_cast<uint32_t>(p.wx_box_b)};
-  if (make_tensor_map(&map, wx, Cfg::WX_ES, 5, dims, box) != 0) return -4;
+  if (at_once == nullptr && make_tensor_map(&map, wx, Cfg::WX_ES, 5, dims, box) != 0) return -4;
   auto kern = frnn_fwd_kernel<CELL, BV, U, WX_BF16, XG, EXT>;
   const int fit = fit_tmem_budget(kern, kFwdThreads, tmem_cols_pow2(Cfg::A_COL0 + Cfg::MT * (p.D / 2), 32u), &smem, p.C > 8 && !XG);
   if (fit != 0) return fit;
@@ -540,6 +540,12 @@ int launch_fwd_ext(const FwdParams& p, const void* wx, cudaStream_t stream) {
   }
   cfg.attrs = attr;
   cfg.numAttrs = 1;
+  if (at_once != nullptr) {  // asked only how many groups run at once
+    if (p.C > 1) return static_cast<int>(cudaOccupancyMaxActiveClusters(at_once, kern, &cfg));
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(at_once, kern, static_cast<int>(cfg.blockDim.x), cfg.dynamicSmemBytes);
+    *at_once *= sm_count();
+    return static_cast<int>(e);
+  }
   if (!XG && p.C > 1) {
     // a cluster that cannot be placed (too many CTAs or too much shared memory per GPC) is reported, not launched
     int max_clusters = 0;
@@ -552,38 +558,38 @@ int launch_fwd_ext(const FwdParams& p, const void* wx, cudaStream_t stream) {
 }
 
 template <int CELL, int BV, int U, bool WX_BF16, bool XG>
-int launch_fwd(const FwdParams& p, const void* wx, cudaStream_t stream) {
+int launch_fwd(const FwdParams& p, const void* wx, cudaStream_t stream, int* at_once) {
   const bool ext = p.T_total != p.T || p.t0 != 0 || p.out_bf16 != 0 || p.fwd_clip < INFINITY;
-  return ext ? launch_fwd_ext<CELL, BV, U, WX_BF16, XG, true>(p, wx, stream)
-             : launch_fwd_ext<CELL, BV, U, WX_BF16, XG, false>(p, wx, stream);
+  return ext ? launch_fwd_ext<CELL, BV, U, WX_BF16, XG, true>(p, wx, stream, at_once)
+             : launch_fwd_ext<CELL, BV, U, WX_BF16, XG, false>(p, wx, stream, at_once);
 }
 
 template <int CELL, int BV, int U>
-int launch_fwd_dt(const FwdParams& p, const void* wx, int wx_bf16, cudaStream_t s) {
+int launch_fwd_dt(const FwdParams& p, const void* wx, int wx_bf16, cudaStream_t s, int* at_once) {
   if constexpr (U == 32) {  // groups wider than a cluster exchange through global memory (32-unit slices only)
     if (p.xg_data != nullptr)
-      return wx_bf16 ? launch_fwd<CELL, BV, U, true, true>(p, wx, s) : launch_fwd<CELL, BV, U, false, true>(p, wx, s);
+      return wx_bf16 ? launch_fwd<CELL, BV, U, true, true>(p, wx, s, at_once) : launch_fwd<CELL, BV, U, false, true>(p, wx, s, at_once);
   }
   if (p.xg_data != nullptr) return -2;
-  return wx_bf16 ? launch_fwd<CELL, BV, U, true, false>(p, wx, s) : launch_fwd<CELL, BV, U, false, false>(p, wx, s);
+  return wx_bf16 ? launch_fwd<CELL, BV, U, true, false>(p, wx, s, at_once) : launch_fwd<CELL, BV, U, false, false>(p, wx, s, at_once);
 }
 template <int CELL>
-int launch_fwd_cell(const FwdParams& p, const void* wx, int wx_bf16, int bv, int unit, cudaStream_t s) {
-  if (bv == 8 && unit == 32) return launch_fwd_dt<CELL, 8, 32>(p, wx, wx_bf16, s);
-  if (bv == 16 && unit == 32) return launch_fwd_dt<CELL, 16, 32>(p, wx, wx_bf16, s);
-  if (bv == 8 && unit == 16) return launch_fwd_dt<CELL, 8, 16>(p, wx, wx_bf16, s);
-  if (bv == 16 && unit == 16) return launch_fwd_dt<CELL, 16, 16>(p, wx, wx_bf16, s);
+int launch_fwd_cell(const FwdParams& p, const void* wx, int wx_bf16, int bv, int unit, cudaStream_t s, int* at_once) {
+  if (bv == 8 && unit == 32) return launch_fwd_dt<CELL, 8, 32>(p, wx, wx_bf16, s, at_once);
+  if (bv == 16 && unit == 32) return launch_fwd_dt<CELL, 16, 32>(p, wx, wx_bf16, s, at_once);
+  if (bv == 8 && unit == 16) return launch_fwd_dt<CELL, 8, 16>(p, wx, wx_bf16, s, at_once);
+  if (bv == 16 && unit == 16) return launch_fwd_dt<CELL, 16, 16>(p, wx, wx_bf16, s, at_once);
   return -2;
 }
 
 }  // namespace
 
-int forward_dispatch(int cell, const FwdParams& p, const void* wx, int wx_bf16, int bv, int unit, cudaStream_t s) {
+int forward_dispatch(int cell, const FwdParams& p, const void* wx, int wx_bf16, int bv, int unit, cudaStream_t s, int* at_once) {
   switch (cell) {
-    case kLSTM: return launch_fwd_cell<kLSTM>(p, wx, wx_bf16, bv, unit, s);
-    case kSLSTM: return launch_fwd_cell<kSLSTM>(p, wx, wx_bf16, bv, unit, s);
-    case kGRU: return launch_fwd_cell<kGRU>(p, wx, wx_bf16, bv, unit, s);
-    case kElman: return launch_fwd_cell<kElman>(p, wx, wx_bf16, bv, unit, s);
+    case kLSTM: return launch_fwd_cell<kLSTM>(p, wx, wx_bf16, bv, unit, s, at_once);
+    case kSLSTM: return launch_fwd_cell<kSLSTM>(p, wx, wx_bf16, bv, unit, s, at_once);
+    case kGRU: return launch_fwd_cell<kGRU>(p, wx, wx_bf16, bv, unit, s, at_once);
+    case kElman: return launch_fwd_cell<kElman>(p, wx, wx_bf16, bv, unit, s, at_once);
     default: return -1;
   }
 }

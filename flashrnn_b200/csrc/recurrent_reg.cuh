@@ -16,7 +16,7 @@
 
 namespace frnn {
 
-constexpr int kRegRows = 8;           // batch rows of one column tile of an mma; a group has one, two or (clusters of 6 CTAs and more) three
+constexpr int kRegRows = 8;           // batch rows of one column tile of an mma; a group has one, two or (clusters of 5 CTAs and more) three
 constexpr int kRegMaxRows = 24;
 constexpr int kRegNoRoom = -100;      // not taken: too many waves, or outputs off the 16-byte grid
 constexpr int kRegTaken = -101;       // answer to a question: the call would run here
@@ -74,11 +74,17 @@ inline int reg_tile_map(CUtensorMap* map, const void* base, int es, int D, int N
   return make_tensor_map_strided(map, base, es, 5, dims, strides, box, chunk * es);
 }
 
-// 0 if a launch of `groups` clusters of `width` CTAs (or plain CTAs: 1) is taken, kRegNoRoom if not, else
-// a cudaError_t. Raises the kernel's shared-memory limit and allows it clusters of 16; the capacity it asks the driver for is
-// remembered. `rival_groups` > 0: plain CTAs may also run in several waves, as long as these are not more than 4/3 of the
-// waves of so many 16-row groups of the tcgen05 kernels.
+// Clusters of `width` CTAs (or plain CTAs: 1) that run at once, or minus a cudaError_t. Raises the kernel's shared-memory limit and allows
+// it clusters of 16; what it asks the driver for is remembered.
+int reg_capacity(const void* kern, const cudaLaunchConfig_t& cfg, int width);
+// 0 if a launch of `groups` clusters is taken, kRegNoRoom if not, else a cudaError_t. `rival_groups` > 0: plain CTAs may also run in several
+// waves, as long as these are not more than 4/3 of the waves of so many 16-row groups of the tcgen05 kernels.
 int reg_room(const void* kern, const cudaLaunchConfig_t& cfg, int width, long long groups, long long rival_groups, int D);
+
+// How the tcgen05 kernels would run a call of at most 512 units: batch rows of a group, waves (0: unknown). Where these need a second
+// wave, register groups of more than 8 rows are always faster.
+struct RegRival { int rows, waves; };
+RegRival reg_rival(bool backward, int cell, int wx_bf16, int N, int B, int D);
 
 #ifdef __CUDACC__
 __device__ __forceinline__ void reg_report(int* err, int code, int detail) {

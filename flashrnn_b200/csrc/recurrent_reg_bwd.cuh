@@ -4,8 +4,7 @@
 //   1. adds up the partial dh_t of its items (fixed order), the external gradient and the pointwise
 //      carry, runs the cell backward and writes round_bf16(dg_t) to shared memory for ldmatrix (one CTA barrier),
 //   2. multiplies with its warp's fragments of R_slice^T [D x GR*U] (rows = units p of h_{t-1}, k = gate rows of this CTA),
-//   3. hands the accumulators to the owners of those units: two lanes swap halves so that each packet is 4 batch rows of
-//      one unit, 16 bytes.
+//   3. hands the accumulators to the owners of those units as they lie: two batch rows of a unit, 8 bytes.
 // The sums of step 2 run over the same gate rows in the same order as in the tcgen05 kernels, whose CTAs own 32 units (16
 // where the width is not a multiple of 32), and step 1 adds them in the same order: every gradient is the same bits, whichever
 // kernels a call takes.
@@ -43,7 +42,8 @@ template <> struct HistPlanes<kSLSTM> { static constexpr int first = 1, count = 
 template <> struct HistPlanes<kGRU> { static constexpr int first = 0, count = 1; };
 template <> struct HistPlanes<kElman> { static constexpr int first = 0, count = 1; };
 
-template <int CELL, int KT, bool LOCAL, bool HALVES, int NB>
+// DENSE: a third CTA on the SM where that saves a wave (see launch_bwd_reg).
+template <int CELL, int KT, bool LOCAL, bool HALVES, int NB, bool DENSE = false>
 struct BwdRegCfg {
   using CT = CellTraits<CELL>;
   static constexpr int UPW = 4;                         // units of a warp
@@ -62,17 +62,17 @@ struct BwdRegCfg {
   // dg is double-buffered; what follows it starts at a multiple of 1 KB
   static constexpr int DG_ALL = reg_round_1k(2 * NB * DG_BYTES);
   // CTAs per SM the register budget is cut for
-  static constexpr int MIN_BLOCKS = LOCAL ? (KT <= 2 ? (NB > 1 || CELL == kLSTM || CELL == kSLSTM ? 2 : 3) : (CELL == kSLSTM ? 1 : 2))
+  static constexpr int MIN_BLOCKS = LOCAL ? (KT <= 2 ? (NB > 1 || ((CELL == kLSTM || CELL == kSLSTM) && !DENSE) ? 2 : 3) : (CELL == kSLSTM ? 1 : 2))
                                           : (KT <= 8 || CELL == kElman ? 2 : 1);
 };
 
-template <int CELL, int KT, bool LOCAL, bool HALVES, int NB>
-__global__ void __launch_bounds__(BwdRegCfg<CELL, KT, LOCAL, HALVES, NB>::THREADS, BwdRegCfg<CELL, KT, LOCAL, HALVES, NB>::MIN_BLOCKS)
+template <int CELL, int KT, bool LOCAL, bool HALVES, int NB, bool DENSE>
+__global__ void __launch_bounds__(BwdRegCfg<CELL, KT, LOCAL, HALVES, NB, DENSE>::THREADS, BwdRegCfg<CELL, KT, LOCAL, HALVES, NB, DENSE>::MIN_BLOCKS)
 frnn_bwd_reg_kernel(const BwdParams p, const float* history, const float* initial, const __grid_constant__ CUtensorMap cache_map,
                     const __grid_constant__ CUtensorMap hist_map,
                     const __grid_constant__ CUtensorMap dhist_map, const __grid_constant__ CUtensorMap dgr_map,
                     const __grid_constant__ CUtensorMap dwx_map, const int wx_bf16, const int own_dwx, const int ring_steps) {
-  using Cfg = BwdRegCfg<CELL, KT, LOCAL, HALVES, NB>;
+  using Cfg = BwdRegCfg<CELL, KT, LOCAL, HALVES, NB, DENSE>;
   using CT = CellTraits<CELL>;
   constexpr int S = CT::S, MTW = Cfg::MTW, KTW = Cfg::KTW, CH = Cfg::CH, GCL = Cfg::GCL, HP = Cfg::HP, HS = Cfg::HS, U = Cfg::U,
                 nwarps = Cfg::NWARPS, UPW = Cfg::UPW, kPlane2 = Cfg::PLANE2, kPlane4 = Cfg::PLANE4;
@@ -275,7 +275,9 @@ frnn_bwd_reg_kernel(const BwdParams p, const float* history, const float* initia
           for (int e = 0; e < NB; ++e) dsum[e] += v[k][e];
       }
     };
-    // The steps, compiled without the options and hooks of a call and with them: their flags are a good part of a step's instructions.
+    // The steps, compiled without the options and hooks of a call, with the options, and with both: their flags are a good part of a
+    // step's instructions, and the phase timers' registers are spilled fragments elsewhere (LSTM B9 T256 N1 D512 with a clip, us: 581 in a loop
+    // with the hooks, 374 without).
     auto run = [&](auto mode_tag) {
       constexpr bool hook = decltype(mode_tag)::value == kRegHooks, any = decltype(mode_tag)::value != kRegPlain;
       long long pc[6] = {0, 0, 0, 0, 0, 0};
@@ -532,10 +534,10 @@ frnn_bwd_reg_kernel(const BwdParams p, const float* history, const float* initia
 }
 
 // Runs the call, or (ask) only says whether it would: kRegTaken / kRegNoRoom.
-template <int CELL, int KT, bool LOCAL, bool HALVES, int NB>
+template <int CELL, int KT, bool LOCAL, bool HALVES, int NB, bool DENSE = false>
 int launch_bwd_reg(const BwdParams& p, const void* cache, const float* history, const float* initial,
                    const float* d_history, int wx_bf16, cudaStream_t stream, bool ask, long long rival_groups = 0) {
-  using Cfg = BwdRegCfg<CELL, KT, LOCAL, HALVES, NB>;
+  using Cfg = BwdRegCfg<CELL, KT, LOCAL, HALVES, NB, DENSE>;
   using CT = CellTraits<CELL>;
   constexpr int U = Cfg::U, ROWS = Cfg::ROWS, chunks = (U + kRegChunk - 1) / kRegChunk;
   const int C = (p.D + U - 1) / U;
@@ -550,7 +552,7 @@ int launch_bwd_reg(const BwdParams& p, const void* cache, const float* history, 
   const uint64_t nd = static_cast<uint64_t>(N) * D, uT = p.T, uB = p.B;
   // bulk stores start on 16-byte boundaries; the tcgen05 kernels write these outputs with plain stores
   if (((reinterpret_cast<uintptr_t>(p.dwx) | reinterpret_cast<uintptr_t>(p.dgr)) & 15u) != 0) return kRegNoRoom;
-  auto kern = frnn_bwd_reg_kernel<CELL, KT, LOCAL, HALVES, NB>;
+  auto kern = frnn_bwd_reg_kernel<CELL, KT, LOCAL, HALVES, NB, DENSE>;
   BwdParams q = p;
   q.C = C;
   const long long groups = static_cast<long long>(N) * reg_batch_tiles(B, ROWS);
@@ -566,6 +568,14 @@ int launch_bwd_reg(const BwdParams& p, const void* cache, const float* history, 
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = LOCAL ? 0 : 1;
+  if constexpr (LOCAL && KT == 2 && NB == 1 && !DENSE && (CELL == kLSTM || CELL == kSLSTM)) {
+    // Heads of 32 units have 288 threads: two CTAs an SM within 96 registers, three within 72 and some spills, which are a seventh (LSTM) to a
+    // third (sLSTM) of a step. B304 T48 N8 (three fit, two do not), us: LSTM 52 against 59 with 16 rows, sLSTM 76 / 84; B600 89 / 105 and 142 / 167.
+    const int two = reg_capacity(reinterpret_cast<const void*>(kern), cfg, 1), three = two / 2 * 3;
+    const long long waves = two > 0 ? (groups + two - 1) / two : 0, dense = three > 0 ? (groups + three - 1) / three : 0;
+    if (20 * waves > (CELL == kLSTM ? 23 : 27) * dense)
+      return launch_bwd_reg<CELL, KT, LOCAL, HALVES, NB, true>(p, cache, history, initial, d_history, wx_bf16, stream, ask, rival_groups);
+  }
   // whether the call is taken at all comes first: one that is not pays for nothing else
   const int rc = reg_room(reinterpret_cast<const void*>(kern), cfg, C, groups, rival_groups, D);
   if (rc != 0 || ask) return rc != 0 ? rc : kRegTaken;
@@ -609,13 +619,18 @@ int launch_bwd_reg_rows(const BwdRegCall& v) {
   // clusters of 9 still run two to an SM, more rows per group are no faster than that kernel. T48 N1 - 4, us, against it: 16 rows sLSTM B64
   // D320 127 / 157, D288 126 / 120, D448 322 / 253, B256 D112 177 / 168; 24 rows LSTM B64 D384 162 / 245, B256 D288 160 / 149, B56
   // D512 (T64) 400 / 354; GRU B256 D288 95 / 131.
+  // 16 rows of an LSTM from 448 units on with fp32 Wx (a second output to stage) win by the second wave that the tcgen05 groups need, and
+  // lose against a single one: D512 189 / 213 and 193 / 145. tcgen05 groups of 8 rows (db_rows: few groups) beat 24 rows of four gates, LSTM B22
+  // N4 D384 146 / 105.
   constexpr bool tight = CELL == kLSTM || CELL == kSLSTM;
+  const bool few = v.p.db_rows == kRegRows;
   if (v.rows == 2 * kRegRows) {
     if ((CELL == kSLSTM && (HALVES || KT == 32 || v.p.D == 288))) return kRegNoRoom;
+    if (CELL == kLSTM && v.p.D >= 448 && !v.wx_bf16 && reg_rival(true, CELL, v.wx_bf16, v.p.N, v.p.B, v.p.D).waves == 1) return kRegNoRoom;
     return launch_bwd_reg<CELL, KT, LOCAL, HALVES, 2>(v.p, v.cache, v.history, v.initial, v.d_history, v.wx_bf16, v.stream, v.ask, rivals);
   }
   if constexpr (KT >= 16 && !HALVES && !(tight && KT == 32)) {
-    if (tight && v.p.D == 288) return kRegNoRoom;
+    if (tight && (v.p.D == 288 || few)) return kRegNoRoom;
     return launch_bwd_reg<CELL, KT, LOCAL, HALVES, 3>(v.p, v.cache, v.history, v.initial, v.d_history, v.wx_bf16, v.stream, v.ask);
   }
   return kRegNoRoom;

@@ -12,8 +12,9 @@
 // One more warp moves data: TMA tiles of Wx in, staged outputs (history, gate cache, bf16 h) out, both under the swizzle
 // that lets units x batch rows be read and written without bank conflicts, several steps per transfer (reg_transfer_steps). The
 // compute warps' own stores of these outputs cost 800 cycles per step in address arithmetic and partial-line stores, their own
-// TMA issue about as much. The loop over the steps is compiled for the outputs that the call has (kRegTrain, kRegPlain, kRegAny):
-// flags and offsets at run time were 5 to 25 % of a step.
+// TMA issue about as much. The loop over the steps is compiled for the outputs that the call has (kRegHooks ...):
+// flags and offsets at run time were 5 to 25 % of a step, the hooks' tests alone 3 to 6 (LSTM B9 T256 N1 D512, us: hidden states alone 337
+// in one loop for everything, 271 in their own; with a clip in training 348 / 298).
 //
 // A group cannot overtake itself: a half of the operand double buffer is written again only after every warp has published
 // the step in between, and a warp publishes after its own reads of that half.
@@ -36,7 +37,8 @@ namespace frnn {
 
 namespace {
 
-template <int CELL, int KT, bool LOCAL, int NB>
+// DENSE: a third CTA on the SM where all groups run at once with it only (see launch_fwd_reg).
+template <int CELL, int KT, bool LOCAL, int NB, bool DENSE = false>
 struct FwdRegCfg {
   static constexpr int UPW = CELL == kElman ? 8 : 4;         // units of a warp: one 16-row tile holds all gates of four
   static constexpr int IT = UPW / 4, NI = NB * IT;           // items (unit, batch row) of a thread, per column tile and in all
@@ -46,16 +48,18 @@ struct FwdRegCfg {
   static constexpr int THREADS = (U / UPW + 1) * 32;
   // h_t goes to a peer as the words of two batch rows, or (GATHER) as packets of eight that a quad of lanes puts together
   static constexpr bool GATHER = UPW == 8 && MAX_C > 4;
-  // CTAs per SM the register budget is cut for
-  static constexpr int MIN_BLOCKS = LOCAL ? (KT <= 2 ? 4 : (CELL == kSLSTM ? 1 : 2)) : (KT <= 8 || CELL == kElman ? 2 : 1);
+  // CTAs per SM the register budget is cut for. Elman: four compute warps; 124 registers instead of 132 at 256 units let a third CTA in (B304
+  // T64 D224 59 / 47 us, where two take 16 rows a group), and cost nothing where it has no work.
+  static constexpr int MIN_BLOCKS = LOCAL ? (KT <= 2 ? 4 : (CELL == kSLSTM ? 1 : 2))
+                                          : ((CELL == kElman && KT <= 16 && NB == 1) || DENSE ? 3 : (KT <= 8 || CELL == kElman ? 2 : 1));
 };
 
-template <int CELL, int KT, bool LOCAL, int NB>
-__global__ void __launch_bounds__(FwdRegCfg<CELL, KT, LOCAL, NB>::THREADS, FwdRegCfg<CELL, KT, LOCAL, NB>::MIN_BLOCKS)
+template <int CELL, int KT, bool LOCAL, int NB, bool DENSE>
+__global__ void __launch_bounds__(FwdRegCfg<CELL, KT, LOCAL, NB, DENSE>::THREADS, FwdRegCfg<CELL, KT, LOCAL, NB, DENSE>::MIN_BLOCKS)
 frnn_fwd_reg_kernel(const FwdParams p, const __grid_constant__ CUtensorMap wx_map, const __grid_constant__ CUtensorMap hist_map,
                     const __grid_constant__ CUtensorMap cache_map, const __grid_constant__ CUtensorMap hbf_map, const int wx_bf16,
                     const int ring_steps, const int hist_states) {
-  using Cfg = FwdRegCfg<CELL, KT, LOCAL, NB>;
+  using Cfg = FwdRegCfg<CELL, KT, LOCAL, NB, DENSE>;
   using CT = CellTraits<CELL>;
   constexpr int UPW = Cfg::UPW, IT = Cfg::IT, NI = Cfg::NI, CHUNK = kRegChunk, ROWS = Cfg::ROWS, U = Cfg::U, nwarps = U / UPW;
   constexpr int kPlane2 = ROWS * CHUNK * 2, kPlane4 = ROWS * CHUNK * 4, kPlaneC = ROWS * CHUNK * CT::CES;
@@ -222,8 +226,7 @@ frnn_fwd_reg_kernel(const FwdParams p, const __grid_constant__ CUtensorMap wx_ma
     }
     if (prof) p.err[20] = static_cast<int>(clock64() - t_entry);
 
-    // The steps, compiled for the outputs of a training call, for those of a whole history without one, and for anything (with the
-    // hooks): the flags of a call cost a fifth of a step's instructions.
+    // The steps, compiled for what the call writes, and for anything (with the hooks): see above.
     auto run = [&](auto mode_tag) {
       constexpr int MODE = decltype(mode_tag)::value;
       constexpr bool hook = MODE == kRegHooks, any = hook || MODE == kRegAny, train = MODE == kRegTrain || MODE == kRegClipped;
@@ -453,9 +456,9 @@ frnn_fwd_reg_kernel(const FwdParams p, const __grid_constant__ CUtensorMap wx_ma
 }
 
 // Runs the call, or (ask) only says whether it would: kRegTaken / kRegNoRoom.
-template <int CELL, int KT, bool LOCAL, int NB>
+template <int CELL, int KT, bool LOCAL, int NB, bool DENSE = false>
 int launch_fwd_reg(const FwdParams& p, const void* wx, int wx_bf16, cudaStream_t stream, bool ask, long long rival_groups = 0) {
-  using Cfg = FwdRegCfg<CELL, KT, LOCAL, NB>;
+  using Cfg = FwdRegCfg<CELL, KT, LOCAL, NB, DENSE>;
   using CT = CellTraits<CELL>;
   constexpr int U = Cfg::U, ROWS = Cfg::ROWS, CHUNK = kRegChunk, plane = ROWS * CHUNK, chunks = (U + CHUNK - 1) / CHUNK;
   const int es = wx_bf16 ? 2 : 4;
@@ -472,7 +475,7 @@ int launch_fwd_reg(const FwdParams& p, const void* wx, int wx_bf16, cudaStream_t
   // bulk stores start on 16-byte boundaries; the tcgen05 kernels write these outputs with plain stores
   if (((reinterpret_cast<uintptr_t>(p.history) | reinterpret_cast<uintptr_t>(p.cache) | reinterpret_cast<uintptr_t>(p.hbf)) & 15u) != 0)
     return kRegNoRoom;
-  auto kern = frnn_fwd_reg_kernel<CELL, KT, LOCAL, NB>;
+  auto kern = frnn_fwd_reg_kernel<CELL, KT, LOCAL, NB, DENSE>;
   FwdParams q = p;
   q.C = (p.D + U - 1) / U;
   const long long groups = static_cast<long long>(p.N) * reg_batch_tiles(p.B, ROWS);
@@ -488,6 +491,12 @@ int launch_fwd_reg(const FwdParams& p, const void* wx, int wx_bf16, cudaStream_t
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = LOCAL ? 0 : 1;
+  if constexpr (KT == 4 && NB == 1 && !DENSE && CELL != kElman) {
+    // Heads of 64 units: three CTAs of nine warps an SM within 72 registers cost a step 3 to 9 %, but hold groups that would need 16 rows. B304
+    // T64 N4, us, 16 rows / three CTAs: LSTM 58 / 52, sLSTM 81 / 66, GRU 52 / 48. The sLSTM with fp32 Wx, 82 / 74, stays with 16 rows.
+    const int two = reg_capacity(reinterpret_cast<const void*>(kern), cfg, q.C);
+    if (two >= 0 && groups > two && (CELL != kSLSTM || wx_bf16)) return launch_fwd_reg<CELL, KT, LOCAL, NB, true>(p, wx, wx_bf16, stream, ask, rival_groups);
+  }
   // whether the call is taken at all comes first: one that is not pays for nothing else
   const int rc = reg_room(reinterpret_cast<const void*>(kern), cfg, q.C, groups, rival_groups, p.D);
   if (rc != 0 || ask) return rc != 0 ? rc : kRegTaken;
@@ -512,8 +521,13 @@ int launch_fwd_reg_rows(const FwdParams& p, const void* wx, int wx_bf16, cudaStr
   // More rows per group: 13 to 14 cycles of a scheduler per mma and column tile, while a tcgen05.mma costs the same for 16 rows as for 8
   // and its kernel has two CTAs of up to 448 units on an SM. T48 N1 - 4, us, against that kernel: 16 rows LSTM B64 D448 105 / 102, D512
   // 120 / 222; 24 rows B96 D256 344 / 411 (T256), B256 D288 108 / 99, B64 D384 116 / 108. The Elman cell has half the tiles: D512 153 / 327.
+  // Of 16-row groups of the sLSTM from 480 units on, a training call with bf16 Wx loses to tcgen05 groups that run in one wave, and wins
+  // where these need a second one: B112 T48 D512 151 / 133 us, B64 144 / 221 (fp32 Wx 117 / 134, inference 111 / 123).
   if (rows == 2 * kRegRows) {
     if (CELL != kElman && p.D > 384 && p.D <= 448) return kRegNoRoom;
+    if constexpr (CELL == kSLSTM && KT == 32) {
+      if (p.D >= 480 && wx_bf16 && p.cache != nullptr && reg_rival(false, CELL, wx_bf16, p.N, p.B, p.D).waves == 1) return kRegNoRoom;
+    }
     return launch_fwd_reg<CELL, KT, LOCAL, 2>(p, wx, wx_bf16, s, ask, rivals);
   }
   if constexpr (KT == 12 || KT == 16 || (CELL == kElman && KT > 16)) return launch_fwd_reg<CELL, KT, LOCAL, 3>(p, wx, wx_bf16, s, ask);
