@@ -429,7 +429,7 @@ extern "C" int frnn_b200_register_rows(int cell, int wx_bf16, int B, int N, int 
   if (rc != 0) return rc;
   if (!plan.supported) return -2;
   FwdParams f{};
-  f.B = B; f.T = 1; f.T_total = 1; f.N = N; f.D = D;
+  f.B = B; f.T = 1; f.T_total = 1; f.N = N; f.D = D; f.fwd_clip = INFINITY;
   f.cache = reinterpret_cast<void*>(16);  // a training call: cache and bf16 h are staged; never dereferenced
   f.hbf = reinterpret_cast<__nv_bfloat16*>(16);
   BwdParams b{};

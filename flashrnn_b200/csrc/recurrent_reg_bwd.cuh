@@ -66,7 +66,7 @@ struct BwdRegCfg {
                                           : (KT <= 8 || CELL == kElman ? 2 : 1);
 };
 
-template <int CELL, int KT, bool LOCAL, bool HALVES, int NB, bool DENSE>
+template <int CELL, int KT, bool LOCAL, bool HALVES, int NB, bool DENSE, bool EXTRA>
 __global__ void __launch_bounds__(BwdRegCfg<CELL, KT, LOCAL, HALVES, NB, DENSE>::THREADS, BwdRegCfg<CELL, KT, LOCAL, HALVES, NB, DENSE>::MIN_BLOCKS)
 frnn_bwd_reg_kernel(const BwdParams p, const float* history, const float* initial, const __grid_constant__ CUtensorMap cache_map,
                     const __grid_constant__ CUtensorMap hist_map,
@@ -496,8 +496,7 @@ frnn_bwd_reg_kernel(const BwdParams p, const float* history, const float* initia
       }
     };
     if (hooks) run(std::integral_constant<int, kRegHooks>{});
-    else if (cut || clip_on || v1) run(std::integral_constant<int, kRegAny>{});
-    else run(std::integral_constant<int, kRegPlain>{});
+    else run(std::integral_constant<int, EXTRA ? kRegAny : kRegPlain>{});
 #pragma unroll
     for (int e = 0; e < NB; ++e)
       if (act[e]) {
@@ -552,7 +551,7 @@ int launch_bwd_reg(const BwdParams& p, const void* cache, const float* history, 
   const uint64_t nd = static_cast<uint64_t>(N) * D, uT = p.T, uB = p.B;
   // bulk stores start on 16-byte boundaries; the tcgen05 kernels write these outputs with plain stores
   if (((reinterpret_cast<uintptr_t>(p.dwx) | reinterpret_cast<uintptr_t>(p.dgr)) & 15u) != 0) return kRegNoRoom;
-  auto kern = frnn_bwd_reg_kernel<CELL, KT, LOCAL, HALVES, NB, DENSE>;
+  auto kern = reg_extra(p) ? frnn_bwd_reg_kernel<CELL, KT, LOCAL, HALVES, NB, DENSE, true> : frnn_bwd_reg_kernel<CELL, KT, LOCAL, HALVES, NB, DENSE, false>;
   BwdParams q = p;
   q.C = C;
   const long long groups = static_cast<long long>(N) * reg_batch_tiles(B, ROWS);

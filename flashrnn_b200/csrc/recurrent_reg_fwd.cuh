@@ -54,7 +54,7 @@ struct FwdRegCfg {
                                           : ((CELL == kElman && KT <= 16 && NB == 1) || DENSE ? 3 : (KT <= 8 || CELL == kElman ? 2 : 1));
 };
 
-template <int CELL, int KT, bool LOCAL, int NB, bool DENSE>
+template <int CELL, int KT, bool LOCAL, int NB, bool DENSE, bool EXTRA>
 __global__ void __launch_bounds__(FwdRegCfg<CELL, KT, LOCAL, NB, DENSE>::THREADS, FwdRegCfg<CELL, KT, LOCAL, NB, DENSE>::MIN_BLOCKS)
 frnn_fwd_reg_kernel(const FwdParams p, const __grid_constant__ CUtensorMap wx_map, const __grid_constant__ CUtensorMap hist_map,
                     const __grid_constant__ CUtensorMap cache_map, const __grid_constant__ CUtensorMap hbf_map, const int wx_bf16,
@@ -424,16 +424,22 @@ frnn_fwd_reg_kernel(const FwdParams p, const __grid_constant__ CUtensorMap wx_ma
         p.err[17] = static_cast<int>(pc[2]);   // ldmatrix, mma
       }
     };
-    const bool alone = !has_cache && !has_hbf, whole = hist_states == CT::S && !out_bf16;
-    if (hooks) run(std::integral_constant<int, kRegHooks>{});
-    else if (whole && has_hbf && (has_cache || CELL == kElman)) {
-      if (clip_on) run(std::integral_constant<int, kRegClipped>{});
-      else run(std::integral_constant<int, kRegTrain>{});
-    } else if (clip_on || !alone) run(std::integral_constant<int, kRegAny>{});
-    else if (hist_states == 0) run(std::integral_constant<int, kRegLast>{});
-    else if (out_bf16) run(std::integral_constant<int, kRegNarrow>{});
-    else if (whole) run(std::integral_constant<int, kRegPlain>{});
-    else run(std::integral_constant<int, kRegHidden>{});
+    if constexpr (!EXTRA) {
+      // The hooks' loop takes any call. Its second mention costs nothing, and without it these loops were scheduled worse: LSTM 16 rows D128 57.6
+      // us against 55.5 (B288 T48 N2), D32 19.3 against 17.7.
+      if (hooks || hist_states != CT::S || out_bf16 || clip_on) run(std::integral_constant<int, kRegHooks>{});
+      else if (has_hbf && (has_cache || CELL == kElman)) run(std::integral_constant<int, kRegTrain>{});
+      else if (!has_hbf && !has_cache) run(std::integral_constant<int, kRegPlain>{});
+      else run(std::integral_constant<int, kRegHooks>{});
+    } else {
+      const bool whole = hist_states == CT::S && !out_bf16;
+      if (hooks) run(std::integral_constant<int, kRegHooks>{});
+      else if (whole && has_hbf && (has_cache || CELL == kElman)) run(std::integral_constant<int, kRegClipped>{});
+      else if (clip_on || has_cache || has_hbf) run(std::integral_constant<int, kRegAny>{});
+      else if (hist_states == 0) run(std::integral_constant<int, kRegLast>{});
+      else if (out_bf16) run(std::integral_constant<int, kRegNarrow>{});
+      else run(std::integral_constant<int, kRegHidden>{});
+    }
 #pragma unroll
     for (int i = 0; i < NI; ++i) {
       if (!act[i]) continue;
@@ -475,7 +481,8 @@ int launch_fwd_reg(const FwdParams& p, const void* wx, int wx_bf16, cudaStream_t
   // bulk stores start on 16-byte boundaries; the tcgen05 kernels write these outputs with plain stores
   if (((reinterpret_cast<uintptr_t>(p.history) | reinterpret_cast<uintptr_t>(p.cache) | reinterpret_cast<uintptr_t>(p.hbf)) & 15u) != 0)
     return kRegNoRoom;
-  auto kern = frnn_fwd_reg_kernel<CELL, KT, LOCAL, NB, DENSE>;
+  const bool extra = reg_extra<CELL>(p, hist_states, has_cache);
+  auto kern = extra ? frnn_fwd_reg_kernel<CELL, KT, LOCAL, NB, DENSE, true> : frnn_fwd_reg_kernel<CELL, KT, LOCAL, NB, DENSE, false>;
   FwdParams q = p;
   q.C = (p.D + U - 1) / U;
   const long long groups = static_cast<long long>(p.N) * reg_batch_tiles(p.B, ROWS);

@@ -44,7 +44,7 @@ struct BwdWideCfg {
   static_assert(2 * PART >= NB * 8 * CT::GB * UO * 4, "the bias sums of the last step fit the buffers of the partial sums");
 };
 
-template <int CELL, int KS, int NB, int KT>
+template <int CELL, int KS, int NB, int KT, bool EXTRA>
 __global__ void __launch_bounds__(BwdWideCfg<CELL, KS, NB, KT>::THREADS, 1)
 frnn_bwd_wide_kernel(const BwdParams p, const float* history, const float* initial, const __grid_constant__ CUtensorMap cache_map,
                      const __grid_constant__ CUtensorMap hist_map, const __grid_constant__ CUtensorMap dhist_map,
@@ -223,7 +223,7 @@ frnn_bwd_wide_kernel(const BwdParams p, const float* history, const float* initi
         for (int s = 0; s < KS; ++s) dsum[i] += v[s];
       }
     };
-    // The steps, compiled without the options and hooks of a call and with them.
+    // The steps, compiled without the options and hooks of a call, with the options, and with both.
     auto run = [&](auto mode_tag) {
       constexpr bool hook = decltype(mode_tag)::value == kRegHooks, any = decltype(mode_tag)::value != kRegPlain;
       long long pc[6] = {0, 0, 0, 0, 0, 0};
@@ -428,8 +428,7 @@ frnn_bwd_wide_kernel(const BwdParams p, const float* history, const float* initi
       }
     };
     if (hooks) run(std::integral_constant<int, kRegHooks>{});
-    else if (cut || clip_on || v1) run(std::integral_constant<int, kRegAny>{});
-    else run(std::integral_constant<int, kRegPlain>{});
+    else run(std::integral_constant<int, EXTRA ? kRegAny : kRegPlain>{});
     // bias gradient of the batch rows of the group, added in their order: through the buffers of the partial sums, which the last wait
     // of every owner warp left
     asm volatile("bar.sync 1, 256;" ::: "memory");
@@ -479,7 +478,7 @@ int launch_bwd_wide(const BwdParams& p, const void* cache, const float* history,
   const int smem = bytes(steps);
   if (smem > kRegSmemLimit) return kRegNoRoom;
   if (((reinterpret_cast<uintptr_t>(p.dwx) | reinterpret_cast<uintptr_t>(p.dgr)) & 15u) != 0) return kRegNoRoom;  // off the grid of bulk stores
-  auto kern = frnn_bwd_wide_kernel<CELL, KS, NB, KT>;
+  auto kern = reg_extra(p) ? frnn_bwd_wide_kernel<CELL, KS, NB, KT, true> : frnn_bwd_wide_kernel<CELL, KS, NB, KT, false>;
   const int D = p.D, N = p.N, B = p.B;
   const long long groups = static_cast<long long>(N) * reg_batch_tiles(B, Cfg::ROWS), clusters = groups * (D / 128);
   cudaLaunchConfig_t cfg = {};

@@ -42,7 +42,7 @@ struct FwdWideCfg {
   static_assert(OWNERS <= 8, "an item per thread");
 };
 
-template <int CELL, int KS, int NB, int KT>
+template <int CELL, int KS, int NB, int KT, bool EXTRA>
 __global__ void __launch_bounds__(FwdWideCfg<CELL, KS, NB, KT>::THREADS, 1)
 frnn_fwd_wide_kernel(const FwdParams p, const __grid_constant__ CUtensorMap wx_map, const __grid_constant__ CUtensorMap hist_map,
                      const __grid_constant__ CUtensorMap cache_map, const __grid_constant__ CUtensorMap hbf_map, const int wx_bf16,
@@ -185,8 +185,7 @@ frnn_fwd_wide_kernel(const FwdParams p, const __grid_constant__ CUtensorMap wx_m
     cluster_sync_all();
     if (prof) p.err[20] = static_cast<int>(clock64() - t_entry);
 
-    // The steps, compiled for the outputs of a training call, for those of a whole history without one, and for anything (with the
-    // hooks): see recurrent_reg_fwd.cuh.
+    // The steps, compiled for what the call writes, and for anything (with the hooks): see recurrent_reg_fwd.cuh.
     auto run = [&](auto mode_tag) {
       constexpr int MODE = decltype(mode_tag)::value;
       constexpr bool hook = MODE == kRegHooks, any = hook || MODE == kRegAny, train = MODE == kRegTrain || MODE == kRegClipped;
@@ -347,16 +346,22 @@ frnn_fwd_wide_kernel(const FwdParams p, const __grid_constant__ CUtensorMap wx_m
         p.err[17] = static_cast<int>(pc[2]);   // ldmatrix, mma, partial gates sent
       }
     };
-    const bool alone = !has_cache && !has_hbf, whole = hist_states == CT::S && !out_bf16;
-    if (hooks) run(std::integral_constant<int, kRegHooks>{});
-    else if (whole && has_hbf && (has_cache || CELL == kElman)) {
-      if (clip_on) run(std::integral_constant<int, kRegClipped>{});
-      else run(std::integral_constant<int, kRegTrain>{});
-    } else if (clip_on || !alone) run(std::integral_constant<int, kRegAny>{});
-    else if (hist_states == 0) run(std::integral_constant<int, kRegLast>{});
-    else if (out_bf16) run(std::integral_constant<int, kRegNarrow>{});
-    else if (whole) run(std::integral_constant<int, kRegPlain>{});
-    else run(std::integral_constant<int, kRegHidden>{});
+    if constexpr (!EXTRA) {
+      // The hooks' loop takes any call. Its second mention costs nothing, and without it these loops were scheduled worse: LSTM 16 rows D128 57.6
+      // us against 55.5 (B288 T48 N2), D32 19.3 against 17.7.
+      if (hooks || hist_states != CT::S || out_bf16 || clip_on) run(std::integral_constant<int, kRegHooks>{});
+      else if (has_hbf && (has_cache || CELL == kElman)) run(std::integral_constant<int, kRegTrain>{});
+      else if (!has_hbf && !has_cache) run(std::integral_constant<int, kRegPlain>{});
+      else run(std::integral_constant<int, kRegHooks>{});
+    } else {
+      const bool whole = hist_states == CT::S && !out_bf16;
+      if (hooks) run(std::integral_constant<int, kRegHooks>{});
+      else if (whole && has_hbf && (has_cache || CELL == kElman)) run(std::integral_constant<int, kRegClipped>{});
+      else if (clip_on || has_cache || has_hbf) run(std::integral_constant<int, kRegAny>{});
+      else if (hist_states == 0) run(std::integral_constant<int, kRegLast>{});
+      else if (out_bf16) run(std::integral_constant<int, kRegNarrow>{});
+      else run(std::integral_constant<int, kRegHidden>{});
+    }
     if (act) {
 #pragma unroll
       for (int k = 0; k < CT::S; ++k) p.carry[static_cast<size_t>(k) * B * ND + item] = st[k];
@@ -390,7 +395,7 @@ int launch_fwd_wide(const FwdParams& p, const void* wx, int wx_bf16, cudaStream_
   if (smem > kRegSmemLimit) return kRegNoRoom;
   if (((reinterpret_cast<uintptr_t>(p.history) | reinterpret_cast<uintptr_t>(p.cache) | reinterpret_cast<uintptr_t>(p.hbf)) & 15u) != 0)
     return kRegNoRoom;  // bulk stores start on 16-byte boundaries
-  auto kern = frnn_fwd_wide_kernel<CELL, KS, NB, KT>;
+  auto kern = reg_extra<CELL>(p, hist_states, has_cache) ? frnn_fwd_wide_kernel<CELL, KS, NB, KT, true> : frnn_fwd_wide_kernel<CELL, KS, NB, KT, false>;
   const long long clusters = static_cast<long long>(p.N) * reg_batch_tiles(p.B, Cfg::ROWS) * (p.D / 32);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(static_cast<unsigned>(clusters * KS));
