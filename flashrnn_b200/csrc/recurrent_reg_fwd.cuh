@@ -96,7 +96,7 @@ frnn_fwd_reg_kernel(const FwdParams p, const __grid_constant__ CUtensorMap wx_ma
   const bool prof = p.err[3] != 0 && blockIdx.x == 0 && tid == 0;
   const int mute_from = p.err[4] != 0 ? p.err[5] : 0x7fffffff;
   const uint32_t jitter = wx_bf16 ? 0u : static_cast<uint32_t>(p.err[6]);
-  const bool hooks = p.err[3] != 0 || p.err[4] != 0 || jitter != 0u;
+  const bool hooks = p.err[3] != 0 || p.err[4] != 0 || (jitter != 0u && p.err[7] == 0);  // err[7]: only the I/O warp is late
 
   if (tid == 0) {
     for (int i = 0; i < 2; ++i) mbar_init(smem_u32(&s_hbar[i]), 1);

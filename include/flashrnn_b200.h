@@ -23,6 +23,9 @@
  * Test hook for the failure path: with err[4] = 1 the CTAs stop publishing their per-step exchange
  * data from step err[5] on, so the next bounded wait (limit = wait_limit_ms) runs out and the call
  * reports err[0] = 101 (forward) / 106 or 107 (backward) and returns normally.
+ * Test hook for races: with err[6] = seed (and fp32 Wx) the warp roles of pseudo-randomly chosen CTAs are late by up to
+ * 8 us in a quarter of the steps; with err[7] = 1 as well only the I/O warps of the kernels with R in registers, whose
+ * compute warps then run the loops of a call without hooks.
  *
  * Counterparts in the reference (0z5a/flashrnn):
  *   flashrnn/flashrnn/fused/flashrnn.cc:56-347      pybind class FlashRNNFuncFused

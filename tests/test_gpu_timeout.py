@@ -41,16 +41,19 @@ def _backward(lib, _lib, cell, B, T, N, D, t, err, limit_ms):
                                   limit_ms, err.data_ptr(), torch.cuda.current_stream().cuda_stream)
 
 
-# R in registers as a cluster and as one CTA, clusters of the tcgen05 kernels, and three ways through global memory
-@pytest.mark.parametrize("shape", [("lstm", 8, 24, 2, 128), ("lstm", 8, 24, 2, 48), ("lstm", 8, 24, 1, 512), ("lstm", 4, 12, 1, 576),
-                                   ("lstm", 4, 12, 1, 768), ("lstm", 64, 12, 1, 768)],
-                         ids=["registers-cluster", "registers-one-cta", "tcgen05-cluster", "global", "global-ksplit", "global-1d"])
-def test_stalled_exchange_is_reported_and_context_survives(shape, cuda_device):
+# R in registers as a cluster, as one CTA and over global memory; R in tensor memory as a cluster and three ways through global memory.
+# `rows`: batch rows of a forward and a backward group with R in registers
+@pytest.mark.parametrize("shape,rows", [(("lstm", 8, 24, 2, 128), (8, 8)), (("lstm", 8, 24, 2, 48), (8, 8)), (("lstm", 8, 24, 1, 512), (8, 8)),
+                                        (("lstm", 4, 12, 1, 768), (8, 8)), (("lstm", 152, 24, 3, 256), (0, 0)), (("lstm", 4, 12, 1, 576), (8, 0)),
+                                        (("lstm", 4, 12, 1, 1280), (0, 0)), (("lstm", 64, 12, 1, 768), (0, 0))],
+                         ids=["registers-cluster", "registers-one-cta", "registers-cluster-16", "registers-global", "tcgen05-cluster", "global",
+                              "global-ksplit", "global-1d"])
+def test_stalled_exchange_is_reported_and_context_survives(shape, rows, cuda_device):
     from flashrnn_b200 import _lib
 
     lib = _lib.load()
     cell, B, T, N, D = shape
-    assert _lib.register_kernels(cell, False, B, N, D) == (D <= 128,) * 2
+    assert _lib.register_rows(cell, False, B, N, D) == rows
     t = _buffers(_lib, cell, B, T, N, D, cuda_device)
     err = torch.zeros(32, dtype=torch.int32, device=cuda_device)
     assert _forward(lib, _lib, cell, B, T, N, D, t, err, 0) == 0
