@@ -53,7 +53,8 @@ struct WgradParams {
 // not stored.
 // Us with the reductions, against the plain-load kernel that such widths (and 320, 448, 640, whose equal tiles were no whole boxes)
 // had, one chunk at a time: GRU B13 T333 N2 D208 22.9 / 55.6, LSTM B16 T256 N16 D48 20.0 / 76.0, B32 T512 N2 D320 66 / 1079, B96
-// T256 N8 D176 91 / 1705, B8 T1024 N1 D640 58 / 851.
+// T256 N8 D176 91 / 1705, B8 T1024 N1 D640 58 / 851. Several batch rows to a chunk, against one: LSTM B448 T1 D288 16.8 / 50.4, B430 T2 N9 D112
+// 13.6 / 67.6, B4 T3 D640 11.5 / 15.2.
 constexpr int kTmaThreads = 192;
 constexpr int kTmaStages = 4;
 // Every launch asks for the limit of the widest tile: the attribute belongs to the kernel, and a thread with narrower tiles would take it from

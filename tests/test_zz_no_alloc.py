@@ -58,8 +58,8 @@ def test_noalloc_wgrad_matches_regular_entry_point_twice(cuda_device):
 
 
 def test_noalloc_packed_and_plain_load_kernels_back_to_back(cuda_device):
-    """The built-in array also serves the kernel for widths that are not multiples of 64 (plain loads) and the
-    narrow-head kernel that packs several heads into one tile. Different shapes and seeds in a row: whatever an
+    """The built-in array also serves widths that are not multiples of 64 (boxes that reach past a head) and
+    narrow heads, several to a tile. Different shapes and seeds in a row: whatever an
     earlier call left in the array must not show up in a later result. dR against an fp32 einsum of the same bf16
     operands, db against the plain sum of the per-tile partials."""
     from flashrnn_b200 import _lib
