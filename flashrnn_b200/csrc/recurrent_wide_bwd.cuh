@@ -427,7 +427,7 @@ frnn_bwd_wide_kernel(const BwdParams p, const float* history, const float* initi
         p.err[12] = static_cast<int>(pc[4]);  // mma and scatter
       }
     };
-    if (hooks) run(std::integral_constant<int, kRegHooks>{});
+    if (hooks || (!EXTRA && (cut || clip_on || v1))) run(std::integral_constant<int, kRegHooks>{});
     else run(std::integral_constant<int, EXTRA ? kRegAny : kRegPlain>{});
     // bias gradient of the batch rows of the group, added in their order: through the buffers of the partial sums, which the last wait
     // of every owner warp left
