@@ -37,7 +37,7 @@ namespace frnn {
 
 namespace {
 
-// DENSE: a third CTA on the SM where all groups run at once with it only (see launch_fwd_reg).
+// DENSE: one more CTA on the SM where all groups run at once with it only (see launch_fwd_reg).
 template <int CELL, int KT, bool LOCAL, int NB, bool DENSE = false>
 struct FwdRegCfg {
   static constexpr int UPW = CELL == kElman ? 8 : 4;         // units of a warp: one 16-row tile holds all gates of four
@@ -51,7 +51,7 @@ struct FwdRegCfg {
   // CTAs per SM the register budget is cut for. Elman: four compute warps; 124 registers instead of 132 at 256 units let a third CTA in (B304
   // T64 D224 59 / 47 us, where two take 16 rows a group), and cost nothing where it has no work.
   static constexpr int MIN_BLOCKS = LOCAL ? (KT <= 2 ? 4 : (CELL == kSLSTM ? 1 : 2))
-                                          : ((CELL == kElman && KT <= 16 && NB == 1) || DENSE ? 3 : (KT <= 8 || CELL == kElman ? 2 : 1));
+                                          : ((CELL == kElman && KT <= 16 && NB == 1) || (DENSE && KT == 4) ? 3 : (KT <= 8 || CELL == kElman || DENSE ? 2 : 1));
 };
 
 template <int CELL, int KT, bool LOCAL, int NB, bool DENSE, bool EXTRA>
@@ -503,6 +503,12 @@ int launch_fwd_reg(const FwdParams& p, const void* wx, int wx_bf16, cudaStream_t
     // T64 N4, us, 16 rows / three CTAs: LSTM 58 / 52, sLSTM 81 / 66, GRU 52 / 48. The sLSTM with fp32 Wx, 82 / 74, stays with 16 rows.
     const int two = reg_capacity(reinterpret_cast<const void*>(kern), cfg, q.C);
     if (two >= 0 && groups > two && (CELL != kSLSTM || wx_bf16)) return launch_fwd_reg<CELL, KT, LOCAL, NB, true>(p, wx, wx_bf16, stream, ask, rival_groups);
+  }
+  if constexpr (KT == 12 && NB == 1 && !DENSE && CELL != kElman) {
+    // Heads of 144 to 192 units: two CTAs an SM within 96 registers, where wider groups would not be fewer. B8 T48, us, tcgen05 / these: N34
+    // D144 LSTM 105 / 43, sLSTM 116 / 50, GRU 61 / 40; N24 D192 LSTM 65 / 43, GRU 61 / 40. Heads that fit with one CTA an SM have 118 to 124 registers.
+    const int one = reg_capacity(reinterpret_cast<const void*>(kern), cfg, q.C);
+    if (one >= 0 && groups > one && p.B <= kRegRows) return launch_fwd_reg<CELL, KT, LOCAL, NB, true>(p, wx, wx_bf16, stream, ask, rival_groups);
   }
   // whether the call is taken at all comes first: one that is not pays for nothing else
   const int rc = reg_room(reinterpret_cast<const void*>(kern), cfg, q.C, groups, rival_groups, p.D);

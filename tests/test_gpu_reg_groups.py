@@ -17,7 +17,8 @@ CASES = [
     (("elman", 266, 6, 4, 128), (16, 16)), (("lstm", 57, 7, 4, 160), (16, 16)), (("gru", 64, 3, 3, 256), (16, 16)),
     (("lstm", 64, 2, 1, 384), (16, 16)), (("gru", 57, 5, 1, 448), (0, 16)), (("slstm", 64, 3, 1, 512), (16, 0)), (("lstm", 200, 4, 4, 112), (16, 16)),
     (("lstm", 84, 5, 3, 256), (24, 24)), (("gru", 100, 3, 3, 240), (24, 0)), (("slstm", 90, 2, 3, 224), (24, 24)), (("elman", 720, 2, 1, 256), (24, 24)),
-    # a third CTA on the SM: the first batch that needs it; the other side of the rules for wider groups
+    # one more CTA on the SM: the first batch that needs it, many heads of few rows; the other side of the rules for wider groups
+    (("lstm", 3, 5, 34, 144), (8, 0)), (("slstm", 8, 3, 30, 160), (8, 0)), (("gru", 1, 4, 30, 144), (8, 0)),
     (("lstm", 304, 5, 8, 32), (8, 8)), (("slstm", 310, 3, 8, 32), (8, 8)), (("lstm", 304, 6, 4, 64), (8, 16)), (("slstm", 301, 3, 4, 64), (16, 16)),
     (("gru", 304, 5, 4, 64), (8, 16)), (("elman", 304, 3, 1, 224), (8, 16)), (("lstm", 112, 3, 1, 512), (16, 0)), (("slstm", 64, 3, 1, 384), (16, 16)),
     (("lstm", 22, 3, 4, 384), (0, 0)),
